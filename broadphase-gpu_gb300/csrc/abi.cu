@@ -468,14 +468,7 @@ void stq_context_destroy(stq_context *ctx) {
     if (ctx->graph_stream) cudaStreamDestroy(ctx->graph_stream);
     if (ctx->graph_event) cudaEventDestroy(ctx->graph_event);
     if (ctx->owns_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
-    for (DevBuf *b : {&ctx->points, &ctx->in_dev, &ctx->scenes, &ctx->cell_base, &ctx->scene_pairs, &ctx->counts, &ctx->box_cells,
-                      &ctx->offsets, &ctx->scan_ws, &ctx->keys64[0], &ctx->keys64[1], &ctx->vals[0],
-                      &ctx->vals[1], &ctx->sort_ws, &ctx->xmin, &ctx->xmax, &ctx->syz, &ctx->sv, &ctx->sflag, &ctx->sfloor, &ctx->cell_floor, &ctx->partner, &ctx->run_end, &ctx->long_list,
-                      &ctx->seg_scan, &ctx->bkeys[0], &ctx->bkeys[1],
-                      &ctx->bvals[0], &ctx->bvals[1],
-                      &ctx->box_counts, &ctx->prefix_ws, &ctx->pair_keys[0], &ctx->pair_keys[1],
-                      &ctx->batch_boxes, &ctx->e2e_boxes, &ctx->e2e_pairs, &ctx->e2e_mesh, &ctx->aux,
-                      &ctx->window_pairs, &ctx->window_long_list, &ctx->window_cursors})
+    for (DevBuf *b : ctx->buffers())
       b->release();
     if (ctx->in_host) cudaFreeHost(ctx->in_host);
     if (ctx->h_hdr) cudaFreeHost(ctx->h_hdr);
@@ -868,6 +861,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     for (int o = 0; o < 16; ++o) key.opts[o] = ctx->options[o];
     key.opts[16] = int64_t(inflation_radius * 1e9f);
     key.stream = caller;
+    for (const DevBuf *b : ctx->buffers()) key.bufs.push_back(b->ptr);
     int st = STQ_OK;
     if (!ctx->graph || !(key == ctx->graph_key)) {
       if (ctx->graph) cudaGraphExecDestroy(ctx->graph);

@@ -45,12 +45,15 @@ struct Staging {
 
 struct GraphKey {
   const void *ptr[7] = {};
+  // every buffer of the context: any call on it may have moved one since the
+  // capture (a sort of more pairs than the batch has replicas, a larger scene)
+  std::vector<const void *> bufs;
   int64_t sizes[9] = {};
   int64_t opts[17] = {};  // every context option, then the inflation radius
   cudaStream_t stream = nullptr;
   bool operator==(const GraphKey &o) const {
     return std::memcmp(ptr, o.ptr, sizeof ptr) == 0 && std::memcmp(sizes, o.sizes, sizeof sizes) == 0 &&
-           std::memcmp(opts, o.opts, sizeof opts) == 0 && stream == o.stream;
+           std::memcmp(opts, o.opts, sizeof opts) == 0 && stream == o.stream && bufs == o.bufs;
   }
 };
 
@@ -122,6 +125,15 @@ struct stq_context {
   bool pending[kStages] = {};
   double stage_ms[kStages] = {};
   int64_t stage_calls[kStages] = {};
+
+  // every device buffer of the context
+  std::vector<DevBuf *> buffers() {
+    return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &counts, &box_cells, &offsets, &scan_ws,
+            &keys64[0], &keys64[1], &vals[0], &vals[1], &sort_ws, &xmin, &xmax, &syz, &sv, &sflag, &sfloor,
+            &cell_floor, &partner, &run_end, &long_list, &seg_scan, &bkeys[0], &bkeys[1], &bvals[0], &bvals[1],
+            &box_counts, &prefix_ws, &pair_keys[0], &pair_keys[1], &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh,
+            &aux, &window_pairs, &window_long_list, &window_cursors};
+  }
 };
 
 

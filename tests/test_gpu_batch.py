@@ -211,3 +211,33 @@ def test_autotune_keeps_results_exact_and_caches(ctx, stq, oracle, cuda, scenes)
     check_batch(oracle, pairs[: r.count].cpu().numpy(), bo, want, ctx.batch_scene_pairs(len(meshes)))
     ms2, settings2 = ctx.autotune(boxes, bo, pairs, cap)  # same shape bucket: cached
     assert ms2 == 0 and settings2 == settings
+
+
+@pytest.mark.parametrize("between", ["sort_pairs", "prepare"])
+def test_batch_graph_follows_buffers_that_another_call_moved(stq, oracle, cuda, scenes, between):
+    """A captured batch holds the context's buffers: a call between two batches
+    that grows one of them (a sort of more pairs than the batch has replicas, a
+    larger scene of one cell) makes the second batch capture again."""
+    import torch
+
+    meshes, want = scenes
+    meshes, want = meshes[:4], want[:4]
+    V0, V1, E, F, vo, eo, fo = stq.concat_meshes(meshes)
+    d = [dev(x, cuda) for x in (V0, V1, E, F)]
+    bo = np.concatenate([[0], np.cumsum([m.num_boxes for m in meshes])])
+    cap = sum(len(w) for w in want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    with stq.Context(0, torch.cuda.current_stream(cuda).cuda_stream) as ctx:
+        for rep in range(2):
+            r, per = ctx.batch_broadphase(d[0], d[1], vo, d[2], eo, d[3], fo, pairs, cap)
+            assert r.status == stq.STQ_OK
+            check_batch(oracle, pairs[: r.count].cpu().numpy(), bo, want, per)
+            if between == "sort_pairs":
+                n = 40 * int(bo[-1])
+                many = torch.randint(0, 1 << 20, (n, 2), dtype=torch.int32, device=cuda)
+                ctx.sort_pairs(many, n)
+            else:
+                b = stq.random_boxes(3 * int(bo[-1]), seed=3)
+                ctx.set_option(stq.OPT_CELLS, 1)
+                ctx.prepare(dev(b.view(np.int32).reshape(-1, 11), cuda), len(b), 0)
+                ctx.set_option(stq.OPT_CELLS, 0)
