@@ -859,7 +859,9 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     std::memcpy(key.sizes, sizes, sizeof sizes);
     static_assert(sizeof(ctx->options) / sizeof(ctx->options[0]) == 16, "options in the graph key");
     for (int o = 0; o < 16; ++o) key.opts[o] = ctx->options[o];
-    key.opts[16] = int64_t(inflation_radius * 1e9f);
+    uint32_t radius_bits = 0;  // the exact radius: the graph holds it as a kernel argument
+    std::memcpy(&radius_bits, &inflation_radius, sizeof radius_bits);
+    key.opts[16] = int64_t(radius_bits);
     key.stream = caller;
     for (const DevBuf *b : ctx->buffers()) key.bufs.push_back(b->ptr);
     int st = STQ_OK;

@@ -241,3 +241,23 @@ def test_batch_graph_follows_buffers_that_another_call_moved(stq, oracle, cuda, 
                 ctx.set_option(stq.OPT_CELLS, 1)
                 ctx.prepare(dev(b.view(np.int32).reshape(-1, 11), cuda), len(b), 0)
                 ctx.set_option(stq.OPT_CELLS, 0)
+
+
+def test_batch_graph_follows_small_radii(ctx, stq, oracle, cuda, scenes):
+    """Two inflation radii below 1e-9 are two graphs: the pairs of a scene scaled
+    to 1e-9 depend on which of them was asked for."""
+    import torch
+
+    m = scenes[0][0]
+    V0, V1 = m.V0 * 1e-9, m.V1 * 1e-9
+    vo, eo, fo = ([0, len(x)] for x in (V0, m.E, m.F))
+    d = [dev(x, cuda) for x in (V0, V1, m.E, m.F)]
+    cap, counts = 64 * m.num_boxes, set()
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    for r in (0.0, 2e-11, 0.0):
+        want = oracle.broadphase(oracle.construct_boxes(V0, V1, m.E, m.F, stq.AABB_DTYPE, r))
+        res, _ = ctx.batch_broadphase(d[0], d[1], vo, d[2], eo, d[3], fo, pairs, cap, inflation_radius=r)
+        assert res.status == stq.STQ_OK
+        assert np.array_equal(oracle.canonical(pairs[: res.count].cpu().numpy()), want)
+        counts.add(len(want))
+    assert len(counts) == 2
