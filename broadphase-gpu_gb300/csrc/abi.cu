@@ -84,19 +84,24 @@ void apply_options(stq_context *ctx) {
 BatchHeader *dev_hdr(stq_context *ctx) {
   return reinterpret_cast<BatchHeader *>(ctx->in_dev.as<char>() + ctx->layout.hdr);
 }
-int read_header(stq_context *ctx, const BatchHeader *src) {
-  STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_hdr, src ? src : dev_hdr(ctx), sizeof(BatchHeader),
-                                cudaMemcpyDeviceToHost, ctx->stream),
-           "read back batch header");
-  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
-  collect_stages(ctx);
+int check_header(stq_context *ctx) {
   const int f = ctx->h_hdr->flags;
   if (f & kFlagNaN) return fail(ctx, STQ_ERR_INVALID_INPUT, "a box bound is NaN");
   if (f & kFlagBadIndex)
     return fail(ctx, STQ_ERR_INVALID_INPUT, "an edge or face vertex index is out of range");
   if (f & kFlagReplicaOverflow)
     return fail(ctx, STQ_ERR_NO_MEMORY, "cell replicas exceed the replica buffers");
+  if (ctx->h_hdr->fault) return fail(ctx, STQ_ERR_TIMEOUT, "a bounded wait of the sort expired");
   return STQ_OK;
+}
+
+int read_header(stq_context *ctx, const BatchHeader *src) {
+  STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_hdr, src ? src : dev_hdr(ctx), sizeof(BatchHeader),
+                                cudaMemcpyDeviceToHost, ctx->stream),
+           "read back batch header");
+  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
+  collect_stages(ctx);
+  return check_header(ctx);
 }
 
 int64_t tiles_for(const int64_t *box_off, int S) {
@@ -200,8 +205,8 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
   b.box_vals = ctx->bvals[0].as<uint32_t>();
   b.box_keys2 = ctx->bkeys[1].as<uint32_t>();
   b.box_vals2 = ctx->bvals[1].as<uint32_t>();
-  b.order = ctx->bvals[ctx->order_buf].as<uint32_t>();
-  b.sorted_keys = ctx->bkeys[ctx->order_buf].as<uint32_t>();
+  b.order = ctx->bvals[0].as<uint32_t>();
+  b.sorted_keys = ctx->bkeys[0].as<uint32_t>();
   b.seg_scan = ctx->seg_scan.as<uint32_t>();
   b.seg_cap = ctx->seg_cap;
   b.box_cap = ctx->box_cap;
@@ -220,9 +225,7 @@ int ensure_box_buffers(stq_context *ctx, int64_t box_cap) {
     STQ_CUDA(ctx, ctx->bkeys[b].ensure(sizeof(uint32_t) * n), "allocate box keys");
     STQ_CUDA(ctx, ctx->bvals[b].ensure(sizeof(uint32_t) * n), "allocate box order");
   }
-  STQ_CUDA(ctx, ctx->sort_ws.ensure(std::max(radix_workspace_bytes(int64_t(n), 4, 8),
-                                              radix_workspace_bytes(int64_t(n), 4, 4))),
-           "allocate sort workspace");
+  STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(int64_t(n))), "allocate sort workspace");
   ctx->box_cap = int64_t(n);
   return STQ_OK;
 }
@@ -233,9 +236,7 @@ int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap)
     STQ_CUDA(ctx, ctx->keys64[b].ensure(sizeof(unsigned long long) * r), "allocate keys");
     STQ_CUDA(ctx, ctx->vals[b].ensure(sizeof(uint32_t) * r), "allocate values");
   }
-  STQ_CUDA(ctx, ctx->sort_ws.ensure(std::max(radix_workspace_bytes(int64_t(r), 8, 8),
-                                              radix_workspace_bytes(int64_t(r), 8, 4))),
-           "allocate sort workspace");
+  STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(int64_t(r))), "allocate sort workspace");
   // three lists (vertices, edges, faces) per cell, each followed by a sentinel
   const int64_t segs = std::max<int64_t>(3 * cells_cap, ctx->seg_cap);
   STQ_CUDA(ctx, ctx->seg_scan.ensure(sizeof(uint32_t) * size_t(segs + 1)), "allocate segment offsets");
@@ -272,17 +273,13 @@ int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t n_box
   STQ_CUDA(ctx, launch_batch_box_keys(ctx->stream, b), "launch box keys");
   uint32_t *kb[2] = {ctx->bkeys[0].as<uint32_t>(), ctx->bkeys[1].as<uint32_t>()};
   uint32_t *vb[2] = {ctx->bvals[0].as<uint32_t>(), ctx->bvals[1].as<uint32_t>()};
-  const int rbits = ctx->options[STQ_OPT_RADIX_BITS] == 4 ? 4 : 8;
   const int64_t n = n_boxes >= 0 ? n_boxes : ctx->box_cap;
-  STQ_CUDA(ctx, radix_sort_u32(ctx->stream, kb, vb, n, rbits, ctx->sort_ws.ptr, &ctx->order_buf, &ctx->launches,
+  STQ_CUDA(ctx, radix_sort_u32(ctx->stream, kb, vb, n, ctx->sort_ws.ptr, &b.hdr->fault, &ctx->launches,
                                n_boxes >= 0 ? nullptr : &b.hdr->box_count),
            "launch box sort");
   stage_end(ctx, kSort);
-  BatchBuffers bs = b;
-  bs.order = vb[ctx->order_buf];
-  bs.sorted_keys = kb[ctx->order_buf];
   stage_begin(ctx, kKeys);
-  STQ_CUDA(ctx, launch_batch_counts(ctx->stream, bs, n), "launch replica counts");
+  STQ_CUDA(ctx, launch_batch_counts(ctx->stream, b, n), "launch replica counts");
   STQ_CUDA(ctx, exclusive_scan_u32(ctx->stream, b.counts, b.offsets, ctx->box_cap, ctx->scan_ws.ptr,
                                    &b.hdr->replicas, &ctx->launches),
            "launch replica scan");
@@ -292,10 +289,7 @@ int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t n_box
 
 int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int seg_bits, int64_t n_boxes,
                          int64_t replicas) {
-  BatchBuffers bs = b;
-  bs.order = ctx->bvals[ctx->order_buf].as<uint32_t>();
-  bs.sorted_keys = ctx->bkeys[ctx->order_buf].as<uint32_t>();
-  STQ_CUDA(ctx, launch_batch_emit(ctx->stream, bs, n_boxes >= 0 ? n_boxes : ctx->box_cap, ctx->num_sms),
+  STQ_CUDA(ctx, launch_batch_emit(ctx->stream, b, n_boxes >= 0 ? n_boxes : ctx->box_cap, ctx->num_sms),
            "launch replica emit");
   stage_end(ctx, kKeys);
   // the replicas arrive in sweep-axis order: a stable sort by list id alone
@@ -305,11 +299,10 @@ int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int seg_bits, 
   uint32_t *vb[2] = {ctx->vals[0].as<uint32_t>(), ctx->vals[1].as<uint32_t>()};
   int which = 0;
   stage_begin(ctx, kSort);
-  const int rbits = ctx->options[STQ_OPT_RADIX_BITS] == 4 ? 4 : 8;
   const int64_t r = replicas >= 0 ? replicas : ctx->rep_cap;
-  // seg_bits covers the capacity; passes above the actual list count copy through
+  // seg_bits covers the capacity; the digits that no list id uses are skipped
   STQ_CUDA(ctx, radix_sort_u64_vals(ctx->stream, kb, vb, r, 32, 32 + std::max(seg_bits, 1), ctx->sort_ws.ptr,
-                                    &which, &ctx->launches, &b.hdr->replicas, rbits, &b.hdr->lists),
+                                    &which, &b.hdr->fault, &ctx->launches, replicas >= 0 ? nullptr : &b.hdr->replicas),
            "launch list sort");
   stage_end(ctx, kSort);
   ctx->scene.xmin = ctx->xmin.as<float>();
@@ -450,6 +443,7 @@ int stq_context_create(int device, void *stream, stq_context **out) {
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   apply_options(ctx);
   if (cudaMallocHost(&ctx->h_hdr, sizeof(BatchHeader)) != cudaSuccess ||
+      cudaMallocHost(&ctx->h_fault, sizeof(int)) != cudaSuccess ||
       ctx->aux.ensure(sizeof(BatchHeader)) != cudaSuccess || ensure_staging(ctx, 1, 1) != STQ_OK) {
     stq_context_destroy(ctx);
     return STQ_ERR_NO_MEMORY;
@@ -472,6 +466,7 @@ void stq_context_destroy(stq_context *ctx) {
       b->release();
     if (ctx->in_host) cudaFreeHost(ctx->in_host);
     if (ctx->h_hdr) cudaFreeHost(ctx->h_hdr);
+    if (ctx->h_fault) cudaFreeHost(ctx->h_fault);
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     if (ctx->copy_stream) {
       cudaStreamSynchronize(ctx->copy_stream);
@@ -895,10 +890,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
   STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
   collect_stages(ctx);
   const BatchHeader &h = *ctx->h_hdr;
-  if (h.flags & kFlagNaN) return fail(ctx, STQ_ERR_INVALID_INPUT, "a box bound is NaN");
-  if (h.flags & kFlagBadIndex) return fail(ctx, STQ_ERR_INVALID_INPUT, "an edge or face vertex index is out of range");
-  if (h.flags & kFlagReplicaOverflow)
-    return fail(ctx, STQ_ERR_NO_MEMORY, "cell replicas exceed the replica buffers");
+  STQ_TRY(check_header(ctx));
   ctx->n_scenes = n_scenes;
   ctx->n_boxes = N;
   ctx->length = int64_t(h.length);
@@ -1065,23 +1057,17 @@ int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count) {
   if (!ctx || count < 0 || (count > 0 && !d_pairs)) return STQ_ERR_INVALID_ARG;
   if (count < 2) return STQ_OK;
   DeviceGuard g(ctx->device);
-  for (int b = 0; b < 2; ++b)
-    STQ_CUDA(ctx, ctx->pair_keys[b].ensure(sizeof(unsigned long long) * size_t(count)),
-             "allocate pair keys");
-  STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(count, 8, 8)), "allocate sort workspace");
-  unsigned long long *kb[2] = {ctx->pair_keys[0].as<unsigned long long>(),
-                               ctx->pair_keys[1].as<unsigned long long>()};
+  STQ_CUDA(ctx, ctx->pair_tmp.ensure(sizeof(stq_pair) * size_t(count)), "allocate pair buffer");
+  STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(count)), "allocate sort workspace");
+  *ctx->h_fault = 0;
   stage_begin(ctx, kPairSort);
-  STQ_CUDA(ctx, launch_pairs_to_keys(ctx->stream, d_pairs, count, kb[0], true), "pairs to keys");
-  int which = 0;
-  STQ_CUDA(ctx, radix_sort_u64(ctx->stream, kb, count, 0, 64, ctx->sort_ws.ptr, &which,
-                               &ctx->launches),
+  STQ_CUDA(ctx, radix_sort_pairs(ctx->stream, d_pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->sort_ws.ptr,
+                                 ctx->h_fault, &ctx->launches),
            "launch pair sort");
-  STQ_CUDA(ctx, launch_pairs_to_keys(ctx->stream, d_pairs, count, kb[which], false), "keys to pairs");
   stage_end(ctx, kPairSort);
-  ctx->launches += 2;
   STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
   collect_stages(ctx);
+  if (*ctx->h_fault) return fail(ctx, STQ_ERR_TIMEOUT, "a bounded wait of the sort expired");
   return STQ_OK;
 }
 
@@ -1207,20 +1193,9 @@ int stq_autotune(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *h_box
   int st = STQ_OK;
   for (int64_t scale : {1, 2, 4, 8}) {
     if ((st = stq_context_set_option(ctx, STQ_OPT_CELL_SCALE, scale)) != STQ_OK) break;
-    // the radix width changes the prepare only: the sorted scene is the same
     float t_prep = 1e30f;
-    int64_t best_radix = 8;
-    for (int64_t radix : {8, 4}) {
-      if ((st = stq_context_set_option(ctx, STQ_OPT_RADIX_BITS, radix)) != STQ_OK) break;
-      float t = 0.f;
-      st = elapsed([&] { return stq_batch_prepare(ctx, d_boxes, h_box_off, n_scenes, nullptr, STQ_AXIS_AUTO); },
-                   &t);
-      if (st != STQ_OK) break;
-      if (t < t_prep) {
-        t_prep = t;
-        best_radix = radix;
-      }
-    }
+    st = elapsed([&] { return stq_batch_prepare(ctx, d_boxes, h_box_off, n_scenes, nullptr, STQ_AXIS_AUTO); },
+                 &t_prep);
     if (st != STQ_OK) break;
     for (const Shape &sh : space) {
       stq_context_set_option(ctx, STQ_OPT_SWEEP_SHAPE, sh.shape);
@@ -1238,7 +1213,7 @@ int stq_autotune(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *h_box
       if (st != STQ_OK) break;
       if (t_prep + t_sweep < best_total) {
         best_total = t_prep + t_sweep;
-        best_set = {sh.lanes, sh.queue, sh.block, best_radix, scale, sh.per_lane, sh.shape, sh.run_cap};
+        best_set = {sh.lanes, sh.queue, sh.block, 8, scale, sh.per_lane, sh.shape, sh.run_cap};
       }
     }
     if (st != STQ_OK) break;

@@ -79,6 +79,7 @@ batch_reset_kernel(SceneRecord *scenes, const SceneInput *__restrict__ inputs,
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     hdr->flags = 0;
+    hdr->fault = 0;
     hdr->replicas = 0;
     hdr->cells = 0;
     hdr->lists = 0;

@@ -78,12 +78,11 @@ struct stq_context {
   size_t in_host_bytes = 0;
   DevBuf scenes, cell_base, scene_pairs, counts, offsets, box_cells, scan_ws, keys64[2], vals[2], sort_ws;
   DevBuf points;  // fp64 vertex positions rounded to float once (box builds)
-  DevBuf xmin, xmax, syz, sv, sflag, sfloor, partner, run_end, box_counts, prefix_ws, pair_keys[2];
+  DevBuf xmin, xmax, syz, sv, sflag, sfloor, partner, run_end, box_counts, prefix_ws, pair_tmp;
   DevBuf cell_floor;  // lower bounds of each cell on b and c
   DevBuf long_list;  // runs handed from the lane sweep to the warp pass
   DevBuf seg_scan;  // first sorted replica of each (cell, type) list
   DevBuf bkeys[2], bvals[2];  // box sort: keys and box indices, double-buffered
-  int order_buf = 0;          // which bvals buffer holds the sorted box order
   int64_t seg_cap = 0;
   DevBuf batch_boxes, e2e_boxes, e2e_pairs, e2e_mesh;
   DevBuf aux;  // header of calls outside a batch (box build, all-pairs check)
@@ -94,6 +93,7 @@ struct stq_context {
   int64_t n_boxes = 0, length = 0;
   SortedScene scene;
   BatchHeader *h_hdr = nullptr;             // pinned readback
+  int *h_fault = nullptr;  // pinned, written by a pair sort whose wait ran out
   unsigned long long *h_scene_pairs = nullptr;  // pinned readback
   int h_scene_pairs_cap = 0;
 
@@ -131,7 +131,7 @@ struct stq_context {
     return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &counts, &box_cells, &offsets, &scan_ws,
             &keys64[0], &keys64[1], &vals[0], &vals[1], &sort_ws, &xmin, &xmax, &syz, &sv, &sflag, &sfloor,
             &cell_floor, &partner, &run_end, &long_list, &seg_scan, &bkeys[0], &bkeys[1], &bvals[0], &bvals[1],
-            &box_counts, &prefix_ws, &pair_keys[0], &pair_keys[1], &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh,
+            &box_counts, &prefix_ws, &pair_tmp, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh,
             &aux, &window_pairs, &window_long_list, &window_cursors};
   }
 };
@@ -152,6 +152,8 @@ void collect_stages(stq_context *ctx);
 void stage_begin(stq_context *ctx, int st);
 void stage_end(stq_context *ctx, int st);
 BatchHeader *dev_hdr(stq_context *ctx);
+// Status of a batch header read back into ctx->h_hdr.
+int check_header(stq_context *ctx);
 int read_header(stq_context *ctx, const BatchHeader *src = nullptr);
 int64_t tiles_for(const int64_t *box_off, int S);
 int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap);

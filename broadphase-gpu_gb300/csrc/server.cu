@@ -358,7 +358,7 @@ int collect(stq_server *sv, int64_t *done_ids, int max_done, int *n_done) {
   sv->in_flight = false;
   const BatchHeader &h = *ctx->h_hdr;
   if (h.flags & (kFlagNaN | kFlagBadIndex)) return sfail(sv, STQ_ERR_INVALID_INPUT, "invalid request mesh");
-  if (h.flags & kFlagReplicaOverflow) return sfail(sv, STQ_ERR_NO_MEMORY, "replica buffers exceeded");
+  STQ_TRY(check_header(ctx));
   if (int64_t(h.pairs) > sv->pair_cap) {
     // the pair estimate was short: grow the buffer and sweep this step again
     // (positions are already advanced, so no second advance)

@@ -28,7 +28,7 @@ constexpr size_t kOffKeys1 = kOffKeys0 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kOffVals0 = kOffKeys1 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kOffVals1 = kOffVals0 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kOffSortWs = kOffVals1 + up256(sizeof(uint32_t) * kMax);
-constexpr size_t kSortWsBytes = sizeof(uint32_t) * (256 * ((kMax + kRadixTile - 1) / kRadixTile) + 256) + 256;
+constexpr size_t kSortWsBytes = radix_workspace_bytes(kMax);
 constexpr size_t kOffXmin = kOffSortWs + up256(kSortWsBytes);
 constexpr size_t kOffXmax = kOffXmin + up256(sizeof(float) * kSlots);
 constexpr size_t kOffSyz = kOffXmax + up256(sizeof(float) * kSlots);
@@ -139,10 +139,10 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
                      reinterpret_cast<uint32_t *>(scratch + kOffKeys1)};
   uint32_t *vb[2] = {reinterpret_cast<uint32_t *>(scratch + kOffVals0),
                      reinterpret_cast<uint32_t *>(scratch + kOffVals1)};
-  int which = 0;
-  if (radix_sort_u32(s, kb, vb, n, 8, scratch + kOffSortWs, &which, nullptr) != cudaSuccess)
+  BatchHeader *hdr = reinterpret_cast<BatchHeader *>(scratch + kOffHdr);
+  if (radix_sort_u32(s, kb, vb, n, scratch + kOffSortWs, &hdr->fault, nullptr) != cudaSuccess)
     return STQ_ERR_CUDA;
-  static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, vb[which], scratch);
+  static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, vb[0], scratch);
   SweepParams p;
   p.xmin = reinterpret_cast<const float *>(scratch + kOffXmin);
   p.xmax = reinterpret_cast<const float *>(scratch + kOffXmax);
@@ -157,7 +157,6 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   p.chunk = 32;
   p.pairs = d_pairs;
   p.capacity = capacity;
-  BatchHeader *hdr = reinterpret_cast<BatchHeader *>(scratch + kOffHdr);
   p.count = &hdr->pairs;
   p.work = &hdr->work;
   p.box_counts = nullptr;
@@ -177,6 +176,7 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
       cudaStreamSynchronize(s) != cudaSuccess)
     return STQ_ERR_CUDA;
   if (h.flags & kFlagNaN) return STQ_ERR_INVALID_INPUT;
+  if (h.fault) return STQ_ERR_TIMEOUT;
   const int64_t found = int64_t(h.pairs);
   if (total) *total = found;
   *count = found < capacity ? found : capacity;

@@ -129,7 +129,7 @@ struct BatchHeader {
   unsigned int box_count;   // input: n_boxes as the element count of the box sort
   unsigned long long candidates;  // candidates tested by the last sweep
   unsigned int lists;       // (cell, type) lists: 3 * cells
-  unsigned int pad;
+  int fault;                // a bounded wait between blocks ran out
 };
 
 // A tile of at most kTileBoxes consecutive boxes of one scene (built by the
@@ -310,27 +310,31 @@ cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long l
 // host_count: device address of page-locked, mapped host memory
 cudaError_t launch_window_step(cudaStream_t s, WindowCounters *wc, unsigned long long *host_count);
 
-// LSD radix sort of (uint32 key, uint32 value) or (uint64 key) pairs.
-// kbuf/vbuf are double buffers; *which receives the buffer index holding the
-// result. Returns workspace bytes when called with workspace == nullptr.
-size_t radix_workspace_bytes(int64_t n, int key_bytes, int bits);
-constexpr int kRadixTile = 2048;  // keys per radix tile (one per-digit count each)
-cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *kbuf[2], uint32_t *vbuf[2],
-                           int64_t n, int bits, void *workspace, int *which,
-                           int64_t *launches, const unsigned int *d_n = nullptr);
-cudaError_t radix_sort_u64(cudaStream_t s, unsigned long long *kbuf[2],
-                           int64_t n, int begin_bit, int end_bit, void *workspace,
-                           int *which, int64_t *launches);
-// d_hi (may be null): on the device, the number of distinct values of the
-// keys' bits from begin_bit up; a pass whose digit is 0 in every key (all those
-// values below 2^(its shift - begin_bit)) copies the keys through instead of
-// ranking them, so a sort sized for a capacity (a captured graph) pays for
-// the digits the actual keys use.
-cudaError_t radix_sort_u64_vals(cudaStream_t s, unsigned long long *kbuf[2],
-                                uint32_t *vbuf[2], int64_t n, int begin_bit, int end_bit,
-                                void *workspace, int *which, int64_t *launches,
-                                const unsigned int *d_n = nullptr, int bits = 8,
-                                const unsigned int *d_hi = nullptr);
+// Stable LSD radix sorts (8-bit digits). kbuf/vbuf are double buffers.
+// fault: device-visible word set to 1 if a bounded wait between blocks ran out
+// (the result is then not sorted). d_n (may be null): on the device, the number
+// of elements (at most n).
+constexpr int kRadixMinTile = 2048;       // keys of the smallest tile of a pass
+constexpr size_t kRadixHeadBytes = 8704;  // digit counts, cursors
+// Workspace of a sort of up to n elements: the head and 256 status words per
+// tile. The smallest tiles are used below a fixed size, larger ones (at least
+// twice as long) above it.
+constexpr size_t radix_workspace_bytes(int64_t n) {
+  const size_t tiles = size_t((n > 0 ? n : 1) + kRadixMinTile - 1) / kRadixMinTile;
+  const size_t half = (tiles + 1) / 2, small_max = size_t(1) << 13;
+  const size_t small = tiles < small_max ? tiles : small_max;
+  return kRadixHeadBytes + sizeof(unsigned long long) * 256 * (small > half ? small : half);
+}
+// result in kbuf[0], vbuf[0]
+cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *kbuf[2], uint32_t *vbuf[2], int64_t n, void *workspace,
+                           int *fault, int64_t *launches, const unsigned int *d_n = nullptr);
+// by bits [begin_bit, end_bit); *which receives the buffer that holds the result
+cudaError_t radix_sort_u64_vals(cudaStream_t s, unsigned long long *kbuf[2], uint32_t *vbuf[2], int64_t n,
+                                int begin_bit, int end_bit, void *workspace, int *which, int *fault,
+                                int64_t *launches, const unsigned int *d_n = nullptr);
+// lexicographic by (first, second) as unsigned ids, in place; tmp holds n pairs
+cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,
+                             int64_t *launches);
 // exclusive scan of n uint32 counts; *d_total receives the sum
 size_t scan_workspace_bytes(int64_t n);
 cudaError_t exclusive_scan_u32(cudaStream_t s, const uint32_t *in, uint32_t *out, int64_t n,
@@ -348,7 +352,5 @@ cudaError_t launch_prefix_select(cudaStream_t s, const int32_t *box_counts,
 cudaError_t launch_brute_force(cudaStream_t s, const stq_aabb *boxes, int64_t n,
                                stq_pair *pairs, long long capacity,
                                unsigned long long *count);
-cudaError_t launch_pairs_to_keys(cudaStream_t s, const stq_pair *pairs, int64_t n,
-                                 unsigned long long *keys, bool to_keys);
 
 }  // namespace stq

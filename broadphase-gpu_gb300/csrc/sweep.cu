@@ -873,20 +873,6 @@ brute_force_kernel(const stq_aabb *__restrict__ boxes, int64_t n,
   }
 }
 
-__global__ void pairs_keys_kernel(stq_pair *pairs, int64_t n, unsigned long long *keys,
-                                  bool to_keys) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    if (to_keys) {
-      keys[i] = (static_cast<unsigned long long>(uint32_t(pairs[i].first)) << 32) |
-                uint32_t(pairs[i].second);
-    } else {
-      pairs[i].first = int32_t(keys[i] >> 32);
-      pairs[i].second = int32_t(keys[i] & 0xffffffffu);
-    }
-  }
-}
-
 }  // namespace
 
 static cudaError_t launch_long_runs(cudaStream_t s, const SweepParams &p, bool count_mode, int num_sms) {
@@ -959,15 +945,6 @@ cudaError_t launch_brute_force(cudaStream_t s, const stq_aabb *boxes, int64_t n,
   const int64_t tiles = (n + kBruteTile - 1) / kBruteTile;
   dim3 grid(unsigned(tiles), unsigned(tiles < 64 ? tiles : 64));
   brute_force_kernel<<<grid, kBruteTile, 0, s>>>(boxes, n, pairs, capacity, count);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pairs_to_keys(cudaStream_t s, const stq_pair *pairs, int64_t n,
-                                 unsigned long long *keys, bool to_keys) {
-  if (n == 0) return cudaSuccess;
-  int64_t g = (n + 255) / 256;
-  if (g > 152 * 16) g = 152 * 16;
-  pairs_keys_kernel<<<unsigned(g), 256, 0, s>>>(const_cast<stq_pair *>(pairs), n, keys, to_keys);
   return cudaGetLastError();
 }
 

@@ -90,7 +90,8 @@ typedef enum stq_option {
   STQ_OPT_BLOCK_SIZE = 3,      /* sweep block size: 128, 256 (default) or 512     */
   STQ_OPT_CELLS = 4,           /* cell grid on the two non-sweep axes: 0 automatic,
                                   1 no cells (plain sweep), k > 1 a k x k grid      */
-  STQ_OPT_RADIX_BITS = 5,      /* radix digit width: 4 or 8 (single-cell sort)     */
+  STQ_OPT_RADIX_BITS = 5,      /* 4 or 8: accepted and reported; the sorts always use
+                                  8-bit digits, which are faster at every size    */
   STQ_OPT_CELL_SCALE = 6,      /* automatic cell side in median box extents (1..64,
                                   default 2); a scene of n boxes gets at most
                                   n / max(16, 8 * scale) cells                      */
@@ -270,7 +271,7 @@ int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count);
 /* ---- autotuning --------------------------------------------------------------
  * Times prepare + sweep of the given batch (as stq_batch_prepare, all start
  * boxes), each setting five times (the fastest counts), over cell scale
- * {1, 2, 4, 8} and radix digit width {4, 8} (the prepare), and over the sweep
+ * {1, 2, 4, 8} (the prepare), and over the sweep
  * shapes (the work split of the start boxes' runs): one start box per lane
  * with 2, 4 or 8 candidates per step (queue depth {32, 64}), lane groups of
  * 4, 8 or 16 lanes (queue depth {16, 32, 64}), each with block size
