@@ -247,10 +247,9 @@ int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap)
   STQ_CUDA(ctx, ctx->syz.ensure(sizeof(float4) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->sv.ensure(sizeof(int4) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->sflag.ensure(sizeof(int) * slots), "allocate sorted scene");
-  STQ_CUDA(ctx, ctx->sfloor.ensure(sizeof(float2) * slots), "allocate sorted scene");
+  STQ_CUDA(ctx, ctx->scode.ensure(sizeof(uint32_t) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->partner.ensure(sizeof(int) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->run_end.ensure(sizeof(int) * slots), "allocate sorted scene");
-  STQ_CUDA(ctx, ctx->cell_floor.ensure(sizeof(float2) * size_t(segs / 3 + 1)), "allocate cell bounds");
   STQ_CUDA(ctx, ctx->long_list.ensure(sizeof(int2) * slots), "allocate long-run list");
   ctx->rep_cap = int64_t(r);
   ctx->slot_cap = int64_t(slots);
@@ -310,18 +309,17 @@ int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int seg_bits, 
   ctx->scene.syz = ctx->syz.as<float4>();
   ctx->scene.sv = ctx->sv.as<int4>();
   ctx->scene.sflag = ctx->sflag.as<int>();
-  ctx->scene.sfloor = ctx->sfloor.as<float2>();
+  ctx->scene.scode = ctx->scode.as<uint32_t>();
   ctx->scene.partner = ctx->partner.as<int>();
   ctx->scene.run_end = ctx->run_end.as<int>();
   stage_begin(ctx, kGather);
   STQ_CUDA(ctx, launch_list_offsets(ctx->stream, kb[which], b.hdr, b.seg_scan, b.seg_cap, ctx->scene, ctx->slot_cap),
            "launch list offsets");
   STQ_CUDA(ctx, launch_gather_cells(ctx->stream, b.boxes, kb[which], vb[which], b.hdr, r, b.cell_base, b.scenes,
-                                    b.seg_scan, ctx->cell_floor.as<float2>(), ctx->seg_cap / 3,
-                                    ctx->scene),
+                                    b.seg_scan, ctx->scene),
            "launch gather");
   stage_end(ctx, kGather);
-  ctx->launches += 4;
+  ctx->launches += 3;
   return STQ_OK;
 }
 
@@ -376,7 +374,7 @@ int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
   p.work = &hdr->work;
   p.box_counts = ctx->box_counts.as<int32_t>();
   p.sflag = ctx->scene.sflag;
-  p.sfloor = ctx->scene.sfloor;
+  p.scode = ctx->scene.scode;
   p.partner = ctx->scene.partner;
   p.run_end = ctx->scene.run_end;
   p.scene_pairs = ctx->scene_pairs.as<unsigned long long>();

@@ -25,11 +25,6 @@ constexpr int kBlock = 256;
 constexpr int kHistBias = 40;  // extent bucket = binary exponent + 40
 constexpr int kSampleBoxes = 1024;
 
-__device__ __forceinline__ float key_float(uint32_t k) {
-  const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-  return __uint_as_float(b);
-}
-
 __device__ __forceinline__ void axes_bc(int a, int &b, int &c) {
   b = a == 0 ? 1 : 0;
   c = a == 2 ? 1 : 2;
@@ -346,6 +341,11 @@ batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
       g.nb = ((g.nb0 - 1) >> level) + 1;
       g.nc = ((g.nc0 - 1) >> level) + 1;
       g.ncells = g.nb * g.nc;
+      // 64 code steps per cell of the chosen level; a cell is 2^level level-0
+      // cells, of which there are nb0 over Lb (one cell: the whole extent)
+      const float steps = 64.f / float(1 << level);
+      g.sb = g.Lb > 0.f && isfinite(g.Lb) ? (level >= kCoordBits ? 64.f : steps * float(g.nb0)) / g.Lb : 0.f;
+      g.sc = g.Lc > 0.f && isfinite(g.Lc) ? (level >= kCoordBits ? 64.f : steps * float(g.nc0)) / g.Lc : 0.f;
       cells = unsigned(g.ncells);
     }
     // block exclusive scan of the cell counts
@@ -542,30 +542,6 @@ list_offsets_kernel(const unsigned long long *__restrict__ keys, BatchHeader *__
   if ((threadIdx.x & 31) == 0 && mx) atomicMax(&hdr->max_list, mx);
 }
 
-// Lower bounds of every cell on the two non-sweep axes (-inf for the first
-// row or column, where no box can start below the cell).
-__global__ void __launch_bounds__(kBlock)
-cell_floor_kernel(const unsigned int *__restrict__ cell_base, const SceneRecord *__restrict__ scenes,
-                  const BatchHeader *hdr, float2 *__restrict__ cell_floor, long long cells_cap) {
-  // more cells than the buffers hold is the replica overflow: nothing is swept
-  const unsigned int cells = (long long)hdr->cells <= cells_cap ? hdr->cells : 0u;
-  const int S = hdr->n_scenes;
-  for (unsigned int cell = blockIdx.x * kBlock + threadIdx.x; cell < cells; cell += gridDim.x * kBlock) {
-    int lo = 0, hi = S - 1;  // scene of the cell
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (cell_base[mid] <= cell) lo = mid;
-      else hi = mid - 1;
-    }
-    const GridParams g = scenes[lo].grid;
-    const int local = int(cell - cell_base[lo]);
-    const int cb = local / g.nc, cc = local - cb * g.nc;
-    // cell cb of the chosen level starts at level-0 cell cb << shift
-    cell_floor[cell] = make_float2(cb > 0 ? cell_lower_bound(cb << g.shift, g.ob, g.ib) : -INFINITY,
-                                   cc > 0 ? cell_lower_bound(cc << g.shift, g.oc, g.ic) : -INFINITY);
-  }
-}
-
 // Sorted replica p of segment s (cell c, type t; s = 3c + t) goes to
 // position p + s: every list is followed by one NaN slot, which ends every
 // run at its list (and cell, and scene) boundary.
@@ -575,10 +551,9 @@ cell_floor_kernel(const unsigned int *__restrict__ cell_base, const SceneRecord 
 // two minima on b, on c) is the max of the two boxes' first cells; both boxes
 // lie in this cell, so the reference point is here exactly when, on each of
 // b and c, one of the two replicas is its box's first cell.
-// sfloor of a position: on b and on c, -inf if the cell is the box's first
-// cell there, else the cell's lower bound; a candidate is in its first cell
-// on an axis exactly when its minimum there is >= that bound, so the sweep
-// tests the rule on the candidate's bounds, which it loads anyway.
+// scode of a position: its box's y/z interval in the cell and the inverted
+// first-cell bits (stq_device.cuh): one integer that the sweep tests against
+// the start box's before it loads any bound.
 // partner of a position: its first candidate. An edge's candidates are the
 // edges after it in its list; a vertex's are the cell's faces whose min is
 // >= its min (lower bound), a face's the cell's vertices whose min is > its
@@ -592,8 +567,8 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const unsigned long long
                     const SceneRecord *__restrict__ scenes, const uint32_t *__restrict__ seg_scan,
                     float *__restrict__ xmin,
                     float *__restrict__ xmax,
-                    const float2 *__restrict__ cell_floor, float4 *__restrict__ syz,
-                    int4 *__restrict__ sv, int *__restrict__ sflag, float2 *__restrict__ sfloor,
+                    float4 *__restrict__ syz,
+                    int4 *__restrict__ sv, int *__restrict__ sflag, uint32_t *__restrict__ scode,
                     int *__restrict__ partner, int *__restrict__ run_end) {
   const int64_t R = hdr->replicas;
   const int S = hdr->n_scenes;
@@ -662,13 +637,8 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const unsigned long long
     syz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
     sv[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
     sflag[k] = (lo << 2) | (fc << 1) | fb;
-    float2 fl = make_float2(-INFINITY, -INFINITY);
-    if (!(fb && fc)) {
-      const float2 cf = cell_floor[cell];
-      if (!fb) fl.x = cf.x;
-      if (!fc) fl.y = cf.y;
-    }
-    sfloor[k] = fl;
+    scode[k] = code_pack(code_step(x.min[b], g.ob, g.sb, cb), code_step(x.min[c], g.oc, g.sc, cc),
+                         code_step(x.max[b], g.ob, g.sb, cb), code_step(x.max[c], g.oc, g.sc, cc), !fb, !fc);
     partner[k] = int(first);
   }
 }
@@ -791,12 +761,10 @@ cudaError_t launch_gather_cells(cudaStream_t s, const stq_aabb *boxes,
                                 const unsigned long long *keys, const uint32_t *order,
                                 const BatchHeader *hdr, int64_t rep_cap,
                                 const unsigned int *cell_base, const SceneRecord *scenes,
-                                const uint32_t *seg_scan, float2 *cell_floor, int64_t cells_cap,
-                                SortedScene scene) {
-  cell_floor_kernel<<<blocks_for(cells_cap), kBlock, 0, s>>>(cell_base, scenes, hdr, cell_floor, cells_cap);
+                                const uint32_t *seg_scan, SortedScene scene) {
   gather_cells_kernel<<<wave_blocks((const void *)gather_cells_kernel, rep_cap), kBlock, 0, s>>>(
-      boxes, keys, order, hdr, cell_base, scenes, seg_scan, scene.xmin, scene.xmax, cell_floor, scene.syz,
-      scene.sv, scene.sflag, scene.sfloor, scene.partner, scene.run_end);
+      boxes, keys, order, hdr, cell_base, scenes, seg_scan, scene.xmin, scene.xmax, scene.syz,
+      scene.sv, scene.sflag, scene.scode, scene.partner, scene.run_end);
   return cudaGetLastError();
 }
 

@@ -78,8 +78,7 @@ struct stq_context {
   size_t in_host_bytes = 0;
   DevBuf scenes, cell_base, scene_pairs, counts, offsets, box_cells, scan_ws, keys64[2], vals[2], sort_ws;
   DevBuf points;  // fp64 vertex positions rounded to float once (box builds)
-  DevBuf xmin, xmax, syz, sv, sflag, sfloor, partner, run_end, box_counts, prefix_ws, pair_tmp;
-  DevBuf cell_floor;  // lower bounds of each cell on b and c
+  DevBuf xmin, xmax, syz, sv, sflag, scode, partner, run_end, box_counts, prefix_ws, pair_tmp;
   DevBuf long_list;  // runs handed from the lane sweep to the warp pass
   DevBuf seg_scan;  // first sorted replica of each (cell, type) list
   DevBuf bkeys[2], bvals[2];  // box sort: keys and box indices, double-buffered
@@ -129,8 +128,8 @@ struct stq_context {
   // every device buffer of the context
   std::vector<DevBuf *> buffers() {
     return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &counts, &box_cells, &offsets, &scan_ws,
-            &keys64[0], &keys64[1], &vals[0], &vals[1], &sort_ws, &xmin, &xmax, &syz, &sv, &sflag, &sfloor,
-            &cell_floor, &partner, &run_end, &long_list, &seg_scan, &bkeys[0], &bkeys[1], &bvals[0], &bvals[1],
+            &keys64[0], &keys64[1], &vals[0], &vals[1], &sort_ws, &xmin, &xmax, &syz, &sv, &sflag, &scode,
+            &partner, &run_end, &long_list, &seg_scan, &bkeys[0], &bkeys[1], &bvals[0], &bvals[1],
             &box_counts, &prefix_ws, &pair_tmp, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh,
             &aux, &window_pairs, &window_long_list, &window_cursors};
   }

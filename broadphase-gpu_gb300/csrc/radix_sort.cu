@@ -19,7 +19,6 @@
 // run, two skipped; 9.6 GB at 3.1 TB/s), 2.1 M pairs 249 -> 138 us, 346,000
 // pairs 158 -> 70 us, 6,700 pairs 138 -> 22 us.
 #include <algorithm>
-#include <atomic>
 
 #include "stq_device.cuh"
 #include "stq_internal.h"
@@ -444,20 +443,6 @@ radix_block_kernel(const K *kin, K *kout, const uint32_t *vin, uint32_t *vout, i
       kout[first + i * 32] = key[i];
       if (VALS) vout[first + i * 32] = val[i];
     }
-}
-
-// Lets a kernel take more than 48 KB of shared memory; asked once per kernel
-// and device.
-template <auto Kern>
-cudaError_t allow_smem(size_t bytes) {
-  static std::atomic<unsigned long long> done{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 64 && (done.load() >> dev & 1ull)) return cudaSuccess;
-  e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-  if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev);
-  return e;
 }
 
 int sm_count() {

@@ -34,10 +34,12 @@ constexpr size_t kOffXmax = kOffXmin + up256(sizeof(float) * kSlots);
 constexpr size_t kOffSyz = kOffXmax + up256(sizeof(float) * kSlots);
 constexpr size_t kOffSv = kOffSyz + up256(sizeof(float4) * kSlots);
 constexpr size_t kOffFlag = kOffSv + up256(sizeof(int4) * kSlots);
-constexpr size_t kOffFloor = kOffFlag + up256(sizeof(int) * kSlots);
-constexpr size_t kOffPartner = kOffFloor + up256(sizeof(float2) * kSlots);
-constexpr size_t kOffHdr = kOffPartner + up256(sizeof(int) * kSlots);
-constexpr size_t kOffScenePairs = kOffHdr + up256(sizeof(BatchHeader));
+constexpr size_t kOffCode = kOffFlag + up256(sizeof(int) * kSlots);
+constexpr size_t kOffPartner = kOffCode + up256(sizeof(uint32_t) * kSlots);
+constexpr size_t kOffRunEnd = kOffPartner + up256(sizeof(int) * kSlots);
+constexpr size_t kOffHdr = kOffRunEnd + up256(sizeof(int) * kSlots);
+constexpr size_t kOffExtent = kOffHdr + up256(sizeof(BatchHeader));  // see static_keys_kernel
+constexpr size_t kOffScenePairs = kOffExtent + 256;
 constexpr size_t kScratchBytes = kOffScenePairs + up256(sizeof(unsigned long long));
 
 // The scratch of every stq_sweep_static call on this device (about 4.5 MB).
@@ -45,7 +47,8 @@ static __device__ __align__(256) unsigned char g_static_scratch[kScratchBytes];
 
 // Writes the scene's sizes into the header (zeroed by the host before this
 // launch, so the NaN flag that any block may set is never cleared after it),
-// the sort keys and the box indices.
+// the sort keys and the box indices, and the scene's extent on the two other
+// axes: the largest ~key(min) and key(max) of each (zero before this launch).
 __global__ void static_keys_kernel(const stq_aabb *__restrict__ boxes, int n, int axis,
                                    unsigned char *scratch) {
   BatchHeader *hdr = reinterpret_cast<BatchHeader *>(scratch + kOffHdr);
@@ -60,25 +63,40 @@ __global__ void static_keys_kernel(const stq_aabb *__restrict__ boxes, int n, in
     hdr->length = unsigned(n);
   }
   bool nan = false;
+  uint32_t ext[4] = {0u, 0u, 0u, 0u};
   if (i < n) {
     const stq_aabb &b = boxes[i];
     for (int k = 0; k < 3; ++k) nan |= (b.min[k] != b.min[k]) | (b.max[k] != b.max[k]);
     keys[i] = float_key(b.min[axis]);
     vals[i] = uint32_t(i);
+    const int bb = axis == 0 ? 1 : 0, cc = axis == 2 ? 1 : 2;
+    ext[0] = ~float_key(b.min[bb]);
+    ext[1] = ~float_key(b.min[cc]);
+    ext[2] = float_key(b.max[bb]);
+    ext[3] = float_key(b.max[cc]);
   }
   if (__any_sync(kFullMask, nan) && (threadIdx.x & 31) == 0) atomicOr(&hdr->flags, kFlagNaN);
+  uint32_t *extent = reinterpret_cast<uint32_t *>(scratch + kOffExtent);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const uint32_t m = __reduce_max_sync(kFullMask, ext[e]);
+    if ((threadIdx.x & 31) == 0) atomicMax(&extent[e], m);
+  }
 }
 
 // Sorted positions 0..n-1 (one cell), then the NaN sentinel and the padding.
 __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, int axis,
-                                     const uint32_t *__restrict__ order, unsigned char *scratch) {
+                                     const uint32_t *__restrict__ keys, const uint32_t *__restrict__ order,
+                                     unsigned char *scratch) {
   float *xmin = reinterpret_cast<float *>(scratch + kOffXmin);
   float *xmax = reinterpret_cast<float *>(scratch + kOffXmax);
   float4 *syz = reinterpret_cast<float4 *>(scratch + kOffSyz);
   int4 *sv = reinterpret_cast<int4 *>(scratch + kOffSv);
   int *sflag = reinterpret_cast<int *>(scratch + kOffFlag);
-  float2 *sfloor = reinterpret_cast<float2 *>(scratch + kOffFloor);
+  uint32_t *scode = reinterpret_cast<uint32_t *>(scratch + kOffCode);
   int *partner = reinterpret_cast<int *>(scratch + kOffPartner);
+  int *run_end = reinterpret_cast<int *>(scratch + kOffRunEnd);
+  const uint32_t *extent = reinterpret_cast<const uint32_t *>(scratch + kOffExtent);
   const int b = axis == 0 ? 1 : 0, c = axis == 2 ? 1 : 2;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) {
@@ -88,13 +106,27 @@ __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, 
     syz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
     sv[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
     sflag[k] = 3;  // one cell: every box is in its first cell on both axes
-    sfloor[k] = make_float2(-INFINITY, -INFINITY);
+    const float ob = key_float(~extent[0]), oc = key_float(~extent[1]);
+    const float lb = key_float(extent[2]) - ob, lc = key_float(extent[3]) - oc;
+    const float sb = lb > 0.f && isfinite(lb) ? 64.f / lb : 0.f, sc = lc > 0.f && isfinite(lc) ? 64.f / lc : 0.f;
+    scode[k] = code_pack(code_step(x.min[b], ob, sb, 0), code_step(x.min[c], oc, sc, 0), code_step(x.max[b], ob, sb, 0),
+                         code_step(x.max[c], oc, sc, 0), false, false);
     partner[k] = k + 1;  // one list: candidates follow in sort order
+    // one past the last minimum that is not above this maximum
+    const uint32_t xk = float_key(x.max[axis]);
+    int lo = k + 1, hi = n;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (keys[mid] <= xk) lo = mid + 1;
+      else hi = mid;
+    }
+    run_end[k] = lo;
   } else if (k < n + 1 + kSortedPad) {
     const float q = __int_as_float(0x7fc00000);
     xmin[k] = q;
     xmax[k] = q;
     partner[k] = k;
+    run_end[k] = k;
   }
 }
 
@@ -142,16 +174,16 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   BatchHeader *hdr = reinterpret_cast<BatchHeader *>(scratch + kOffHdr);
   if (radix_sort_u32(s, kb, vb, n, scratch + kOffSortWs, &hdr->fault, nullptr) != cudaSuccess)
     return STQ_ERR_CUDA;
-  static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, vb[0], scratch);
+  static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, kb[0], vb[0], scratch);
   SweepParams p;
   p.xmin = reinterpret_cast<const float *>(scratch + kOffXmin);
   p.xmax = reinterpret_cast<const float *>(scratch + kOffXmax);
   p.syz = reinterpret_cast<const float4 *>(scratch + kOffSyz);
   p.sv = reinterpret_cast<const int4 *>(scratch + kOffSv);
   p.sflag = reinterpret_cast<const int *>(scratch + kOffFlag);
-  p.sfloor = reinterpret_cast<const float2 *>(scratch + kOffFloor);
+  p.scode = reinterpret_cast<const uint32_t *>(scratch + kOffCode);
   p.partner = reinterpret_cast<const int *>(scratch + kOffPartner);
-  p.run_end = nullptr;  // run ends are not computed here; the sweep takes the queue shape
+  p.run_end = reinterpret_cast<const int *>(scratch + kOffRunEnd);
   p.begin = 0;
   p.end = ni;
   p.chunk = 32;

@@ -66,6 +66,12 @@ __device__ __forceinline__ uint32_t float_key(float f) {
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// The float of a key (-0 comes back as +0).
+__device__ __forceinline__ float key_float(uint32_t k) {
+  const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+  return __uint_as_float(b);
+}
+
 // Box type from the signs of vertexIds (src/aabb.cu:12-31): vertex 0, edge
 // 1, face 2.
 __device__ __forceinline__ int type_of(int v1, int v2) {
@@ -82,29 +88,38 @@ __device__ __forceinline__ int cell_coord(float v, float origin, float inv, int 
   return int(t);
 }
 
-// Lower bound of cell C (1 <= C <= n - 1) on one axis: the smallest float v
-// with cell_coord(v, origin, inv, n) >= C, i.e. with (v - origin) * inv >= C
-// in the same round-to-nearest steps. That test is monotone in v, so a binary
-// search over the floats in order (ordered bit patterns from -inf to +inf,
-// -0 just below +0; no NaN lies between) finds v exactly in 32 steps. For a
-// box of a replica in cell C, "C is the cell of the box's minimum" is then
-// "minimum >= the lower bound of C": the cell of the minimum is at most C.
-__device__ __forceinline__ float cell_lower_bound(int C, float origin, float inv) {
-  auto ordered = [](float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-  };
-  auto from_ordered = [](uint32_t k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
-  };
-  const float fc = float(C);
-  uint32_t lo = ordered(-INFINITY), hi = ordered(INFINITY);  // test fails at lo, holds at hi
-  while (hi - lo > 1u) {
-    const uint32_t mid = lo + ((hi - lo) >> 1);
-    if (__fmul_rn(__fsub_rn(from_ordered(mid), origin), inv) >= fc) hi = mid;
-    else lo = mid;
-  }
-  return from_ordered(hi);
+// ---- position codes -----------------------------------------------------------
+// A sorted position's code holds its box's y/z interval in its cell, in 64
+// steps per axis, and whether the cell is not the box's first along b and c:
+//   bits 0-5 lo_b | 7-12 lo_c | 14-19 63 - hi_b | 21-26 63 - hi_c | 28 nf_b | 30 nf_c
+// Every field has a zero guard bit above it. For a start box with code A and a
+// candidate with code B, every guard bit of code_start(A) - B is set exactly
+// when hi_a >= lo_b and hi_b >= lo_a on both axes (in steps) and neither axis
+// has the flag set in both: the fields of code_start(A) are 64 + hi_a, 64 + 63 -
+// lo_a and 2 + 1 - nf_a, so that no field borrows. Steps are a monotone function
+// of the bound, clamped to the cell, so boxes that overlap always pass: one
+// subtraction and one test stand for six float comparisons, and the exact test
+// is left to the pairs that pass.
+constexpr uint32_t kCodeGuard = 0xa8102040u;
+constexpr uint32_t kCodeNotFirst = 0x50000000u;
+
+__host__ __device__ __forceinline__ uint32_t code_pack(uint32_t lo_b, uint32_t lo_c, uint32_t hi_b, uint32_t hi_c,
+                                                       bool nf_b, bool nf_c) {
+  return lo_b | lo_c << 7 | (63u - hi_b) << 14 | (63u - hi_c) << 21 | (nf_b ? 1u << 28 : 0u) | (nf_c ? 1u << 30 : 0u);
+}
+__host__ __device__ __forceinline__ uint32_t code_start(uint32_t c) {
+  return ~((c >> 14 & 0x3fffu) | (c & 0x3fffu) << 14 | (c & 0xf0000000u));
+}
+__host__ __device__ __forceinline__ bool code_pass(uint32_t start, uint32_t cand) {
+  return (~(start - cand) & kCodeGuard) == 0u;
+}
+
+// Step of a bound in cell `cell`: scale is steps (64 per cell) per unit length.
+// Monotone in v (round-to-nearest steps, clamped; NaN, which only an infinite
+// origin gives, counts as 0).
+__device__ __forceinline__ uint32_t code_step(float v, float origin, float scale, int cell) {
+  const float t = __fsub_rn(__fmul_rn(__fsub_rn(v, origin), scale), 64.f * float(cell));
+  return uint32_t(fminf(fmaxf(t, 0.f), 63.f));
 }
 
 // ---- box type and pair filter ------------------------------------------------

@@ -3,6 +3,7 @@
 // kernel launch wrappers.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 
@@ -33,6 +34,20 @@ struct DevBuf {
   }
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
+
+// Lets a kernel take more than 48 KB of shared memory; asked once per kernel
+// and device.
+template <auto Kern>
+cudaError_t allow_smem(size_t bytes) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 64 && (done.load() >> dev & 1ull)) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+  if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev);
+  return e;
+}
 
 // Device-side scalars of one sweep: counters, flags and results read back
 // by the host in a single copy.
@@ -74,7 +89,7 @@ struct GridParams {
   int nb0, nc0;   // level-0 cells along b and c
   int shift;      // cell coordinate = level-0 coordinate >> shift (the chosen
                   // level; kCoordBits when no level fits: one cell)
-  int pad;
+  float sb, sc;   // code steps (64 per cell of the chosen level) per unit length
 };
 
 constexpr int kGridLevels = 6;  // level L halves the level-0 grid L times
@@ -166,8 +181,8 @@ struct SortedScene {
   float4 *syz = nullptr;  // (min_b, min_c, max_b, max_c) on the other axes
   int4 *sv = nullptr;     // (vertexIds[0..2], id)
   int *sflag = nullptr;   // first-cell bits (0: along b, 1: along c), scene << 2
-  float2 *sfloor = nullptr;  // per axis b, c: -inf where the cell is the box's
-                             // first, else the cell's lower bound
+  uint32_t *scode = nullptr;  // y/z interval in the cell and first-cell bits
+                              // (position codes, stq_device.cuh)
   int *partner = nullptr; // first candidate position of each start position
   int *run_end = nullptr; // one past its last candidate on the sweep axis
   int64_t length = 0;     // sweep positions (boxes; sentinels excluded at the end)
@@ -205,8 +220,7 @@ struct SweepParams {
   int *work;
   int32_t *box_counts;       // count mode: pairs per start position (k - begin)
   const int *sflag;          // first-cell bits and scene of each position
-  const float2 *sfloor;      // first-cell rule of a start position on b and c:
-                             // a candidate passes if its minima are >= these
+  const uint32_t *scode;     // position codes
   const int *partner;        // first candidate position of each start position
   const int *run_end;        // one past its last candidate (null: not computed;
                              // the flat shape needs it)
@@ -278,8 +292,7 @@ cudaError_t launch_gather_cells(cudaStream_t s, const stq_aabb *boxes,
                                 const unsigned long long *keys, const uint32_t *order,
                                 const BatchHeader *hdr, int64_t rep_cap,
                                 const unsigned int *cell_base, const SceneRecord *scenes,
-                                const uint32_t *seg_scan, float2 *cell_floor, int64_t cells_cap,
-                                SortedScene scene);
+                                const uint32_t *seg_scan, SortedScene scene);
 // Batched box build: scene s has vertices [voff[s], voff[s+1]) etc.; box ids
 // are global (box_off[s] + local), vertex ids local to the scene.
 // points: 2 * vert_cap float4 of scratch for the rounded positions

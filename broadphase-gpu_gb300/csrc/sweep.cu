@@ -46,7 +46,7 @@ __device__ __forceinline__ void flush_staged(const int2 *st, int n, int lane, co
   __syncwarp();
 }
 
-template <int G, int Q, int BLOCK, bool COUNT>
+template <int G, int Q, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_kernel(const SweepParams p) {
   static_assert(32 % G == 0, "lane group must divide the warp");
@@ -55,7 +55,7 @@ stq_sweep_kernel(const SweepParams p) {
   constexpr int E = 32 / G;  // lane groups per warp
   constexpr int STAGE = 64;  // pairs staged per warp before one global append
   __shared__ int ring[BLOCK / 32][Q];
-  __shared__ int2 stage[COUNT ? 1 : BLOCK / 32][COUNT ? 1 : STAGE];
+  __shared__ int2 stage[BLOCK / 32][STAGE];
 
   const int lane = threadIdx.x & 31;
   const int gl = lane % G;              // lane within group
@@ -70,11 +70,11 @@ stq_sweep_kernel(const SweepParams p) {
   int next_k = 0, chunk_end = 0;
   bool more = true;
   // lane-group state (identical in the G lanes of a group)
-  int k = -1, j0 = 0, acc = 0, taken = 0;
+  int k = -1, j0 = 0, taken = 0;
   float kmax = 0.f;
   float4 kb = make_float4(0.f, 0.f, 0.f, 0.f);
   int4 kv = make_int4(0, 0, 0, 0);
-  float2 kfl = make_float2(0.f, 0.f);  // first-cell rule of the current start box
+  uint32_t knf = 0;  // not-first bits of the current start box
   const int end = min(p.end, int(p.hdr->length));
   const int span = end - p.begin;
   int kf = 0;  // scene of the current start box (above the first-cell bits)
@@ -85,7 +85,7 @@ stq_sweep_kernel(const SweepParams p) {
   int wscene = 0;
   unsigned long long wpairs = 0;
   const bool multi = p.hdr->n_scenes > 1;  // per-scene counts need the scene of each hit
-  int2 *st = stage[COUNT ? 0 : (threadIdx.x >> 5)];
+  int2 *st = stage[threadIdx.x >> 5];
 
   while (true) {
     // 1. Refill the ring with start boxes that have at least one candidate.
@@ -123,8 +123,7 @@ stq_sweep_kernel(const SweepParams p) {
         kmax = p.xmax[k];
         kb = p.syz[k];
         kv = p.sv[k];
-        kfl = p.sfloor[k];
-        acc = 0;
+        knf = p.scode[k] & kCodeNotFirst;
         taken = 0;
         kf = multi ? p.sflag[k] : 0;
       }
@@ -150,8 +149,8 @@ stq_sweep_kernel(const SweepParams p) {
       const float4 b = p.syz[j];
       // a pair found in several cells is emitted only in the cell of its
       // reference point: on b and on c, one of the two replicas must be its
-      // box's first cell (the candidate's: minimum >= the cell's lower bound)
-      if (overlap_bc(kb, b) && b.x >= kfl.x && b.y >= kfl.y) {  // ids only for these
+      // box's first cell
+      if (overlap_bc(kb, b) && (p.scode[j] & knf) == 0u) {  // ids only for these
         const int4 bv = p.sv[j];
         hit = (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
         lo_id = min(kv.w, bv.w);
@@ -162,9 +161,7 @@ stq_sweep_kernel(const SweepParams p) {
     //    it to the pair list with one global atomic per 32 or more pairs.
     const unsigned hm = __ballot_sync(kFullMask, hit);
     const int ghits = __popc(hm & grp_mask);
-    if (COUNT) {
-      acc += ghits;
-    } else if (hm) {
+    if (hm) {
       if (hit) st[staged + __popc(hm & lanemask_lt())] = make_int2(lo_id, hi_id);
       staged += __popc(hm);
       // per-scene counts: one register while the warp stays in one scene
@@ -198,23 +195,19 @@ stq_sweep_kernel(const SweepParams p) {
         if (p.run_cap && taken >= p.run_cap) {  // a long run: the warp pass takes the rest
           if (gl == 0) {
             p.long_list[atomicAdd(p.long_items, 1u)] = make_int2(k, j0);
-            if (COUNT) p.box_counts[k - p.begin] = acc;
           }
           k = -1;
         }
       } else {
-        if (COUNT && gl == 0) p.box_counts[k - p.begin] = acc;
         k = -1;
       }
     }
   }
-  if (!COUNT) {
-    __syncwarp();
-    if (staged) flush_staged(st, staged, lane, p);
-    if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
-    const unsigned t = __reduce_add_sync(kFullMask, tested);
-    if (lane == 0 && p.stats) atomicAdd(p.stats, (unsigned long long)t);
-  }
+  __syncwarp();
+  if (staged) flush_staged(st, staged, lane, p);
+  if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
+  const unsigned t = __reduce_add_sync(kFullMask, tested);
+  if (lane == 0 && p.stats) atomicAdd(p.stats, (unsigned long long)t);
 }
 
 // One start box per lane. A lane walks its own run, U consecutive candidates
@@ -223,7 +216,7 @@ stq_sweep_kernel(const SweepParams p) {
 // (lane-local: no ballot), and a lane whose run ended takes the next pending
 // box from the warp's ring. Otherwise as stq_sweep_kernel: ring refill by
 // ballot compaction, lazy vertex-id loads, per-warp staging of pairs.
-template <int U, int Q, int BLOCK, bool COUNT>
+template <int U, int Q, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_lane_kernel(const SweepParams p) {
   static_assert(U == 1 || U == 2 || U == 4 || U == 8, "candidates per lane step: 1, 2, 4 or 8");
@@ -235,21 +228,21 @@ stq_sweep_lane_kernel(const SweepParams p) {
   constexpr bool kWide = (BLOCK / 32) * (Q * 8 + STAGE * 8) <= 48 * 1024;
   using Entry = typename std::conditional<kWide, int2, int>::type;
   __shared__ Entry ring[BLOCK / 32][Q];
-  __shared__ int2 stage[COUNT ? 1 : BLOCK / 32][COUNT ? 1 : STAGE];
+  __shared__ int2 stage[BLOCK / 32][STAGE];
 
   const int lane = threadIdx.x & 31;
   const unsigned below = lanemask_lt();
   Entry *q = ring[threadIdx.x >> 5];
-  int2 *st = stage[COUNT ? 0 : (threadIdx.x >> 5)];
+  int2 *st = stage[threadIdx.x >> 5];
 
   int qhead = 0, qsize = 0;
   int next_k = 0, chunk_end = 0;
   bool more = true;
-  int k = -1, j = 0, acc = 0, kf = 0, taken = 0;
+  int k = -1, j = 0, kf = 0, taken = 0;
   float kmax = 0.f;
   float4 kb = make_float4(0.f, 0.f, 0.f, 0.f);
   int4 kv = make_int4(0, 0, 0, 0);
-  float2 kfl = make_float2(0.f, 0.f);  // first-cell rule of the start box
+  uint32_t knf = 0;  // not-first bits of the start box
   const int end = min(p.end, int(p.hdr->length));
   const int span = end - p.begin;
   unsigned tested = 0;
@@ -307,9 +300,8 @@ stq_sweep_lane_kernel(const SweepParams p) {
         kmax = p.xmax[k];
         kb = p.syz[k];
         kv = p.sv[k];
-        kfl = p.sfloor[k];
+        knf = p.scode[k] & kCodeNotFirst;
         kf = multi ? p.sflag[k] : 0;
-        acc = 0;
         taken = 0;
       }
     }
@@ -340,7 +332,7 @@ stq_sweep_lane_kernel(const SweepParams p) {
     for (int u = 0; u < U; ++u) {
       if (u < nvalid) {
         const float4 b = p.syz[j + u];
-        if (overlap_bc(kb, b) && b.x >= kfl.x && b.y >= kfl.y) {  // and the first-cell rule
+        if (overlap_bc(kb, b) && (p.scode[j + u] & knf) == 0u) {  // and the first-cell rule
           const int4 bv = p.sv[j + u];
           if ((p.typed || valid_pair(kv, bv)) && !covertex(kv, bv)) hits |= 1u << u;
         }
@@ -348,44 +340,40 @@ stq_sweep_lane_kernel(const SweepParams p) {
     }
     // 4. Emit the step's hits through the warp's staging buffer.
     const int nh = __popc(hits);
-    if (COUNT) {
-      acc += nh;
-    } else {
-      const unsigned anym = __ballot_sync(kFullMask, nh > 0);
-      if (anym) {
-        int total = 0;
+    const unsigned anym = __ballot_sync(kFullMask, nh > 0);
+    if (anym) {
+      int total = 0;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const bool hit = (hits >> u) & 1u;
-          const unsigned hm = __ballot_sync(kFullMask, hit);
-          if (hit) {
-            const int id = p.sv[j + u].w;
-            st[staged + __popc(hm & below)] = make_int2(min(kv.w, id), max(kv.w, id));
-          }
-          staged += __popc(hm);
-          total += __popc(hm);
+      for (int u = 0; u < U; ++u) {
+        const bool hit = (hits >> u) & 1u;
+        const unsigned hm = __ballot_sync(kFullMask, hit);
+        if (hit) {
+          const int id = p.sv[j + u].w;
+          st[staged + __popc(hm & below)] = make_int2(min(kv.w, id), max(kv.w, id));
         }
-        // per-scene counts: one register while the warp stays in one scene
-        if (!multi) {
+        staged += __popc(hm);
+        total += __popc(hm);
+      }
+      // per-scene counts: one register while the warp stays in one scene
+      if (!multi) {
+        wpairs += unsigned(total);
+      } else {
+        const int lead = __shfl_sync(kFullMask, kf >> 2, __ffs(anym) - 1);
+        if (__all_sync(kFullMask, nh == 0 || (kf >> 2) == lead)) {
+          if (lead != wscene) {
+            if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
+            wscene = lead;
+            wpairs = 0;
+          }
           wpairs += unsigned(total);
-        } else {
-          const int lead = __shfl_sync(kFullMask, kf >> 2, __ffs(anym) - 1);
-          if (__all_sync(kFullMask, nh == 0 || (kf >> 2) == lead)) {
-            if (lead != wscene) {
-              if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
-              wscene = lead;
-              wpairs = 0;
-            }
-            wpairs += unsigned(total);
-          } else if (nh) {
-            atomicAdd(&p.scene_pairs[kf >> 2], (unsigned long long)nh);
-          }
+        } else if (nh) {
+          atomicAdd(&p.scene_pairs[kf >> 2], (unsigned long long)nh);
         }
-        if (staged >= 32) {
-          __syncwarp();
-          flush_staged(st, staged, lane, p);
-          staged = 0;
-        }
+      }
+      if (staged >= 32) {
+        __syncwarp();
+        flush_staged(st, staged, lane, p);
+        staged = 0;
       }
     }
     // 5. A lane whose U candidates all passed continues; otherwise its run ended.
@@ -395,66 +383,84 @@ stq_sweep_lane_kernel(const SweepParams p) {
         taken += U;
         if (p.run_cap && taken >= p.run_cap) {  // a long run: the warp pass takes the rest
           p.long_list[atomicAdd(p.long_items, 1u)] = make_int2(k, j);
-          if (COUNT) p.box_counts[k - p.begin] = acc;
           k = -1;
         }
       } else {
-        if (COUNT) p.box_counts[k - p.begin] = acc;
         k = -1;
       }
     }
   }
-  if (!COUNT) {
-    __syncwarp();
-    if (staged) flush_staged(st, staged, lane, p);
-    if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
-    const unsigned t = __reduce_add_sync(kFullMask, tested);
-    if (lane == 0 && p.stats) atomicAdd(p.stats, (unsigned long long)t);
-  }
+  __syncwarp();
+  if (staged) flush_staged(st, staged, lane, p);
+  if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
+  const unsigned t = __reduce_add_sync(kFullMask, tested);
+  if (lane == 0 && p.stats) atomicAdd(p.stats, (unsigned long long)t);
 }
 
 // Flat shape. A warp takes 32 consecutive start positions; each one's run on
 // the sweep axis is [partner, run_end), both found by the gather (runs longer
-// than run_cap are cut there and the rest goes to the warp pass). The runs of
-// the starts that have candidates are laid end to end, and the warp walks
-// that flat sequence 32 candidates per step, one per lane: lane l of the step
-// at `base` takes flat candidate f = base + l, whose start is the last one
-// whose run begins at or before f (a bit mask of the run beginnings inside the
-// step, one OR-reduction, and a population count). Consecutive lanes read
-// consecutive positions of a run, and every lane works except in the last
-// step of the 32 starts.
-// Two passes per warp. The filter tests the y/z overlap and the first-cell
-// rule on the candidate's (min_b, min_c, max_b, max_c) record, V steps with
-// their loads issued together, and compacts the candidates that pass into a
-// per-warp shared-memory queue. Once 32 are queued, the check takes them one
-// per lane: the vertex ids of both boxes, is_valid_pair and covertex, and the
-// hits go through the staging buffer as in the other shapes. The starts'
-// records sit in shared memory, so the queue is drained before the next 32
-// starts replace them.
+// than run_cap are cut there and the rest goes to the warp pass).
+//
+// The filter compares position codes (stq_device.cuh): one integer per
+// candidate and one per start box, a subtraction and a test for the y/z
+// overlap and the first-cell rule. It has two forms, chosen for each 32 starts:
+//   - band: the starts' runs lie in one window of positions. One start per
+//     lane, the window's codes 32 at a time through shared memory, every lane
+//     tests all 32 (three integer instructions each) and keeps the bits inside
+//     its own run. The cost goes with the window, whatever the runs cover of it.
+//   - flat: the runs are laid end to end and the warp takes 32 candidates per
+//     step, one per lane: lane l of the step at `base` takes flat candidate
+//     base + l, whose start is the last one whose run begins at or before it (a
+//     bit mask of the run beginnings inside the step, one OR-reduction, and a
+//     population count). The cost goes with the candidates.
+// Candidates that pass are queued in shared memory (start slot and offset in
+// its run), and taken 32 at a time, one per lane, for the exact y/z test, the
+// vertex ids, is_valid_pair and covertex. The hits go through the staging
+// buffer. The starts' records sit in shared memory, so the queue is drained
+// before the next 32 starts replace them.
 struct FlatStart {
-  float4 kb;   // start box (min_b, min_c, max_b, max_c)
-  float2 kfl;  // first-cell rule
-  int joff;    // position of flat candidate f is joff + f
-  int kf;      // first-cell bits and scene
-  int4 kv;     // vertex ids and id
+  float4 kb;      // start box (min_b, min_c, max_b, max_c)
+  uint32_t code;  // code_start of its code
+  int joff;       // position of flat candidate f is joff + f
+  int j;          // first position of its run
+  int kf;         // first-cell bits and scene
+  int4 kv;        // vertex ids and id
 };
 static_assert(sizeof(FlatStart) == 48, "FlatStart: three 16-byte words");
 
-template <int BLOCK, int V>
+// Band or flat: a band step takes some 500 instructions for 32 positions, 130 of
+// them the filter, and a flat step some 30 for its 32 candidates. The line is
+// flat between 3 and 8 candidates per position of the window (1.16 to 1.18 ms
+// on the 6 M-box scene, where 98% of the candidates are in bands); without
+// bands that sweep takes 1.36 ms.
+constexpr int kBandRatio = 6;
+// Pairs staged per warp, appended with one atomic on the pair counter once
+// fewer than 32 places are left. All warps share that counter: with 64 places
+// the same sweep takes 1.61 ms, with 128 1.16, with 192 1.12; larger stages take
+// resident blocks away (384: 1.20, 768: 1.38 ms).
+constexpr int kFlatStage = 192;
+constexpr int kFlatRound = 256;  // candidates queued at once by a band step (or 32 V by a flat one)
+constexpr int kFlatQueue = 32 + kFlatRound;
+struct FlatWarp {
+  FlatStart rec[32];
+  int2 stage[kFlatStage];
+  uint32_t queue[kFlatQueue];  // slot | offset in the run << 5 (run_cap < 2^27)
+  uint4 code[8];               // a band step's 32 candidate codes
+  int hits[32];                // count mode: pairs per slot
+};
+
+template <int BLOCK, int V, bool COUNT>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_flat_kernel(const SweepParams p) {
-  constexpr int STAGE = 64;  // < 32 left over + at most 32 new pairs per check
-  constexpr int QUEUE = 32 * (V + 1);  // < 32 left over + at most 32 * V per filter round
-  __shared__ FlatStart recs[BLOCK / 32][32];
-  __shared__ int2 stage[BLOCK / 32][STAGE];
-  __shared__ int2 queue[BLOCK / 32][QUEUE];  // (start record, candidate position)
-
+  static_assert(32 * V <= kFlatRound, "queue holds a flat round");
+  extern __shared__ __align__(16) unsigned char flat_smem[];
+  FlatWarp &sw = reinterpret_cast<FlatWarp *>(flat_smem)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const unsigned below = lanemask_lt();
   const unsigned upto = below | (1u << lane);
-  FlatStart *rec = recs[threadIdx.x >> 5];
-  int2 *st = stage[threadIdx.x >> 5];
-  int2 *qu = queue[threadIdx.x >> 5];
+  FlatStart *rec = sw.rec;
+  int2 *st = sw.stage;
+  uint32_t *qu = sw.queue;
 
   const int end = min(p.end, int(p.hdr->length));
   const int span = end - p.begin;
@@ -471,14 +477,22 @@ stq_sweep_flat_kernel(const SweepParams p) {
     int2 pr = make_int2(0, 0);
     int kf = 0;
     if (lane < n) {
-      const int2 e = qu[queued - n + lane];
-      const int4 bv = p.sv[e.y];
-      const int4 kv = rec[e.x].kv;
-      if (multi) kf = rec[e.x].kf;
-      hit = (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
-      pr = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
+      const uint32_t e = qu[queued - n + lane];
+      const FlatStart &r = rec[e & 31u];
+      const int j = r.j + int(e >> 5);
+      const float4 b = p.syz[j];
+      const int4 bv = p.sv[j];
+      const int4 kv = r.kv;
+      if (multi) kf = r.kf;
+      hit = overlap_bc(r.kb, b) && (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
+      if (COUNT) {
+        if (hit) atomicAdd(&sw.hits[e & 31u], 1);
+      } else {
+        pr = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
+      }
     }
     queued -= n;
+    if (COUNT) return;
     const unsigned hm = __ballot_sync(kFullMask, hit);
     if (hm) {
       if (hit) st[staged + __popc(hm & below)] = pr;
@@ -498,7 +512,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
           atomicAdd(&p.scene_pairs[kf >> 2], 1ull);
         }
       }
-      if (staged >= 32) {
+      if (staged > kFlatStage - 32) {
         __syncwarp();
         flush_staged(st, staged, lane, p);
         staged = 0;
@@ -531,8 +545,8 @@ stq_sweep_flat_kernel(const SweepParams p) {
     }
     const unsigned nz = __ballot_sync(kFullMask, len > 0);
     if (nz == 0) continue;
-    // 2. Lay the runs end to end: exclusive prefix of the lengths; the starts
-    //    with candidates keep their records in shared memory, in lane order.
+    // 2. Exclusive prefix of the lengths; the starts with candidates keep their
+    //    records in shared memory, in lane order.
     int incl = len;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -541,60 +555,116 @@ stq_sweep_flat_kernel(const SweepParams p) {
     }
     const int excl = incl - len;
     const int total = __shfl_sync(kFullMask, incl, 31);
+    const int slot = __popc(nz & below);
+    uint32_t code = 0;
     if (len > 0) {
       FlatStart r;
       r.kb = p.syz[k];
-      r.kfl = p.sfloor[k];
+      code = code_start(p.scode[k]);
+      r.code = code;
       r.joff = j - excl;
+      r.j = j;
       r.kf = multi ? p.sflag[k] : 0;
       r.kv = p.sv[k];
-      rec[__popc(nz & below)] = r;
+      rec[slot] = r;
     }
-    __syncwarp();
+    if (COUNT) sw.hits[lane] = 0;
     tested += unsigned(total);
-    // a run that begins inside the step at `base` marks bit (excl - base)
-    const unsigned my_begin = len > 0 ? unsigned(excl) : 0xffffffffu;
-    // 3. The filter over the flat candidates, V steps of 32 at a time.
-    int begun = 0;  // starts whose run began before the current step
-    for (int base = 0; base < total; base += 32 * V) {
-      int si[V], jj[V];
-      float4 kfj[V];  // (rule b, rule c, joff, -) of each lane's start
-      float4 b[V];
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const unsigned d = my_begin - unsigned(base + 32 * v);
-        const unsigned heads = __reduce_or_sync(kFullMask, d < 32u ? (1u << d) : 0u);
-        si[v] = begun + __popc(heads & upto) - 1;
-        begun += __popc(heads);
-        const int f = base + 32 * v + lane;
-        kfj[v] = *reinterpret_cast<const float4 *>(&rec[si[v]].kfl);
-        jj[v] = f < total ? __float_as_int(kfj[v].z) + f : -1;
-      }
-#pragma unroll
-      for (int v = 0; v < V; ++v)
-        if (jj[v] >= 0) b[v] = p.syz[jj[v]];
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        bool pass = false;
-        if (jj[v] >= 0) {
-          const float4 kb = rec[si[v]].kb;
-          // the first-cell rule as in the other shapes
-          pass = overlap_bc(kb, b[v]) && b[v].x >= kfj[v].x && b[v].y >= kfj[v].y;
-        }
-        const unsigned pm = __ballot_sync(kFullMask, pass);
-        if (pass) qu[queued + __popc(pm & below)] = make_int2(si[v], jj[v]);
-        queued += __popc(pm);
-      }
-      __syncwarp();
-      // 4. The check, 32 queued candidates at a time.
-      while (queued >= 32) {
-        check(32);
+    const int jlo = __reduce_min_sync(kFullMask, len > 0 ? j : 0x7fffffff);
+    const int jhi = __reduce_max_sync(kFullMask, len > 0 ? j + len : 0);
+    __syncwarp();
+    if (jhi - jlo <= total / kBandRatio) {
+      // 3a. The band: 32 positions of the window per step.
+      for (int j0 = jlo; j0 < jhi; j0 += 32) {
+        const int lo = j - j0, hi = lo + len;
+        uint32_t mine = 0;  // positions of this step inside the lane's run
+        if (len > 0 && lo < 32 && hi > 0)
+          mine = (kFullMask << max(lo, 0)) & (hi >= 32 ? kFullMask : ~(kFullMask << hi));
+        if (__ballot_sync(kFullMask, mine != 0u) == 0u) continue;
+        reinterpret_cast<uint32_t *>(sw.code)[lane] = p.scode[j0 + lane];
         __syncwarp();
+        uint32_t hits = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const uint4 c = sw.code[q];
+          if (code_pass(code, c.x)) hits |= 1u << (4 * q);
+          if (code_pass(code, c.y)) hits |= 2u << (4 * q);
+          if (code_pass(code, c.z)) hits |= 4u << (4 * q);
+          if (code_pass(code, c.w)) hits |= 8u << (4 * q);
+        }
+        hits &= mine;
+        // queue them, places by a prefix sum of the lanes' counts; more than
+        // the queue holds go 8 positions (at most 256 candidates) at a time
+        uint32_t part = __reduce_add_sync(kFullMask, __popc(hits)) <= unsigned(kFlatRound) ? kFullMask : 0xffu;
+        do {
+          uint32_t h = hits & part;
+          hits ^= h;
+          part <<= 8;
+          const int count = __popc(h);
+          int at = count;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFullMask, at, o);
+            if (lane >= o) at += v;
+          }
+          const int all = __shfl_sync(kFullMask, at, 31);
+          at += queued - count;
+          while (h) {
+            const int c = __ffs(h) - 1;
+            h &= h - 1u;
+            qu[at++] = unsigned(slot) | unsigned(c - lo) << 5;
+          }
+          queued += all;
+          __syncwarp();
+          while (queued >= 32) {
+            check(32);
+            __syncwarp();
+          }
+        } while (__any_sync(kFullMask, hits != 0u));
+      }
+    } else {
+      // 3b. Flat: V steps of 32 candidates at a time. A run that begins inside
+      //     the step at `base` marks bit (excl - base).
+      const unsigned my_begin = len > 0 ? unsigned(excl) : 0xffffffffu;
+      int begun = 0;  // starts whose run began before the current step
+      for (int base = 0; base < total; base += 32 * V) {
+        int si[V], rel[V];
+        uint32_t sc[V], cc[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const unsigned d = my_begin - unsigned(base + 32 * v);
+          const unsigned heads = __reduce_or_sync(kFullMask, d < 32u ? (1u << d) : 0u);
+          si[v] = begun + __popc(heads & upto) - 1;
+          begun += __popc(heads);
+          const int f = base + 32 * v + lane;
+          const uint4 r = *reinterpret_cast<const uint4 *>(&rec[si[v]].code);
+          const int jj = int(r.y) + f;
+          sc[v] = r.x;
+          rel[v] = f < total ? jj - int(r.z) : -1;
+          cc[v] = f < total ? p.scode[jj] : 0u;
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const bool pass = rel[v] >= 0 && code_pass(sc[v], cc[v]);
+          const unsigned pm = __ballot_sync(kFullMask, pass);
+          if (pass) qu[queued + __popc(pm & below)] = unsigned(si[v]) | unsigned(rel[v]) << 5;
+          queued += __popc(pm);
+        }
+        __syncwarp();
+        while (queued >= 32) {
+          check(32);
+          __syncwarp();
+        }
       }
     }
     if (queued) check(queued);
     __syncwarp();  // the records are rewritten by the next 32 starts
+    if (COUNT) {
+      if (len > 0) p.box_counts[k - p.begin] = sw.hits[slot];
+      __syncwarp();
+    }
   }
+  if (COUNT) return;
   __syncwarp();
   if (staged) flush_staged(st, staged, lane, p);
   if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
@@ -630,7 +700,7 @@ stq_long_run_kernel(const SweepParams p) {
     const float kmax = p.xmax[k];
     const float4 kb = p.syz[k];
     const int4 kv = p.sv[k];
-    const float2 kfl = p.sfloor[k];
+    const uint32_t knf = p.scode[k] & kCodeNotFirst;
     const int kf = p.sflag[k];
     unsigned run_hits = 0;  // warp-uniform (emit) or this lane's (count mode)
     while (true) {
@@ -651,7 +721,7 @@ stq_long_run_kernel(const SweepParams p) {
         if (off < first) {
           ++tested;
           const float4 b = p.syz[j + off];
-          if (overlap_bc(kb, b) && b.x >= kfl.x && b.y >= kfl.y) {  // and the first-cell rule
+          if (overlap_bc(kb, b) && (p.scode[j + off] & knf) == 0u) {  // and the first-cell rule
             const int4 bv = p.sv[j + off];
             hit = (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
             pr = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
@@ -693,7 +763,7 @@ stq_long_run_kernel(const SweepParams p) {
 // device: the query costs host time on every launch otherwise, and the host
 // calls launch one sweep per window back to back.
 template <typename Kern>
-cudaError_t resident_blocks(Kern kern, int block, int *per_sm) {
+cudaError_t resident_blocks(Kern kern, int block, size_t smem, int *per_sm) {
   static std::mutex mu;
   static std::map<std::pair<const void *, int>, int> known;
   int dev = 0;
@@ -704,7 +774,7 @@ cudaError_t resident_blocks(Kern kern, int block, int *per_sm) {
   auto it = known.find(key);
   if (it == known.end()) {
     int v = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, block, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, block, smem);
     if (e != cudaSuccess) return e;
     it = known.emplace(key, v).first;
   }
@@ -713,9 +783,10 @@ cudaError_t resident_blocks(Kern kern, int block, int *per_sm) {
 }
 
 template <typename Kern>
-cudaError_t launch_persistent(Kern kern, int block, cudaStream_t s, const SweepParams &p, int num_sms) {
+cudaError_t launch_persistent(Kern kern, int block, cudaStream_t s, const SweepParams &p, int num_sms,
+                              size_t smem = 0) {
   int per_sm = 0;
-  cudaError_t e = resident_blocks(kern, block, &per_sm);
+  cudaError_t e = resident_blocks(kern, block, smem, &per_sm);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   // persistent grid: all resident blocks, capped by the available work
@@ -724,21 +795,21 @@ cudaError_t launch_persistent(Kern kern, int block, cudaStream_t s, const SweepP
   const int64_t max_useful = (warps_needed + block / 32 - 1) / (block / 32);
   if (blocks > max_useful) blocks = max_useful;
   if (blocks < 1) blocks = 1;
-  kern<<<unsigned(blocks), block, 0, s>>>(p);
+  kern<<<unsigned(blocks), block, smem, s>>>(p);
   return cudaGetLastError();
 }
 
-template <int G, int Q, int BLOCK, bool COUNT>
+template <int G, int Q, int BLOCK>
 cudaError_t launch_variant(cudaStream_t s, const SweepParams &p, int num_sms) {
-  return launch_persistent(stq_sweep_kernel<G, Q, BLOCK, COUNT>, BLOCK, s, p, num_sms);
+  return launch_persistent(stq_sweep_kernel<G, Q, BLOCK>, BLOCK, s, p, num_sms);
 }
 
 template <int G, int Q>
 cudaError_t launch_gq(cudaStream_t s, const SweepParams &p, int block, int sms) {
   switch (block) {
-    case 128: return launch_variant<G, Q, 128, false>(s, p, sms);
-    case 512: return launch_variant<G, Q, 512, false>(s, p, sms);
-    default: return launch_variant<G, Q, 256, false>(s, p, sms);
+    case 128: return launch_variant<G, Q, 128>(s, p, sms);
+    case 512: return launch_variant<G, Q, 512>(s, p, sms);
+    default: return launch_variant<G, Q, 256>(s, p, sms);
   }
 }
 
@@ -757,9 +828,9 @@ cudaError_t launch_g(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
 template <int U, int Q>
 cudaError_t launch_uq(cudaStream_t s, const SweepParams &p, int block, int sms) {
   switch (block) {
-    case 128: return launch_persistent(stq_sweep_lane_kernel<U, Q, 128, false>, 128, s, p, sms);
-    case 512: return launch_persistent(stq_sweep_lane_kernel<U, Q, 512, false>, 512, s, p, sms);
-    default: return launch_persistent(stq_sweep_lane_kernel<U, Q, 256, false>, 256, s, p, sms);
+    case 128: return launch_persistent(stq_sweep_lane_kernel<U, Q, 128>, 128, s, p, sms);
+    case 512: return launch_persistent(stq_sweep_lane_kernel<U, Q, 512>, 512, s, p, sms);
+    default: return launch_persistent(stq_sweep_lane_kernel<U, Q, 256>, 256, s, p, sms);
   }
 }
 
@@ -773,12 +844,20 @@ cudaError_t launch_u(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
   }
 }
 
-// The flat shape's blocks are 128 or 256 threads (512 would pass the 48 KB of
-// static shared memory a block may hold).
+// The flat shape's blocks are 128 or 256 threads.
+template <int BLOCK, int V, bool COUNT>
+cudaError_t launch_flat_block(cudaStream_t s, const SweepParams &p, int sms) {
+  constexpr auto kern = stq_sweep_flat_kernel<BLOCK, V, COUNT>;
+  constexpr size_t smem = sizeof(FlatWarp) * (BLOCK / 32);
+  cudaError_t e = allow_smem<kern>(smem);
+  if (e != cudaSuccess) return e;
+  return launch_persistent(kern, BLOCK, s, p, sms, smem);
+}
+
 template <int V>
 cudaError_t launch_flat(cudaStream_t s, const SweepParams &p, int block, int sms) {
-  if (block == 128) return launch_persistent(stq_sweep_flat_kernel<128, V>, 128, s, p, sms);
-  return launch_persistent(stq_sweep_flat_kernel<256, V>, 256, s, p, sms);
+  if (block == 128) return launch_flat_block<128, V, false>(s, p, sms);
+  return launch_flat_block<256, V, false>(s, p, sms);
 }
 
 // ---- overflow: longest prefix of start boxes whose pairs fit ------------------
@@ -896,7 +975,7 @@ cudaError_t launch_sweep(cudaStream_t s, const SweepParams &p, const SweepTuning
 static cudaError_t launch_sweep_lanes(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
                                       bool count_mode, int num_sms) {
   if (count_mode)  // per-start-box counts do not depend on the tuning
-    return launch_variant<8, 64, 256, true>(s, p, num_sms);
+    return launch_flat_block<256, 4, true>(s, p, num_sms);
   if (t.shape == kShapeFlat && p.run_end) {
     switch (t.per_lane) {  // filter steps per round
       case 2: return launch_flat<2>(s, p, t.block, num_sms);

@@ -113,9 +113,9 @@ typedef enum stq_option {
   STQ_OPT_HOST_WINDOWS = 12,   /* stq_sweep_host / stq_broadphase_host: windows a
                                   sweep is cut into (2..32, default 16; fewer when
                                   the scene has under 2^19 positions per window) */
-  STQ_OPT_SWEEP_SHAPE = 13     /* 2 (default): flat, each warp lays the runs of 32
-                                  start boxes end to end and tests one candidate
-                                  per lane and step (block size 128 or 256; 512
+  STQ_OPT_SWEEP_SHAPE = 13     /* 2 (default): flat, each warp takes the runs of 32
+                                  start boxes together, as one window of positions
+                                  or laid end to end (block size 128 or 256; 512
                                   acts as 256); 1: a per-warp queue of pending
                                   start boxes taken by lanes or lane groups
                                   (STQ_OPT_LANES_PER_ENTRY, STQ_OPT_QUEUE_DEPTH)  */

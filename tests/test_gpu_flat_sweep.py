@@ -1,0 +1,48 @@
+"""The flat sweep's forms: windows where every code passes (32 x 32 candidates per
+step, more than a queue round), runs cut by the cap, a mix of dense and sparse
+starts, and overflow counts from the same kernel; all against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def dense_boxes(stq, n, seed, spread):
+    """n boxes of which most overlap: side 1, centres within `spread`."""
+    b = stq.random_boxes(n, sliver_frac=0.0, seed=seed)
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(0, spread, (n, 3)).astype(np.float32)
+    b["min"], b["max"] = c - np.float32(0.5), c + np.float32(0.5)
+    # unrelated ids, so that few pairs share a vertex
+    b["vertex_ids"][:, 0] = np.arange(n)
+    b["vertex_ids"][:, 1] = np.where(b["vertex_ids"][:, 1] >= 0, n + np.arange(n), -np.arange(n) - 1)
+    b["vertex_ids"][:, 2] = np.where(b["vertex_ids"][:, 2] >= 0, 2 * n + np.arange(n), -np.arange(n) - 1)
+    return b
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 64, 65, 300, 1100, 2500])
+@pytest.mark.parametrize("spread", [0.0, 1.0, 40.0])
+@pytest.mark.parametrize("run_cap", [0, 40])
+def test_dense_windows_vs_oracle(ctx, stq, oracle, cuda, n, spread, run_cap):
+    import torch
+
+    b = dense_boxes(stq, n, 5 + n, spread)
+    want = oracle.broadphase(b)
+    d = torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+    ctx.set_option(stq.OPT_RUN_CAP, run_cap)
+    cap = len(want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    for axis in (0, -1):
+        r = ctx.sweep(d, n, pairs, cap, axis=axis)
+        assert r.status == stq.STQ_OK and r.count == len(want)
+        assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+    if len(want) < 64:
+        return
+    most = 1 + max(len(want) // 5, 4 * n)  # one start box has at most n pairs
+    start, parts = 0, []
+    while start < ctx.prepared_length:
+        r = ctx.sweep_prepared(pairs, min(most, cap), start=start)
+        parts.append(pairs[: r.count].cpu().numpy().copy())
+        start = r.next_start
+    got = np.concatenate(parts)
+    assert len(got) == len(want) and np.array_equal(oracle.canonical(got), want)
