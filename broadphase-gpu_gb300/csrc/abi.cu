@@ -106,7 +106,8 @@ int read_header(stq_context *ctx, const BatchHeader *src) {
 
 int64_t tiles_for(const int64_t *box_off, int S) {
   int64_t t = 0;
-  for (int s = 0; s < S; ++s) t += (box_off[s + 1] - box_off[s] + kTileBoxes - 1) / kTileBoxes;
+  const int size = tile_boxes(box_off[S]);
+  for (int s = 0; s < S; ++s) t += (box_off[s + 1] - box_off[s] + size - 1) / size;
   return t;
 }
 
@@ -129,6 +130,7 @@ int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap) {
   STQ_CUDA(ctx, ctx->cell_base.ensure(sizeof(unsigned) * size_t(scene_cap + 1)), "allocate cell bases");
   STQ_CUDA(ctx, ctx->scene_pairs.ensure(sizeof(unsigned long long) * size_t(scene_cap)),
            "allocate scene pair counters");
+  STQ_CUDA(ctx, ctx->emit_status.ensure(sizeof(unsigned long long) * size_t(tile_cap)), "allocate emit status");
   if (scene_cap > ctx->h_scene_pairs_cap) {
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     ctx->h_scene_pairs = nullptr;
@@ -149,7 +151,6 @@ void fill_staging(stq_context *ctx, const int64_t *box_off, int S, const int *ax
   BatchHeader *h = host_at<BatchHeader>(ctx, L.hdr);
   std::memset(h, 0, sizeof(BatchHeader));
   h->n_boxes = box_off[S];
-  h->box_count = uint32_t(box_off[S]);
   h->n_scenes = S;
   h->budget = ctx->budget;
   long long *bo = host_at<long long>(ctx, L.box_off);
@@ -168,10 +169,11 @@ void fill_staging(stq_context *ctx, const int64_t *box_off, int S, const int *ax
   }
   TileRec *tr = host_at<TileRec>(ctx, L.tiles);
   int t = 0;
+  const int size = tile_boxes(box_off[S]);
   for (int s = 0; s < S; ++s)
-    for (int64_t b = box_off[s]; b < box_off[s + 1]; b += kTileBoxes) {
+    for (int64_t b = box_off[s]; b < box_off[s + 1]; b += size) {
       tr[t].begin = b;
-      tr[t].count = int(std::min<int64_t>(kTileBoxes, box_off[s + 1] - b));
+      tr[t].count = int(std::min<int64_t>(size, box_off[s + 1] - b));
       tr[t].scene = s;
       ++t;
     }
@@ -196,17 +198,13 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
   b.scenes = ctx->scenes.as<SceneRecord>();
   b.cell_base = ctx->cell_base.as<unsigned>();
   b.hdr = dev_hdr(ctx);
-  b.counts = ctx->counts.as<uint32_t>();
-  b.offsets = ctx->offsets.as<uint32_t>();
   b.box_cells = ctx->box_cells.as<uint2>();
-  b.keys = ctx->keys64[0].as<unsigned long long>();
-  b.vals = ctx->vals[0].as<uint32_t>();
-  b.box_keys = ctx->bkeys[0].as<uint32_t>();
-  b.box_vals = ctx->bvals[0].as<uint32_t>();
-  b.box_keys2 = ctx->bkeys[1].as<uint32_t>();
-  b.box_vals2 = ctx->bvals[1].as<uint32_t>();
-  b.order = ctx->bvals[0].as<uint32_t>();
-  b.sorted_keys = ctx->bkeys[0].as<uint32_t>();
+  b.box_q = ctx->box_q.as<uint32_t>();
+  b.emit_status = ctx->emit_status.as<unsigned long long>();
+  for (int k = 0; k < 2; ++k) {
+    b.keys[k] = ctx->keys[k].as<uint32_t>();
+    b.vals[k] = ctx->vals[k].as<uint32_t>();
+  }
   b.seg_scan = ctx->seg_scan.as<uint32_t>();
   b.seg_cap = ctx->seg_cap;
   b.box_cap = ctx->box_cap;
@@ -217,15 +215,8 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
 
 int ensure_box_buffers(stq_context *ctx, int64_t box_cap) {
   const size_t n = size_t(std::max<int64_t>(box_cap, 1));
-  STQ_CUDA(ctx, ctx->counts.ensure(sizeof(uint32_t) * n), "allocate replica counts");
-  STQ_CUDA(ctx, ctx->offsets.ensure(sizeof(uint32_t) * n), "allocate replica offsets");
   STQ_CUDA(ctx, ctx->box_cells.ensure(sizeof(uint2) * n), "allocate box cell ranges");
-  STQ_CUDA(ctx, ctx->scan_ws.ensure(scan_workspace_bytes(int64_t(n))), "allocate scan workspace");
-  for (int b = 0; b < 2; ++b) {
-    STQ_CUDA(ctx, ctx->bkeys[b].ensure(sizeof(uint32_t) * n), "allocate box keys");
-    STQ_CUDA(ctx, ctx->bvals[b].ensure(sizeof(uint32_t) * n), "allocate box order");
-  }
-  STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(int64_t(n))), "allocate sort workspace");
+  STQ_CUDA(ctx, ctx->box_q.ensure(sizeof(uint32_t) * n), "allocate box codes");
   ctx->box_cap = int64_t(n);
   return STQ_OK;
 }
@@ -233,7 +224,7 @@ int ensure_box_buffers(stq_context *ctx, int64_t box_cap) {
 int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap) {
   const size_t r = size_t(std::max<int64_t>(rep_cap, 1));
   for (int b = 0; b < 2; ++b) {
-    STQ_CUDA(ctx, ctx->keys64[b].ensure(sizeof(unsigned long long) * r), "allocate keys");
+    STQ_CUDA(ctx, ctx->keys[b].ensure(sizeof(uint32_t) * r), "allocate keys");
     STQ_CUDA(ctx, ctx->vals[b].ensure(sizeof(uint32_t) * r), "allocate values");
   }
   STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(int64_t(r))), "allocate sort workspace");
@@ -242,11 +233,10 @@ int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap)
   STQ_CUDA(ctx, ctx->seg_scan.ensure(sizeof(uint32_t) * size_t(segs + 1)), "allocate segment offsets");
   ctx->seg_cap = segs;
   const size_t slots = r + size_t(segs) + 1 + kSortedPad;
-  STQ_CUDA(ctx, ctx->xmin.ensure(sizeof(float) * slots), "allocate sorted scene");
-  STQ_CUDA(ctx, ctx->xmax.ensure(sizeof(float) * slots), "allocate sorted scene");
-  STQ_CUDA(ctx, ctx->syz.ensure(sizeof(float4) * slots), "allocate sorted scene");
-  STQ_CUDA(ctx, ctx->sv.ensure(sizeof(int4) * slots), "allocate sorted scene");
-  STQ_CUDA(ctx, ctx->sflag.ensure(sizeof(int) * slots), "allocate sorted scene");
+  STQ_CUDA(ctx, ctx->yz.ensure(sizeof(float4) * slots), "allocate sorted scene");
+  STQ_CUDA(ctx, ctx->xx.ensure(sizeof(float2) * slots), "allocate sorted scene");
+  STQ_CUDA(ctx, ctx->vv.ensure(sizeof(int4) * slots), "allocate sorted scene");
+  STQ_CUDA(ctx, ctx->flag.ensure(sizeof(int) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->scode.ensure(sizeof(uint32_t) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->partner.ensure(sizeof(int) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->run_end.ensure(sizeof(int) * slots), "allocate sorted scene");
@@ -262,64 +252,39 @@ int bits_for(int64_t v) {
   return b;
 }
 
-int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t n_boxes) {
+int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap) {
   stage_begin(ctx, kAxis);
   STQ_CUDA(ctx, launch_batch_stats(ctx->stream, b), "launch batch statistics");
   STQ_CUDA(ctx, launch_batch_policy(ctx->stream, b), "launch batch policy");
   stage_end(ctx, kAxis);
-  // boxes in sweep-axis order: the emit then writes every list in key order
-  stage_begin(ctx, kSort);
-  STQ_CUDA(ctx, launch_batch_box_keys(ctx->stream, b), "launch box keys");
-  uint32_t *kb[2] = {ctx->bkeys[0].as<uint32_t>(), ctx->bkeys[1].as<uint32_t>()};
-  uint32_t *vb[2] = {ctx->bvals[0].as<uint32_t>(), ctx->bvals[1].as<uint32_t>()};
-  const int64_t n = n_boxes >= 0 ? n_boxes : ctx->box_cap;
-  STQ_CUDA(ctx, radix_sort_u32(ctx->stream, kb, vb, n, ctx->sort_ws.ptr, &b.hdr->fault, &ctx->launches,
-                               n_boxes >= 0 ? nullptr : &b.hdr->box_count),
-           "launch box sort");
-  stage_end(ctx, kSort);
   stage_begin(ctx, kKeys);
-  STQ_CUDA(ctx, launch_batch_counts(ctx->stream, b, n), "launch replica counts");
-  STQ_CUDA(ctx, exclusive_scan_u32(ctx->stream, b.counts, b.offsets, ctx->box_cap, ctx->scan_ws.ptr,
-                                   &b.hdr->replicas, &ctx->launches),
-           "launch replica scan");
-  ctx->launches += 6;  // reset, statistics, policy, box keys, choose, counts
+  STQ_CUDA(ctx, launch_batch_box_keys(ctx->stream, b, rep_cap, seg_cap), "launch box keys");
+  ctx->launches += 5;  // reset, statistics, policy, box keys, choose
   return STQ_OK;
 }
 
-int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int seg_bits, int64_t n_boxes,
-                         int64_t replicas) {
-  STQ_CUDA(ctx, launch_batch_emit(ctx->stream, b, n_boxes >= 0 ? n_boxes : ctx->box_cap, ctx->num_sms),
-           "launch replica emit");
+int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes) {
+  STQ_CUDA(ctx, launch_batch_emit(ctx->stream, b), "launch replica emit");
   stage_end(ctx, kKeys);
-  // the replicas arrive in sweep-axis order: a stable sort by list id alone
-  // (the key's high half) leaves every list sorted by its minima
-  unsigned long long *kb[2] = {ctx->keys64[0].as<unsigned long long>(),
-                               ctx->keys64[1].as<unsigned long long>()};
-  uint32_t *vb[2] = {ctx->vals[0].as<uint32_t>(), ctx->vals[1].as<uint32_t>()};
-  int which = 0;
   stage_begin(ctx, kSort);
   const int64_t r = replicas >= 0 ? replicas : ctx->rep_cap;
-  // seg_bits covers the capacity; the digits that no list id uses are skipped
-  STQ_CUDA(ctx, radix_sort_u64_vals(ctx->stream, kb, vb, r, 32, 32 + std::max(seg_bits, 1), ctx->sort_ws.ptr,
-                                    &which, &b.hdr->fault, &ctx->launches, replicas >= 0 ? nullptr : &b.hdr->replicas),
-           "launch list sort");
+  STQ_CUDA(ctx, radix_sort_u32(ctx->stream, b.keys, b.vals, r, ctx->sort_ws.ptr, &b.hdr->fault, &ctx->launches,
+                               replicas >= 0 ? nullptr : &b.hdr->replicas, &b.hdr->passes, passes >= 0 ? passes : 4),
+           "launch replica sort");
   stage_end(ctx, kSort);
-  ctx->scene.xmin = ctx->xmin.as<float>();
-  ctx->scene.xmax = ctx->xmax.as<float>();
-  ctx->scene.syz = ctx->syz.as<float4>();
-  ctx->scene.sv = ctx->sv.as<int4>();
-  ctx->scene.sflag = ctx->sflag.as<int>();
+  ctx->scene.yz = ctx->yz.as<float4>();
+  ctx->scene.x = ctx->xx.as<float2>();
+  ctx->scene.v = ctx->vv.as<int4>();
+  ctx->scene.flag = ctx->flag.as<int>();
   ctx->scene.scode = ctx->scode.as<uint32_t>();
   ctx->scene.partner = ctx->partner.as<int>();
   ctx->scene.run_end = ctx->run_end.as<int>();
   stage_begin(ctx, kGather);
-  STQ_CUDA(ctx, launch_list_offsets(ctx->stream, kb[which], b.hdr, b.seg_scan, b.seg_cap, ctx->scene, ctx->slot_cap),
+  STQ_CUDA(ctx, launch_list_offsets(ctx->stream, b.keys[0], b.hdr, b.seg_scan, b.seg_cap, ctx->scene, ctx->slot_cap),
            "launch list offsets");
-  STQ_CUDA(ctx, launch_gather_cells(ctx->stream, b.boxes, kb[which], vb[which], b.hdr, r, b.cell_base, b.scenes,
-                                    b.seg_scan, ctx->scene),
-           "launch gather");
+  STQ_CUDA(ctx, launch_gather_cells(ctx->stream, b, r, ctx->scene), "launch gather");
   stage_end(ctx, kGather);
-  ctx->launches += 3;
+  ctx->launches += 3;  // emit, list offsets, gather
   return STQ_OK;
 }
 
@@ -335,14 +300,14 @@ int prepare_exact(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_
   fill_staging(ctx, box_off, S, axes, axis, nullptr, nullptr, nullptr);
   STQ_TRY(upload_staging(ctx));
   BatchBuffers b = batch_buffers(ctx, d_boxes);
-  STQ_TRY(enqueue_prepare_front(ctx, b, N));
+  STQ_TRY(enqueue_prepare_front(ctx, b, -1, -1));
   STQ_TRY(read_header(ctx));
   const int64_t R = ctx->h_hdr->replicas, cells = ctx->h_hdr->cells;
   if (R + 3 * cells + 1 + kSortedPad > int64_t(INT32_MAX))
     return fail(ctx, STQ_ERR_NO_MEMORY, "too many cell replicas for 32-bit positions");
   STQ_TRY(ensure_replica_buffers(ctx, std::max(R, ctx->rep_cap), cells));
   b = batch_buffers(ctx, d_boxes);
-  STQ_TRY(enqueue_prepare_back(ctx, b, bits_for(3 * cells), N, R));
+  STQ_TRY(enqueue_prepare_back(ctx, b, R, int(ctx->h_hdr->passes)));
   ctx->n_scenes = S;
   ctx->n_boxes = N;
   ctx->length = R > 0 ? R + 3 * cells - 1 : 0;
@@ -357,10 +322,13 @@ int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
   BatchHeader *hdr = dev_hdr(ctx);
   cudaStream_t s = cursors && stream ? stream : ctx->stream;
   SweepParams p;
-  p.xmin = ctx->scene.xmin;
-  p.xmax = ctx->scene.xmax;
-  p.syz = ctx->scene.syz;
-  p.sv = ctx->scene.sv;
+  p.yz = ctx->scene.yz;
+  p.x = ctx->scene.x;
+  p.v = ctx->scene.v;
+  p.flag = ctx->scene.flag;
+  p.scode = ctx->scene.scode;
+  p.partner = ctx->scene.partner;
+  p.run_end = ctx->scene.run_end;
   p.begin = int32_t(begin);
   p.end = int32_t(std::min<int64_t>(end, INT32_MAX));
   // start positions per work grab: at least ~4 grabs per resident warp
@@ -373,10 +341,6 @@ int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
   p.count = &hdr->pairs;
   p.work = &hdr->work;
   p.box_counts = ctx->box_counts.as<int32_t>();
-  p.sflag = ctx->scene.sflag;
-  p.scode = ctx->scene.scode;
-  p.partner = ctx->scene.partner;
-  p.run_end = ctx->scene.run_end;
   p.scene_pairs = ctx->scene_pairs.as<unsigned long long>();
   p.hdr = hdr;
   p.stats = &hdr->candidates;
@@ -804,7 +768,6 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
   const int64_t vert_cap = int64_t(ctx->points.bytes / (2 * sizeof(float4)));
   fill_staging(ctx, box_off.data(), n_scenes, nullptr, axis, h_vert_off, h_edge_off, h_face_off);
   const stq_aabb *boxes = ctx->batch_boxes.as<stq_aabb>();
-  const int cell_bits = bits_for(3 * cells_cap);
   auto enqueue_all = [&]() -> int {
     STQ_TRY(upload_staging(ctx));
     stage_begin(ctx, kBuild);
@@ -818,8 +781,8 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     ctx->launches += 1;  // the rounding of the positions
     stage_end(ctx, kBuild);
     const BatchBuffers b = batch_buffers(ctx, boxes);
-    STQ_TRY(enqueue_prepare_front(ctx, b, -1));
-    STQ_TRY(enqueue_prepare_back(ctx, b, cell_bits, -1, -1));
+    STQ_TRY(enqueue_prepare_front(ctx, b, ctx->rep_cap, ctx->seg_cap));
+    STQ_TRY(enqueue_prepare_back(ctx, b, -1, -1));
     STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, d_pairs, capacity, false));
     STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_hdr, dev_hdr(ctx), sizeof(BatchHeader),
                                   cudaMemcpyDeviceToHost, ctx->stream),
@@ -848,7 +811,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     const void *ptrs[7] = {d_V0, d_V1, d_E, d_F, d_pairs, boxes, ctx->points.ptr};
     std::memcpy(key.ptr, ptrs, sizeof ptrs);
     const int64_t sizes[9] = {ctx->box_cap, ctx->rep_cap, ctx->slot_cap, ctx->scene_cap,
-                              ctx->tile_cap, capacity, n_scenes, cell_bits, vert_cap};
+                              ctx->tile_cap, capacity, n_scenes, ctx->seg_cap, vert_cap};
     std::memcpy(key.sizes, sizes, sizeof sizes);
     static_assert(sizeof(ctx->options) / sizeof(ctx->options[0]) == 16, "options in the graph key");
     for (int o = 0; o < 16; ++o) key.opts[o] = ctx->options[o];

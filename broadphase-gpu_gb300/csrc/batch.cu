@@ -1,12 +1,16 @@
 // batch.cu - prepare kernels of the scene table: per-scene statistics, sweep
 // axis and cell grid, cell replicas with their sort keys, and the sorted-scene
-// gather with one NaN sentinel after every cell.
+// gather with one empty position after every list.
 //
 // Reference: create_ds (src/sweep.cu:125-161) and the axis choice of
 // calc_mean / calc_variance (src/sweep.cu:93-123); the reference sorts one
 // scene along x. Here every scene of a batch gets its own sweep axis and
 // y/z cell grid, all scenes' cells get global ids, and one sort orders every
-// replica by (cell, min on the sweep axis).
+// replica by (cell, box type, sweep-axis code). The code is a monotone 16-bit
+// image of the minimum: a list is sorted up to boxes of one code, its runs hold
+// every candidate of a code that can overlap, and the sweep tests the sweep axis
+// exactly for the pairs that pass its filter. So the whole key fits 24 or 32
+// bits, and the boxes need no sort of their own.
 //
 // All sizes are read from the BatchHeader on the device, so one captured
 // graph serves any batch within the buffer capacities.
@@ -24,6 +28,7 @@ namespace {
 constexpr int kBlock = 256;
 constexpr int kHistBias = 40;  // extent bucket = binary exponent + 40
 constexpr int kSampleBoxes = 1024;
+constexpr int kSampleMins = 512;  // of these, for the sweep-axis code segments
 
 __device__ __forceinline__ void axes_bc(int a, int &b, int &c) {
   b = a == 0 ? 1 : 0;
@@ -55,8 +60,9 @@ __device__ void block_sums(const T (&v)[K], T (&out)[K], T (*red)[K]) {
 // ---- 0. reset the per-scene accumulators ------------------------------------------
 __global__ void __launch_bounds__(kBlock)
 batch_reset_kernel(SceneRecord *scenes, const SceneInput *__restrict__ inputs,
-                   unsigned long long *scene_pairs, BatchHeader *hdr) {
+                   unsigned long long *scene_pairs, BatchHeader *hdr, unsigned long long *emit_status) {
   const int S = hdr->n_scenes;
+  for (int t = blockIdx.x * kBlock + threadIdx.x; t < hdr->n_tiles; t += gridDim.x * kBlock) emit_status[t] = 0ull;
   for (int s = blockIdx.x * kBlock + threadIdx.x; s < S; s += gridDim.x * kBlock) {
     SceneRecord &r = scenes[s];
     r.axis_mode = inputs[s].axis_mode;
@@ -75,6 +81,7 @@ batch_reset_kernel(SceneRecord *scenes, const SceneInput *__restrict__ inputs,
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     hdr->flags = 0;
     hdr->fault = 0;
+    hdr->emit_ticket = 0;
     hdr->replicas = 0;
     hdr->cells = 0;
     hdr->lists = 0;
@@ -211,13 +218,21 @@ batch_policy_kernel(const stq_aabb *__restrict__ boxes, const long long *__restr
   int b, c;
   axes_bc(axis, b, c);
   __shared__ unsigned hist[2][64];
+  __shared__ float sample[kSampleMins];
+  __shared__ float median[2];
   for (int i = threadIdx.x; i < 128; i += kBlock) (&hist[0][0])[i] = 0u;
+  for (int i = threadIdx.x; i < kSampleMins; i += kBlock) sample[i] = INFINITY;
   __syncthreads();
   const bool automatic = r.cells_opt == 0 && !r.inverted && n > 1;
-  if (automatic) {
+  {
     const long long step = n > kSampleBoxes ? n / kSampleBoxes : 1;
+    // every second sample gives a minimum on the sweep axis (all of them in
+    // scenes of fewer boxes than minima wanted)
+    const int every = n > kSampleMins ? kSampleBoxes / kSampleMins : 1;
     for (long long i = threadIdx.x; i < kSampleBoxes && i * step < n; i += kBlock) {
       const stq_aabb &x = boxes[b0 + i * step];
+      if (i % every == 0 && i / every < kSampleMins) sample[i / every] = x.min[axis];
+      if (!automatic) continue;
       const int ax[2] = {b, c};
       for (int q = 0; q < 2; ++q) {
         const float ext = x.max[ax[q]] - x.min[ax[q]];
@@ -231,6 +246,51 @@ batch_policy_kernel(const stq_aabb *__restrict__ boxes, const long long *__restr
       }
     }
   }
+  // the sampled minima in order (bitonic; missing ones are +inf, at the end)
+  static_assert(kSampleMins == 2 * kBlock, "one comparison per thread and step");
+  for (int size = 2; size <= kSampleMins; size <<= 1)
+    for (int d = size >> 1; d > 0; d >>= 1) {
+      __syncthreads();
+      const int i = 2 * int(threadIdx.x) - (int(threadIdx.x) & (d - 1)), j = i + d;
+      const float x = sample[i], y = sample[j];
+      if ((x > y) == ((i & size) == 0)) {
+        sample[i] = y;
+        sample[j] = x;
+      }
+    }
+  __syncthreads();
+  // median extents: one warp per axis, two buckets per lane
+  if (threadIdx.x < 64) {
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned h0 = hist[q][2 * lane], h1 = hist[q][2 * lane + 1];
+    unsigned run = h0 + h1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(kFullMask, run, o);
+      if (lane >= o) run += y;
+    }
+    const unsigned total = __shfl_sync(kFullMask, run, 31);
+    // first bucket whose running count reaches half
+    const unsigned m = __ballot_sync(kFullMask, total > 0 && 2 * run >= total);
+    if (lane == 0) median[q] = 0.f;
+    __syncwarp();
+    if (m && lane == __ffs(m) - 1) {
+      const int k = 2 * (run - h1) >= total ? 2 * lane : 2 * lane + 1;
+      median[q] = k == 0 ? 0.f : 0.75f * exp2f(float(k - kHistBias));
+    }
+  }
+  // sweep-axis code segments: their ends are quantiles of the sample, the first
+  // and the last reach to the scene's bounds
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + kSplits) {
+    const int i = threadIdx.x - 64;
+    const int m = int(n < kSampleMins ? (n > 0 ? n : 1) : kSampleMins);
+    const float lo = key_float(r.lo_key[axis]), hi = key_float(r.hi_key[axis]);
+    const float s0 = i == 0 && isfinite(lo) ? lo : sample[i * m / kSplits];
+    const float s1 = i == kSplits - 1 ? (isfinite(hi) ? hi : sample[m - 1]) : sample[(i + 1) * m / kSplits];
+    const float w = s1 - s0;
+    r.split[i] = s0;
+    r.split_inv[i] = w > 0.f && isfinite(w) ? float(kSplitSteps) / w : 0.f;
+  }
   __syncthreads();
   if (threadIdx.x != 0) return;
   const float lob = key_float(r.lo_key[b]), hib = key_float(r.hi_key[b]);
@@ -240,19 +300,7 @@ batch_policy_kernel(const stq_aabb *__restrict__ boxes, const long long *__restr
   if (r.cells_opt > 1 && !r.inverted && n > 1) {
     nb = nc = r.cells_opt;
   } else if (automatic) {
-    float w[2];
-    for (int q = 0; q < 2; ++q) {
-      unsigned total = 0, run = 0;
-      for (int k = 0; k < 64; ++k) total += hist[q][k];
-      w[q] = 0.f;
-      for (int k = 0; k < 64; ++k) {
-        run += hist[q][k];
-        if (2 * run >= total && total > 0) {
-          w[q] = k == 0 ? 0.f : 0.75f * exp2f(float(k - kHistBias));
-          break;
-        }
-      }
-    }
+    float w[2] = {median[0], median[1]};
     if (!(w[0] > 0.f)) w[0] = Lb / 1024.f;
     if (!(w[1] > 0.f)) w[1] = Lc / 1024.f;
     nb = grid_side(Lb, r.cell_scale * w[0]);
@@ -298,24 +346,14 @@ __device__ __forceinline__ Range cell_range(const stq_aabb &x, int a, float ob, 
   return r;
 }
 
-// Scene of box bi: the last scene whose first box is <= bi.
-__device__ __forceinline__ int scene_of(const long long *__restrict__ box_off, int S, uint32_t bi) {
-  int lo = 0, hi = S - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (box_off[mid] <= (long long)bi) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
 // ---- 4. choose the finest level within the replica budget; cell bases ----------
 __global__ void __launch_bounds__(1024)
 batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
-                    unsigned int *cell_base, BatchHeader *hdr) {
+                    unsigned int *cell_base, BatchHeader *hdr, long long rep_cap, long long seg_cap) {
   __shared__ unsigned int warp_tot[32];
   __shared__ unsigned int carry;
-  if (threadIdx.x == 0) carry = 0;
+  __shared__ unsigned long long reps;
+  if (threadIdx.x == 0) carry = 0, reps = 0;
   __syncthreads();
   const int S = hdr->n_scenes;
   const long long budget = hdr->budget;
@@ -341,6 +379,7 @@ batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
       g.nb = ((g.nb0 - 1) >> level) + 1;
       g.nc = ((g.nc0 - 1) >> level) + 1;
       g.ncells = g.nb * g.nc;
+      atomicAdd(&reps, level < kGridLevels ? r.level_reps[level] : (unsigned long long)n);
       // 64 code steps per cell of the chosen level; a cell is 2^level level-0
       // cells, of which there are nb0 over Lb (one cell: the whole extent)
       const float steps = 64.f / float(1 << level);
@@ -373,107 +412,68 @@ batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
   }
   if (threadIdx.x == 0) {
     cell_base[S] = carry;
-    hdr->cells = carry;
-    hdr->lists = 3u * carry;
-  }
-}
-
-// ---- 5. per-box replica counts in sweep-axis order (zero past the last box, up
-// to the capacity), from the level-0 cell ranges by box index that the
-// box-key kernel wrote, at the scene's chosen level
-__device__ __forceinline__ uint32_t cells_count(uint2 r, int shift) {
-  return (((r.x >> 11 & 2047u) >> shift) - ((r.x & 2047u) >> shift) + 1u) *
-         (((r.y >> 11 & 2047u) >> shift) - ((r.y & 2047u) >> shift) + 1u);
-}
-
-__global__ void __launch_bounds__(kBlock)
-batch_count_kernel(const uint32_t *__restrict__ order, const uint2 *__restrict__ box_cells,
-                   const long long *__restrict__ box_off, const SceneRecord *__restrict__ scenes,
-                   const BatchHeader *hdr, uint32_t *__restrict__ counts, long long box_cap) {
-  const long long N = hdr->n_boxes;
-  const int S = hdr->n_scenes;
-  for (long long p = blockIdx.x * (long long)kBlock + threadIdx.x; p < N; p += (long long)gridDim.x * kBlock) {
-    const uint32_t bi = order[p];
-    counts[p] = cells_count(box_cells[bi], scenes[scene_of(box_off, S, bi)].grid.shift);
-  }
-  // positions past the batch contribute nothing to the scan
-  for (long long i = N + blockIdx.x * (long long)kBlock + threadIdx.x; i < box_cap;
-       i += (long long)gridDim.x * kBlock)
-    counts[i] = 0u;
-}
-
-// ---- 6. replica keys: (segment << 32) | order-preserving min, where the
-// segment is (global cell, box type): every cell holds a vertex, an edge and
-// a face list.
-__global__ void __launch_bounds__(kBlock)
-batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restrict__ sorted_keys,
-                  const uint32_t *__restrict__ order,
-                  const long long *__restrict__ box_off, const SceneRecord *__restrict__ scenes,
-                  const unsigned int *__restrict__ cell_base, BatchHeader *hdr,
-                  const uint32_t *__restrict__ offsets, unsigned long long *__restrict__ keys,
-                  uint32_t *__restrict__ vals, long long rep_cap, long long seg_cap) {
-  const bool fits = (long long)hdr->replicas <= rep_cap && 3ll * hdr->cells <= seg_cap;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    // each of the 3 lists of a cell is followed by its sentinel; the last
-    // sentinel is not a start position. On overflow nothing is emitted.
-    hdr->length = fits && hdr->cells > 0 && hdr->replicas > 0 ? hdr->replicas + 3 * hdr->cells - 1 : 0u;
+    const unsigned long long R = reps, lists = 3ull * carry;
+    // more than the buffers hold: the scenes are flagged and left empty (the
+    // caller without limits checks that positions fit 31 bits)
+    const bool fits = R < 0xffffffffull && (rep_cap < 0 || ((long long)R <= rep_cap && (long long)lists <= seg_cap));
+    if (!fits) atomicOr(&hdr->flags, kFlagReplicaOverflow);
+    hdr->replicas = fits ? unsigned(R) : 0u;
+    hdr->cells = fits ? carry : 0u;
+    hdr->lists = fits ? unsigned(lists) : 0u;
+    // each of the 3 lists of a cell is followed by its empty position; the last
+    // of these is not a start position
+    hdr->length = fits && carry > 0 && R > 0 ? unsigned(R + lists - 1) : 0u;
     hdr->max_list = 0u;
-    if (!fits) {
-      atomicOr(&hdr->flags, kFlagReplicaOverflow);
-      hdr->replicas = 0;
-    }
-  }
-  if (!fits) return;
-  const long long N = hdr->n_boxes;
-  const int S = hdr->n_scenes;
-  // positions in sweep-axis order: every list receives its replicas in key
-  // order, which the stable sort by list id keeps
-  for (long long p = blockIdx.x * (long long)kBlock + threadIdx.x; p < N; p += (long long)gridDim.x * kBlock) {
-    const uint32_t bi = order[p];
-    const int sc = scene_of(box_off, S, bi);
-    const int nc = scenes[sc].grid.nc, sh = scenes[sc].grid.shift;
-    const unsigned long long cb0 = cell_base[sc];
-    // the box's level-0 cell range and type (8 bytes, by box index) and its
-    // sort key, instead of the 44-byte box
-    const uint2 r = box_cells[bi];
-    const int b0 = int(r.x & 2047u) >> sh, b1 = int(r.x >> 11 & 2047u) >> sh;
-    const int c0 = int(r.y & 2047u) >> sh, c1 = int(r.y >> 11 & 2047u) >> sh;
-    const unsigned long long type = r.x >> 22;
-    const unsigned long long xk = sorted_keys[p];
-    uint32_t o = offsets[p];
-    for (int cb = b0; cb <= b1; ++cb)
-      for (int cc = c0; cc <= c1; ++cc) {
-        const unsigned long long seg = (cb0 + (unsigned long long)(cb * nc + cc)) * 3ull + type;
-        keys[o] = (seg << 32) | xk;
-        vals[o] = bi;
-        ++o;
-      }
+    // key: list id above the top bits of the sweep-axis code, 24 bits in all (three
+    // digits) where that leaves the code 10 bits or more, else 32. At 10 bits the
+    // 6 M-box scene (14 bits of lists) tests 9% more candidates and sorts a digit
+    // less: sort + sweep 0.22 + 1.26 ms against 0.29 + 1.19 with 32 bits.
+    int seg_bits = 0;
+    while (seg_bits < 32 && (1ull << seg_bits) < lists) ++seg_bits;
+    const int key_bits = seg_bits <= 14 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
+    hdr->key_bits = key_bits;
+    hdr->passes = unsigned(max(seg_bits + key_bits + 7, 8)) / 8u;
   }
 }
 
-// ---- 3. sort keys of the boxes (the order-preserving image of the minimum on
-// the scene's sweep axis, with the box index as value), each box's level-0
-// cell range and type, and the replicas of every grid level, per scene
+// ---- 3. per box: the level-0 cell range and type, the sweep-axis codes of its
+// minimum and maximum, and the replicas of every grid level, per scene
+__device__ __forceinline__ uint32_t axis_code(float v, const float *split, const float *inv) {
+  int i = 0;
+#pragma unroll
+  for (int step = kSplits / 2; step > 0; step >>= 1)
+    if (v >= split[i + step]) i += step;
+  // monotone: the segment is, and so is the step inside it (round-to-nearest
+  // operations, clamped; NaN, which only infinite ends give, counts as 0)
+  const float t = __fmul_rn(__fsub_rn(v, split[i]), inv[i]);
+  return uint32_t(i * kSplitSteps) + uint32_t(fminf(fmaxf(t, 0.f), float(kSplitSteps - 1)));
+}
+
 __global__ void __launch_bounds__(kBlock)
 batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
                       SceneRecord *scenes, const BatchHeader *hdr,
-                      uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, uint2 *__restrict__ box_cells) {
+                      uint2 *__restrict__ box_cells, uint32_t *__restrict__ box_q) {
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
   SceneRecord &r = scenes[t.scene];
   const GridParams g = r.grid;
+  __shared__ float split[kSplits], inv[kSplits];
+  if (threadIdx.x < kSplits) {
+    split[threadIdx.x] = r.split[threadIdx.x];
+    inv[threadIdx.x] = r.split_inv[threadIdx.x];
+  }
+  __syncthreads();
   // a thread sees at most kTileBoxes / kBlock = 16 boxes of at most 2048^2
   // cells each: 32-bit sums per thread, 64-bit per block
   static_assert(uint64_t(kTileBoxes / kBlock) * kMaxGridSide * kMaxGridSide < (uint64_t(1) << 32),
                 "per-thread level sums");
   unsigned reps[kGridLevels] = {};
+#pragma unroll 2
   for (int i = threadIdx.x; i < t.count; i += kBlock) {
     const long long bi = t.begin + i;
     const stq_aabb &x = boxes[bi];
-    keys[bi] = float_key(x.min[g.axis]);
-    vals[bi] = uint32_t(bi);
-    // the box's cell range and type, by box index, while the box is read in
-    // order (level-0 coordinates fit kCoordBits = 11 bits)
+    box_q[bi] = axis_code(x.min[g.axis], split, inv) | axis_code(x.max[g.axis], split, inv) << 16;
+    // level-0 coordinates fit kCoordBits = 11 bits
     const Range q = cell_range(x, g.axis, g.ob, g.ib, g.nb0, g.oc, g.ic, g.nc0);
     const unsigned type = unsigned(type_of(x.vertex_ids[1], x.vertex_ids[2]));
     box_cells[bi] = make_uint2(unsigned(q.b0) | unsigned(q.b1) << 11 | type << 22,
@@ -492,26 +492,145 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
     for (int l = 0; l < kGridLevels; ++l) atomicAdd(&r.level_reps[l], tot[l]);
 }
 
+// ---- 5. replica keys in box order: (list id << key_bits) | sweep-axis code, where
+// the list is (global cell, box type). A block takes a tile (one scene), counts
+// its replicas at the chosen level, publishes the count, and finds its first
+// output position by looking back over the tiles before it (which hold their
+// tickets, so they are running; the wait is bounded all the same). Status word:
+// 1 << 62 | count, or 2 << 62 | sum up to and with the tile.
+constexpr int kEmitSpins = 1 << 20;
+
+__device__ __forceinline__ uint32_t cells_count(uint2 r, int shift) {
+  return (((r.x >> 11 & 2047u) >> shift) - ((r.x & 2047u) >> shift) + 1u) *
+         (((r.y >> 11 & 2047u) >> shift) - ((r.y & 2047u) >> shift) + 1u);
+}
+
+__global__ void __launch_bounds__(kBlock)
+batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restrict__ box_q,
+                  const TileRec *__restrict__ tiles, const SceneRecord *__restrict__ scenes,
+                  const unsigned int *__restrict__ cell_base, BatchHeader *hdr, unsigned long long *status,
+                  uint32_t *k0, uint32_t *k1, uint32_t *v0, uint32_t *v1) {
+  if (hdr->replicas == 0u) return;
+  const int n_tiles = hdr->n_tiles, key_bits = hdr->key_bits;
+  const bool second = hdr->passes & 1u;
+  uint32_t *__restrict__ keys = second ? k1 : k0;
+  uint32_t *__restrict__ vals = second ? v1 : v0;
+  constexpr int kWarps = kBlock / 32;
+  __shared__ uint32_t warp_count[kWarps];
+  __shared__ unsigned long long before;
+  __shared__ int ticket, gave_up;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  while (true) {
+    if (threadIdx.x == 0) {
+      ticket = int(atomicAdd(&hdr->emit_ticket, 1u));
+      gave_up = 0;
+    }
+    __syncthreads();
+    const int tile = ticket;
+    if (tile >= n_tiles) return;
+    const TileRec t = tiles[tile];
+    const GridParams &g = scenes[t.scene].grid;
+    const int sh = g.shift, nc = g.nc;
+    const unsigned cb0 = cell_base[t.scene];
+    // a warp takes consecutive boxes of the tile, 32 at a time
+    const int share = (t.count + kWarps * 32 - 1) / (kWarps * 32) * 32;
+    const int w0 = min(warp * share, t.count), w1 = min(w0 + share, t.count);
+    uint32_t mine = 0;
+    for (int i = w0 + lane; i < w1; i += 32) mine += cells_count(box_cells[t.begin + i], sh);
+    mine = __reduce_add_sync(kFullMask, mine);
+    if (lane == 0) warp_count[warp] = mine;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t total = 0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) total += warp_count[w];
+      volatile unsigned long long *st = status;
+      if (lane == 0) st[tile] = (tile == 0 ? 2ull : 1ull) << 62 | total;
+      // look back 32 tiles at a time
+      unsigned long long sum = 0;
+      int spins = 0;
+      for (int at = tile - 1; at >= 0;) {
+        const unsigned long long w = at - lane >= 0 ? st[at - lane] : 2ull << 62;
+        const unsigned empty = __ballot_sync(kFullMask, (w >> 62) == 0ull);
+        const unsigned full = __ballot_sync(kFullMask, (w >> 62) == 2ull);
+        const int stop = full ? __ffs(full) - 1 : 31;  // last lane to add
+        if (empty & (stop == 31 ? kFullMask : (2u << stop) - 1u)) {  // a tile before that is not ready
+          if (++spins > kEmitSpins) {
+            if (lane == 0) gave_up = 1;
+            break;
+          }
+          continue;
+        }
+        unsigned long long v = lane <= stop ? w & ~(3ull << 62) : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
+        sum += v;
+        if (full) break;
+        at -= 32;
+      }
+      if (lane == 0) {
+        if (tile > 0) st[tile] = 2ull << 62 | (sum + total);
+        before = sum;
+      }
+    }
+    __syncthreads();
+    if (gave_up) {  // positions are not known: nothing is written
+      if (threadIdx.x == 0) hdr->fault = 1;
+      __syncthreads();
+      continue;
+    }
+    uint32_t o = uint32_t(before);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) o += w < warp ? warp_count[w] : 0u;
+    for (int i = w0 + lane; i - lane < w1; i += 32) {
+      uint2 r = make_uint2(0u, 0u);
+      uint32_t n = 0, q = 0;
+      if (i < w1) {
+        r = box_cells[t.begin + i];
+        q = (box_q[t.begin + i] & 0xffffu) >> (kAxisCodeBits - key_bits);
+        n = cells_count(r, sh);
+      }
+      uint32_t x = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFullMask, x, d);
+        if (lane >= d) x += y;
+      }
+      uint32_t at = o + x - n;
+      o += __shfl_sync(kFullMask, x, 31);
+      if (i < w1) {
+        const unsigned b0 = (r.x & 2047u) >> sh, b1 = (r.x >> 11 & 2047u) >> sh;
+        const unsigned c0 = (r.y & 2047u) >> sh, c1 = (r.y >> 11 & 2047u) >> sh;
+        const unsigned type = r.x >> 22;
+        for (unsigned cb = b0; cb <= b1; ++cb)
+          for (unsigned cc = c0; cc <= c1; ++cc) {
+            const unsigned seg = (cb0 + cb * unsigned(nc) + cc) * 3u + type;
+            keys[at] = seg << key_bits | q;
+            vals[at] = uint32_t(t.begin + i);
+            ++at;
+          }
+      }
+    }
+    __syncthreads();  // warp_count, before and ticket are rewritten
+  }
+}
+
 // First position of every (cell, type) list in the sorted replicas, and one
 // entry past the last (the replica count): the keys are sorted by list id, so
 // each offset is the lower bound of its id. Sorted replica p of list s sits at
 // position p + s, so list s ends at position offset[s + 1] + s: the slot after
-// it gets the NaN sentinel (NaN bounds end every run there; its partner is
-// itself, so the sweep's refill test of a sentinel reads inside the scene and
-// fails), and so do kSortedPad slots of padding after the last list. The
-// gather writes every other position. Also the longest list, a statistic of
-// the prepared scene.
+// it is an empty position (its run starts and ends at itself), and so are
+// kSortedPad slots of padding after the last list. The gather writes every
+// other position. Also the longest list, a statistic of the prepared scene.
 __global__ void __launch_bounds__(kBlock)
-list_offsets_kernel(const unsigned long long *__restrict__ keys, BatchHeader *__restrict__ hdr,
+list_offsets_kernel(const uint32_t *__restrict__ keys, BatchHeader *__restrict__ hdr,
                     uint32_t *__restrict__ seg_scan, long long seg_cap, SortedScene scene, int64_t slots_cap) {
-  // nothing was emitted past the capacity (the emit flags that overflow)
+  // (cells past the capacity are flagged and counted as none)
   const uint32_t nseg = uint32_t(min(3ll * hdr->cells, seg_cap));
   const uint32_t R = hdr->replicas;
-  const float q = __int_as_float(0x7fc00000);
-  auto sentinel = [&](int64_t k) {
+  const int key_bits = hdr->key_bits;
+  auto empty = [&](int64_t k) {
     if (k < slots_cap) {
-      scene.xmin[k] = q;
-      scene.xmax[k] = q;
       scene.partner[k] = int(k);
       scene.run_end[k] = int(k);
     }
@@ -521,7 +640,7 @@ list_offsets_kernel(const unsigned long long *__restrict__ keys, BatchHeader *__
     uint32_t a = 0, e = R;
     while (a < e) {
       const uint32_t mid = (a + e) >> 1;
-      if (uint32_t(keys[mid] >> 32) < s) a = mid + 1;
+      if (keys[mid] >> key_bits < s) a = mid + 1;
       else e = mid;
     }
     return a;
@@ -533,51 +652,53 @@ list_offsets_kernel(const unsigned long long *__restrict__ keys, BatchHeader *__
     if (s < nseg) {
       const uint32_t hi = lower(s + 1);
       mx = max(mx, hi - lo);
-      sentinel(int64_t(hi) + s);
+      empty(int64_t(hi) + s);
     }
   }
   for (uint32_t t = blockIdx.x * kBlock + threadIdx.x; t < uint32_t(kSortedPad); t += stride)
-    sentinel(int64_t(R) + nseg + t);
+    empty(int64_t(R) + nseg + t);
   mx = __reduce_max_sync(kFullMask, mx);
   if ((threadIdx.x & 31) == 0 && mx) atomicMax(&hdr->max_list, mx);
 }
 
 // Sorted replica p of segment s (cell c, type t; s = 3c + t) goes to
-// position p + s: every list is followed by one NaN slot, which ends every
-// run at its list (and cell, and scene) boundary.
-// sflag of a position: bit 0 set if the cell is the box's first cell along b,
-// bit 1 if it is its first cell along c, scene index above. Since the cell
-// coordinate is monotone, the cell of a pair's reference point (max of the
-// two minima on b, on c) is the max of the two boxes' first cells; both boxes
-// lie in this cell, so the reference point is here exactly when, on each of
-// b and c, one of the two replicas is its box's first cell.
+// position p + s.
+// First-cell bits of a position: bit 0 set if the cell is the box's first cell
+// along b, bit 1 if it is its first cell along c. Since the cell coordinate is
+// monotone, the cell of a pair's reference point (max of the two minima on b,
+// on c) is the max of the two boxes' first cells; both boxes lie in this cell,
+// so the reference point is here exactly when, on each of b and c, one of the
+// two replicas is its box's first cell.
 // scode of a position: its box's y/z interval in the cell and the inverted
 // first-cell bits (stq_device.cuh): one integer that the sweep tests against
 // the start box's before it loads any bound.
 // partner of a position: its first candidate. An edge's candidates are the
-// edges after it in its list; a vertex's are the cell's faces whose min is
-// >= its min (lower bound), a face's the cell's vertices whose min is > its
-// min (upper bound): every V-F pair that overlaps on the sweep axis is found
-// once, from the box with the smaller min (the vertex on ties), and vertex-
-// vertex, edge-face and face-face candidates are never tested.
+// edges after it in its list; a vertex's are the cell's faces whose code is
+// >= its code (lower bound), a face's the cell's vertices whose code is > its
+// code (upper bound): every V-F pair that can overlap on the sweep axis is found
+// once, and vertex-vertex, edge-face and face-face candidates are never tested.
+// run_end: one past the last candidate whose code is at most that of the box's
+// maximum (or its own, if that is larger: an inverted box still meets the boxes
+// of its code). Codes are monotone, so every candidate with a minimum at or
+// below the maximum is in the run; those of an equal code that are not are left
+// to the exact test.
 __global__ void __launch_bounds__(kBlock)
-gather_cells_kernel(const stq_aabb *__restrict__ boxes, const unsigned long long *__restrict__ keys,
-                    const uint32_t *__restrict__ order, const BatchHeader *hdr,
+gather_cells_kernel(const stq_aabb *__restrict__ boxes, const uint32_t *__restrict__ keys,
+                    const uint32_t *__restrict__ order, const uint32_t *__restrict__ box_q, const BatchHeader *hdr,
                     const unsigned int *__restrict__ cell_base,
                     const SceneRecord *__restrict__ scenes, const uint32_t *__restrict__ seg_scan,
-                    float *__restrict__ xmin,
-                    float *__restrict__ xmax,
-                    float4 *__restrict__ syz,
-                    int4 *__restrict__ sv, int *__restrict__ sflag, uint32_t *__restrict__ scode,
-                    int *__restrict__ partner, int *__restrict__ run_end) {
+                    SortedScene scene) {
   const int64_t R = hdr->replicas;
   const int S = hdr->n_scenes;
+  const int key_bits = hdr->key_bits;
   for (int64_t p = blockIdx.x * int64_t(kBlock) + threadIdx.x; p < R;
        p += int64_t(gridDim.x) * kBlock) {
-    const unsigned long long key = keys[p];
-    const unsigned int seg = unsigned(key >> 32);
-    const unsigned int cell = seg / 3u, type = seg - 3u * cell;
+    const uint32_t key = keys[p];
     const uint32_t bi = order[p];
+    const stq_aabb &x = boxes[bi];
+    const uint32_t qmax = (box_q[bi] >> 16) >> (kAxisCodeBits - key_bits);
+    const unsigned int seg = key >> key_bits;
+    const unsigned int cell = seg / 3u, type = seg - 3u * cell;
     int lo = 0, hi = S - 1;  // scene of the cell
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -587,7 +708,6 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const unsigned long long
     const GridParams g = scenes[lo].grid;
     int b, c;
     axes_bc(g.axis, b, c);
-    const stq_aabb &x = boxes[bi];
     const int local = int(cell - cell_base[lo]);
     const int cb = local / g.nc, cc = local - cb * g.nc;
     const int fb = (cell_coord(x.min[b], g.ob, g.ib, g.nb0) >> g.shift) == cb;
@@ -598,48 +718,42 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const unsigned long long
     // list of the cell from the bound search below
     unsigned int cand = seg;
     uint32_t run_a = uint32_t(p) + 1u, run_e = seg_scan[seg + 1];
+    const uint32_t q = key - (seg << key_bits);
     if (type != 1u) {
-      // bound search of this min among the other list's sorted keys
-      const unsigned int other = 3u * cell + (type == 0u ? 2u : 0u);
-      const uint32_t xk = uint32_t(key & 0xffffffffu);
-      uint32_t a = seg_scan[other], e = seg_scan[other + 1];
+      cand = 3u * cell + (type == 0u ? 2u : 0u);
+      const uint32_t want = cand << key_bits | q;
+      uint32_t a = seg_scan[cand], e = seg_scan[cand + 1];
       run_e = e;
       while (a < e) {
         const uint32_t mid = (a + e) >> 1;
-        const uint32_t mk = uint32_t(keys[mid] & 0xffffffffu);
-        if (type == 0u ? mk < xk : mk <= xk) a = mid + 1;
+        const uint32_t mk = keys[mid];
+        if (type == 0u ? mk < want : mk <= want) a = mid + 1;
         else e = mid;
       }
-      first = int64_t(a) + other;
-      cand = other;
+      first = int64_t(a) + cand;
       run_a = a;
     }
-    if (run_end) {
-      // end of the run: the first candidate whose min is above this max
-      // (keys order as floats, -0 = +0, so the key test is the sweep's x
-      // test); galloping from the run's start, then a bisection
-      const uint32_t xk = float_key(x.max[g.axis]);
-      uint32_t a = run_a, step = 8;
-      while (a + step <= run_e && uint32_t(keys[a + step - 1] & 0xffffffffu) <= xk) {
-        a += step;
-        step <<= 1;
-      }
-      uint32_t e = min(a + step, run_e);
-      while (a < e) {
-        const uint32_t mid = (a + e) >> 1;
-        if (uint32_t(keys[mid] & 0xffffffffu) <= xk) a = mid + 1;
-        else e = mid;
-      }
-      run_end[k] = int(int64_t(a) + cand);
+    // galloping from the run's start, then a bisection
+    const uint32_t last = cand << key_bits | max(qmax, q);
+    uint32_t a = run_a, step = 8;
+    while (a + step <= run_e && keys[a + step - 1] <= last) {
+      a += step;
+      step <<= 1;
     }
-    xmin[k] = x.min[g.axis];
-    xmax[k] = x.max[g.axis];
-    syz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
-    sv[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
-    sflag[k] = (lo << 2) | (fc << 1) | fb;
-    scode[k] = code_pack(code_step(x.min[b], g.ob, g.sb, cb), code_step(x.min[c], g.oc, g.sc, cc),
-                         code_step(x.max[b], g.ob, g.sb, cb), code_step(x.max[c], g.oc, g.sc, cc), !fb, !fc);
-    partner[k] = int(first);
+    uint32_t e = min(a + step, run_e);
+    while (a < e) {
+      const uint32_t mid = (a + e) >> 1;
+      if (keys[mid] <= last) a = mid + 1;
+      else e = mid;
+    }
+    scene.yz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
+    scene.x[k] = make_float2(x.min[g.axis], x.max[g.axis]);
+    scene.v[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
+    scene.flag[k] = (lo << 2) | (fc << 1) | fb;
+    scene.scode[k] = code_pack(code_step(x.min[b], g.ob, g.sb, cb), code_step(x.min[c], g.oc, g.sc, cc),
+                               code_step(x.max[b], g.ob, g.sb, cb), code_step(x.max[c], g.oc, g.sc, cc), !fb, !fc);
+    scene.partner[k] = int(first);
+    scene.run_end[k] = int(int64_t(a) + cand);
   }
 }
 
@@ -720,7 +834,7 @@ cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long l
 
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b) {
   batch_reset_kernel<<<blocks_for(b.scene_cap, 64), kBlock, 0, s>>>(b.scenes, b.inputs,
-                                                                      b.scene_pairs, b.hdr);
+                                                                      b.scene_pairs, b.hdr, b.emit_status);
   batch_stats_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.scenes, b.hdr);
   return cudaGetLastError();
 }
@@ -730,41 +844,28 @@ cudaError_t launch_batch_policy(cudaStream_t s, const BatchBuffers &b) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b) {
-  batch_box_keys_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.scenes, b.hdr, b.box_keys,
-                                                                b.box_vals, b.box_cells);
-  batch_choose_kernel<<<1, 1024, 0, s>>>(b.box_off, b.scenes, b.cell_base, b.hdr);
+cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap) {
+  batch_box_keys_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.scenes, b.hdr, b.box_cells, b.box_q);
+  batch_choose_kernel<<<1, 1024, 0, s>>>(b.box_off, b.scenes, b.cell_base, b.hdr, rep_cap, seg_cap);
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_counts(cudaStream_t s, const BatchBuffers &b, int64_t n) {
-  const int64_t m = std::max<int64_t>(n, b.box_cap);
-  batch_count_kernel<<<wave_blocks((const void *)batch_count_kernel, m), kBlock, 0, s>>>(
-      b.order, b.box_cells, b.box_off, b.scenes, b.hdr, b.counts, b.box_cap);
+cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b) {
+  batch_emit_kernel<<<wave_blocks((const void *)batch_emit_kernel, int64_t(b.tile_cap) * kBlock), kBlock, 0, s>>>(
+      b.box_cells, b.box_q, b.tiles, b.scenes, b.cell_base, b.hdr, b.emit_status, b.keys[0], b.keys[1], b.vals[0],
+      b.vals[1]);
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b, int64_t n, int num_sms) {
-  batch_emit_kernel<<<wave_blocks((const void *)batch_emit_kernel, n), kBlock, 0, s>>>(
-      b.box_cells, b.sorted_keys, b.order, b.box_off, b.scenes, b.cell_base, b.hdr, b.offsets, b.keys, b.vals,
-      b.rep_cap, b.seg_cap);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_list_offsets(cudaStream_t s, const unsigned long long *keys, BatchHeader *hdr, uint32_t *seg_scan,
+cudaError_t launch_list_offsets(cudaStream_t s, const uint32_t *keys, BatchHeader *hdr, uint32_t *seg_scan,
                                 int64_t seg_cap, const SortedScene &scene, int64_t slots_cap) {
   list_offsets_kernel<<<blocks_for(seg_cap + 1), kBlock, 0, s>>>(keys, hdr, seg_scan, seg_cap, scene, slots_cap);
   return cudaGetLastError();
 }
 
-cudaError_t launch_gather_cells(cudaStream_t s, const stq_aabb *boxes,
-                                const unsigned long long *keys, const uint32_t *order,
-                                const BatchHeader *hdr, int64_t rep_cap,
-                                const unsigned int *cell_base, const SceneRecord *scenes,
-                                const uint32_t *seg_scan, SortedScene scene) {
-  gather_cells_kernel<<<wave_blocks((const void *)gather_cells_kernel, rep_cap), kBlock, 0, s>>>(
-      boxes, keys, order, hdr, cell_base, scenes, seg_scan, scene.xmin, scene.xmax, scene.syz,
-      scene.sv, scene.sflag, scene.scode, scene.partner, scene.run_end);
+cudaError_t launch_gather_cells(cudaStream_t s, const BatchBuffers &b, int64_t replicas, const SortedScene &scene) {
+  gather_cells_kernel<<<wave_blocks((const void *)gather_cells_kernel, replicas), kBlock, 0, s>>>(
+      b.boxes, b.keys[0], b.vals[0], b.box_q, b.hdr, b.cell_base, b.scenes, b.seg_scan, scene);
   return cudaGetLastError();
 }
 

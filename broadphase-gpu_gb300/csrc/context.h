@@ -76,12 +76,11 @@ struct stq_context {
   DevBuf in_dev;
   char *in_host = nullptr;
   size_t in_host_bytes = 0;
-  DevBuf scenes, cell_base, scene_pairs, counts, offsets, box_cells, scan_ws, keys64[2], vals[2], sort_ws;
+  DevBuf scenes, cell_base, scene_pairs, box_cells, box_q, emit_status, keys[2], vals[2], sort_ws;
   DevBuf points;  // fp64 vertex positions rounded to float once (box builds)
-  DevBuf xmin, xmax, syz, sv, sflag, scode, partner, run_end, box_counts, prefix_ws, pair_tmp;
+  DevBuf yz, xx, vv, flag, scode, partner, run_end, box_counts, prefix_ws, pair_tmp;
   DevBuf long_list;  // runs handed from the lane sweep to the warp pass
   DevBuf seg_scan;  // first sorted replica of each (cell, type) list
-  DevBuf bkeys[2], bvals[2];  // box sort: keys and box indices, double-buffered
   int64_t seg_cap = 0;
   DevBuf batch_boxes, e2e_boxes, e2e_pairs, e2e_mesh;
   DevBuf aux;  // header of calls outside a batch (box build, all-pairs check)
@@ -127,11 +126,10 @@ struct stq_context {
 
   // every device buffer of the context
   std::vector<DevBuf *> buffers() {
-    return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &counts, &box_cells, &offsets, &scan_ws,
-            &keys64[0], &keys64[1], &vals[0], &vals[1], &sort_ws, &xmin, &xmax, &syz, &sv, &sflag, &scode,
-            &partner, &run_end, &long_list, &seg_scan, &bkeys[0], &bkeys[1], &bvals[0], &bvals[1],
-            &box_counts, &prefix_ws, &pair_tmp, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh,
-            &aux, &window_pairs, &window_long_list, &window_cursors};
+    return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &box_cells, &box_q, &emit_status, &keys[0], &keys[1],
+            &vals[0], &vals[1], &sort_ws, &yz, &xx, &vv, &flag, &scode, &partner, &run_end, &long_list, &seg_scan, &box_counts,
+            &prefix_ws, &pair_tmp, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh, &aux, &window_pairs,
+            &window_long_list, &window_cursors};
   }
 };
 
@@ -163,15 +161,14 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes);
 int ensure_box_buffers(stq_context *ctx, int64_t box_cap);
 int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap);
 int bits_for(int64_t v);
-// Statistics, axis and grid per scene, the box sort along the sweep axis,
-// replica counts per sorted position and their scan. n_boxes: the box count,
-// or -1 when only the device knows it (graph capture, serving).
-int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t n_boxes);
-// Replica emit in sweep-axis order, list counts and offsets, and the stable
-// sort by list id (seg_bits bits) that turns it into x-sorted cell lists;
-// then the sorted scene. replicas: the replica count, or -1 (device count).
-int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int seg_bits, int64_t n_boxes,
-                         int64_t replicas);
+// Statistics, axis, grid and sweep-axis codes per scene, the grid level and the
+// replica count. Scenes that need more than rep_cap replicas or seg_cap lists
+// are flagged and left empty (-1: no limit).
+int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap);
+// Replica emit in box order, their sort by (list, sweep-axis code), list offsets
+// and the sorted scene. replicas, passes: the replica count and the digits of
+// its sort, or -1 when only the device knows them (graph capture, serving).
+int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes);
 // Launches one sweep over start positions [begin, end). With cursors null it
 // first clears the batch header's pair counter, cursors, per-scene counts and
 // statistics and uses them and the context's long-run list; otherwise it uses

@@ -54,6 +54,9 @@ static_assert(sizeof(SortHead) <= kRadixHeadBytes, "workspace sizing");
 struct Digits {
   int passes;
   uint8_t shift[kMaxPasses];
+  // on the device, the passes to run (null: those whose digit is not the same
+  // in every key); the input is in buffer *d_passes & 1, the result in buffer 0
+  const unsigned int *d_passes;
 };
 
 __device__ __forceinline__ unsigned long long load_status(const unsigned long long *p) {
@@ -88,13 +91,14 @@ __device__ __forceinline__ uint32_t scan_bins(uint32_t v, uint32_t *scratch) {
 // Digit counts of every pass (one read of the keys) and, in the last block to
 // finish, the first position of every digit, the passes to run and the buffer
 // each reads. Also clears the tiles' status words. A digit that all keys share
-// is skipped, unless that would leave the result in the other buffer than the
-// host expects (buffer passes & 1): then one such pass is run as a copy.
+// is skipped, unless that would leave the result in the second buffer: then one
+// such pass is run as a copy (the number of passes is even).
 template <typename K>
 __global__ void __launch_bounds__(kHistBlock)
-radix_hist_kernel(const K *__restrict__ keys, int64_t n, const unsigned int *d_n, Digits dg, SortHead *head,
-                  unsigned long long *status, int tile) {
+radix_hist_kernel(const K *__restrict__ k0, const K *__restrict__ k1, int64_t n, const unsigned int *d_n, Digits dg,
+                  SortHead *head, unsigned long long *status, int tile) {
   if (d_n && int64_t(*d_n) < n) n = *d_n;
+  const K *__restrict__ keys = dg.d_passes && (*dg.d_passes & 1u) ? k1 : k0;
   __shared__ uint32_t h[kMaxPasses][kBins];
   __shared__ unsigned same;  // passes whose digit all keys share
   __shared__ uint32_t last;
@@ -158,8 +162,13 @@ radix_hist_kernel(const K *__restrict__ keys, int64_t n, const unsigned int *d_n
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned skip = same;
-    if (__popc(skip) & 1) skip &= skip - 1;  // run one of them: the parity the host expects
+    if (__popc(skip) & 1) skip &= skip - 1;  // run one of them: the result ends in the first buffer
     uint32_t src = 0;
+    if (dg.d_passes) {
+      const unsigned run = min(*dg.d_passes, unsigned(dg.passes));
+      skip = ~((1u << run) - 1u);
+      src = *dg.d_passes & 1u;
+    }
     for (int q = 0; q < dg.passes; ++q) {
       const uint32_t run = (skip >> q & 1u) ? 0u : 1u;
       head->run[q] = run;
@@ -360,7 +369,11 @@ struct BlockShared {
 
 template <typename K, bool VALS, int ITEMS>
 __global__ void __launch_bounds__(kPassBlock)
-radix_block_kernel(const K *kin, K *kout, const uint32_t *vin, uint32_t *vout, int n, Digits dg) {
+radix_block_kernel(const K *k0, const K *k1, K *kout, const uint32_t *v0, const uint32_t *v1, uint32_t *vout, int n,
+                   Digits dg) {
+  const bool second = dg.d_passes && (*dg.d_passes & 1u);
+  const K *kin = second ? k1 : k0;
+  const uint32_t *vin = second ? v1 : v0;
   using S = BlockShared<K, VALS, ITEMS>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   S &sm = *reinterpret_cast<S *>(smem_raw);
@@ -480,8 +493,8 @@ cudaError_t launch_block(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[
   constexpr size_t smem = sizeof(BlockShared<K, VALS, ITEMS>);
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  const int to = dg.passes & 1;
-  kern<<<1, kPassBlock, smem, s>>>(kbuf[0], kbuf[to], VALS ? vbuf[0] : nullptr, VALS ? vbuf[to] : nullptr, int(n), dg);
+  kern<<<1, kPassBlock, smem, s>>>(kbuf[0], kbuf[1], kbuf[0], VALS ? vbuf[0] : nullptr, VALS ? vbuf[1] : nullptr,
+                                   VALS ? vbuf[0] : nullptr, int(n), dg);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
@@ -489,7 +502,7 @@ cudaError_t launch_block(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[
 template <typename K, bool VALS>
 cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const unsigned int *d_n,
                       const Digits &dg, void *workspace, int *fault, int64_t *launches) {
-  if (n <= 1 || dg.passes == 0) return cudaSuccess;
+  if (dg.passes == 0 || (n <= 1 && !dg.d_passes)) return cudaSuccess;
   if (!d_n) {  // one block up to its 16 keys per thread
     if (n <= kPassBlock * 2) return launch_block<K, VALS, 2>(s, kbuf, vbuf, n, dg, launches);
     if (n <= kPassBlock * 8) return launch_block<K, VALS, 8>(s, kbuf, vbuf, n, dg, launches);
@@ -504,13 +517,13 @@ cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2],
   // inputs take small ones, so that every SM gets a tile. The line is at half a
   // large tile per SM: 1.0 M u32 keys take 74 us in large tiles and 91 in small
   // ones, 346,000 pairs 78 us in large and 70 in small ones.
-  constexpr int kLarge = sizeof(K) == 8 && VALS ? 8 : 16;
+  constexpr int kLarge = 16;
   static_assert(kPassBlock * kLarge >= 2 * kMinTile, "workspace sizing: status words of large tiles");
   const bool large = n >= int64_t(sm_count()) * 4096;
   const int tile = large ? kPassBlock * kLarge : kMinTile;
   const int64_t hist_blocks = (n + kHistBlock * 4 - 1) / (kHistBlock * 4);
   radix_hist_kernel<K><<<unsigned(std::min<int64_t>(hist_blocks, int64_t(sm_count()) * 4)), kHistBlock, 0, s>>>(
-      kbuf[0], n, d_n, dg, head, status, tile);
+      kbuf[0], kbuf[1], n, d_n, dg, head, status, tile);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   e = large ? launch_passes<K, VALS, kLarge>(s, kbuf, vbuf, n, d_n, dg, head, status, fault)
@@ -521,9 +534,11 @@ cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2],
 
 }  // namespace
 
-cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *kbuf[2], uint32_t *vbuf[2], int64_t n, void *workspace,
-                           int *fault, int64_t *launches, const unsigned int *d_n) {
-  return sort_impl<uint32_t, true>(s, kbuf, vbuf, n, d_n, Digits{4, {0, 8, 16, 24}}, workspace, fault, launches);
+cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, void *workspace,
+                           int *fault, int64_t *launches, const unsigned int *d_n, const unsigned int *d_passes,
+                           int passes) {
+  return sort_impl<uint32_t, true>(s, kbuf, vbuf, n, d_n, Digits{passes, {0, 8, 16, 24}, d_passes}, workspace, fault,
+                                   launches);
 }
 
 cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,
@@ -533,139 +548,8 @@ cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int
   unsigned long long *kb[2] = {reinterpret_cast<unsigned long long *>(pairs),
                                reinterpret_cast<unsigned long long *>(tmp)};
   return sort_impl<unsigned long long, false>(s, kb, nullptr, n, nullptr,
-                                              Digits{8, {32, 40, 48, 56, 0, 8, 16, 24}}, workspace, fault, launches);
-}
-
-cudaError_t radix_sort_u64_vals(cudaStream_t s, unsigned long long *kbuf[2], uint32_t *vbuf[2], int64_t n,
-                                int begin_bit, int end_bit, void *workspace, int *which, int *fault,
-                                int64_t *launches, const unsigned int *d_n) {
-  Digits dg{};
-  for (int shift = begin_bit; shift < end_bit; shift += 8) dg.shift[dg.passes++] = uint8_t(shift);
-  *which = n <= 1 ? 0 : dg.passes & 1;
-  return sort_impl<unsigned long long, true>(s, kbuf, vbuf, n, d_n, dg, workspace, fault, launches);
-}
-
-// ---- exclusive scan of uint32 counts (reduce-then-scan, no waiting) -------------
-namespace {
-
-constexpr int kSortBlock = 256;
-constexpr int kSortWarps = kSortBlock / 32;
-
-// Block-wide exclusive scan of one value per thread (kSortBlock threads).
-__device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *total, uint32_t *scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(kFullMask, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) scratch[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t w = lane < kSortWarps ? scratch[lane] : 0;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(kFullMask, w, o);
-      if (lane >= o) w += y;
-    }
-    if (lane < kSortWarps) scratch[lane] = w;  // inclusive warp totals
-  }
-  __syncthreads();
-  const uint32_t warp_base = warp > 0 ? scratch[warp - 1] : 0;
-  *total = scratch[kSortWarps - 1];
-  __syncthreads();
-  return warp_base + x - v;
-}
-
-// Exclusive scan of in[b, b + 2048) (clipped to n) into out, starting from
-// carry, by one block with 8 entries per thread: coalesced loads into shared
-// memory, each thread scans 8 consecutive entries (padded indices: no bank
-// conflicts), one block scan. Returns the chunk's total (in every thread).
-constexpr int kChunkPer = 8, kChunk = kSortBlock * kChunkPer;
-__device__ uint32_t scan_chunk(const uint32_t *in, uint32_t *out, int64_t b, int64_t n, uint32_t carry) {
-  __shared__ uint32_t buf[kChunk + kChunk / 32];
-  __shared__ uint32_t scratch[32];
-  auto at = [](int x) { return x + (x >> 5); };
-#pragma unroll
-  for (int i = 0; i < kChunkPer; ++i) {
-    const int x = i * kSortBlock + threadIdx.x;
-    buf[at(x)] = b + x < n ? in[b + x] : 0u;
-  }
-  __syncthreads();
-  uint32_t v[kChunkPer], sum = 0;
-#pragma unroll
-  for (int i = 0; i < kChunkPer; ++i) {
-    v[i] = buf[at(threadIdx.x * kChunkPer + i)];
-    sum += v[i];
-  }
-  uint32_t tot;
-  uint32_t run = carry + block_exclusive_scan(sum, &tot, scratch);
-#pragma unroll
-  for (int i = 0; i < kChunkPer; ++i) {
-    buf[at(threadIdx.x * kChunkPer + i)] = run;
-    run += v[i];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kChunkPer; ++i) {
-    const int x = i * kSortBlock + threadIdx.x;
-    if (b + x < n) out[b + x] = buf[at(x)];
-  }
-  __syncthreads();  // the next chunk overwrites buf
-  return tot;
-}
-
-// Exclusive scan of row[0..n) in place by one block; returns the total.
-__device__ uint32_t block_scan_row(uint32_t *row, int64_t n) {
-  uint32_t carry = 0;
-  for (int64_t b = 0; b < n; b += kChunk) carry += scan_chunk(row, row, b, n, carry);
-  return carry;
-}
-
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kSortBlock * kScanItems;
-
-__global__ void __launch_bounds__(kSortBlock)
-scan_reduce_kernel(const uint32_t *__restrict__ in, int64_t n, uint32_t *__restrict__ sums) {
-  __shared__ uint32_t scratch[32];
-  const int64_t base = int64_t(blockIdx.x) * kScanTile + threadIdx.x;
-  uint32_t s = 0;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i)  // coalesced; a sum needs no order
-    if (base + i * kSortBlock < n) s += in[base + i * kSortBlock];
-  uint32_t tot;
-  block_exclusive_scan(s, &tot, scratch);
-  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
-
-__global__ void __launch_bounds__(kSortBlock)
-scan_sums_kernel(uint32_t *__restrict__ sums, int64_t ntiles, uint32_t *__restrict__ total) {
-  const uint32_t t = block_scan_row(sums, ntiles);
-  if (threadIdx.x == 0) *total = t;
-}
-
-__global__ void __launch_bounds__(kSortBlock)
-scan_apply_kernel(const uint32_t *__restrict__ in, int64_t n, const uint32_t *__restrict__ sums,
-                  uint32_t *__restrict__ out) {
-  static_assert(kScanTile == kChunk, "one chunk per scan tile");
-  scan_chunk(in, out, int64_t(blockIdx.x) * kScanTile, n, sums[blockIdx.x]);
-}
-
-}  // namespace
-
-size_t scan_workspace_bytes(int64_t n) {
-  const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-  return sizeof(uint32_t) * size_t(ntiles + 1);
-}
-
-cudaError_t exclusive_scan_u32(cudaStream_t s, const uint32_t *in, uint32_t *out, int64_t n,
-                               void *workspace, uint32_t *d_total, int64_t *launches) {
-  const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
-  uint32_t *sums = static_cast<uint32_t *>(workspace);
-  if (n > 0) scan_reduce_kernel<<<unsigned(ntiles), kSortBlock, 0, s>>>(in, n, sums);
-  scan_sums_kernel<<<1, kSortBlock, 0, s>>>(sums, ntiles, d_total);
-  if (n > 0) scan_apply_kernel<<<unsigned(ntiles), kSortBlock, 0, s>>>(in, n, sums, out);
-  if (launches) *launches += n > 0 ? 3 : 1;
-  return cudaGetLastError();
+                                              Digits{8, {32, 40, 48, 56, 0, 8, 16, 24}, nullptr},
+                                              workspace, fault, launches);
 }
 
 }  // namespace stq

@@ -264,8 +264,8 @@ int enqueue_tick(stq_server *sv, bool advance) {
                                         ref_next_up(0.f), ctx->batch_boxes.as<stq_aabb>()),
            "launch box build");
   const BatchBuffers b = batch_buffers(ctx, ctx->batch_boxes.as<stq_aabb>());
-  STQ_TRY(enqueue_prepare_front(ctx, b, -1));
-  STQ_TRY(enqueue_prepare_back(ctx, b, bits_for(3 * (sv->max_boxes / 16 + sv->max_scenes + 1)), -1, -1));
+  STQ_TRY(enqueue_prepare_front(ctx, b, ctx->rep_cap, ctx->seg_cap));
+  STQ_TRY(enqueue_prepare_back(ctx, b, -1, -1));
   STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, sv->pairs.as<stq_pair>(), sv->pair_cap, false));
   STQ_CUDA(ctx, launch_pair_checksums(ctx->stream, sv->pairs.as<stq_pair>(), sv->pair_cap, hdr, box_off,
                                       sv->checks_dev.as<unsigned long long>(), sv->max_scenes),
@@ -428,7 +428,9 @@ int stq_server_create(int device, void *stream, int64_t budget_bytes, int64_t ma
       cudaEventCreateWithFlags(&sv->copy_done, cudaEventDisableTiming) != cudaSuccess)
     return bad(STQ_ERR_CUDA);
   // pipeline buffers for the largest batch, counted against the budget
-  const int64_t tiles = max_boxes / kTileBoxes + max_scenes + 1;
+  // small ticks are cut into small tiles, of which there are fewer than kSmallBatch
+  // / kSmallTile and one per scene
+  const int64_t tiles = std::max(max_boxes / kTileBoxes, kSmallBatch / kSmallTile) + max_scenes + 1;
   if (ensure_staging(ctx, max_scenes, int(tiles)) != STQ_OK || ensure_box_buffers(ctx, max_boxes) != STQ_OK ||
       ensure_replica_buffers(ctx, int64_t(ctx->budget) * max_boxes, max_boxes / 16 + max_scenes + 1) != STQ_OK ||
       ctx->batch_boxes.ensure(sizeof(stq_aabb) * size_t(max_boxes)) != cudaSuccess ||
@@ -443,11 +445,8 @@ int stq_server_create(int device, void *stream, int64_t budget_bytes, int64_t ma
   std::memset(sv->voff_host, 0, sizeof(long long) * size_t(max_scenes + 1));
   size_t free_b = 0, total = 0;
   cudaMemGetInfo(&free_b, &total);
-  sv->fixed = int64_t(ctx->in_dev.bytes + ctx->counts.bytes + ctx->offsets.bytes + ctx->scan_ws.bytes +
-                      ctx->keys64[0].bytes * 2 + ctx->vals[0].bytes * 2 + ctx->sort_ws.bytes + ctx->xmin.bytes + ctx->xmax.bytes +
-                      ctx->syz.bytes + ctx->sv.bytes + ctx->sflag.bytes + ctx->scode.bytes +
-                      ctx->partner.bytes + ctx->run_end.bytes +
-                      ctx->seg_scan.bytes + ctx->batch_boxes.bytes);
+  sv->fixed = 0;
+  for (const DevBuf *b : ctx->buffers()) sv->fixed += int64_t(b->bytes);
   if (sv->fixed >= budget_bytes) return bad(STQ_ERR_NO_MEMORY);
   *out = sv.release();
   return STQ_OK;

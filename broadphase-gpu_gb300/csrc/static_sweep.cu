@@ -29,12 +29,10 @@ constexpr size_t kOffVals0 = kOffKeys1 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kOffVals1 = kOffVals0 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kOffSortWs = kOffVals1 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kSortWsBytes = radix_workspace_bytes(kMax);
-constexpr size_t kOffXmin = kOffSortWs + up256(kSortWsBytes);
-constexpr size_t kOffXmax = kOffXmin + up256(sizeof(float) * kSlots);
-constexpr size_t kOffSyz = kOffXmax + up256(sizeof(float) * kSlots);
-constexpr size_t kOffSv = kOffSyz + up256(sizeof(float4) * kSlots);
-constexpr size_t kOffFlag = kOffSv + up256(sizeof(int4) * kSlots);
-constexpr size_t kOffCode = kOffFlag + up256(sizeof(int) * kSlots);
+constexpr size_t kOffYz = kOffSortWs + up256(kSortWsBytes);
+constexpr size_t kOffX = kOffYz + up256(sizeof(float4) * kSlots);
+constexpr size_t kOffV = kOffX + up256(sizeof(float2) * kSlots);
+constexpr size_t kOffCode = kOffV + up256(sizeof(int4) * kSlots);
 constexpr size_t kOffPartner = kOffCode + up256(sizeof(uint32_t) * kSlots);
 constexpr size_t kOffRunEnd = kOffPartner + up256(sizeof(int) * kSlots);
 constexpr size_t kOffHdr = kOffRunEnd + up256(sizeof(int) * kSlots);
@@ -88,11 +86,9 @@ __global__ void static_keys_kernel(const stq_aabb *__restrict__ boxes, int n, in
 __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, int axis,
                                      const uint32_t *__restrict__ keys, const uint32_t *__restrict__ order,
                                      unsigned char *scratch) {
-  float *xmin = reinterpret_cast<float *>(scratch + kOffXmin);
-  float *xmax = reinterpret_cast<float *>(scratch + kOffXmax);
-  float4 *syz = reinterpret_cast<float4 *>(scratch + kOffSyz);
-  int4 *sv = reinterpret_cast<int4 *>(scratch + kOffSv);
-  int *sflag = reinterpret_cast<int *>(scratch + kOffFlag);
+  float4 *yz = reinterpret_cast<float4 *>(scratch + kOffYz);
+  float2 *xx = reinterpret_cast<float2 *>(scratch + kOffX);
+  int4 *v = reinterpret_cast<int4 *>(scratch + kOffV);
   uint32_t *scode = reinterpret_cast<uint32_t *>(scratch + kOffCode);
   int *partner = reinterpret_cast<int *>(scratch + kOffPartner);
   int *run_end = reinterpret_cast<int *>(scratch + kOffRunEnd);
@@ -101,11 +97,9 @@ __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, 
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) {
     const stq_aabb &x = boxes[order[k]];
-    xmin[k] = x.min[axis];
-    xmax[k] = x.max[axis];
-    syz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
-    sv[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
-    sflag[k] = 3;  // one cell: every box is in its first cell on both axes
+    yz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
+    xx[k] = make_float2(x.min[axis], x.max[axis]);
+    v[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
     const float ob = key_float(~extent[0]), oc = key_float(~extent[1]);
     const float lb = key_float(extent[2]) - ob, lc = key_float(extent[3]) - oc;
     const float sb = lb > 0.f && isfinite(lb) ? 64.f / lb : 0.f, sc = lc > 0.f && isfinite(lc) ? 64.f / lc : 0.f;
@@ -122,9 +116,6 @@ __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, 
     }
     run_end[k] = lo;
   } else if (k < n + 1 + kSortedPad) {
-    const float q = __int_as_float(0x7fc00000);
-    xmin[k] = q;
-    xmax[k] = q;
     partner[k] = k;
     run_end[k] = k;
   }
@@ -176,11 +167,10 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
     return STQ_ERR_CUDA;
   static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, kb[0], vb[0], scratch);
   SweepParams p;
-  p.xmin = reinterpret_cast<const float *>(scratch + kOffXmin);
-  p.xmax = reinterpret_cast<const float *>(scratch + kOffXmax);
-  p.syz = reinterpret_cast<const float4 *>(scratch + kOffSyz);
-  p.sv = reinterpret_cast<const int4 *>(scratch + kOffSv);
-  p.sflag = reinterpret_cast<const int *>(scratch + kOffFlag);
+  p.yz = reinterpret_cast<const float4 *>(scratch + kOffYz);
+  p.x = reinterpret_cast<const float2 *>(scratch + kOffX);
+  p.v = reinterpret_cast<const int4 *>(scratch + kOffV);
+  p.flag = nullptr;  // one scene, and no runs for the warp pass
   p.scode = reinterpret_cast<const uint32_t *>(scratch + kOffCode);
   p.partner = reinterpret_cast<const int *>(scratch + kOffPartner);
   p.run_end = reinterpret_cast<const int *>(scratch + kOffRunEnd);

@@ -96,6 +96,14 @@ constexpr int kGridLevels = 6;  // level L halves the level-0 grid L times
 constexpr int kCoordBits = 11;  // level-0 cell coordinates are below 2^11
 static_assert(kMaxGridSide <= (1 << kCoordBits), "level-0 cell coordinates fit kCoordBits");
 
+// Sweep-axis codes: 16 bits, 64 segments of 1,024 steps. The segments hold
+// about the same number of boxes each (their ends are quantiles of a sample), so
+// that no spread of the boxes, however uneven, puts many of them on one step.
+constexpr int kSplits = 64;
+constexpr int kSplitSteps = 1024;
+constexpr int kAxisCodeBits = 16;
+static_assert(kSplits * kSplitSteps == 1 << kAxisCodeBits, "16-bit codes");
+
 // One scene of a batch: inputs written by the host, the rest computed on the
 // device by the prepare kernels.
 struct SceneRecord {
@@ -107,7 +115,8 @@ struct SceneRecord {
   // statistics
   double s1[3], s2[3];              // sum(min + max), sum(min^2 + max^2)
   unsigned int lo_key[3], hi_key[3];  // order-preserving min / max bounds
-  unsigned int hist[3][64];         // log2 histogram of the extents
+  float split[kSplits];             // sweep-axis codes: lower ends of the segments
+  float split_inv[kSplits];         // code steps per unit length in each
   int inverted;                     // some box has min > max on an axis
   int pad1;
   unsigned long long level_reps[kGridLevels];  // replicas per grid level
@@ -141,15 +150,21 @@ struct BatchHeader {
   int budget;               // replica budget: replicas <= budget * boxes per scene
   int n_tiles;              // input: entries of the tile table
   unsigned int max_list;    // longest (cell, type) list
-  unsigned int box_count;   // input: n_boxes as the element count of the box sort
+  int key_bits;             // sweep-axis bits of a replica key (the list id is above)
   unsigned long long candidates;  // candidates tested by the last sweep
   unsigned int lists;       // (cell, type) lists: 3 * cells
   int fault;                // a bounded wait between blocks ran out
+  unsigned int passes;      // digits of the replica sort; its input is in buffer passes & 1
+  unsigned int emit_ticket; // next tile of the replica emit
 };
 
 // A tile of at most kTileBoxes consecutive boxes of one scene (built by the
 // host from the scene offsets), so that a block reduces per-scene values once.
 constexpr int kTileBoxes = 4096;
+// Batches of up to kSmallBatch boxes take tiles of 1,024, so that most SMs get one.
+constexpr int kSmallTile = 1024;
+constexpr int64_t kSmallBatch = 152 * 4 * kSmallTile;
+constexpr int tile_boxes(int64_t n) { return n <= kSmallBatch ? kSmallTile : kTileBoxes; }
 struct TileRec {
   long long begin;  // first box of the tile
   int count;        // boxes in the tile
@@ -173,19 +188,25 @@ struct SweepTuning {
   int chunk = 256;      // start boxes per work grab
 };
 
-// Sorted scene in HBM, structure of arrays, one sentinel after the boxes
-// (xmin = xmax = NaN) followed by kSortedPad padding entries.
+// One sorted position: what the exact test of a pair reads.
+struct PosRec {
+  float4 yz;  // (min_b, min_c, max_b, max_c) on the non-sweep axes
+  float2 x;   // (min, max) on the sweep axis
+  int4 v;     // vertexIds[0..2], id
+};
+
+// Sorted scene in HBM, structure of arrays. Every list is followed by one empty
+// position (partner = run_end = itself).
 struct SortedScene {
-  float *xmin = nullptr;  // min on the sweep axis (all a candidate needs)
-  float *xmax = nullptr;  // max on the sweep axis (read once per start box)
-  float4 *syz = nullptr;  // (min_b, min_c, max_b, max_c) on the other axes
-  int4 *sv = nullptr;     // (vertexIds[0..2], id)
-  int *sflag = nullptr;   // first-cell bits (0: along b, 1: along c), scene << 2
+  float4 *yz = nullptr;
+  float2 *x = nullptr;
+  int4 *v = nullptr;
+  int *flag = nullptr;        // first-cell bits (0: along b, 1: along c), scene << 2
   uint32_t *scode = nullptr;  // y/z interval in the cell and first-cell bits
                               // (position codes, stq_device.cuh)
-  int *partner = nullptr; // first candidate position of each start position
-  int *run_end = nullptr; // one past its last candidate on the sweep axis
-  int64_t length = 0;     // sweep positions (boxes; sentinels excluded at the end)
+  int *partner = nullptr;     // first candidate position of each start position
+  int *run_end = nullptr;     // one past its last candidate
+  int64_t length = 0;         // sweep positions (boxes; sentinels excluded at the end)
 };
 
 // Counters of one sweep launch that runs beside another (a host call's
@@ -208,10 +229,13 @@ struct SweepCursors {
 };
 
 struct SweepParams {
-  const float *xmin;
-  const float *xmax;
-  const float4 *syz;
-  const int4 *sv;
+  const float4 *yz;          // bounds on the non-sweep axes
+  const float2 *x;           // on the sweep axis
+  const int4 *v;             // vertex ids and id
+  const int *flag;           // first-cell bits and scene
+  const uint32_t *scode;     // position codes
+  const int *partner;        // first candidate position of each start position
+  const int *run_end;        // one past its last candidate
   int32_t begin, end;        // start positions [begin, min(end, hdr->length))
   int32_t chunk;             // start positions per grab
   stq_pair *pairs;
@@ -219,11 +243,6 @@ struct SweepParams {
   unsigned long long *count;
   int *work;
   int32_t *box_counts;       // count mode: pairs per start position (k - begin)
-  const int *sflag;          // first-cell bits and scene of each position
-  const uint32_t *scode;     // position codes
-  const int *partner;        // first candidate position of each start position
-  const int *run_end;        // one past its last candidate (null: not computed;
-                             // the flat shape needs it)
   unsigned long long *scene_pairs;  // per-scene pair counters
   const BatchHeader *hdr;    // device sizes (length bounds the sweep range)
   unsigned long long *stats; // candidates tested (may be null)
@@ -256,15 +275,12 @@ struct BatchBuffers {
   SceneRecord *scenes;
   unsigned int *cell_base;      // n_scenes + 1
   BatchHeader *hdr;
-  uint32_t *counts, *offsets;   // per box position in sweep-axis order
-  uint2 *box_cells;             // per box index: cell range and type
+  uint2 *box_cells;             // per box: cell range and type
                                 // (b0 | b1 << 11 | type << 22, c0 | c1 << 11)
-  uint32_t *box_keys, *box_vals;  // box sort input (key, box index), double-buffered with
-  uint32_t *box_keys2, *box_vals2;
-  const uint32_t *order;        // boxes in sweep-axis order (box sort output)
-  const uint32_t *sorted_keys;  // their sort keys (sweep-axis minimum images)
-  unsigned long long *keys;     // replica keys (sort input)
-  uint32_t *vals;               // replica box indices (sort input)
+  uint32_t *box_q;              // per box: sweep-axis codes of its min | its max << 16
+  unsigned long long *emit_status;  // per tile: running replica counts of the emit
+  uint32_t *keys[2];            // replica keys: list id << key_bits | sweep-axis code
+  uint32_t *vals[2];            // replica box indices
   uint32_t *seg_scan;           // first sorted replica of each segment (cell x type),
                                 // seg_cap + 1 entries
   long long seg_cap;
@@ -276,23 +292,19 @@ struct BatchBuffers {
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b);
 // sweep axis and level-0 grid per scene (1 launch)
 cudaError_t launch_batch_policy(cudaStream_t s, const BatchBuffers &b);
-// box sort keys, level-0 cell ranges and every level's replica count; then the
-// level within the replica budget and the cell bases (2 launches)
-cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b);
-// n: positions to cover (the box count, or the box capacity when only the
-// device knows the count)
-cudaError_t launch_batch_counts(cudaStream_t s, const BatchBuffers &b, int64_t n);
-cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b, int64_t n, int num_sms);
-// list offsets from the list-sorted keys (and the longest list); the NaN
-// sentinel after every list and the padding after the last
-cudaError_t launch_list_offsets(cudaStream_t s, const unsigned long long *keys, BatchHeader *hdr, uint32_t *seg_scan,
+// level-0 cell ranges, sweep-axis codes and every level's replica count; then the
+// level within the replica budget, the cell bases and the key layout (2 launches).
+// Scenes that need more than rep_cap replicas or seg_cap lists are flagged and
+// left empty (no limit: -1).
+cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap);
+// replicas in box order (1 launch)
+cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b);
+// list offsets from the sorted keys (and the longest list); the empty position
+// after every list and the padding after the last
+cudaError_t launch_list_offsets(cudaStream_t s, const uint32_t *keys, BatchHeader *hdr, uint32_t *seg_scan,
                                 int64_t seg_cap, const SortedScene &scene, int64_t slots_cap);
 
-cudaError_t launch_gather_cells(cudaStream_t s, const stq_aabb *boxes,
-                                const unsigned long long *keys, const uint32_t *order,
-                                const BatchHeader *hdr, int64_t rep_cap,
-                                const unsigned int *cell_base, const SceneRecord *scenes,
-                                const uint32_t *seg_scan, SortedScene scene);
+cudaError_t launch_gather_cells(cudaStream_t s, const BatchBuffers &b, int64_t replicas, const SortedScene &scene);
 // Batched box build: scene s has vertices [voff[s], voff[s+1]) etc.; box ids
 // are global (box_off[s] + local), vertex ids local to the scene.
 // points: 2 * vert_cap float4 of scratch for the rounded positions
@@ -338,22 +350,15 @@ constexpr size_t radix_workspace_bytes(int64_t n) {
   const size_t small = tiles < small_max ? tiles : small_max;
   return kRadixHeadBytes + sizeof(unsigned long long) * 256 * (small > half ? small : half);
 }
-// result in kbuf[0], vbuf[0]
-cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *kbuf[2], uint32_t *vbuf[2], int64_t n, void *workspace,
-                           int *fault, int64_t *launches, const unsigned int *d_n = nullptr);
-// by bits [begin_bit, end_bit); *which receives the buffer that holds the result
-cudaError_t radix_sort_u64_vals(cudaStream_t s, unsigned long long *kbuf[2], uint32_t *vbuf[2], int64_t n,
-                                int begin_bit, int end_bit, void *workspace, int *which, int *fault,
-                                int64_t *launches, const unsigned int *d_n = nullptr);
+// result in kbuf[0], vbuf[0]. d_passes (may be null: 4): on the device, the
+// number of low digits to sort by, at most `passes`; the input is then in
+// buffer *d_passes & 1, else in buffer 0.
+cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, void *workspace,
+                           int *fault, int64_t *launches, const unsigned int *d_n = nullptr,
+                           const unsigned int *d_passes = nullptr, int passes = 4);
 // lexicographic by (first, second) as unsigned ids, in place; tmp holds n pairs
 cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,
                              int64_t *launches);
-// exclusive scan of n uint32 counts; *d_total receives the sum
-size_t scan_workspace_bytes(int64_t n);
-cudaError_t exclusive_scan_u32(cudaStream_t s, const uint32_t *in, uint32_t *out, int64_t n,
-                               void *workspace, uint32_t *d_total, int64_t *launches);
-
-
 cudaError_t launch_sweep(cudaStream_t s, const SweepParams &p,
                          const SweepTuning &t, bool count_mode, int num_sms);
 // inclusive scan of box_counts[0..m) and the longest prefix whose pair sum

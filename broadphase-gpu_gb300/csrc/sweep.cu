@@ -6,19 +6,19 @@
 // is_valid_pair (src/collision.cu:38-48, src/aabb.cu:33-40) and add_overlap
 // (src/collision.cu:50-74).
 //
-// GB300 design. A start box k's candidates are its x-run
-// j = partner[k], partner[k]+1, ... up to the first j whose min exceeds k's
-// max (a NaN sentinel ends every list); partner[k] is k+1 for an edge, and the
-// first face (for a vertex) or vertex (for a face) of the same cell's list at
-// or after k's min. Two shapes walk the runs:
+// GB300 design. A start box k's candidates are its run [partner[k], run_end[k])
+// of one list, found by the gather: the edges after it for an edge, the faces (for
+// a vertex) or vertices (for a face) of the same cell. A run holds every
+// candidate that can overlap on the sweep axis, and a few that do not (those of
+// an equal sweep-axis code); a candidate's position code is tested first, then
+// the pair exactly. Two shapes walk the runs:
 //   - queue (stq_sweep_lane_kernel, stq_sweep_kernel): each warp owns a
 //     shared-memory ring of pending start boxes (the "tiniest queue"); a lane,
 //     or a group of G lanes, takes one start box from the ring and walks its
 //     run, and takes the next pending box when the run ends, so a long run
 //     never stalls the others;
-//   - flat (stq_sweep_flat_kernel, the default): the gather has found every
-//     run's end (run_end), so a warp lays the runs of 32 consecutive start
-//     positions end to end and tests one candidate per lane and step.
+//   - flat (stq_sweep_flat_kernel, the default): a warp takes the runs of 32
+//     consecutive start positions together.
 // Runs longer than a cap go to a warp pass (stq_long_run_kernel). Refill,
 // hand-out and pair output use __ballot_sync/__popc compaction: no
 // shared-memory atomics, and one global atomic per 32 or more pairs.
@@ -33,6 +33,17 @@
 namespace stq {
 
 namespace {
+
+__device__ __forceinline__ PosRec load_pos(const SweepParams &p, int j) { return PosRec{p.yz[j], p.x[j], p.v[j]}; }
+
+// The exact test of a pair that passed the filter: overlap on the non-sweep
+// axes and on the sweep axis (the box with the smaller minimum reaches the other's
+// minimum; on ties the start box a goes first), is_valid_pair where the lists
+// mix types, and covertex.
+__device__ __forceinline__ bool pair_hit(const PosRec &a, const PosRec &b, int typed) {
+  const bool x = b.x.x >= a.x.x ? b.x.x <= a.x.y : a.x.x <= b.x.y;
+  return x && overlap_bc(a.yz, b.yz) && (typed || valid_pair(a.v, b.v)) && !covertex(a.v, b.v);
+}
 
 // Appends the warp's n staged pairs with one atomic; pairs past the capacity
 // are counted but not written.
@@ -61,7 +72,6 @@ stq_sweep_kernel(const SweepParams p) {
   const int gl = lane % G;              // lane within group
   const int grp = lane / G;             // group within warp
   const unsigned grp_mask = G == 32 ? kFullMask : (((1u << G) - 1u) << (grp * G));
-  const unsigned upto_me = grp_mask & (lane == 31 ? kFullMask : ((2u << lane) - 1u));
   const unsigned leaders_below = (grp * G) == 0 ? 0u : ((1u << (grp * G)) - 1u);
   int *q = ring[threadIdx.x >> 5];
 
@@ -71,13 +81,12 @@ stq_sweep_kernel(const SweepParams p) {
   bool more = true;
   // lane-group state (identical in the G lanes of a group)
   int k = -1, j0 = 0, taken = 0;
-  float kmax = 0.f;
-  float4 kb = make_float4(0.f, 0.f, 0.f, 0.f);
-  int4 kv = make_int4(0, 0, 0, 0);
-  uint32_t knf = 0;  // not-first bits of the current start box
+  int jend = 0;       // one past the run of the current start box
+  PosRec kr = {};     // the current start box
+  uint32_t code = 0;  // and its code
+  int kf = 0;         // its scene, above the first-cell bits
   const int end = min(p.end, int(p.hdr->length));
   const int span = end - p.begin;
-  int kf = 0;  // scene of the current start box (above the first-cell bits)
   unsigned tested = 0;  // candidates this lane tested (statistics)
   // warp-uniform: staged pairs, and pairs of the current scene not yet added
   // to its counter
@@ -104,7 +113,7 @@ stq_sweep_kernel(const SweepParams p) {
       const int take = min(32, min(Q - qsize, chunk_end - next_k));
       const int kk = next_k + lane;
       bool push = false;
-      if (lane < take) push = p.xmin[p.partner[kk]] <= p.xmax[kk];
+      if (lane < take) push = p.partner[kk] < p.run_end[kk];
       const unsigned m = __ballot_sync(kFullMask, push);
       if (push) q[(qhead + qsize + __popc(m & lanemask_lt())) & (Q - 1)] = kk;
       qsize += __popc(m);
@@ -120,12 +129,11 @@ stq_sweep_kernel(const SweepParams p) {
       if (r < ntake) {
         k = q[(qhead + r) & (Q - 1)];
         j0 = p.partner[k];
-        kmax = p.xmax[k];
-        kb = p.syz[k];
-        kv = p.sv[k];
-        knf = p.scode[k] & kCodeNotFirst;
+        jend = p.run_end[k];
+        kr = load_pos(p, k);
+        code = code_start(p.scode[k]);
+        kf = multi ? p.flag[k] : 0;
         taken = 0;
-        kf = multi ? p.sflag[k] : 0;
       }
     }
     qhead = (qhead + ntake) & (Q - 1);
@@ -136,25 +144,19 @@ stq_sweep_kernel(const SweepParams p) {
       if (!more && qsize == 0) break;
       continue;
     }
-    // 3. Test G consecutive candidates per group. Valid lanes form the
-    //    prefix of the group before the first x-test failure.
+    // 3. Test G consecutive candidates per group: those before the run's end,
+    //    by their codes, then exactly.
     const int j = j0 + gl;
-    const bool xok = active && p.xmin[j] <= kmax;
-    const unsigned failm = __ballot_sync(kFullMask, active && !xok);
-    const bool valid = active && (failm & upto_me) == 0;
+    const bool valid = active && j < jend;
     bool hit = false;
     int lo_id = 0, hi_id = 0;
     if (valid) {
       ++tested;
-      const float4 b = p.syz[j];
-      // a pair found in several cells is emitted only in the cell of its
-      // reference point: on b and on c, one of the two replicas must be its
-      // box's first cell
-      if (overlap_bc(kb, b) && (p.scode[j] & knf) == 0u) {  // ids only for these
-        const int4 bv = p.sv[j];
-        hit = (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
-        lo_id = min(kv.w, bv.w);
-        hi_id = max(kv.w, bv.w);
+      if (code_pass(code, p.scode[j])) {
+        const PosRec c = load_pos(p, j);
+        hit = pair_hit(kr, c, p.typed);
+        lo_id = min(kr.v.w, c.v.w);
+        hi_id = max(kr.v.w, c.v.w);
       }
     }
     // 4. Emit: compact the step's hits into the warp's staging buffer; append
@@ -211,11 +213,10 @@ stq_sweep_kernel(const SweepParams p) {
 }
 
 // One start box per lane. A lane walks its own run, U consecutive candidates
-// per step: the U minima are loaded together (U independent loads in flight
-// per lane), the valid ones are the prefix before the first x-test failure
-// (lane-local: no ballot), and a lane whose run ended takes the next pending
-// box from the warp's ring. Otherwise as stq_sweep_kernel: ring refill by
-// ballot compaction, lazy vertex-id loads, per-warp staging of pairs.
+// per step: the U codes are loaded together (U independent loads in flight per
+// lane), and a lane whose run ended takes the next pending box from the warp's
+// ring. Otherwise as stq_sweep_kernel: ring refill by ballot compaction, per-warp
+// staging of pairs.
 template <int U, int Q, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_lane_kernel(const SweepParams p) {
@@ -238,11 +239,10 @@ stq_sweep_lane_kernel(const SweepParams p) {
   int qhead = 0, qsize = 0;
   int next_k = 0, chunk_end = 0;
   bool more = true;
-  int k = -1, j = 0, kf = 0, taken = 0;
-  float kmax = 0.f;
-  float4 kb = make_float4(0.f, 0.f, 0.f, 0.f);
-  int4 kv = make_int4(0, 0, 0, 0);
-  uint32_t knf = 0;  // not-first bits of the start box
+  int k = -1, j = 0, jend = 0, taken = 0;
+  PosRec kr = {};     // the start box
+  uint32_t code = 0;  // and its code
+  int kf = 0;         // its scene, above the first-cell bits
   const int end = min(p.end, int(p.hdr->length));
   const int span = end - p.begin;
   unsigned tested = 0;
@@ -271,7 +271,7 @@ stq_sweep_lane_kernel(const SweepParams p) {
       int pk = 0;
       if (lane < take) {
         pk = p.partner[kk];
-        push = p.xmin[pk] <= p.xmax[kk];
+        push = pk < p.run_end[kk];
       }
       const unsigned m = __ballot_sync(kFullMask, push);
       if (push) {
@@ -297,11 +297,10 @@ stq_sweep_lane_kernel(const SweepParams p) {
           k = e;
           j = p.partner[k];
         }
-        kmax = p.xmax[k];
-        kb = p.syz[k];
-        kv = p.sv[k];
-        knf = p.scode[k] & kCodeNotFirst;
-        kf = multi ? p.sflag[k] : 0;
+        jend = p.run_end[k];
+        kr = load_pos(p, k);
+        code = code_start(p.scode[k]);
+        kf = multi ? p.flag[k] : 0;
         taken = 0;
       }
     }
@@ -313,31 +312,18 @@ stq_sweep_lane_kernel(const SweepParams p) {
       if (!more && qsize == 0) break;
       continue;
     }
-    // 3. U candidates of the lane's run: the valid ones are the prefix before
-    //    the first x-test failure (a NaN sentinel ends every list).
-    float xm[U];
+    // 3. U candidates of the lane's run (their codes are loaded together), by
+    //    their codes, then exactly. Hits as bits; a hit's id is loaded again on
+    //    output (an L1 hit) rather than kept in registers for the whole step.
+    const int nvalid = active ? min(U, jend - j) : 0;
+    uint32_t cc[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) xm[u] = active ? p.xmin[j + u] : 0.f;
-    int nvalid = 0;
-    if (active) {
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (nvalid == u && xm[u] <= kmax) ++nvalid;
-    }
+    for (int u = 0; u < U; ++u) cc[u] = u < nvalid ? p.scode[j + u] : 0u;
     tested += unsigned(nvalid);
-    // hits as bits; a hit's id is loaded again on output (an L1 hit) rather
-    // than kept in registers for the whole step
     unsigned hits = 0;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (u < nvalid) {
-        const float4 b = p.syz[j + u];
-        if (overlap_bc(kb, b) && (p.scode[j + u] & knf) == 0u) {  // and the first-cell rule
-          const int4 bv = p.sv[j + u];
-          if ((p.typed || valid_pair(kv, bv)) && !covertex(kv, bv)) hits |= 1u << u;
-        }
-      }
-    }
+    for (int u = 0; u < U; ++u)
+      if (u < nvalid && code_pass(code, cc[u]) && pair_hit(kr, load_pos(p, j + u), p.typed)) hits |= 1u << u;
     // 4. Emit the step's hits through the warp's staging buffer.
     const int nh = __popc(hits);
     const unsigned anym = __ballot_sync(kFullMask, nh > 0);
@@ -348,8 +334,8 @@ stq_sweep_lane_kernel(const SweepParams p) {
         const bool hit = (hits >> u) & 1u;
         const unsigned hm = __ballot_sync(kFullMask, hit);
         if (hit) {
-          const int id = p.sv[j + u].w;
-          st[staged + __popc(hm & below)] = make_int2(min(kv.w, id), max(kv.w, id));
+          const int id = p.v[j + u].w;
+          st[staged + __popc(hm & below)] = make_int2(min(kr.v.w, id), max(kr.v.w, id));
         }
         staged += __popc(hm);
         total += __popc(hm);
@@ -419,30 +405,31 @@ stq_sweep_lane_kernel(const SweepParams p) {
 // buffer. The starts' records sit in shared memory, so the queue is drained
 // before the next 32 starts replace them.
 struct FlatStart {
-  float4 kb;      // start box (min_b, min_c, max_b, max_c)
-  uint32_t code;  // code_start of its code
-  int joff;       // position of flat candidate f is joff + f
-  int j;          // first position of its run
+  float4 yz;      // the start box (PosRec)
+  int4 v;
+  float2 x;
   int kf;         // first-cell bits and scene
-  int4 kv;        // vertex ids and id
+  int j;          // first position of its run
 };
 static_assert(sizeof(FlatStart) == 48, "FlatStart: three 16-byte words");
 
 // Band or flat: a band step takes some 500 instructions for 32 positions, 130 of
-// them the filter, and a flat step some 30 for its 32 candidates. The line is
-// flat between 3 and 8 candidates per position of the window (1.16 to 1.18 ms
-// on the 6 M-box scene, where 98% of the candidates are in bands); without
-// bands that sweep takes 1.36 ms.
+// them the filter, and a flat step some 30 for its 32 candidates. The time is
+// level between 3 and 8 candidates per position of the window (within 2% on the
+// 6 M-box scene, where 98% of the candidates are in bands); without bands that
+// sweep takes 18% longer.
 constexpr int kBandRatio = 6;
 // Pairs staged per warp, appended with one atomic on the pair counter once
-// fewer than 32 places are left. All warps share that counter: with 64 places
-// the same sweep takes 1.61 ms, with 128 1.16, with 192 1.12; larger stages take
-// resident blocks away (384: 1.20, 768: 1.38 ms).
+// fewer than 32 places are left. All warps share that counter: on the 6 M-box
+// scene (92 M pairs) 64 places took 1.61 ms, 128 1.16, 192 1.12; larger stages
+// take resident blocks away (384: 1.20, 768: 1.38 ms).
 constexpr int kFlatStage = 192;
 constexpr int kFlatRound = 256;  // candidates queued at once by a band step (or 32 V by a flat one)
 constexpr int kFlatQueue = 32 + kFlatRound;
 struct FlatWarp {
   FlatStart rec[32];
+  int2 lookup[32];             // flat form: code_start of a start's code, and joff: its
+                               // run's flat candidate f is at position joff + f
   int2 stage[kFlatStage];
   uint32_t queue[kFlatQueue];  // slot | offset in the run << 5 (run_cap < 2^27)
   uint4 code[8];               // a band step's 32 candidate codes
@@ -480,15 +467,13 @@ stq_sweep_flat_kernel(const SweepParams p) {
       const uint32_t e = qu[queued - n + lane];
       const FlatStart &r = rec[e & 31u];
       const int j = r.j + int(e >> 5);
-      const float4 b = p.syz[j];
-      const int4 bv = p.sv[j];
-      const int4 kv = r.kv;
+      const PosRec c = load_pos(p, j);
       if (multi) kf = r.kf;
-      hit = overlap_bc(r.kb, b) && (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
+      hit = pair_hit(PosRec{r.yz, r.x, r.v}, c, p.typed);
       if (COUNT) {
         if (hit) atomicAdd(&sw.hits[e & 31u], 1);
       } else {
-        pr = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
+        pr = make_int2(min(r.v.w, c.v.w), max(r.v.w, c.v.w));
       }
     }
     queued -= n;
@@ -532,8 +517,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
     const int take = min(32, chunk_end - next_k);
     const int k = next_k + lane;
     next_k += take;
-    // 1. Runs: the candidates before the first minimum above the start's
-    //    maximum (a sentinel position has an empty run).
+    // 1. Runs (that of the position after a list is empty).
     int len = 0, j = 0;
     if (lane < take) {
       j = p.partner[k];
@@ -559,14 +543,14 @@ stq_sweep_flat_kernel(const SweepParams p) {
     uint32_t code = 0;
     if (len > 0) {
       FlatStart r;
-      r.kb = p.syz[k];
+      r.yz = p.yz[k];
+      r.x = p.x[k];
+      r.v = p.v[k];
+      r.kf = multi ? p.flag[k] : 0;
       code = code_start(p.scode[k]);
-      r.code = code;
-      r.joff = j - excl;
       r.j = j;
-      r.kf = multi ? p.sflag[k] : 0;
-      r.kv = p.sv[k];
       rec[slot] = r;
+      sw.lookup[slot] = make_int2(int(code), j - excl);
     }
     if (COUNT) sw.hits[lane] = 0;
     tested += unsigned(total);
@@ -637,10 +621,10 @@ stq_sweep_flat_kernel(const SweepParams p) {
           si[v] = begun + __popc(heads & upto) - 1;
           begun += __popc(heads);
           const int f = base + 32 * v + lane;
-          const uint4 r = *reinterpret_cast<const uint4 *>(&rec[si[v]].code);
-          const int jj = int(r.y) + f;
-          sc[v] = r.x;
-          rel[v] = f < total ? jj - int(r.z) : -1;
+          const int2 r = sw.lookup[si[v]];
+          const int jj = r.y + f;
+          sc[v] = uint32_t(r.x);
+          rel[v] = f < total ? jj - rec[si[v]].j : -1;
           cc[v] = f < total ? p.scode[jj] : 0u;
         }
 #pragma unroll
@@ -674,9 +658,8 @@ stq_sweep_flat_kernel(const SweepParams p) {
 // The warp pass over the runs the lane sweep handed over (runs longer than
 // SweepParams::run_cap, which would keep one lane or group busy long after the
 // others finished). One warp per run; each step tests 32 * U consecutive
-// candidates, lane l taking j + 32u + l; the valid ones are those before the
-// first x-test failure in position order (the padding after the last list
-// covers the reads past it). All pairs of a run belong to its start box's scene.
+// candidates, lane l taking j + 32u + l. All pairs of a run belong to its start
+// box's scene.
 template <int U, bool COUNT>
 __global__ void __launch_bounds__(256)
 stq_long_run_kernel(const SweepParams p) {
@@ -697,34 +680,26 @@ stq_long_run_kernel(const SweepParams p) {
     const int2 it = p.long_list[item];
     const int k = it.x;
     int j = it.y;
-    const float kmax = p.xmax[k];
-    const float4 kb = p.syz[k];
-    const int4 kv = p.sv[k];
-    const uint32_t knf = p.scode[k] & kCodeNotFirst;
-    const int kf = p.sflag[k];
+    const int jend = p.run_end[k];
+    const PosRec kr = load_pos(p, k);
+    const uint32_t code = code_start(p.scode[k]);
+    const int kf = p.flag[k];
     unsigned run_hits = 0;  // warp-uniform (emit) or this lane's (count mode)
-    while (true) {
-      float xm[U];
+    for (; j < jend; j += 32 * U) {
+      uint32_t cc[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) xm[u] = p.xmin[j + 32 * u + lane];
-      int first = 32 * U;  // offset of the first x-test failure
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const unsigned fm = __ballot_sync(kFullMask, !(xm[u] <= kmax));
-        if (first == 32 * U && fm) first = 32 * u + __ffs(fm) - 1;
-      }
+      for (int u = 0; u < U; ++u) cc[u] = j + 32 * u + lane < jend ? p.scode[j + 32 * u + lane] : 0u;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int off = 32 * u + lane;
+        const int at = j + 32 * u + lane;
         bool hit = false;
         int2 pr = make_int2(0, 0);
-        if (off < first) {
+        if (at < jend) {
           ++tested;
-          const float4 b = p.syz[j + off];
-          if (overlap_bc(kb, b) && (p.scode[j + off] & knf) == 0u) {  // and the first-cell rule
-            const int4 bv = p.sv[j + off];
-            hit = (p.typed || valid_pair(kv, bv)) && !covertex(kv, bv);
-            pr = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
+          if (code_pass(code, cc[u])) {
+            const PosRec c = load_pos(p, at);
+            hit = pair_hit(kr, c, p.typed);
+            pr = make_int2(min(kr.v.w, c.v.w), max(kr.v.w, c.v.w));
           }
         }
         if (COUNT) {
@@ -741,8 +716,6 @@ stq_long_run_kernel(const SweepParams p) {
         flush_staged(st, staged, lane, p);
         staged = 0;
       }
-      if (first < 32 * U) break;
-      j += 32 * U;
     }
     if (COUNT) {
       const unsigned total = __reduce_add_sync(kFullMask, run_hits);
@@ -976,7 +949,7 @@ static cudaError_t launch_sweep_lanes(cudaStream_t s, const SweepParams &p, cons
                                       bool count_mode, int num_sms) {
   if (count_mode)  // per-start-box counts do not depend on the tuning
     return launch_flat_block<256, 4, true>(s, p, num_sms);
-  if (t.shape == kShapeFlat && p.run_end) {
+  if (t.shape == kShapeFlat) {
     switch (t.per_lane) {  // filter steps per round
       case 2: return launch_flat<2>(s, p, t.block, num_sms);
       default: return launch_flat<4>(s, p, t.block, num_sms);
