@@ -24,15 +24,19 @@ constexpr int64_t kSlots = kMax + 1 + kSortedPad;
 // Byte layout of the scratch array (offsets are multiples of 256).
 constexpr size_t up256(size_t v) { return (v + 255) & ~size_t(255); }
 constexpr size_t kOffKeys0 = 0;
-constexpr size_t kOffKeys1 = kOffKeys0 + up256(sizeof(uint32_t) * kMax);
-constexpr size_t kOffVals0 = kOffKeys1 + up256(sizeof(uint32_t) * kMax);
-constexpr size_t kOffVals1 = kOffVals0 + up256(sizeof(uint32_t) * kMax);
+constexpr size_t kOffVals0 = kOffKeys0 + up256(sizeof(uint32_t) * kMax);
+// the sort's second buffers; the sweep's list of long runs takes their place
+constexpr size_t kOffKeys1 = kOffVals0 + up256(sizeof(uint32_t) * kMax);
+constexpr size_t kOffVals1 = kOffKeys1 + up256(sizeof(uint32_t) * kMax);
+constexpr size_t kOffLong = kOffKeys1;
+static_assert(sizeof(int2) * kMax <= 2 * up256(sizeof(uint32_t) * kMax), "long runs fit the sort's second buffers");
 constexpr size_t kOffSortWs = kOffVals1 + up256(sizeof(uint32_t) * kMax);
 constexpr size_t kSortWsBytes = radix_workspace_bytes(kMax);
 constexpr size_t kOffYz = kOffSortWs + up256(kSortWsBytes);
 constexpr size_t kOffX = kOffYz + up256(sizeof(float4) * kSlots);
 constexpr size_t kOffV = kOffX + up256(sizeof(float2) * kSlots);
-constexpr size_t kOffCode = kOffV + up256(sizeof(int4) * kSlots);
+constexpr size_t kOffFlag = kOffV + up256(sizeof(int4) * kSlots);
+constexpr size_t kOffCode = kOffFlag + up256(sizeof(int) * kSlots);
 constexpr size_t kOffPartner = kOffCode + up256(sizeof(uint32_t) * kSlots);
 constexpr size_t kOffRunEnd = kOffPartner + up256(sizeof(int) * kSlots);
 constexpr size_t kOffHdr = kOffRunEnd + up256(sizeof(int) * kSlots);
@@ -89,6 +93,7 @@ __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, 
   float4 *yz = reinterpret_cast<float4 *>(scratch + kOffYz);
   float2 *xx = reinterpret_cast<float2 *>(scratch + kOffX);
   int4 *v = reinterpret_cast<int4 *>(scratch + kOffV);
+  int *flag = reinterpret_cast<int *>(scratch + kOffFlag);
   uint32_t *scode = reinterpret_cast<uint32_t *>(scratch + kOffCode);
   int *partner = reinterpret_cast<int *>(scratch + kOffPartner);
   int *run_end = reinterpret_cast<int *>(scratch + kOffRunEnd);
@@ -100,6 +105,7 @@ __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, 
     yz[k] = make_float4(x.min[b], x.min[c], x.max[b], x.max[c]);
     xx[k] = make_float2(x.min[axis], x.max[axis]);
     v[k] = make_int4(x.vertex_ids[0], x.vertex_ids[1], x.vertex_ids[2], x.id);
+    flag[k] = 3;  // one cell, one scene: every box is in its first cell
     const float ob = key_float(~extent[0]), oc = key_float(~extent[1]);
     const float lb = key_float(extent[2]) - ob, lc = key_float(extent[3]) - oc;
     const float sb = lb > 0.f && isfinite(lb) ? 64.f / lb : 0.f, sc = lc > 0.f && isfinite(lc) ? 64.f / lc : 0.f;
@@ -166,17 +172,21 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   if (radix_sort_u32(s, kb, vb, n, scratch + kOffSortWs, &hdr->fault, nullptr) != cudaSuccess)
     return STQ_ERR_CUDA;
   static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, kb[0], vb[0], scratch);
+  int num_sms = 152;
+  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   SweepParams p;
   p.yz = reinterpret_cast<const float4 *>(scratch + kOffYz);
   p.x = reinterpret_cast<const float2 *>(scratch + kOffX);
   p.v = reinterpret_cast<const int4 *>(scratch + kOffV);
-  p.flag = nullptr;  // one scene, and no runs for the warp pass
+  p.flag = reinterpret_cast<const int *>(scratch + kOffFlag);
   p.scode = reinterpret_cast<const uint32_t *>(scratch + kOffCode);
   p.partner = reinterpret_cast<const int *>(scratch + kOffPartner);
   p.run_end = reinterpret_cast<const int *>(scratch + kOffRunEnd);
   p.begin = 0;
   p.end = ni;
-  p.chunk = 32;
+  // start boxes per warp: 8 where 32 would leave warps without any (65,536 boxes
+  // are 2,048 warps of 32)
+  p.chunk = n <= int64_t(num_sms) * 48 * 32 ? 8 : 32;
   p.pairs = d_pairs;
   p.capacity = capacity;
   p.count = &hdr->pairs;
@@ -186,12 +196,10 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   p.hdr = hdr;
   p.stats = nullptr;
   p.typed = 0;  // one list of all box types
-  p.run_cap = 0;  // no warp pass: it would need a list of handed-over runs
-  p.long_list = nullptr;
-  p.long_items = nullptr;
-  p.long_work = nullptr;
-  int num_sms = 152;
-  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  p.run_cap = 512;
+  p.long_list = reinterpret_cast<int2 *>(scratch + kOffLong);
+  p.long_items = &hdr->long_items;
+  p.long_work = &hdr->long_work;
   if (launch_sweep(s, p, SweepTuning(), false, num_sms) != cudaSuccess) return STQ_ERR_CUDA;
   BatchHeader h;
   if (cudaMemcpyAsync(&h, hdr, sizeof(BatchHeader), cudaMemcpyDeviceToHost, s) != cudaSuccess ||

@@ -19,7 +19,7 @@
 //     never stalls the others;
 //   - flat (stq_sweep_flat_kernel, the default): a warp takes the runs of 32
 //     consecutive start positions together.
-// Runs longer than a cap go to a warp pass (stq_long_run_kernel). Refill,
+// Runs longer than a cap go to a warp pass (the flat kernel over a list). Refill,
 // hand-out and pair output use __ballot_sync/__popc compaction: no
 // shared-memory atomics, and one global atomic per 32 or more pairs.
 #include <map>
@@ -404,6 +404,11 @@ stq_sweep_lane_kernel(const SweepParams p) {
 // vertex ids, is_valid_pair and covertex. The hits go through the staging
 // buffer. The starts' records sit in shared memory, so the queue is drained
 // before the next 32 starts replace them.
+//
+// LONG: the warp pass over the runs that were handed over (longer than run_cap,
+// which would keep one lane, group or warp busy long after the others finished).
+// The warp's starts are entries of that list, and when there are fewer of them
+// than warps each run is cut into as many equal parts as give every warp one.
 struct FlatStart {
   float4 yz;      // the start box (PosRec)
   int4 v;
@@ -436,7 +441,7 @@ struct FlatWarp {
   int hits[32];                // count mode: pairs per slot
 };
 
-template <int BLOCK, int V, bool COUNT>
+template <int BLOCK, int V, bool COUNT, bool LONG>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_flat_kernel(const SweepParams p) {
   static_assert(32 * V <= kFlatRound, "queue holds a flat round");
@@ -449,8 +454,19 @@ stq_sweep_flat_kernel(const SweepParams p) {
   int2 *st = sw.stage;
   uint32_t *qu = sw.queue;
 
-  const int end = min(p.end, int(p.hdr->length));
-  const int span = end - p.begin;
+  int end, span, chunk = p.chunk;
+  unsigned parts = 1;  // LONG: parts of a run
+  if (LONG) {
+    const unsigned items = *p.long_items, warps = gridDim.x * (BLOCK / 32);
+    if (items == 0) return;
+    parts = max(1u, min(64u, warps / items));
+    end = span = int(items * parts);
+    chunk = max(1, min(32, span / int(4 * warps)));
+  } else {
+    end = min(p.end, int(p.hdr->length));
+    span = end - p.begin;
+  }
+  const int first = LONG ? 0 : p.begin;
   const bool multi = p.hdr->n_scenes > 1;
   int next_k = 0, chunk_end = 0;
   unsigned long long tested = 0;  // warp-uniform
@@ -458,68 +474,30 @@ stq_sweep_flat_kernel(const SweepParams p) {
   int wscene = 0;
   unsigned long long wpairs = 0;
 
-  // the check of n <= 32 queued candidates (the last n entries)
-  auto check = [&](int n) {
-    bool hit = false;
-    int2 pr = make_int2(0, 0);
-    int kf = 0;
-    if (lane < n) {
-      const uint32_t e = qu[queued - n + lane];
-      const FlatStart &r = rec[e & 31u];
-      const int j = r.j + int(e >> 5);
-      const PosRec c = load_pos(p, j);
-      if (multi) kf = r.kf;
-      hit = pair_hit(PosRec{r.yz, r.x, r.v}, c, p.typed);
-      if (COUNT) {
-        if (hit) atomicAdd(&sw.hits[e & 31u], 1);
-      } else {
-        pr = make_int2(min(r.v.w, c.v.w), max(r.v.w, c.v.w));
-      }
-    }
-    queued -= n;
-    if (COUNT) return;
-    const unsigned hm = __ballot_sync(kFullMask, hit);
-    if (hm) {
-      if (hit) st[staged + __popc(hm & below)] = pr;
-      staged += __popc(hm);
-      if (!multi) {
-        wpairs += __popc(hm);
-      } else {
-        const int lead = __shfl_sync(kFullMask, kf >> 2, __ffs(hm) - 1);
-        if (__all_sync(kFullMask, !hit || (kf >> 2) == lead)) {
-          if (lead != wscene) {
-            if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
-            wscene = lead;
-            wpairs = 0;
-          }
-          wpairs += __popc(hm);
-        } else if (hit) {
-          atomicAdd(&p.scene_pairs[kf >> 2], 1ull);
-        }
-      }
-      if (staged > kFlatStage - 32) {
-        __syncwarp();
-        flush_staged(st, staged, lane, p);
-        staged = 0;
-      }
-    }
-  };
-
   while (true) {
     if (next_k >= chunk_end) {
       int c = 0;
-      if (lane == 0) c = atomicAdd(p.work, p.chunk);
+      if (lane == 0) c = LONG ? int(atomicAdd(p.long_work, unsigned(chunk))) : atomicAdd(p.work, chunk);
       c = __shfl_sync(kFullMask, c, 0);
       if (c >= span) break;
-      next_k = p.begin + c;
-      chunk_end = min(next_k + p.chunk, end);
+      next_k = first + c;
+      chunk_end = min(next_k + chunk, end);
     }
     const int take = min(32, chunk_end - next_k);
-    const int k = next_k + lane;
+    int k = next_k + lane;
     next_k += take;
     // 1. Runs (that of the position after a list is empty).
     int len = 0, j = 0;
-    if (lane < take) {
+    if (LONG) {
+      if (lane < take) {
+        const int2 it = p.long_list[unsigned(k) / parts];
+        const int part = int(unsigned(k) % parts), run_end = p.run_end[it.x];
+        const int each = (run_end - it.y + int(parts) - 1) / int(parts);
+        k = it.x;
+        j = it.y + part * each;
+        len = max(min(each, run_end - j), 0);
+      }
+    } else if (lane < take) {
       j = p.partner[k];
       len = max(p.run_end[k] - j, 0);
       if (p.run_cap && len > p.run_cap) {  // a long run: the warp pass takes the rest
@@ -557,76 +535,78 @@ stq_sweep_flat_kernel(const SweepParams p) {
     const int jlo = __reduce_min_sync(kFullMask, len > 0 ? j : 0x7fffffff);
     const int jhi = __reduce_max_sync(kFullMask, len > 0 ? j + len : 0);
     __syncwarp();
-    if (jhi - jlo <= total / kBandRatio) {
-      // 3a. The band: 32 positions of the window per step.
-      for (int j0 = jlo; j0 < jhi; j0 += 32) {
-        const int lo = j - j0, hi = lo + len;
-        uint32_t mine = 0;  // positions of this step inside the lane's run
-        if (len > 0 && lo < 32 && hi > 0)
-          mine = (kFullMask << max(lo, 0)) & (hi >= 32 ? kFullMask : ~(kFullMask << hi));
-        if (__ballot_sync(kFullMask, mine != 0u) == 0u) continue;
-        reinterpret_cast<uint32_t *>(sw.code)[lane] = p.scode[j0 + lane];
-        __syncwarp();
-        uint32_t hits = 0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const uint4 c = sw.code[q];
-          if (code_pass(code, c.x)) hits |= 1u << (4 * q);
-          if (code_pass(code, c.y)) hits |= 2u << (4 * q);
-          if (code_pass(code, c.z)) hits |= 4u << (4 * q);
-          if (code_pass(code, c.w)) hits |= 8u << (4 * q);
-        }
-        hits &= mine;
-        // queue them, places by a prefix sum of the lanes' counts; more than
-        // the queue holds go 8 positions (at most 256 candidates) at a time
-        uint32_t part = __reduce_add_sync(kFullMask, __popc(hits)) <= unsigned(kFlatRound) ? kFullMask : 0xffu;
-        do {
-          uint32_t h = hits & part;
-          hits ^= h;
-          part <<= 8;
-          const int count = __popc(h);
-          int at = count;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(kFullMask, at, o);
-            if (lane >= o) at += v;
-          }
-          const int all = __shfl_sync(kFullMask, at, 31);
-          at += queued - count;
-          while (h) {
-            const int c = __ffs(h) - 1;
-            h &= h - 1u;
-            qu[at++] = unsigned(slot) | unsigned(c - lo) << 5;
-          }
-          queued += all;
+    const bool band = jhi - jlo <= total / kBandRatio;
+    const unsigned my_begin = len > 0 ? unsigned(excl) : 0xffffffffu;
+    int at = band ? jlo : 0;  // next position (band) or flat candidate
+    const int stop = band ? jhi : total;
+    int begun = 0;      // flat: starts whose run began before the current step
+    int lo = 0;         // band: the lane's run begins lo positions into the step
+    uint32_t hits = 0;  // band: candidates of the step that are not queued yet,
+    uint32_t part = 0;  // and those of them that go next
+    bool more;
+    do {
+      if (band) {
+        // 3a. The band: 32 positions of the window per step.
+        if (part == 0u) {
+          lo = j - at;
+          const int hi = lo + len;
+          uint32_t mine = 0;  // positions of this step inside the lane's run
+          if (len > 0 && lo < 32 && hi > 0)
+            mine = (kFullMask << max(lo, 0)) & (hi >= 32 ? kFullMask : ~(kFullMask << hi));
+          reinterpret_cast<uint32_t *>(sw.code)[lane] = p.scode[at + lane];
           __syncwarp();
-          while (queued >= 32) {
-            check(32);
-            __syncwarp();
+          at += 32;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint4 c = sw.code[q];
+            if (code_pass(code, c.x)) hits |= 1u << (4 * q);
+            if (code_pass(code, c.y)) hits |= 2u << (4 * q);
+            if (code_pass(code, c.z)) hits |= 4u << (4 * q);
+            if (code_pass(code, c.w)) hits |= 8u << (4 * q);
           }
-        } while (__any_sync(kFullMask, hits != 0u));
-      }
-    } else {
-      // 3b. Flat: V steps of 32 candidates at a time. A run that begins inside
-      //     the step at `base` marks bit (excl - base).
-      const unsigned my_begin = len > 0 ? unsigned(excl) : 0xffffffffu;
-      int begun = 0;  // starts whose run began before the current step
-      for (int base = 0; base < total; base += 32 * V) {
+          hits &= mine;
+          // more than the queue holds go 8 positions (at most 256) at a time
+          part = __reduce_add_sync(kFullMask, __popc(hits)) <= unsigned(kFlatRound) ? kFullMask : 0xffu;
+        }
+        uint32_t h = hits & part;
+        hits ^= h;
+        part <<= 8;
+        if (part == kFullMask << 8) part = 0u;  // all of them went
+        // places by a prefix sum of the lanes' counts
+        const int count = __popc(h);
+        int to = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(kFullMask, to, o);
+          if (lane >= o) to += v;
+        }
+        const int all = __shfl_sync(kFullMask, to, 31);
+        to += queued - count;
+        while (h) {
+          const int c = __ffs(h) - 1;
+          h &= h - 1u;
+          qu[to++] = unsigned(slot) | unsigned(c - lo) << 5;
+        }
+        queued += all;
+      } else {
+        // 3b. Flat: V steps of 32 candidates at a time. A run that begins inside
+        //     the step at `at` marks bit (excl - at).
         int si[V], rel[V];
         uint32_t sc[V], cc[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-          const unsigned d = my_begin - unsigned(base + 32 * v);
+          const unsigned d = my_begin - unsigned(at + 32 * v);
           const unsigned heads = __reduce_or_sync(kFullMask, d < 32u ? (1u << d) : 0u);
           si[v] = begun + __popc(heads & upto) - 1;
           begun += __popc(heads);
-          const int f = base + 32 * v + lane;
+          const int f = at + 32 * v + lane;
           const int2 r = sw.lookup[si[v]];
           const int jj = r.y + f;
           sc[v] = uint32_t(r.x);
           rel[v] = f < total ? jj - rec[si[v]].j : -1;
           cc[v] = f < total ? p.scode[jj] : 0u;
         }
+        at += 32 * V;
 #pragma unroll
         for (int v = 0; v < V; ++v) {
           const bool pass = rel[v] >= 0 && code_pass(sc[v], cc[v]);
@@ -634,17 +614,57 @@ stq_sweep_flat_kernel(const SweepParams p) {
           if (pass) qu[queued + __popc(pm & below)] = unsigned(si[v]) | unsigned(rel[v]) << 5;
           queued += __popc(pm);
         }
-        __syncwarp();
-        while (queued >= 32) {
-          check(32);
-          __syncwarp();
-        }
       }
-    }
-    if (queued) check(queued);
-    __syncwarp();  // the records are rewritten by the next 32 starts
+      __syncwarp();
+      more = at < stop || part != 0u;
+      // 4. The check of the last queued candidates, one per lane (idle lanes
+      //    take a queued one again).
+      while (queued >= 32 || (!more && queued > 0)) {
+        const int n = min(queued, 32);
+        const uint32_t e = qu[queued - 1 - (lane < n ? lane : 0)];
+        queued -= n;
+        const FlatStart &r = rec[e & 31u];
+        const int c = r.j + int(e >> 5);
+        const float4 b = p.yz[c];
+        const int4 bv = p.v[c];
+        const int4 kv = r.v;
+        const bool hit = lane < n && pair_hit(PosRec{r.yz, r.x, kv}, PosRec{b, p.x[c], bv}, p.typed);
+        if (COUNT) {
+          if (hit) atomicAdd(&sw.hits[e & 31u], 1);
+        } else {
+          const unsigned hm = __ballot_sync(kFullMask, hit);
+          if (hit) st[staged + __popc(hm & below)] = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
+          staged += __popc(hm);
+          if (!multi) {
+            wpairs += __popc(hm);
+          } else if (hm) {
+            const int kf = r.kf;
+            const int lead = __shfl_sync(kFullMask, kf >> 2, __ffs(hm) - 1);
+            if (__all_sync(kFullMask, !hit || (kf >> 2) == lead)) {
+              if (lead != wscene) {
+                if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
+                wscene = lead;
+                wpairs = 0;
+              }
+              wpairs += __popc(hm);
+            } else if (hit) {
+              atomicAdd(&p.scene_pairs[kf >> 2], 1ull);
+            }
+          }
+          if (staged > kFlatStage - 32) {
+            __syncwarp();
+            flush_staged(st, staged, lane, p);
+            staged = 0;
+          }
+        }
+        __syncwarp();
+      }
+    } while (more);
     if (COUNT) {
-      if (len > 0) p.box_counts[k - p.begin] = sw.hits[slot];
+      if (len > 0) {
+        if (LONG) atomicAdd(&p.box_counts[k - p.begin], sw.hits[slot]);
+        else p.box_counts[k - p.begin] = sw.hits[slot];
+      }
       __syncwarp();
     }
   }
@@ -653,83 +673,6 @@ stq_sweep_flat_kernel(const SweepParams p) {
   if (staged) flush_staged(st, staged, lane, p);
   if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
   if (lane == 0 && p.stats) atomicAdd(p.stats, tested);
-}
-
-// The warp pass over the runs the lane sweep handed over (runs longer than
-// SweepParams::run_cap, which would keep one lane or group busy long after the
-// others finished). One warp per run; each step tests 32 * U consecutive
-// candidates, lane l taking j + 32u + l. All pairs of a run belong to its start
-// box's scene.
-template <int U, bool COUNT>
-__global__ void __launch_bounds__(256)
-stq_long_run_kernel(const SweepParams p) {
-  constexpr int STAGE = 32 * (U + 1);
-  __shared__ int2 stage[COUNT ? 1 : 8][COUNT ? 1 : STAGE];
-  const int lane = threadIdx.x & 31;
-  const unsigned below = lanemask_lt();
-  int2 *st = stage[COUNT ? 0 : (threadIdx.x >> 5)];
-  const unsigned n_items = *p.long_items;
-  if (n_items == 0) return;
-  int staged = 0;
-  unsigned tested = 0;
-  while (true) {
-    unsigned item = 0;
-    if (lane == 0) item = atomicAdd(p.long_work, 1u);
-    item = __shfl_sync(kFullMask, item, 0);
-    if (item >= n_items) break;
-    const int2 it = p.long_list[item];
-    const int k = it.x;
-    int j = it.y;
-    const int jend = p.run_end[k];
-    const PosRec kr = load_pos(p, k);
-    const uint32_t code = code_start(p.scode[k]);
-    const int kf = p.flag[k];
-    unsigned run_hits = 0;  // warp-uniform (emit) or this lane's (count mode)
-    for (; j < jend; j += 32 * U) {
-      uint32_t cc[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) cc[u] = j + 32 * u + lane < jend ? p.scode[j + 32 * u + lane] : 0u;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int at = j + 32 * u + lane;
-        bool hit = false;
-        int2 pr = make_int2(0, 0);
-        if (at < jend) {
-          ++tested;
-          if (code_pass(code, cc[u])) {
-            const PosRec c = load_pos(p, at);
-            hit = pair_hit(kr, c, p.typed);
-            pr = make_int2(min(kr.v.w, c.v.w), max(kr.v.w, c.v.w));
-          }
-        }
-        if (COUNT) {
-          run_hits += hit ? 1u : 0u;
-        } else {
-          const unsigned hm = __ballot_sync(kFullMask, hit);
-          if (hit) st[staged + __popc(hm & below)] = pr;
-          staged += __popc(hm);
-          run_hits += unsigned(__popc(hm));
-        }
-      }
-      if (!COUNT && staged >= 32) {
-        __syncwarp();
-        flush_staged(st, staged, lane, p);
-        staged = 0;
-      }
-    }
-    if (COUNT) {
-      const unsigned total = __reduce_add_sync(kFullMask, run_hits);
-      if (lane == 0 && total) atomicAdd(&p.box_counts[k - p.begin], int(total));
-    } else if (lane == 0 && run_hits) {
-      atomicAdd(&p.scene_pairs[kf >> 2], (unsigned long long)run_hits);
-    }
-  }
-  if (!COUNT) {
-    __syncwarp();
-    if (staged) flush_staged(st, staged, lane, p);
-    const unsigned t = __reduce_add_sync(kFullMask, tested);
-    if (lane == 0 && p.stats) atomicAdd(p.stats, (unsigned long long)t);
-  }
 }
 
 // Resident blocks per SM of a sweep kernel, queried once per kernel and
@@ -820,11 +763,23 @@ cudaError_t launch_u(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
 // The flat shape's blocks are 128 or 256 threads.
 template <int BLOCK, int V, bool COUNT>
 cudaError_t launch_flat_block(cudaStream_t s, const SweepParams &p, int sms) {
-  constexpr auto kern = stq_sweep_flat_kernel<BLOCK, V, COUNT>;
+  constexpr auto kern = stq_sweep_flat_kernel<BLOCK, V, COUNT, false>;
   constexpr size_t smem = sizeof(FlatWarp) * (BLOCK / 32);
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   return launch_persistent(kern, BLOCK, s, p, sms, smem);
+}
+
+// The warp pass: four blocks per SM (most sweeps hand nothing over, and the
+// blocks leave at once).
+template <bool COUNT>
+cudaError_t launch_long_runs(cudaStream_t s, const SweepParams &p, int sms) {
+  constexpr auto kern = stq_sweep_flat_kernel<256, 4, COUNT, true>;
+  constexpr size_t smem = sizeof(FlatWarp) * 8;
+  cudaError_t e = allow_smem<kern>(smem);
+  if (e != cudaSuccess) return e;
+  kern<<<unsigned(sms * 4), 256, smem, s>>>(p);
+  return cudaGetLastError();
 }
 
 template <int V>
@@ -927,13 +882,6 @@ brute_force_kernel(const stq_aabb *__restrict__ boxes, int64_t n,
 
 }  // namespace
 
-static cudaError_t launch_long_runs(cudaStream_t s, const SweepParams &p, bool count_mode, int num_sms) {
-  if (!p.run_cap) return cudaSuccess;
-  if (count_mode) stq_long_run_kernel<4, true><<<unsigned(num_sms * 2), 256, 0, s>>>(p);
-  else stq_long_run_kernel<4, false><<<unsigned(num_sms * 2), 256, 0, s>>>(p);
-  return cudaGetLastError();
-}
-
 static cudaError_t launch_sweep_lanes(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
                                       bool count_mode, int num_sms);
 
@@ -942,7 +890,8 @@ cudaError_t launch_sweep(cudaStream_t s, const SweepParams &p, const SweepTuning
   if (p.end <= p.begin) return cudaSuccess;
   cudaError_t e = launch_sweep_lanes(s, p, t, count_mode, num_sms);
   if (e != cudaSuccess) return e;
-  return launch_long_runs(s, p, count_mode, num_sms);
+  if (!p.run_cap) return cudaSuccess;
+  return count_mode ? launch_long_runs<true>(s, p, num_sms) : launch_long_runs<false>(s, p, num_sms);
 }
 
 static cudaError_t launch_sweep_lanes(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
