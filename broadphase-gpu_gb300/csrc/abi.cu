@@ -107,7 +107,7 @@ int read_header(stq_context *ctx, const BatchHeader *src) {
 int64_t tiles_for(const int64_t *box_off, int S) {
   int64_t t = 0;
   const int size = tile_boxes(box_off[S]);
-  for (int s = 0; s < S; ++s) t += (box_off[s + 1] - box_off[s] + size - 1) / size;
+  for (int s = 0; s < S; ++s) t += std::max<int64_t>((box_off[s + 1] - box_off[s] + size - 1) / size, 1);
   return t;
 }
 
@@ -130,7 +130,9 @@ int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap) {
   STQ_CUDA(ctx, ctx->cell_base.ensure(sizeof(unsigned) * size_t(scene_cap + 1)), "allocate cell bases");
   STQ_CUDA(ctx, ctx->scene_pairs.ensure(sizeof(unsigned long long) * size_t(scene_cap)),
            "allocate scene pair counters");
-  STQ_CUDA(ctx, ctx->emit_status.ensure(sizeof(unsigned long long) * size_t(tile_cap)), "allocate emit status");
+  STQ_CUDA(ctx, ctx->tile_reps.ensure(sizeof(unsigned long long) * kGridLevels * size_t(tile_cap)),
+           "allocate tile replica counts");
+  STQ_CUDA(ctx, ctx->tile_off.ensure(sizeof(uint32_t) * size_t(tile_cap)), "allocate tile offsets");
   if (scene_cap > ctx->h_scene_pairs_cap) {
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     ctx->h_scene_pairs = nullptr;
@@ -165,18 +167,30 @@ void fill_staging(stq_context *ctx, const int64_t *box_off, int S, const int *ax
     in[s].axis_mode = axes ? axes[s] : axis;
     in[s].cells_opt = int(ctx->options[STQ_OPT_CELLS]);
     in[s].cell_scale = ctx->cell_scale;
-    in[s].pad = 0;
+    in[s].tiles = 0;  // counted below
+    for (int k = 0; k < 3; ++k) {
+      in[s].s1[k] = in[s].s2[k] = 0.0;
+      in[s].lo_key[k] = 0xffffffffu;
+      in[s].hi_key[k] = 0u;
+    }
+    in[s].inverted = 0;
+    in[s].done = 0;
+    for (int l = 0; l < kGridLevels; ++l) in[s].level_reps[l] = 0;
   }
   TileRec *tr = host_at<TileRec>(ctx, L.tiles);
   int t = 0;
   const int size = tile_boxes(box_off[S]);
-  for (int s = 0; s < S; ++s)
-    for (int64_t b = box_off[s]; b < box_off[s + 1]; b += size) {
+  for (int s = 0; s < S; ++s) {
+    int64_t b = box_off[s];
+    do {  // an empty scene has one tile, whose block sets up its grid
       tr[t].begin = b;
       tr[t].count = int(std::min<int64_t>(size, box_off[s + 1] - b));
       tr[t].scene = s;
+      ++in[s].tiles;
       ++t;
-    }
+      b += size;
+    } while (b < box_off[s + 1]);
+  }
   h->n_tiles = t;
 }
 
@@ -200,7 +214,8 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
   b.hdr = dev_hdr(ctx);
   b.box_cells = ctx->box_cells.as<uint2>();
   b.box_q = ctx->box_q.as<uint32_t>();
-  b.emit_status = ctx->emit_status.as<unsigned long long>();
+  b.tile_reps = ctx->tile_reps.as<unsigned long long>();
+  b.tile_off = ctx->tile_off.as<uint32_t>();
   for (int k = 0; k < 2; ++k) {
     b.keys[k] = ctx->keys[k].as<uint32_t>();
     b.vals[k] = ctx->vals[k].as<uint32_t>();
@@ -255,11 +270,10 @@ int bits_for(int64_t v) {
 int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap) {
   stage_begin(ctx, kAxis);
   STQ_CUDA(ctx, launch_batch_stats(ctx->stream, b), "launch batch statistics");
-  STQ_CUDA(ctx, launch_batch_policy(ctx->stream, b), "launch batch policy");
   stage_end(ctx, kAxis);
   stage_begin(ctx, kKeys);
   STQ_CUDA(ctx, launch_batch_box_keys(ctx->stream, b, rep_cap, seg_cap), "launch box keys");
-  ctx->launches += 5;  // reset, statistics, policy, box keys, choose
+  ctx->launches += 2;
   return STQ_OK;
 }
 
@@ -651,8 +665,7 @@ int stq_select_axis(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int *a
   STQ_TRY(upload_staging(ctx));
   BatchBuffers b = batch_buffers(ctx, d_boxes);
   STQ_CUDA(ctx, launch_batch_stats(ctx->stream, b), "launch statistics");
-  STQ_CUDA(ctx, launch_batch_policy(ctx->stream, b), "launch policy");
-  ctx->launches += 3;
+  ctx->launches += 1;
   STQ_TRY(read_header(ctx));
   *axis_out = ctx->h_hdr->axis;
   return STQ_OK;

@@ -28,7 +28,7 @@ namespace {
 constexpr int kBlock = 256;
 constexpr int kHistBias = 40;  // extent bucket = binary exponent + 40
 constexpr int kSampleBoxes = 1024;
-constexpr int kSampleMins = 512;  // of these, for the sweep-axis code segments
+constexpr int kSampleMins = 256;  // of these, for the sweep-axis code segments
 
 __device__ __forceinline__ void axes_bc(int a, int &b, int &c) {
   b = a == 0 ? 1 : 0;
@@ -57,45 +57,201 @@ __device__ void block_sums(const T (&v)[K], T (&out)[K], T (*red)[K]) {
   }
 }
 
-// ---- 0. reset the per-scene accumulators ------------------------------------------
-__global__ void __launch_bounds__(kBlock)
-batch_reset_kernel(SceneRecord *scenes, const SceneInput *__restrict__ inputs,
-                   unsigned long long *scene_pairs, BatchHeader *hdr, unsigned long long *emit_status) {
-  const int S = hdr->n_scenes;
-  for (int t = blockIdx.x * kBlock + threadIdx.x; t < hdr->n_tiles; t += gridDim.x * kBlock) emit_status[t] = 0ull;
-  for (int s = blockIdx.x * kBlock + threadIdx.x; s < S; s += gridDim.x * kBlock) {
-    SceneRecord &r = scenes[s];
-    r.axis_mode = inputs[s].axis_mode;
-    r.cells_opt = inputs[s].cells_opt;
-    r.cell_scale = inputs[s].cell_scale;
-    scene_pairs[s] = 0ull;
-    for (int k = 0; k < 3; ++k) {
-      r.s1[k] = 0.0;
-      r.s2[k] = 0.0;
-      r.lo_key[k] = 0xffffffffu;
-      r.hi_key[k] = 0u;
+// Exclusive scan of one value per thread of the block; *total in every thread.
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *total, uint32_t *scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFullMask, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();  // scratch may be in use
+  if (lane == 31) scratch[warp] = x;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kBlock / 32; ++w) {
+    before += w < warp ? scratch[w] : 0u;
+    all += scratch[w];
+  }
+  *total = all;
+  return before + x - v;
+}
+
+__device__ int grid_side(float L, float h) {
+  if (!(L > 0.f) || !(h > 0.f) || !isfinite(L)) return 1;
+  const float s = ceilf(L / h);
+  return s > float(kMaxGridSide) ? kMaxGridSide : (s < 1.f ? 1 : int(s));
+}
+
+__device__ __forceinline__ float inv_side(int n, float L) { return n > 1 ? float(n) / L : 0.f; }
+
+// ---- 2. policy of a scene, by the block that finished its statistics ---------------
+// Sweep axis of largest corner variance (x, then y, preferred on ties, as
+// src/simulation.cu:630-635) unless fixed; level-0 cell side = cell_scale x
+// median box extent (from a strided sample of the scene's boxes), at most
+// 2048 cells per axis and at most max(1, n / max(16, 8 x cell_scale)) cells.
+__device__ __forceinline__ void
+scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, const SceneInput &in, SceneRecord &r,
+             int scene, BatchHeader *hdr) {
+  // the accumulators were written by other blocks' atomics: read them from L2
+  uint32_t lo_key[3], hi_key[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) lo_key[k] = __ldcg(&in.lo_key[k]), hi_key[k] = __ldcg(&in.hi_key[k]);
+  const bool inverted = __ldcg(&in.inverted) != 0;
+  int axis = in.axis_mode;
+  if (axis < 0) {
+    __shared__ double var[3];
+    if (threadIdx.x < 3) {
+      const double m = n > 0 ? 2.0 * double(n) : 1.0;
+      const double mean = __ldcg(&in.s1[threadIdx.x]) / m;
+      var[threadIdx.x] = __ldcg(&in.s2[threadIdx.x]) - m * mean * mean;
     }
-    r.inverted = 0;
-    for (int l = 0; l < kGridLevels; ++l) r.level_reps[l] = 0ull;
+    __syncthreads();
+    axis = 0;
+    if (var[1] > var[axis]) axis = 1;
+    if (var[2] > var[axis]) axis = 2;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    hdr->flags = 0;
-    hdr->fault = 0;
-    hdr->emit_ticket = 0;
-    hdr->replicas = 0;
-    hdr->cells = 0;
-    hdr->lists = 0;
-    hdr->length = 0;
-    hdr->work = 0;
-    hdr->pairs = 0;
-    hdr->prefix = 0;
+  auto key_of = [&](const uint32_t (&k)[3], int a) { return a == 0 ? k[0] : (a == 1 ? k[1] : k[2]); };
+  int b, c;
+  axes_bc(axis, b, c);
+  __shared__ unsigned hist[2][64];
+  __shared__ __align__(16) float sample[kSampleMins];
+  __shared__ float sorted[kSampleMins];
+  __shared__ float median[2];
+  for (int i = threadIdx.x; i < 128; i += kBlock) (&hist[0][0])[i] = 0u;
+  static_assert(kSampleMins == kBlock, "one sampled minimum per thread");
+  sample[threadIdx.x] = INFINITY;
+  __syncthreads();
+  const bool automatic = in.cells_opt == 0 && !inverted && n > 1;
+  {
+    const long long step = n > kSampleBoxes ? n / kSampleBoxes : 1;
+    // every fourth sample gives a minimum on the sweep axis (all of them in
+    // scenes of fewer boxes than minima wanted)
+    constexpr int kPer = kSampleBoxes / kBlock;
+    const int every = n > kSampleMins ? kPer : 1;
+    const int ax[2] = {b, c};
+    float mins[kPer], ext[kPer][2];  // all loads first
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const long long i = (long long)(u * kBlock + threadIdx.x) * step;
+      if (i < n) {
+        const stq_aabb &x = boxes[b0 + i];
+        mins[u] = x.min[axis];
+        for (int q = 0; q < 2; ++q) ext[u][q] = x.max[ax[q]] - x.min[ax[q]];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = u * kBlock + threadIdx.x;
+      if (i * step >= n) continue;
+      if (i % every == 0 && i / every < kSampleMins) sample[i / every] = mins[u];
+      if (!automatic) continue;
+      for (int q = 0; q < 2; ++q) {
+        int bucket = 0;
+        if (ext[u][q] > 0.f) {
+          int e;
+          frexpf(ext[u][q], &e);
+          bucket = min(63, max(1, e + kHistBias));
+        }
+        atomicAdd(&hist[q][bucket], 1u);
+      }
+    }
   }
+  __syncthreads();
+  // the sampled minima in order: each thread counts those before its own
+  // (missing ones are +inf, at the end)
+  {
+    const float mine = sample[threadIdx.x];
+    int rank = 0;
+#pragma unroll 8
+    for (int i = 0; i < kSampleMins; i += 4) {
+      const float4 v = *reinterpret_cast<const float4 *>(&sample[i]);
+      rank += (v.x < mine || (v.x == mine && i < int(threadIdx.x))) + (v.y < mine || (v.y == mine && i + 1 < int(threadIdx.x))) +
+              (v.z < mine || (v.z == mine && i + 2 < int(threadIdx.x))) + (v.w < mine || (v.w == mine && i + 3 < int(threadIdx.x)));
+    }
+    // (a NaN bound, rejected later, may leave a place empty)
+    sorted[threadIdx.x] = INFINITY;
+    __syncthreads();
+    sorted[min(rank, kSampleMins - 1)] = mine;
+  }
+  __syncthreads();
+  // median extents: one warp per axis, two buckets per lane
+  if (threadIdx.x < 64) {
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned h0 = hist[q][2 * lane], h1 = hist[q][2 * lane + 1];
+    unsigned run = h0 + h1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(kFullMask, run, o);
+      if (lane >= o) run += y;
+    }
+    const unsigned total = __shfl_sync(kFullMask, run, 31);
+    // first bucket whose running count reaches half
+    const unsigned m = __ballot_sync(kFullMask, total > 0 && 2 * run >= total);
+    if (lane == 0) median[q] = 0.f;
+    __syncwarp();
+    if (m && lane == __ffs(m) - 1) {
+      const int k = 2 * (run - h1) >= total ? 2 * lane : 2 * lane + 1;
+      median[q] = k == 0 ? 0.f : 0.75f * exp2f(float(k - kHistBias));
+    }
+  }
+  // sweep-axis code segments: their ends are quantiles of the sample, the first
+  // and the last reach to the scene's bounds
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + kSplits) {
+    const int i = threadIdx.x - 64;
+    const int m = int(n < kSampleMins ? (n > 0 ? n : 1) : kSampleMins);
+    const float lo = key_float(key_of(lo_key, axis)), hi = key_float(key_of(hi_key, axis));
+    const float s0 = i == 0 && isfinite(lo) ? lo : sorted[i * m / kSplits];
+    const float s1 = i == kSplits - 1 ? (isfinite(hi) ? hi : sorted[m - 1]) : sorted[(i + 1) * m / kSplits];
+    const float w = s1 - s0;
+    r.split[i] = s0;
+    r.split_inv[i] = w > 0.f && isfinite(w) ? float(kSplitSteps) / w : 0.f;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const float lob = key_float(key_of(lo_key, b)), hib = key_float(key_of(hi_key, b));
+  const float loc = key_float(key_of(lo_key, c)), hic = key_float(key_of(hi_key, c));
+  const float Lb = hib - lob, Lc = hic - loc;
+  int nb = 1, nc = 1;
+  if (in.cells_opt > 1 && !inverted && n > 1) {
+    nb = nc = in.cells_opt;
+  } else if (automatic) {
+    float w[2] = {median[0], median[1]};
+    if (!(w[0] > 0.f)) w[0] = Lb / 1024.f;
+    if (!(w[1] > 0.f)) w[1] = Lc / 1024.f;
+    nb = grid_side(Lb, in.cell_scale * w[0]);
+    nc = grid_side(Lc, in.cell_scale * w[1]);
+    // at least max(16, 8 * scale) boxes per cell on average: dense scenes of
+    // small boxes would otherwise be cut into lists of a few boxes, and their
+    // prepare would outweigh the sweep (the buffers are sized for n / 16 cells)
+    const long long per_cell = max(16ll, (long long)(8.f * in.cell_scale));
+    const long long max_cells = max(1ll, min(1ll << 20, n / per_cell));
+    while ((long long)nb * nc > max_cells) {
+      if (nb >= nc) nb = (nb + 1) / 2;
+      else nc = (nc + 1) / 2;
+    }
+  }
+  if (!(Lb > 0.f) || !isfinite(Lb)) nb = 1;
+  if (!(Lc > 0.f) || !isfinite(Lc)) nc = 1;
+  GridParams &g = r.grid;
+  g.axis = axis;
+  g.ob = lob;
+  g.oc = loc;
+  g.Lb = Lb;
+  g.Lc = Lc;
+  g.ib = inv_side(nb, Lb);
+  g.ic = inv_side(nc, Lc);
+  g.nb0 = g.ib == 0.f ? 1 : nb;
+  g.nc0 = g.ic == 0.f ? 1 : nc;
+  if (scene == 0) hdr->axis = axis;
 }
 
 // ---- 1. statistics: one tile (one scene) per block ------------------------------
 __global__ void __launch_bounds__(kBlock)
 batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
-                   SceneRecord *scenes, BatchHeader *hdr) {
+                   const long long *__restrict__ box_off, SceneInput *inputs, SceneRecord *scenes, BatchHeader *hdr) {
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
   // moments about the tile's first box centre, in fp32 per thread (fp64 is
@@ -103,7 +259,7 @@ batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict
   float c[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float m = 0.5f * (boxes[t.begin].min[k] + boxes[t.begin].max[k]);
+    const float m = t.count > 0 ? 0.5f * (boxes[t.begin].min[k] + boxes[t.begin].max[k]) : 0.f;
     c[k] = isfinite(m) ? m : 0.f;
   }
   float s1[3] = {0.f, 0.f, 0.f}, s2[3] = {0.f, 0.f, 0.f};
@@ -154,180 +310,44 @@ batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict
     wflag[warp] = fl;
   }
   __syncthreads();
-  if (warp != 0) return;
-  SceneRecord &r = scenes[t.scene];
-  double tot = 0.0;  // lane k < 6: moment k of the block
-  uint32_t key = lane < 3 ? 0xffffffffu : 0u;  // lanes 0-2 minima, 3-5 maxima
-  int flags = 0;
-  if (lane < 6) {
-    for (int w = 0; w < kWarps; ++w) {
-      tot += double(wsum[lane][w]);
-      key = lane < 3 ? min(key, wkey[lane][w]) : max(key, wkey[lane][w]);
-      flags |= wflag[w];
-    }
-  }
-  // sum(l + h) = S1 + 2 n c; sum(l^2 + h^2) = S2 + 2 c S1 + 2 n c^2
-  const double a1 = __shfl_sync(kFullMask, tot, lane < 3 ? lane : lane - 3);
-  if (lane < 6) {
-    const int k = lane < 3 ? lane : lane - 3;
-    const double ck = k == 0 ? c[0] : (k == 1 ? c[1] : c[2]), n = double(t.count);
-    if (lane < 3) {
-      atomicAdd(&r.s1[k], tot + 2.0 * n * ck);
-      atomicMin(&r.lo_key[k], key);
-    } else {
-      atomicAdd(&r.s2[k], tot + 2.0 * ck * a1 + 2.0 * n * ck * ck);
-      atomicMax(&r.hi_key[k], key);
-    }
-  }
-  if (lane == 0 && (flags & 1)) atomicOr(&r.inverted, 1);
-  if (lane == 0 && (flags & 2)) atomicOr(&hdr->flags, kFlagNaN);
-}
-
-__device__ int grid_side(float L, float h) {
-  if (!(L > 0.f) || !(h > 0.f) || !isfinite(L)) return 1;
-  const float s = ceilf(L / h);
-  return s > float(kMaxGridSide) ? kMaxGridSide : (s < 1.f ? 1 : int(s));
-}
-
-__device__ __forceinline__ float inv_side(int n, float L) { return n > 1 ? float(n) / L : 0.f; }
-
-// ---- 2. policy: one block per scene ---------------------------------------------
-// Sweep axis of largest corner variance (x, then y, preferred on ties, as
-// src/simulation.cu:630-635) unless fixed; level-0 cell side = cell_scale x
-// median box extent (from a strided sample of the scene's boxes), at most
-// 2048 cells per axis and at most max(1, n / max(16, 8 x cell_scale)) cells.
-__global__ void __launch_bounds__(kBlock)
-batch_policy_kernel(const stq_aabb *__restrict__ boxes, const long long *__restrict__ box_off,
-                    SceneRecord *scenes, BatchHeader *hdr) {
-  const int s = blockIdx.x;
-  if (s >= hdr->n_scenes) return;
-  SceneRecord &r = scenes[s];
-  const long long b0 = box_off[s], n = box_off[s + 1] - b0;
-  int axis = r.axis_mode;
-  if (axis < 0) {
-    double var[3];
-    const double m = n > 0 ? 2.0 * double(n) : 1.0;
-    for (int k = 0; k < 3; ++k) {
-      const double mean = r.s1[k] / m;
-      var[k] = r.s2[k] - m * mean * mean;
-    }
-    axis = 0;
-    if (var[1] > var[axis]) axis = 1;
-    if (var[2] > var[axis]) axis = 2;
-  }
-  int b, c;
-  axes_bc(axis, b, c);
-  __shared__ unsigned hist[2][64];
-  __shared__ float sample[kSampleMins];
-  __shared__ float median[2];
-  for (int i = threadIdx.x; i < 128; i += kBlock) (&hist[0][0])[i] = 0u;
-  for (int i = threadIdx.x; i < kSampleMins; i += kBlock) sample[i] = INFINITY;
-  __syncthreads();
-  const bool automatic = r.cells_opt == 0 && !r.inverted && n > 1;
-  {
-    const long long step = n > kSampleBoxes ? n / kSampleBoxes : 1;
-    // every second sample gives a minimum on the sweep axis (all of them in
-    // scenes of fewer boxes than minima wanted)
-    const int every = n > kSampleMins ? kSampleBoxes / kSampleMins : 1;
-    for (long long i = threadIdx.x; i < kSampleBoxes && i * step < n; i += kBlock) {
-      const stq_aabb &x = boxes[b0 + i * step];
-      if (i % every == 0 && i / every < kSampleMins) sample[i / every] = x.min[axis];
-      if (!automatic) continue;
-      const int ax[2] = {b, c};
-      for (int q = 0; q < 2; ++q) {
-        const float ext = x.max[ax[q]] - x.min[ax[q]];
-        int bucket = 0;
-        if (ext > 0.f) {
-          int e;
-          frexpf(ext, &e);
-          bucket = min(63, max(1, e + kHistBias));
-        }
-        atomicAdd(&hist[q][bucket], 1u);
+  SceneInput &r = inputs[t.scene];
+  __shared__ bool last;
+  if (warp == 0) {
+    double tot = 0.0;  // lane k < 6: moment k of the block
+    uint32_t key = lane < 3 ? 0xffffffffu : 0u;  // lanes 0-2 minima, 3-5 maxima
+    int flags = 0;
+    if (lane < 6) {
+      for (int w = 0; w < kWarps; ++w) {
+        tot += double(wsum[lane][w]);
+        key = lane < 3 ? min(key, wkey[lane][w]) : max(key, wkey[lane][w]);
+        flags |= wflag[w];
       }
     }
-  }
-  // the sampled minima in order (bitonic; missing ones are +inf, at the end)
-  static_assert(kSampleMins == 2 * kBlock, "one comparison per thread and step");
-  for (int size = 2; size <= kSampleMins; size <<= 1)
-    for (int d = size >> 1; d > 0; d >>= 1) {
-      __syncthreads();
-      const int i = 2 * int(threadIdx.x) - (int(threadIdx.x) & (d - 1)), j = i + d;
-      const float x = sample[i], y = sample[j];
-      if ((x > y) == ((i & size) == 0)) {
-        sample[i] = y;
-        sample[j] = x;
+    // sum(l + h) = S1 + 2 n c; sum(l^2 + h^2) = S2 + 2 c S1 + 2 n c^2
+    const double a1 = __shfl_sync(kFullMask, tot, lane < 3 ? lane : lane - 3);
+    if (lane < 6) {
+      const int k = lane < 3 ? lane : lane - 3;
+      const double ck = k == 0 ? c[0] : (k == 1 ? c[1] : c[2]), n = double(t.count);
+      if (lane < 3) {
+        atomicAdd(&r.s1[k], tot + 2.0 * n * ck);
+        atomicMin(&r.lo_key[k], key);
+      } else {
+        atomicAdd(&r.s2[k], tot + 2.0 * ck * a1 + 2.0 * n * ck * ck);
+        atomicMax(&r.hi_key[k], key);
       }
     }
-  __syncthreads();
-  // median extents: one warp per axis, two buckets per lane
-  if (threadIdx.x < 64) {
-    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned h0 = hist[q][2 * lane], h1 = hist[q][2 * lane + 1];
-    unsigned run = h0 + h1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(kFullMask, run, o);
-      if (lane >= o) run += y;
-    }
-    const unsigned total = __shfl_sync(kFullMask, run, 31);
-    // first bucket whose running count reaches half
-    const unsigned m = __ballot_sync(kFullMask, total > 0 && 2 * run >= total);
-    if (lane == 0) median[q] = 0.f;
+    if (lane == 0 && (flags & 1)) atomicOr(&r.inverted, 1);
+    if (lane == 0 && (flags & 2)) atomicOr(&hdr->flags, kFlagNaN);
+    // the block whose tile is the scene's last goes on to its policy
+    __threadfence();
     __syncwarp();
-    if (m && lane == __ffs(m) - 1) {
-      const int k = 2 * (run - h1) >= total ? 2 * lane : 2 * lane + 1;
-      median[q] = k == 0 ? 0.f : 0.75f * exp2f(float(k - kHistBias));
-    }
-  }
-  // sweep-axis code segments: their ends are quantiles of the sample, the first
-  // and the last reach to the scene's bounds
-  if (threadIdx.x >= 64 && threadIdx.x < 64 + kSplits) {
-    const int i = threadIdx.x - 64;
-    const int m = int(n < kSampleMins ? (n > 0 ? n : 1) : kSampleMins);
-    const float lo = key_float(r.lo_key[axis]), hi = key_float(r.hi_key[axis]);
-    const float s0 = i == 0 && isfinite(lo) ? lo : sample[i * m / kSplits];
-    const float s1 = i == kSplits - 1 ? (isfinite(hi) ? hi : sample[m - 1]) : sample[(i + 1) * m / kSplits];
-    const float w = s1 - s0;
-    r.split[i] = s0;
-    r.split_inv[i] = w > 0.f && isfinite(w) ? float(kSplitSteps) / w : 0.f;
+    if (lane == 0) last = atomicAdd(&r.done, 1u) + 1u == unsigned(r.tiles);
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  const float lob = key_float(r.lo_key[b]), hib = key_float(r.hi_key[b]);
-  const float loc = key_float(r.lo_key[c]), hic = key_float(r.hi_key[c]);
-  const float Lb = hib - lob, Lc = hic - loc;
-  int nb = 1, nc = 1;
-  if (r.cells_opt > 1 && !r.inverted && n > 1) {
-    nb = nc = r.cells_opt;
-  } else if (automatic) {
-    float w[2] = {median[0], median[1]};
-    if (!(w[0] > 0.f)) w[0] = Lb / 1024.f;
-    if (!(w[1] > 0.f)) w[1] = Lc / 1024.f;
-    nb = grid_side(Lb, r.cell_scale * w[0]);
-    nc = grid_side(Lc, r.cell_scale * w[1]);
-    // at least max(16, 8 * scale) boxes per cell on average: dense scenes of
-    // small boxes would otherwise be cut into lists of a few boxes, and their
-    // prepare would outweigh the sweep (the buffers are sized for n / 16 cells)
-    const long long per_cell = max(16ll, (long long)(8.f * r.cell_scale));
-    const long long max_cells = max(1ll, min(1ll << 20, n / per_cell));
-    while ((long long)nb * nc > max_cells) {
-      if (nb >= nc) nb = (nb + 1) / 2;
-      else nc = (nc + 1) / 2;
-    }
-  }
-  if (!(Lb > 0.f) || !isfinite(Lb)) nb = 1;
-  if (!(Lc > 0.f) || !isfinite(Lc)) nc = 1;
-  GridParams &g = r.grid;
-  g.axis = axis;
-  g.ob = lob;
-  g.oc = loc;
-  g.Lb = Lb;
-  g.Lc = Lc;
-  g.ib = inv_side(nb, Lb);
-  g.ic = inv_side(nc, Lc);
-  g.nb0 = g.ib == 0.f ? 1 : nb;
-  g.nc0 = g.ic == 0.f ? 1 : nc;
-  if (s == 0) hdr->axis = axis;
+  if (!last) return;
+  __threadfence();
+  const long long first = box_off[t.scene];
+  scene_policy(boxes, first, box_off[t.scene + 1] - first, r, scenes[t.scene], t.scene, hdr);
 }
 
 struct Range {
@@ -346,32 +366,40 @@ __device__ __forceinline__ Range cell_range(const stq_aabb &x, int a, float ob, 
   return r;
 }
 
-// ---- 4. choose the finest level within the replica budget; cell bases ----------
-__global__ void __launch_bounds__(1024)
-batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
-                    unsigned int *cell_base, BatchHeader *hdr, long long rep_cap, long long seg_cap) {
-  __shared__ unsigned int warp_tot[32];
-  __shared__ unsigned int carry;
+// ---- 4. the finest level within the replica budget, cell bases, key layout, by the
+// block that finished the box keys
+__device__ __forceinline__ void
+choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__ tiles, const SceneInput *inputs,
+              SceneRecord *scenes, unsigned int *cell_base, const unsigned long long *tile_reps, uint32_t *tile_off,
+              BatchHeader *hdr, long long rep_cap, long long seg_cap) {
+  __shared__ uint32_t scratch[kBlock / 32];
   __shared__ unsigned long long reps;
-  if (threadIdx.x == 0) carry = 0, reps = 0;
+  if (threadIdx.x == 0) reps = 0;
   __syncthreads();
   const int S = hdr->n_scenes;
   const long long budget = hdr->budget;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int base = 0; base < S; base += 1024) {
+  unsigned int carry = 0;
+  for (int base = 0; base < S; base += kBlock) {
     const int s = base + threadIdx.x;
     unsigned int cells = 0;
     if (s < S) {
       SceneRecord &r = scenes[s];
+      const SceneInput &in = inputs[s];
+      unsigned long long level_reps[kGridLevels];
+#pragma unroll
+      for (int l = 0; l < kGridLevels; ++l) level_reps[l] = __ldcg(&in.level_reps[l]);
       const long long n = box_off[s + 1] - box_off[s];
       int level = kCoordBits;  // none fits: every coordinate shifts to cell 0
-      if (r.cells_opt > 1) {
+      unsigned long long used = (unsigned long long)n;  // one cell: each box once
+      if (in.cells_opt > 1) {
         level = 0;  // a requested grid is kept as is
+        used = level_reps[0];
       } else {
-        for (int l = 0; l < kGridLevels; ++l)
-          if ((long long)r.level_reps[l] <= budget * n) {
+#pragma unroll
+        for (int l = kGridLevels - 1; l >= 0; --l)
+          if ((long long)level_reps[l] <= budget * n) {
             level = l;
-            break;
+            used = level_reps[l];
           }
       }
       GridParams &g = r.grid;
@@ -379,7 +407,7 @@ batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
       g.nb = ((g.nb0 - 1) >> level) + 1;
       g.nc = ((g.nc0 - 1) >> level) + 1;
       g.ncells = g.nb * g.nc;
-      atomicAdd(&reps, level < kGridLevels ? r.level_reps[level] : (unsigned long long)n);
+      atomicAdd(&reps, used);
       // 64 code steps per cell of the chosen level; a cell is 2^level level-0
       // cells, of which there are nb0 over Lb (one cell: the whole extent)
       const float steps = 64.f / float(1 << level);
@@ -387,28 +415,26 @@ batch_choose_kernel(const long long *__restrict__ box_off, SceneRecord *scenes,
       g.sc = g.Lc > 0.f && isfinite(g.Lc) ? (level >= kCoordBits ? 64.f : steps * float(g.nc0)) / g.Lc : 0.f;
       cells = unsigned(g.ncells);
     }
-    // block exclusive scan of the cell counts
-    unsigned int x = cells;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned int y = __shfl_up_sync(kFullMask, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      unsigned int w = warp_tot[lane];
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int y = __shfl_up_sync(kFullMask, w, o);
-        if (lane >= o) w += y;
-      }
-      warp_tot[lane] = w;
-    }
-    __syncthreads();
-    const unsigned int excl = carry + (warp > 0 ? warp_tot[warp - 1] : 0u) + x - cells;
+    uint32_t total;
+    const unsigned int excl = carry + block_exclusive(cells, &total, scratch);
     if (s < S) cell_base[s] = excl;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += warp_tot[31];
-    __syncthreads();
+    carry += total;
+  }
+  __syncthreads();
+  // every tile's first replica, at its scene's level
+  const int n_tiles = hdr->n_tiles;
+  uint32_t at = 0;
+  for (int base = 0; base < n_tiles; base += kBlock) {
+    const int t = base + threadIdx.x;
+    uint32_t n = 0;
+    if (t < n_tiles) {
+      const int level = scenes[tiles[t].scene].grid.shift;
+      n = level < kGridLevels ? uint32_t(__ldcg(&tile_reps[size_t(t) * kGridLevels + level])) : uint32_t(tiles[t].count);
+    }
+    uint32_t total;
+    const uint32_t off = at + block_exclusive(n, &total, scratch);
+    if (t < n_tiles) tile_off[t] = off;
+    at += total;
   }
   if (threadIdx.x == 0) {
     cell_base[S] = carry;
@@ -451,11 +477,13 @@ __device__ __forceinline__ uint32_t axis_code(float v, const float *split, const
 
 __global__ void __launch_bounds__(kBlock)
 batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
-                      SceneRecord *scenes, const BatchHeader *hdr,
+                      const long long *__restrict__ box_off, SceneInput *inputs,
+                      SceneRecord *scenes, unsigned int *cell_base, unsigned long long *tile_reps, uint32_t *tile_off,
+                      BatchHeader *hdr, long long rep_cap, long long seg_cap,
                       uint2 *__restrict__ box_cells, uint32_t *__restrict__ box_q) {
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
-  SceneRecord &r = scenes[t.scene];
+  const SceneRecord &r = scenes[t.scene];
   const GridParams g = r.grid;
   __shared__ float split[kSplits], inv[kSplits];
   if (threadIdx.x < kSplits) {
@@ -487,19 +515,26 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
 #pragma unroll
   for (int l = 0; l < kGridLevels; ++l) wide[l] = reps[l];
   block_sums(wide, tot, red);
-  if (threadIdx.x == 0)
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
 #pragma unroll
-    for (int l = 0; l < kGridLevels; ++l) atomicAdd(&r.level_reps[l], tot[l]);
+    for (int l = 0; l < kGridLevels; ++l) {
+      if (tot[l]) atomicAdd(&inputs[t.scene].level_reps[l], tot[l]);
+      tile_reps[size_t(blockIdx.x) * kGridLevels + l] = tot[l];
+    }
+    // the block whose tile is the batch's last goes on to the levels
+    __threadfence();
+    last = atomicAdd(&hdr->keys_done, 1u) + 1u == unsigned(hdr->n_tiles);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  choose_levels(box_off, tiles, inputs, scenes, cell_base, tile_reps, tile_off, hdr, rep_cap, seg_cap);
 }
 
 // ---- 5. replica keys in box order: (list id << key_bits) | sweep-axis code, where
-// the list is (global cell, box type). A block takes a tile (one scene), counts
-// its replicas at the chosen level, publishes the count, and finds its first
-// output position by looking back over the tiles before it (which hold their
-// tickets, so they are running; the wait is bounded all the same). Status word:
-// 1 << 62 | count, or 2 << 62 | sum up to and with the tile.
-constexpr int kEmitSpins = 1 << 20;
-
+// the list is (global cell, box type). One tile (one scene) per block, from the
+// tile's first replica on.
 __device__ __forceinline__ uint32_t cells_count(uint2 r, int shift) {
   return (((r.x >> 11 & 2047u) >> shift) - ((r.x & 2047u) >> shift) + 1u) *
          (((r.y >> 11 & 2047u) >> shift) - ((r.y & 2047u) >> shift) + 1u);
@@ -507,111 +542,62 @@ __device__ __forceinline__ uint32_t cells_count(uint2 r, int shift) {
 
 __global__ void __launch_bounds__(kBlock)
 batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restrict__ box_q,
-                  const TileRec *__restrict__ tiles, const SceneRecord *__restrict__ scenes,
-                  const unsigned int *__restrict__ cell_base, BatchHeader *hdr, unsigned long long *status,
-                  uint32_t *k0, uint32_t *k1, uint32_t *v0, uint32_t *v1) {
-  if (hdr->replicas == 0u) return;
-  const int n_tiles = hdr->n_tiles, key_bits = hdr->key_bits;
+                  const TileRec *__restrict__ tiles, const uint32_t *__restrict__ tile_off,
+                  const SceneRecord *__restrict__ scenes, const unsigned int *__restrict__ cell_base,
+                  const BatchHeader *hdr, uint32_t *k0, uint32_t *k1, uint32_t *v0, uint32_t *v1) {
+  if (hdr->replicas == 0u || int(blockIdx.x) >= hdr->n_tiles) return;
+  const int key_bits = hdr->key_bits;
   const bool second = hdr->passes & 1u;
   uint32_t *__restrict__ keys = second ? k1 : k0;
   uint32_t *__restrict__ vals = second ? v1 : v0;
   constexpr int kWarps = kBlock / 32;
   __shared__ uint32_t warp_count[kWarps];
-  __shared__ unsigned long long before;
-  __shared__ int ticket, gave_up;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  while (true) {
-    if (threadIdx.x == 0) {
-      ticket = int(atomicAdd(&hdr->emit_ticket, 1u));
-      gave_up = 0;
-    }
-    __syncthreads();
-    const int tile = ticket;
-    if (tile >= n_tiles) return;
-    const TileRec t = tiles[tile];
-    const GridParams &g = scenes[t.scene].grid;
-    const int sh = g.shift, nc = g.nc;
-    const unsigned cb0 = cell_base[t.scene];
-    // a warp takes consecutive boxes of the tile, 32 at a time
-    const int share = (t.count + kWarps * 32 - 1) / (kWarps * 32) * 32;
-    const int w0 = min(warp * share, t.count), w1 = min(w0 + share, t.count);
-    uint32_t mine = 0;
-    for (int i = w0 + lane; i < w1; i += 32) mine += cells_count(box_cells[t.begin + i], sh);
-    mine = __reduce_add_sync(kFullMask, mine);
-    if (lane == 0) warp_count[warp] = mine;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t total = 0;
+  const TileRec t = tiles[blockIdx.x];
+  const GridParams &g = scenes[t.scene].grid;
+  const int sh = g.shift, nc = g.nc;
+  const unsigned cb0 = cell_base[t.scene];
+  uint32_t o = tile_off[blockIdx.x];
+  // a warp takes consecutive boxes of the tile, 32 at a time
+  const int share = (t.count + kWarps * 32 - 1) / (kWarps * 32) * 32;
+  const int w0 = min(warp * share, t.count), w1 = min(w0 + share, t.count);
+  uint32_t mine = 0;
+#pragma unroll 4
+  for (int i = w0 + lane; i < w1; i += 32) mine += cells_count(box_cells[t.begin + i], sh);
+  mine = __reduce_add_sync(kFullMask, mine);
+  if (lane == 0) warp_count[warp] = mine;
+  __syncthreads();
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) total += warp_count[w];
-      volatile unsigned long long *st = status;
-      if (lane == 0) st[tile] = (tile == 0 ? 2ull : 1ull) << 62 | total;
-      // look back 32 tiles at a time
-      unsigned long long sum = 0;
-      int spins = 0;
-      for (int at = tile - 1; at >= 0;) {
-        const unsigned long long w = at - lane >= 0 ? st[at - lane] : 2ull << 62;
-        const unsigned empty = __ballot_sync(kFullMask, (w >> 62) == 0ull);
-        const unsigned full = __ballot_sync(kFullMask, (w >> 62) == 2ull);
-        const int stop = full ? __ffs(full) - 1 : 31;  // last lane to add
-        if (empty & (stop == 31 ? kFullMask : (2u << stop) - 1u)) {  // a tile before that is not ready
-          if (++spins > kEmitSpins) {
-            if (lane == 0) gave_up = 1;
-            break;
-          }
-          continue;
+  for (int w = 0; w < kWarps; ++w) o += w < warp ? warp_count[w] : 0u;
+#pragma unroll 2
+  for (int i = w0 + lane; i - lane < w1; i += 32) {
+    uint2 r = make_uint2(0u, 0u);
+    uint32_t n = 0, q = 0;
+    if (i < w1) {
+      r = box_cells[t.begin + i];
+      q = (box_q[t.begin + i] & 0xffffu) >> (kAxisCodeBits - key_bits);
+      n = cells_count(r, sh);
+    }
+    uint32_t x = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFullMask, x, d);
+      if (lane >= d) x += y;
+    }
+    uint32_t at = o + x - n;
+    o += __shfl_sync(kFullMask, x, 31);
+    if (i < w1) {
+      const unsigned b0 = (r.x & 2047u) >> sh, b1 = (r.x >> 11 & 2047u) >> sh;
+      const unsigned c0 = (r.y & 2047u) >> sh, c1 = (r.y >> 11 & 2047u) >> sh;
+      const unsigned type = r.x >> 22;
+      for (unsigned cb = b0; cb <= b1; ++cb)
+        for (unsigned cc = c0; cc <= c1; ++cc) {
+          const unsigned seg = (cb0 + cb * unsigned(nc) + cc) * 3u + type;
+          keys[at] = seg << key_bits | q;
+          vals[at] = uint32_t(t.begin + i);
+          ++at;
         }
-        unsigned long long v = lane <= stop ? w & ~(3ull << 62) : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
-        sum += v;
-        if (full) break;
-        at -= 32;
-      }
-      if (lane == 0) {
-        if (tile > 0) st[tile] = 2ull << 62 | (sum + total);
-        before = sum;
-      }
     }
-    __syncthreads();
-    if (gave_up) {  // positions are not known: nothing is written
-      if (threadIdx.x == 0) hdr->fault = 1;
-      __syncthreads();
-      continue;
-    }
-    uint32_t o = uint32_t(before);
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) o += w < warp ? warp_count[w] : 0u;
-    for (int i = w0 + lane; i - lane < w1; i += 32) {
-      uint2 r = make_uint2(0u, 0u);
-      uint32_t n = 0, q = 0;
-      if (i < w1) {
-        r = box_cells[t.begin + i];
-        q = (box_q[t.begin + i] & 0xffffu) >> (kAxisCodeBits - key_bits);
-        n = cells_count(r, sh);
-      }
-      uint32_t x = n;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFullMask, x, d);
-        if (lane >= d) x += y;
-      }
-      uint32_t at = o + x - n;
-      o += __shfl_sync(kFullMask, x, 31);
-      if (i < w1) {
-        const unsigned b0 = (r.x & 2047u) >> sh, b1 = (r.x >> 11 & 2047u) >> sh;
-        const unsigned c0 = (r.y & 2047u) >> sh, c1 = (r.y >> 11 & 2047u) >> sh;
-        const unsigned type = r.x >> 22;
-        for (unsigned cb = b0; cb <= b1; ++cb)
-          for (unsigned cc = c0; cc <= c1; ++cc) {
-            const unsigned seg = (cb0 + cb * unsigned(nc) + cc) * 3u + type;
-            keys[at] = seg << key_bits | q;
-            vals[at] = uint32_t(t.begin + i);
-            ++at;
-          }
-      }
-    }
-    __syncthreads();  // warp_count, before and ticket are rewritten
   }
 }
 
@@ -635,26 +621,51 @@ list_offsets_kernel(const uint32_t *__restrict__ keys, BatchHeader *__restrict__
       scene.run_end[k] = int(k);
     }
   };
-  uint32_t mx = 0;
+  // A search goes through a sample of the list ids in shared memory first (ten of
+  // its steps) and then through the part of the keys that is left: a small scene
+  // has too few lists to hide the chain of loads of a whole search.
+  constexpr int kSample = 1024;
+  __shared__ uint32_t sample[kSample];
+  __shared__ uint32_t lows[kBlock];
+  const uint32_t every = R / kSample + 1;  // sample[i] is the list id at i * every
+  for (uint32_t i = threadIdx.x; i < uint32_t(kSample); i += kBlock)
+    sample[i] = uint64_t(i) * every < R ? keys[i * every] >> key_bits : 0xffffffffu;
+  __syncthreads();
   auto lower = [&](uint32_t s) {
-    uint32_t a = 0, e = R;
+    uint32_t a = 0, e = kSample;
     while (a < e) {
       const uint32_t mid = (a + e) >> 1;
-      if (keys[mid] >> key_bits < s) a = mid + 1;
+      if (sample[mid] < s) a = mid + 1;
       else e = mid;
     }
-    return a;
-  };
-  const uint32_t stride = gridDim.x * kBlock;
-  for (uint32_t s = blockIdx.x * kBlock + threadIdx.x; s <= nseg; s += stride) {
-    const uint32_t lo = s < nseg ? lower(s) : R;
-    seg_scan[s] = lo;
-    if (s < nseg) {
-      const uint32_t hi = lower(s + 1);
-      mx = max(mx, hi - lo);
-      empty(int64_t(hi) + s);
+    // sample[a - 1] < s <= sample[a]
+    uint32_t lo = a > 0 ? (a - 1) * every + 1 : 0u, hi = min(uint64_t(a) * every, uint64_t(R));
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (keys[mid] >> key_bits < s) lo = mid + 1;
+      else hi = mid;
     }
+    return lo;
+  };
+  uint32_t mx = 0;
+  // kBlock - 1 lists per block and step: a list's end is the next thread's start
+  constexpr uint32_t kLists = kBlock - 1;
+  for (uint32_t b = blockIdx.x * kLists; b <= nseg; b += gridDim.x * kLists) {
+    const uint32_t s = b + threadIdx.x;
+    const uint32_t lo = s < nseg ? lower(s) : R;
+    lows[threadIdx.x] = lo;
+    __syncthreads();
+    if (threadIdx.x < kLists && s <= nseg) {
+      seg_scan[s] = lo;
+      if (s < nseg) {
+        const uint32_t hi = lows[threadIdx.x + 1];
+        mx = max(mx, hi - lo);
+        empty(int64_t(hi) + s);
+      }
+    }
+    __syncthreads();
   }
+  const uint32_t stride = gridDim.x * kBlock;
   for (uint32_t t = blockIdx.x * kBlock + threadIdx.x; t < uint32_t(kSortedPad); t += stride)
     empty(int64_t(R) + nseg + t);
   mx = __reduce_max_sync(kFullMask, mx);
@@ -833,33 +844,27 @@ cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long l
 }
 
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b) {
-  batch_reset_kernel<<<blocks_for(b.scene_cap, 64), kBlock, 0, s>>>(b.scenes, b.inputs,
-                                                                      b.scene_pairs, b.hdr, b.emit_status);
-  batch_stats_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.scenes, b.hdr);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_batch_policy(cudaStream_t s, const BatchBuffers &b) {
-  batch_policy_kernel<<<unsigned(b.scene_cap), kBlock, 0, s>>>(b.boxes, b.box_off, b.scenes, b.hdr);
+  batch_stats_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.box_off, b.inputs, b.scenes, b.hdr);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap) {
-  batch_box_keys_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.scenes, b.hdr, b.box_cells, b.box_q);
-  batch_choose_kernel<<<1, 1024, 0, s>>>(b.box_off, b.scenes, b.cell_base, b.hdr, rep_cap, seg_cap);
+  batch_box_keys_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.box_off, b.inputs, b.scenes,
+                                                                b.cell_base, b.tile_reps, b.tile_off, b.hdr, rep_cap,
+                                                                seg_cap, b.box_cells, b.box_q);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b) {
-  batch_emit_kernel<<<wave_blocks((const void *)batch_emit_kernel, int64_t(b.tile_cap) * kBlock), kBlock, 0, s>>>(
-      b.box_cells, b.box_q, b.tiles, b.scenes, b.cell_base, b.hdr, b.emit_status, b.keys[0], b.keys[1], b.vals[0],
-      b.vals[1]);
+  batch_emit_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.box_cells, b.box_q, b.tiles, b.tile_off, b.scenes,
+                                                            b.cell_base, b.hdr, b.keys[0], b.keys[1], b.vals[0],
+                                                            b.vals[1]);
   return cudaGetLastError();
 }
 
 cudaError_t launch_list_offsets(cudaStream_t s, const uint32_t *keys, BatchHeader *hdr, uint32_t *seg_scan,
                                 int64_t seg_cap, const SortedScene &scene, int64_t slots_cap) {
-  list_offsets_kernel<<<blocks_for(seg_cap + 1), kBlock, 0, s>>>(keys, hdr, seg_scan, seg_cap, scene, slots_cap);
+  list_offsets_kernel<<<blocks_for((seg_cap + 1) / (kBlock - 1) * kBlock + kBlock), kBlock, 0, s>>>(keys, hdr, seg_scan, seg_cap, scene, slots_cap);
   return cudaGetLastError();
 }
 

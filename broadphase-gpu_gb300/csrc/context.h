@@ -76,7 +76,7 @@ struct stq_context {
   DevBuf in_dev;
   char *in_host = nullptr;
   size_t in_host_bytes = 0;
-  DevBuf scenes, cell_base, scene_pairs, box_cells, box_q, emit_status, keys[2], vals[2], sort_ws;
+  DevBuf scenes, cell_base, scene_pairs, box_cells, box_q, tile_reps, tile_off, keys[2], vals[2], sort_ws;
   DevBuf points;  // fp64 vertex positions rounded to float once (box builds)
   DevBuf yz, xx, vv, flag, scode, partner, run_end, box_counts, prefix_ws, pair_tmp;
   DevBuf long_list;  // runs handed from the lane sweep to the warp pass
@@ -126,7 +126,7 @@ struct stq_context {
 
   // every device buffer of the context
   std::vector<DevBuf *> buffers() {
-    return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &box_cells, &box_q, &emit_status, &keys[0], &keys[1],
+    return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &box_cells, &box_q, &tile_reps, &tile_off, &keys[0], &keys[1],
             &vals[0], &vals[1], &sort_ws, &yz, &xx, &vv, &flag, &scode, &partner, &run_end, &long_list, &seg_scan, &box_counts,
             &prefix_ws, &pair_tmp, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh, &aux, &window_pairs,
             &window_long_list, &window_cursors};

@@ -104,32 +104,26 @@ constexpr int kSplitSteps = 1024;
 constexpr int kAxisCodeBits = 16;
 static_assert(kSplits * kSplitSteps == 1 << kAxisCodeBits, "16-bit codes");
 
-// One scene of a batch: inputs written by the host, the rest computed on the
-// device by the prepare kernels.
+// One scene of a batch, as computed by the prepare kernels.
 struct SceneRecord {
-  // inputs
-  int axis_mode;        // -1: largest variance, else the axis
-  int cells_opt;        // 0 automatic, 1 no cells, k > 1 a k x k grid
-  float cell_scale;     // automatic cell side in median box extents
-  int pad0;
-  // statistics
-  double s1[3], s2[3];              // sum(min + max), sum(min^2 + max^2)
-  unsigned int lo_key[3], hi_key[3];  // order-preserving min / max bounds
   float split[kSplits];             // sweep-axis codes: lower ends of the segments
   float split_inv[kSplits];         // code steps per unit length in each
-  int inverted;                     // some box has min > max on an axis
-  int pad1;
-  unsigned long long level_reps[kGridLevels];  // replicas per grid level
-  // results
   GridParams grid;
 };
 
-// Per-scene inputs written by the host (copied into the records on reset).
+// Per-scene inputs, written by the host before every prepare with the
+// accumulators at their start values.
 struct SceneInput {
-  int axis_mode;
-  int cells_opt;
-  float cell_scale;
-  int pad;
+  int axis_mode;        // -1: largest variance, else the axis
+  int cells_opt;        // 0 automatic, 1 no cells, k > 1 a k x k grid
+  float cell_scale;     // automatic cell side in median box extents
+  int tiles;            // tiles of the scene
+  // accumulators
+  double s1[3], s2[3];                // sum(min + max), sum(min^2 + max^2)
+  unsigned int lo_key[3], hi_key[3];  // order-preserving min / max bounds
+  int inverted;                       // some box has min > max on an axis
+  unsigned int done;                  // tiles whose statistics are in
+  unsigned long long level_reps[kGridLevels];  // replicas per grid level
 };
 
 // Device-side header of a prepared batch: sizes read by every kernel, so a
@@ -155,7 +149,7 @@ struct BatchHeader {
   unsigned int lists;       // (cell, type) lists: 3 * cells
   int fault;                // a bounded wait between blocks ran out
   unsigned int passes;      // digits of the replica sort; its input is in buffer passes & 1
-  unsigned int emit_ticket; // next tile of the replica emit
+  unsigned int keys_done;   // tiles whose box keys and level counts are in
 };
 
 // A tile of at most kTileBoxes consecutive boxes of one scene (built by the
@@ -167,7 +161,7 @@ constexpr int64_t kSmallBatch = 152 * 4 * kSmallTile;
 constexpr int tile_boxes(int64_t n) { return n <= kSmallBatch ? kSmallTile : kTileBoxes; }
 struct TileRec {
   long long begin;  // first box of the tile
-  int count;        // boxes in the tile
+  int count;        // boxes in the tile (0: the one tile of an empty scene)
   int scene;        // scene of the tile
 };
 
@@ -270,7 +264,7 @@ struct BatchBuffers {
   const long long *box_off;     // n_scenes + 1 box offsets
   const TileRec *tiles;         // n_tiles entries
   int tile_cap;
-  const SceneInput *inputs;     // n_scenes entries
+  SceneInput *inputs;           // n_scenes entries
   unsigned long long *scene_pairs;  // n_scenes pair counters
   SceneRecord *scenes;
   unsigned int *cell_base;      // n_scenes + 1
@@ -278,7 +272,8 @@ struct BatchBuffers {
   uint2 *box_cells;             // per box: cell range and type
                                 // (b0 | b1 << 11 | type << 22, c0 | c1 << 11)
   uint32_t *box_q;              // per box: sweep-axis codes of its min | its max << 16
-  unsigned long long *emit_status;  // per tile: running replica counts of the emit
+  unsigned long long *tile_reps;  // per tile: replicas of each grid level
+  uint32_t *tile_off;           // per tile: first replica
   uint32_t *keys[2];            // replica keys: list id << key_bits | sweep-axis code
   uint32_t *vals[2];            // replica box indices
   uint32_t *seg_scan;           // first sorted replica of each segment (cell x type),
@@ -288,14 +283,12 @@ struct BatchBuffers {
   long long rep_cap;
   int scene_cap;
 };
-// reset and per-scene statistics (2 launches)
+// per-scene statistics; sweep axis, level-0 grid and sweep-axis codes (1 launch)
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b);
-// sweep axis and level-0 grid per scene (1 launch)
-cudaError_t launch_batch_policy(cudaStream_t s, const BatchBuffers &b);
 // level-0 cell ranges, sweep-axis codes and every level's replica count; then the
-// level within the replica budget, the cell bases and the key layout (2 launches).
-// Scenes that need more than rep_cap replicas or seg_cap lists are flagged and
-// left empty (no limit: -1).
+// level within the replica budget, the cell bases, the key layout and every
+// tile's first replica (1 launch). Scenes that need more than rep_cap replicas or
+// seg_cap lists are flagged and left empty (no limit: -1).
 cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap);
 // replicas in box order (1 launch)
 cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b);
