@@ -212,6 +212,7 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
   b.scenes = ctx->scenes.as<SceneRecord>();
   b.cell_base = ctx->cell_base.as<unsigned>();
   b.hdr = dev_hdr(ctx);
+  b.front = ctx->h_front;
   b.box_cells = ctx->box_cells.as<uint2>();
   b.box_q = ctx->box_q.as<uint32_t>();
   b.tile_reps = ctx->tile_reps.as<unsigned long long>();
@@ -267,12 +268,12 @@ int bits_for(int64_t v) {
   return b;
 }
 
-int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap) {
+int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap, int passes) {
   stage_begin(ctx, kAxis);
   STQ_CUDA(ctx, launch_batch_stats(ctx->stream, b), "launch batch statistics");
   stage_end(ctx, kAxis);
   stage_begin(ctx, kKeys);
-  STQ_CUDA(ctx, launch_batch_box_keys(ctx->stream, b, rep_cap, seg_cap), "launch box keys");
+  STQ_CUDA(ctx, launch_batch_box_keys(ctx->stream, b, rep_cap, seg_cap, passes), "launch box keys");
   ctx->launches += 2;
   return STQ_OK;
 }
@@ -283,7 +284,7 @@ int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replic
   stage_begin(ctx, kSort);
   const int64_t r = replicas >= 0 ? replicas : ctx->rep_cap;
   STQ_CUDA(ctx, radix_sort_u32(ctx->stream, b.keys, b.vals, r, ctx->sort_ws.ptr, &b.hdr->fault, &ctx->launches,
-                               replicas >= 0 ? nullptr : &b.hdr->replicas, &b.hdr->passes, passes >= 0 ? passes : 4),
+                               replicas >= 0 ? nullptr : &b.hdr->replicas, &b.hdr->passes, passes),
            "launch replica sort");
   stage_end(ctx, kSort);
   ctx->scene.yz = ctx->yz.as<float4>();
@@ -302,32 +303,81 @@ int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replic
   return STQ_OK;
 }
 
-// Prepares a batch with exact buffer sizes (one synchronisation after the
-// replica count). Leaves the batch header read back in ctx->h_hdr.
-int prepare_exact(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_off, int S,
-                  const int *axes, int axis) {
-  ctx->prepared = false;
-  const int64_t N = box_off[S];
-  const int64_t T = tiles_for(box_off, S);
-  STQ_TRY(ensure_staging(ctx, std::max(S, 1), int(std::max<int64_t>(T, 1))));
-  STQ_TRY(ensure_box_buffers(ctx, N));
-  fill_staging(ctx, box_off, S, axes, axis, nullptr, nullptr, nullptr);
-  STQ_TRY(upload_staging(ctx));
-  BatchBuffers b = batch_buffers(ctx, d_boxes);
-  STQ_TRY(enqueue_prepare_front(ctx, b, -1, -1));
-  STQ_TRY(read_header(ctx));
-  const int64_t R = ctx->h_hdr->replicas, cells = ctx->h_hdr->cells;
-  if (R + 3 * cells + 1 + kSortedPad > int64_t(INT32_MAX))
+// Checks what a prepare's first half reported (after front_event, or after the
+// stream) and takes over the sizes. *again: the buffers that the second half was
+// queued for do not hold the scenes; it did nothing.
+int take_front(stq_context *ctx, int S, int64_t N, bool *again) {
+  const FrontInfo &f = *ctx->h_front;
+  *again = false;
+  if (f.flags & ~kFlagReplicaOverflow) {
+    ctx->h_hdr->flags = f.flags & ~kFlagReplicaOverflow;
+    return check_header(ctx);
+  }
+  if (f.replicas + 3 * f.cells + 1 + kSortedPad > (unsigned long long)INT32_MAX)
     return fail(ctx, STQ_ERR_NO_MEMORY, "too many cell replicas for 32-bit positions");
-  STQ_TRY(ensure_replica_buffers(ctx, std::max(R, ctx->rep_cap), cells));
-  b = batch_buffers(ctx, d_boxes);
-  STQ_TRY(enqueue_prepare_back(ctx, b, R, int(ctx->h_hdr->passes)));
+  if (f.flags & kFlagReplicaOverflow) {
+    *again = true;
+    return STQ_OK;
+  }
   ctx->n_scenes = S;
   ctx->n_boxes = N;
-  ctx->length = R > 0 ? R + 3 * cells - 1 : 0;
+  ctx->length = f.replicas > 0 ? int64_t(f.replicas + 3 * f.cells) - 1 : 0;
   ctx->scene.length = ctx->length;
   ctx->prepared = true;
   return STQ_OK;
+}
+
+// Whether the context's buffers, from earlier scenes, may hold a batch of N boxes.
+bool has_room(const stq_context *ctx, int64_t N) {
+  return ctx->passes_seen > 0 && ctx->rep_cap >= N && ctx->seg_cap > 0;
+}
+
+// Queues a whole prepare for the buffers that the context has.
+int enqueue_prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_off, int S, const int *axes, int axis,
+                    bool *whole) {
+  ctx->prepared = false;
+  ctx->swept = false;
+  const int64_t N = box_off[S];
+  STQ_TRY(ensure_staging(ctx, std::max(S, 1), int(std::max<int64_t>(tiles_for(box_off, S), 1))));
+  STQ_TRY(ensure_box_buffers(ctx, N));
+  fill_staging(ctx, box_off, S, axes, axis, nullptr, nullptr, nullptr);
+  STQ_TRY(upload_staging(ctx));
+  const BatchBuffers b = batch_buffers(ctx, d_boxes);
+  STQ_TRY(enqueue_prepare_front(ctx, b, *whole ? ctx->rep_cap : -1, ctx->seg_cap, ctx->passes_seen));
+  if (!ctx->front_event)
+    STQ_CUDA(ctx, cudaEventCreateWithFlags(&ctx->front_event, cudaEventDisableTiming), "create event");
+  STQ_CUDA(ctx, cudaEventRecord(ctx->front_event, ctx->stream), "record prepare");
+  if (*whole) STQ_TRY(enqueue_prepare_back(ctx, b, -1, ctx->passes_seen));
+  return STQ_OK;
+}
+
+// Prepares a batch. Its second half is queued before the host knows the replica
+// count when the buffers of earlier scenes may hold it, so that the stream does
+// not idle while the host waits for that count; if they do not, or there are
+// none, they are sized (an eighth more than needed, for the next step of a
+// moving scene) and the second half is queued then.
+int prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_off, int S, const int *axes, int axis) {
+  const int64_t N = box_off[S];
+  for (bool whole = has_room(ctx, N);; whole = false) {
+    STQ_TRY(enqueue_prepare(ctx, d_boxes, box_off, S, axes, axis, &whole));
+    STQ_CUDA(ctx, cudaEventSynchronize(ctx->front_event), "wait for prepare");
+    bool again = false;
+    STQ_TRY(take_front(ctx, S, N, &again));
+    if (again) continue;
+    if (whole) return STQ_OK;
+    const int64_t R = int64_t(ctx->h_front->replicas), cells = int64_t(ctx->h_front->cells);
+    ctx->prepared = false;
+    if (R > ctx->rep_cap || 3 * cells > ctx->seg_cap) {
+      const int64_t more = std::max(ctx->rep_cap, std::min<int64_t>(R + R / 8 + 256, INT32_MAX / 2));
+      STQ_TRY(ensure_replica_buffers(ctx, std::max(R, more), cells + cells / 8 + 16));
+    } else {
+      STQ_TRY(ensure_replica_buffers(ctx, ctx->rep_cap, cells));
+    }
+    ctx->passes_seen = std::max(ctx->passes_seen, int(ctx->h_front->passes));
+    STQ_TRY(enqueue_prepare_back(ctx, batch_buffers(ctx, d_boxes), R, int(ctx->h_front->passes)));
+    ctx->prepared = true;
+    return STQ_OK;
+  }
 }
 
 int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
@@ -335,6 +385,7 @@ int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
               cudaStream_t stream) {
   BatchHeader *hdr = dev_hdr(ctx);
   cudaStream_t s = cursors && stream ? stream : ctx->stream;
+  ctx->swept = true;
   SweepParams p;
   p.yz = ctx->scene.yz;
   p.x = ctx->scene.x;
@@ -386,6 +437,51 @@ int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
 
 using namespace stq::ctxops;
 
+namespace {
+
+// The results of a sweep of [start, end) whose header has been read back. On
+// overflow: counts pairs per start position, keeps the longest prefix that
+// fits, and emits exactly that prefix again.
+int finish_sweep(stq_context *ctx, int64_t start, int64_t end, stq_pair *d_pairs, int64_t capacity, int64_t *count,
+                 int64_t *next_start, int64_t *total) {
+  const int64_t found = int64_t(ctx->h_hdr->pairs);
+  if (total) *total = found;
+  if (found <= capacity) {
+    *count = found;
+    *next_start = end;
+    return STQ_OK;
+  }
+  const int64_t m = end - start;
+  STQ_CUDA(ctx, ctx->box_counts.ensure(sizeof(int32_t) * size_t(m)), "allocate box counts");
+  STQ_CUDA(ctx, ctx->prefix_ws.ensure(prefix_workspace_bytes(m) + sizeof(DevScalars)),
+           "allocate prefix workspace");
+  STQ_CUDA(ctx, cudaMemsetAsync(ctx->box_counts.ptr, 0, sizeof(int32_t) * size_t(m), ctx->stream),
+           "clear box counts");
+  STQ_TRY(run_sweep(ctx, start, end, nullptr, 0, true));
+  DevScalars *sel = reinterpret_cast<DevScalars *>(ctx->prefix_ws.as<char>() + prefix_workspace_bytes(m));
+  STQ_CUDA(ctx, launch_prefix_select(ctx->stream, ctx->box_counts.as<int32_t>(), m, capacity,
+                                     ctx->prefix_ws.ptr, sel, &ctx->launches),
+           "launch prefix selection");
+  DevScalars h_sel;
+  STQ_CUDA(ctx, cudaMemcpyAsync(&h_sel, sel, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream),
+           "read back prefix");
+  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
+  const int64_t prefix = h_sel.prefix;
+  if (prefix <= 0) {
+    *count = 0;
+    *next_start = start;
+    return fail(ctx, STQ_ERR_CAPACITY, "the first start box has more pairs than capacity");
+  }
+  STQ_TRY(run_sweep(ctx, start, start + prefix, d_pairs, capacity, false));
+  STQ_TRY(read_header(ctx));
+  *count = int64_t(ctx->h_hdr->pairs);
+  *next_start = start + prefix;
+  if (*count > capacity) return fail(ctx, STQ_ERR_CUDA, "prefix re-sweep exceeded capacity");
+  return STQ_OVERFLOW;
+}
+
+}  // namespace
+
 extern "C" {
 
 int stq_abi_version(void) { return STQ_ABI_VERSION; }
@@ -420,6 +516,8 @@ int stq_context_create(int device, void *stream, stq_context **out) {
   apply_options(ctx);
   if (cudaMallocHost(&ctx->h_hdr, sizeof(BatchHeader)) != cudaSuccess ||
       cudaMallocHost(&ctx->h_fault, sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(&ctx->h_flags, sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(&ctx->h_front, sizeof(FrontInfo)) != cudaSuccess ||
       ctx->aux.ensure(sizeof(BatchHeader)) != cudaSuccess || ensure_staging(ctx, 1, 1) != STQ_OK) {
     stq_context_destroy(ctx);
     return STQ_ERR_NO_MEMORY;
@@ -443,6 +541,9 @@ void stq_context_destroy(stq_context *ctx) {
     if (ctx->in_host) cudaFreeHost(ctx->in_host);
     if (ctx->h_hdr) cudaFreeHost(ctx->h_hdr);
     if (ctx->h_fault) cudaFreeHost(ctx->h_fault);
+    if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
+    if (ctx->h_front) cudaFreeHost(ctx->h_front);
+    if (ctx->front_event) cudaEventDestroy(ctx->front_event);
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     if (ctx->copy_stream) {
       cudaStreamSynchronize(ctx->copy_stream);
@@ -576,18 +677,20 @@ int stq_build_boxes(stq_context *ctx, const double *d_V0, const double *d_V1, in
     return fail(ctx, STQ_ERR_INVALID_ARG, "null buffer");
   if (nV + nE + nF == 0) return STQ_OK;
   DeviceGuard g(ctx->device);
-  BatchHeader *aux = ctx->aux.as<BatchHeader>();
-  STQ_CUDA(ctx, cudaMemsetAsync(aux, 0, sizeof(BatchHeader), ctx->stream), "clear flags");
+  *ctx->h_flags = 0;
   STQ_CUDA(ctx, ctx->points.ensure(2 * sizeof(float4) * size_t(std::max<int64_t>(nV, 1))),
            "allocate rounded positions");
   stage_begin(ctx, kBuild);
   STQ_CUDA(ctx, launch_build_boxes(ctx->stream, d_V0, d_V1, nV, d_E, nE, d_F, nF,
-                                   ref_next_up(inflation_radius), d_boxes, &aux->flags,
+                                   ref_next_up(inflation_radius), d_boxes, ctx->h_flags,
                                    ctx->points.as<float4>()),
            "launch box build");
   stage_end(ctx, kBuild);
   ctx->launches += nV > 0 ? 2 : 1;
-  return read_header(ctx, aux);
+  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
+  collect_stages(ctx);
+  if (*ctx->h_flags) return fail(ctx, STQ_ERR_INVALID_INPUT, "an edge or face vertex index is out of range");
+  return STQ_OK;
 }
 
 int stq_batch_build_boxes(stq_context *ctx, const double *d_V0, const double *d_V1,
@@ -644,7 +747,7 @@ int stq_batch_prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *
   if (h_box_off[n_scenes] > kMaxBoxes) return fail(ctx, STQ_ERR_INVALID_ARG, "too many boxes");
   if (h_box_off[n_scenes] > 0 && !d_boxes) return fail(ctx, STQ_ERR_INVALID_ARG, "null boxes");
   DeviceGuard g(ctx->device);
-  return prepare_exact(ctx, d_boxes, h_box_off, n_scenes, h_axis, axis);
+  return prepare(ctx, d_boxes, h_box_off, n_scenes, h_axis, axis);
 }
 
 int stq_prepare(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int axis) {
@@ -687,47 +790,35 @@ int stq_sweep_prepared(stq_context *ctx, int64_t start, int64_t max_start, stq_p
   const int64_t end = (max_start <= 0 || start + max_start > length) ? length : start + max_start;
   STQ_TRY(run_sweep(ctx, start, end, d_pairs, capacity, false));
   STQ_TRY(read_header(ctx));
-  const int64_t found = int64_t(ctx->h_hdr->pairs);
-  if (total) *total = found;
-  if (found <= capacity) {
-    *count = found;
-    *next_start = end;
-    return STQ_OK;
-  }
-  // Overflow: count pairs per start position, keep the longest prefix that
-  // fits, and emit exactly that prefix again.
-  const int64_t m = end - start;
-  STQ_CUDA(ctx, ctx->box_counts.ensure(sizeof(int32_t) * size_t(m)), "allocate box counts");
-  STQ_CUDA(ctx, ctx->prefix_ws.ensure(prefix_workspace_bytes(m) + sizeof(DevScalars)),
-           "allocate prefix workspace");
-  STQ_CUDA(ctx, cudaMemsetAsync(ctx->box_counts.ptr, 0, sizeof(int32_t) * size_t(m), ctx->stream),
-           "clear box counts");
-  STQ_TRY(run_sweep(ctx, start, end, nullptr, 0, true));
-  DevScalars *sel = reinterpret_cast<DevScalars *>(ctx->prefix_ws.as<char>() + prefix_workspace_bytes(m));
-  STQ_CUDA(ctx, launch_prefix_select(ctx->stream, ctx->box_counts.as<int32_t>(), m, capacity,
-                                     ctx->prefix_ws.ptr, sel, &ctx->launches),
-           "launch prefix selection");
-  DevScalars h_sel;
-  STQ_CUDA(ctx, cudaMemcpyAsync(&h_sel, sel, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream),
-           "read back prefix");
-  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
-  const int64_t prefix = h_sel.prefix;
-  if (prefix <= 0) {
-    *count = 0;
-    *next_start = start;
-    return fail(ctx, STQ_ERR_CAPACITY, "the first start box has more pairs than capacity");
-  }
-  STQ_TRY(run_sweep(ctx, start, start + prefix, d_pairs, capacity, false));
-  STQ_TRY(read_header(ctx));
-  *count = int64_t(ctx->h_hdr->pairs);
-  *next_start = start + prefix;
-  if (*count > capacity) return fail(ctx, STQ_ERR_CUDA, "prefix re-sweep exceeded capacity");
-  return STQ_OVERFLOW;
+  return finish_sweep(ctx, start, end, d_pairs, capacity, count, next_start, total);
 }
 
 int stq_sweep(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int axis, int64_t start,
               int64_t max_start, stq_pair *d_pairs, int64_t capacity, int64_t *count,
               int64_t *next_start, int64_t *total) {
+  // the whole scene in buffers of earlier calls: prepare and sweep are queued
+  // together, and the host waits once
+  if (ctx && n > 0 && n <= kMaxBoxes && d_boxes && axis >= STQ_AXIS_AUTO && axis <= STQ_AXIS_Z && start == 0 &&
+      max_start <= 0 && count && next_start && capacity >= 0 && (capacity == 0 || d_pairs) && has_room(ctx, n)) {
+    DeviceGuard g(ctx->device);
+    const int64_t off[2] = {0, n};
+    bool whole = true, again = false;
+    STQ_TRY(enqueue_prepare(ctx, d_boxes, off, 1, nullptr, axis, &whole));
+    STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, d_pairs, capacity, false));
+    STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_hdr, dev_hdr(ctx), sizeof(BatchHeader), cudaMemcpyDeviceToHost, ctx->stream),
+             "read back batch header");
+    STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
+    collect_stages(ctx);
+    STQ_TRY(take_front(ctx, 1, n, &again));
+    if (!again) {
+      const int st = check_header(ctx);
+      if (st != STQ_OK) {
+        ctx->prepared = false;
+        return st;
+      }
+      return finish_sweep(ctx, 0, ctx->length, d_pairs, capacity, count, next_start, total);
+    }
+  }
   STQ_TRY(stq_prepare(ctx, d_boxes, n, axis));
   return stq_sweep_prepared(ctx, start, max_start, d_pairs, capacity, count, next_start, total);
 }
@@ -737,6 +828,10 @@ int stq_batch_scene_pairs(stq_context *ctx, int64_t *h_counts, int n_scenes) {
   if (!ctx->prepared) return fail(ctx, STQ_ERR_NOT_PREPARED, "nothing prepared");
   if (n_scenes > ctx->n_scenes) return fail(ctx, STQ_ERR_INVALID_ARG, "more scenes than prepared");
   DeviceGuard g(ctx->device);
+  if (!ctx->swept) {  // prepared, not swept yet: the counters are from before
+    std::fill(h_counts, h_counts + n_scenes, int64_t(0));
+    return STQ_OK;
+  }
   STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_scene_pairs, ctx->scene_pairs.ptr,
                                 sizeof(unsigned long long) * size_t(n_scenes), cudaMemcpyDeviceToHost,
                                 ctx->stream),
@@ -795,7 +890,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     stage_end(ctx, kBuild);
     const BatchBuffers b = batch_buffers(ctx, boxes);
     STQ_TRY(enqueue_prepare_front(ctx, b, ctx->rep_cap, ctx->seg_cap));
-    STQ_TRY(enqueue_prepare_back(ctx, b, -1, -1));
+    STQ_TRY(enqueue_prepare_back(ctx, b, -1, 4));
     STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, d_pairs, capacity, false));
     STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_hdr, dev_hdr(ctx), sizeof(BatchHeader),
                                   cudaMemcpyDeviceToHost, ctx->stream),
@@ -882,7 +977,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
 
 namespace {
 
-// Sweeps the prepared scene into h_pairs. The start positions are cut into
+// Prepares the boxes and sweeps them into h_pairs. The start positions are cut into
 // windows (STQ_OPT_HOST_WINDOWS, default 16) that alternate between two
 // slots: even windows sweep on the context's stream into e2e_pairs, odd
 // windows on a second stream into window_pairs. A slot's pair counter runs on
@@ -897,18 +992,23 @@ namespace {
 // host-buffer call, runs beside the sweep instead of after it. If the pairs do
 // not fit h_pairs the call falls back to the prefix rule of
 // stq_sweep_prepared and one copy.
-int sweep_to_host(stq_context *ctx, stq_pair *h_pairs, int64_t capacity, int64_t *count,
-                  int64_t *total) {
+int sweep_to_host(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int axis, stq_pair *h_pairs, int64_t capacity,
+                  int64_t *count, int64_t *total) {
+  constexpr int64_t kMinWindow = int64_t(1) << 19;  // start positions
+  // too small for two windows, whatever its replicas: prepared and swept in one
+  const bool one = capacity == 0 || ctx->options[STQ_OPT_HOST_OVERLAP] == 2 ||
+                   (has_room(ctx, n) && ctx->slot_cap < 2 * kMinWindow);
+  if (!one) STQ_TRY(stq_prepare(ctx, d_boxes, n, axis));
   const size_t pair_bytes = sizeof(stq_pair) * size_t(capacity > 0 ? capacity : 1);
   STQ_CUDA(ctx, ctx->e2e_pairs.ensure(pair_bytes), "allocate pair staging");
   stq_pair *d_pairs = ctx->e2e_pairs.as<stq_pair>();
-  const int64_t length = ctx->length;
-  constexpr int64_t kMinWindow = int64_t(1) << 19;  // start positions
+  const int64_t length = one ? 0 : ctx->length;
   const int64_t want = ctx->options[STQ_OPT_HOST_WINDOWS] ? ctx->options[STQ_OPT_HOST_WINDOWS] : 16;
   const int windows = int(std::min<int64_t>(want, length / kMinWindow));
   auto one_copy = [&]() -> int {
     int64_t next = 0;
-    const int st = stq_sweep_prepared(ctx, 0, 0, d_pairs, capacity, count, &next, total);
+    const int st = ctx->prepared && !one ? stq_sweep_prepared(ctx, 0, 0, d_pairs, capacity, count, &next, total)
+                                         : stq_sweep(ctx, d_boxes, n, axis, 0, 0, d_pairs, capacity, count, &next, total);
     if (st != STQ_OK && st != STQ_OVERFLOW) return st;
     if (*count > 0) {
       STQ_CUDA(ctx, cudaMemcpyAsync(h_pairs, d_pairs, sizeof(stq_pair) * size_t(*count),
@@ -918,7 +1018,7 @@ int sweep_to_host(stq_context *ctx, stq_pair *h_pairs, int64_t capacity, int64_t
     }
     return st;
   };
-  if (windows < 2 || capacity == 0 || ctx->options[STQ_OPT_HOST_OVERLAP] == 2) return one_copy();
+  if (windows < 2) return one_copy();
 
   auto windowed = [&]() -> int {
     STQ_CUDA(ctx, ctx->window_pairs.ensure(pair_bytes), "allocate pair staging");
@@ -1023,8 +1123,7 @@ int stq_sweep_host(stq_context *ctx, const stq_aabb *h_boxes, int64_t n, int axi
     STQ_CUDA(ctx, cudaMemcpyAsync(ctx->e2e_boxes.ptr, h_boxes, sizeof(stq_aabb) * size_t(n),
                                   cudaMemcpyHostToDevice, ctx->stream),
              "copy boxes to device");
-  STQ_TRY(stq_prepare(ctx, ctx->e2e_boxes.as<stq_aabb>(), n, axis));
-  return sweep_to_host(ctx, h_pairs, capacity, count, total);
+  return sweep_to_host(ctx, ctx->e2e_boxes.as<stq_aabb>(), n, axis, h_pairs, capacity, count, total);
 }
 
 int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count) {
@@ -1075,8 +1174,7 @@ int stq_broadphase_host(stq_context *ctx, const double *h_V0, const double *h_V1
                           reinterpret_cast<const int32_t *>(base + oE), nE,
                           reinterpret_cast<const int32_t *>(base + oF), nF, inflation_radius,
                           ctx->e2e_boxes.as<stq_aabb>()));
-  STQ_TRY(stq_prepare(ctx, ctx->e2e_boxes.as<stq_aabb>(), n, axis));
-  return sweep_to_host(ctx, h_pairs, capacity, count, total);
+  return sweep_to_host(ctx, ctx->e2e_boxes.as<stq_aabb>(), n, axis, h_pairs, capacity, count, total);
 }
 
 int stq_context_enable_timing(stq_context *ctx, int enable) {

@@ -371,7 +371,7 @@ __device__ __forceinline__ Range cell_range(const stq_aabb &x, int a, float ob, 
 __device__ __forceinline__ void
 choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__ tiles, const SceneInput *inputs,
               SceneRecord *scenes, unsigned int *cell_base, const unsigned long long *tile_reps, uint32_t *tile_off,
-              BatchHeader *hdr, long long rep_cap, long long seg_cap) {
+              BatchHeader *hdr, FrontInfo *front, long long rep_cap, long long seg_cap, int max_passes) {
   __shared__ uint32_t scratch[kBlock / 32];
   __shared__ unsigned long long reps;
   if (threadIdx.x == 0) reps = 0;
@@ -439,9 +439,18 @@ choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__
   if (threadIdx.x == 0) {
     cell_base[S] = carry;
     const unsigned long long R = reps, lists = 3ull * carry;
+    // key: list id above the top bits of the sweep-axis code, 24 bits in all (three
+    // digits) where that leaves the code 10 bits or more, else 32. At 10 bits the
+    // 6 M-box scene (14 bits of lists) tests 9% more candidates and sorts a digit
+    // less: sort + sweep 0.22 + 1.26 ms against 0.29 + 1.19 with 32 bits.
+    int seg_bits = 0;
+    while (seg_bits < 32 && (1ull << seg_bits) < lists) ++seg_bits;
+    const int key_bits = seg_bits <= 14 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
+    const int passes = max(seg_bits + key_bits + 7, 8) / 8;
     // more than the buffers hold: the scenes are flagged and left empty (the
     // caller without limits checks that positions fit 31 bits)
-    const bool fits = R < 0xffffffffull && (rep_cap < 0 || ((long long)R <= rep_cap && (long long)lists <= seg_cap));
+    const bool fits = R < 0xffffffffull && (rep_cap < 0 || ((long long)R <= rep_cap && (long long)lists <= seg_cap &&
+                                                            passes <= max_passes));
     if (!fits) atomicOr(&hdr->flags, kFlagReplicaOverflow);
     hdr->replicas = fits ? unsigned(R) : 0u;
     hdr->cells = fits ? carry : 0u;
@@ -450,15 +459,12 @@ choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__
     // of these is not a start position
     hdr->length = fits && carry > 0 && R > 0 ? unsigned(R + lists - 1) : 0u;
     hdr->max_list = 0u;
-    // key: list id above the top bits of the sweep-axis code, 24 bits in all (three
-    // digits) where that leaves the code 10 bits or more, else 32. At 10 bits the
-    // 6 M-box scene (14 bits of lists) tests 9% more candidates and sorts a digit
-    // less: sort + sweep 0.22 + 1.26 ms against 0.29 + 1.19 with 32 bits.
-    int seg_bits = 0;
-    while (seg_bits < 32 && (1ull << seg_bits) < lists) ++seg_bits;
-    const int key_bits = seg_bits <= 14 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
     hdr->key_bits = key_bits;
-    hdr->passes = unsigned(max(seg_bits + key_bits + 7, 8)) / 8u;
+    hdr->passes = unsigned(passes);
+    front->replicas = R;
+    front->cells = carry;
+    front->passes = unsigned(passes);
+    front->flags = hdr->flags;
   }
 }
 
@@ -479,7 +485,7 @@ __global__ void __launch_bounds__(kBlock)
 batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
                       const long long *__restrict__ box_off, SceneInput *inputs,
                       SceneRecord *scenes, unsigned int *cell_base, unsigned long long *tile_reps, uint32_t *tile_off,
-                      BatchHeader *hdr, long long rep_cap, long long seg_cap,
+                      BatchHeader *hdr, FrontInfo *front, long long rep_cap, long long seg_cap, int max_passes,
                       uint2 *__restrict__ box_cells, uint32_t *__restrict__ box_q) {
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
@@ -529,7 +535,8 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
   __syncthreads();
   if (!last) return;
   __threadfence();
-  choose_levels(box_off, tiles, inputs, scenes, cell_base, tile_reps, tile_off, hdr, rep_cap, seg_cap);
+  choose_levels(box_off, tiles, inputs, scenes, cell_base, tile_reps, tile_off, hdr, front, rep_cap, seg_cap,
+                max_passes);
 }
 
 // ---- 5. replica keys in box order: (list id << key_bits) | sweep-axis code, where
@@ -848,10 +855,10 @@ cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap) {
+cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap, int passes) {
   batch_box_keys_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.box_off, b.inputs, b.scenes,
-                                                                b.cell_base, b.tile_reps, b.tile_off, b.hdr, rep_cap,
-                                                                seg_cap, b.box_cells, b.box_q);
+                                                                b.cell_base, b.tile_reps, b.tile_off, b.hdr, b.front,
+                                                                rep_cap, seg_cap, passes, b.box_cells, b.box_q);
   return cudaGetLastError();
 }
 

@@ -120,7 +120,8 @@ __device__ __forceinline__ stq_aabb build_one(const double *__restrict__ V0,
   for (int q = 0; q < npts; ++q)
     if (idx[q] < 0 || idx[q] >= nV) ok = false;
   if (!ok) {
-    atomicOr(flags, kFlagBadIndex);
+    // no other flag is set before the boxes are built; the word may be in host memory
+    *reinterpret_cast<volatile int *>(flags) = kFlagBadIndex;
     for (int k = 0; k < 3; ++k) b.min[k] = b.max[k] = __int_as_float(0x7fc00000);
     return b;
   }

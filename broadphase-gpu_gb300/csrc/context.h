@@ -92,6 +92,11 @@ struct stq_context {
   SortedScene scene;
   BatchHeader *h_hdr = nullptr;             // pinned readback
   int *h_fault = nullptr;  // pinned, written by a pair sort whose wait ran out
+  int *h_flags = nullptr;  // pinned, written by a box build with a bad index
+  FrontInfo *h_front = nullptr;       // pinned, written by a prepare's first half
+  cudaEvent_t front_event = nullptr;  // after it
+  int passes_seen = 0;  // most digits that a replica sort of this context needed
+  bool swept = false;   // the prepared scenes have been swept (their pair counters hold)
   unsigned long long *h_scene_pairs = nullptr;  // pinned readback
   int h_scene_pairs_cap = 0;
 
@@ -162,12 +167,14 @@ int ensure_box_buffers(stq_context *ctx, int64_t box_cap);
 int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap);
 int bits_for(int64_t v);
 // Statistics, axis, grid and sweep-axis codes per scene, the grid level and the
-// replica count. Scenes that need more than rep_cap replicas or seg_cap lists
-// are flagged and left empty (-1: no limit).
-int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap);
+// replica count. Scenes that need more than rep_cap replicas, seg_cap lists or
+// `passes` digits of the replica sort are flagged and left empty (rep_cap -1: no
+// limit).
+int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap, int passes = 4);
 // Replica emit in box order, their sort by (list, sweep-axis code), list offsets
-// and the sorted scene. replicas, passes: the replica count and the digits of
-// its sort, or -1 when only the device knows them (graph capture, serving).
+// and the sorted scene. replicas: the replica count, or -1 when only the device
+// knows it (graph capture, serving, a prepare that is not waited for). passes:
+// digits of the sort to launch.
 int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes);
 // Launches one sweep over start positions [begin, end). With cursors null it
 // first clears the batch header's pair counter, cursors, per-scene counts and

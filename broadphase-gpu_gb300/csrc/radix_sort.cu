@@ -370,7 +370,8 @@ struct BlockShared {
 template <typename K, bool VALS, int ITEMS>
 __global__ void __launch_bounds__(kPassBlock)
 radix_block_kernel(const K *k0, const K *k1, K *kout, const uint32_t *v0, const uint32_t *v1, uint32_t *vout, int n,
-                   Digits dg) {
+                   const unsigned int *d_n, Digits dg) {
+  if (d_n && int(*d_n) < n) n = int(*d_n);
   const bool second = dg.d_passes && (*dg.d_passes & 1u);
   const K *kin = second ? k1 : k0;
   const uint32_t *vin = second ? v1 : v0;
@@ -488,13 +489,13 @@ cudaError_t launch_passes(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf
 
 template <typename K, bool VALS, int ITEMS>
 cudaError_t launch_block(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const Digits &dg,
-                         int64_t *launches) {
+                         const unsigned int *d_n, int64_t *launches) {
   constexpr auto kern = radix_block_kernel<K, VALS, ITEMS>;
   constexpr size_t smem = sizeof(BlockShared<K, VALS, ITEMS>);
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   kern<<<1, kPassBlock, smem, s>>>(kbuf[0], kbuf[1], kbuf[0], VALS ? vbuf[0] : nullptr, VALS ? vbuf[1] : nullptr,
-                                   VALS ? vbuf[0] : nullptr, int(n), dg);
+                                   VALS ? vbuf[0] : nullptr, int(n), d_n, dg);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
@@ -503,11 +504,10 @@ template <typename K, bool VALS>
 cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const unsigned int *d_n,
                       const Digits &dg, void *workspace, int *fault, int64_t *launches) {
   if (dg.passes == 0 || (n <= 1 && !dg.d_passes)) return cudaSuccess;
-  if (!d_n) {  // one block up to its 16 keys per thread
-    if (n <= kPassBlock * 2) return launch_block<K, VALS, 2>(s, kbuf, vbuf, n, dg, launches);
-    if (n <= kPassBlock * 8) return launch_block<K, VALS, 8>(s, kbuf, vbuf, n, dg, launches);
-    if (n <= kPassBlock * 16) return launch_block<K, VALS, 16>(s, kbuf, vbuf, n, dg, launches);
-  }
+  // one block up to its 16 keys per thread
+  if (n <= kPassBlock * 2) return launch_block<K, VALS, 2>(s, kbuf, vbuf, n, dg, d_n, launches);
+  if (n <= kPassBlock * 8) return launch_block<K, VALS, 8>(s, kbuf, vbuf, n, dg, d_n, launches);
+  if (n <= kPassBlock * 16) return launch_block<K, VALS, 16>(s, kbuf, vbuf, n, dg, d_n, launches);
   SortHead *head = static_cast<SortHead *>(workspace);
   unsigned long long *status = reinterpret_cast<unsigned long long *>(static_cast<char *>(workspace) +
                                                                       kRadixHeadBytes);

@@ -152,6 +152,15 @@ struct BatchHeader {
   unsigned int keys_done;   // tiles whose box keys and level counts are in
 };
 
+// What the host needs of a prepare's first half, written by the device to
+// page-locked memory.
+struct FrontInfo {
+  unsigned long long replicas;  // replicas and cells that the scenes need
+  unsigned long long cells;
+  unsigned int passes;          // digits of the replica sort
+  int flags;                    // kFlag* bits
+};
+
 // A tile of at most kTileBoxes consecutive boxes of one scene (built by the
 // host from the scene offsets), so that a block reduces per-scene values once.
 constexpr int kTileBoxes = 4096;
@@ -269,6 +278,7 @@ struct BatchBuffers {
   SceneRecord *scenes;
   unsigned int *cell_base;      // n_scenes + 1
   BatchHeader *hdr;
+  FrontInfo *front;             // page-locked
   uint2 *box_cells;             // per box: cell range and type
                                 // (b0 | b1 << 11 | type << 22, c0 | c1 << 11)
   uint32_t *box_q;              // per box: sweep-axis codes of its min | its max << 16
@@ -287,9 +297,10 @@ struct BatchBuffers {
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b);
 // level-0 cell ranges, sweep-axis codes and every level's replica count; then the
 // level within the replica budget, the cell bases, the key layout and every
-// tile's first replica (1 launch). Scenes that need more than rep_cap replicas or
-// seg_cap lists are flagged and left empty (no limit: -1).
-cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap);
+// tile's first replica (1 launch). Scenes that need more than rep_cap replicas,
+// seg_cap lists or `passes` digits of the replica sort are flagged and left empty
+// (no limit: rep_cap -1).
+cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap, int passes);
 // replicas in box order (1 launch)
 cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b);
 // list offsets from the sorted keys (and the longest list); the empty position

@@ -1,0 +1,71 @@
+"""One context over scenes that fit, outgrow and leave room in the buffers of the
+scenes before: a sweep is queued whole where they may fit, and again where they
+did not. Every call gives the oracle's pairs, and a bad box is refused from
+either way."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def scene(stq, n, side, seed):
+    b = stq.random_boxes(n, sliver_frac=0.0, seed=seed)
+    c = 0.5 * (b["min"] + b["max"])
+    b["min"], b["max"] = c - np.float32(side / 2), c + np.float32(side / 2)
+    return b
+
+
+def dev(b, cuda):
+    import torch
+
+    return torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_scenes_of_changing_size_and_density(ctx, stq, oracle, cuda, fused):
+    import torch
+
+    # boxes, side of a box: more replicas at the same count, more lists, more
+    # digits of the replica sort, then small ones again; one scene twice
+    steps = [(300, 0.05), (300, 0.05), (300, 0.3), (5000, 0.02), (5000, 0.09), (60_000, 0.01), (60_000, 0.02),
+             (200_000, 0.004), (300, 0.05), (5000, 0.02)]
+    for k, (n, side) in enumerate(steps):
+        b = scene(stq, n, side, seed=50 + k)
+        want = oracle.broadphase(b)
+        pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+        if fused:
+            r = ctx.sweep(dev(b, cuda), n, pairs, len(want) + 16, axis=-1)
+        else:
+            ctx.prepare(dev(b, cuda), n, -1)
+            assert np.array_equal(ctx.batch_scene_pairs(1), [0])  # not swept yet
+            r = ctx.sweep_prepared(pairs, len(want) + 16)
+        assert r.status == stq.STQ_OK and r.count == len(want) and r.next_start == ctx.prepared_length, k
+        assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want), k
+        assert np.array_equal(ctx.batch_scene_pairs(1), [len(want)])
+
+
+def test_bad_boxes_after_good_ones(ctx, stq, oracle, cuda):
+    import torch
+
+    b = scene(stq, 4000, 0.05, seed=7)
+    want = oracle.broadphase(b)
+    pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+    bad = b.copy()
+    bad["max"][17, 1] = np.nan
+    for boxes, ok in ((b, True), (b, True), (bad, False), (b, True)):
+        if ok:
+            r = ctx.sweep(dev(boxes, cuda), len(b), pairs, len(want) + 16)
+            assert r.count == len(want)
+            assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+        else:
+            with pytest.raises(stq.STQError) as e:
+                ctx.sweep(dev(boxes, cuda), len(b), pairs, len(want) + 16)
+            assert e.value.status == stq.STQ_ERR_INVALID_INPUT and ctx.prepared_length == -1
+    small = torch.empty((len(want) // 2, 2), dtype=torch.int32, device=cuda)
+    r = ctx.sweep(dev(b, cuda), len(b), small, len(want) // 2)  # overflow from the whole call
+    assert r.status == stq.STQ_OVERFLOW and r.total == len(want)
+    got = [small[: r.count].cpu().numpy().copy()]
+    while r.status == stq.STQ_OVERFLOW:
+        r = ctx.sweep_prepared(small, len(want) // 2, start=r.next_start)
+        got.append(small[: r.count].cpu().numpy().copy())
+    assert np.array_equal(oracle.canonical(np.concatenate(got)), want)
