@@ -518,6 +518,7 @@ int stq_context_create(int device, void *stream, stq_context **out) {
       cudaMallocHost(&ctx->h_fault, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&ctx->h_flags, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&ctx->h_front, sizeof(FrontInfo)) != cudaSuccess ||
+      cudaMallocHost(&ctx->h_plan, sizeof(PairPlan)) != cudaSuccess ||
       ctx->aux.ensure(sizeof(BatchHeader)) != cudaSuccess || ensure_staging(ctx, 1, 1) != STQ_OK) {
     stq_context_destroy(ctx);
     return STQ_ERR_NO_MEMORY;
@@ -543,6 +544,7 @@ void stq_context_destroy(stq_context *ctx) {
     if (ctx->h_fault) cudaFreeHost(ctx->h_fault);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
     if (ctx->h_front) cudaFreeHost(ctx->h_front);
+    if (ctx->h_plan) cudaFreeHost(ctx->h_plan);
     if (ctx->front_event) cudaEventDestroy(ctx->front_event);
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     if (ctx->copy_stream) {
@@ -1131,11 +1133,11 @@ int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count) {
   if (count < 2) return STQ_OK;
   DeviceGuard g(ctx->device);
   STQ_CUDA(ctx, ctx->pair_tmp.ensure(sizeof(stq_pair) * size_t(count)), "allocate pair buffer");
-  STQ_CUDA(ctx, ctx->sort_ws.ensure(radix_workspace_bytes(count)), "allocate sort workspace");
+  STQ_CUDA(ctx, ctx->sort_ws.ensure(pair_workspace_bytes(count)), "allocate sort workspace");
   *ctx->h_fault = 0;
   stage_begin(ctx, kPairSort);
-  STQ_CUDA(ctx, radix_sort_pairs(ctx->stream, d_pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->sort_ws.ptr,
-                                 ctx->h_fault, &ctx->launches),
+  STQ_CUDA(ctx, sort_pairs(ctx->stream, d_pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->sort_ws.ptr, ctx->h_plan,
+                           &ctx->pair_id_bits, ctx->h_fault, &ctx->launches),
            "launch pair sort");
   stage_end(ctx, kPairSort);
   STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");

@@ -95,6 +95,8 @@ struct stq_context {
   int *h_flags = nullptr;  // pinned, written by a box build with a bad index
   FrontInfo *h_front = nullptr;       // pinned, written by a prepare's first half
   cudaEvent_t front_event = nullptr;  // after it
+  PairPlan *h_plan = nullptr;         // pinned, written by a pair sort's histogram
+  int pair_id_bits = 0;               // of the largest first id of the pairs sorted so far
   int passes_seen = 0;  // most digits that a replica sort of this context needed
   bool swept = false;   // the prepared scenes have been swept (their pair counters hold)
   unsigned long long *h_scene_pairs = nullptr;  // pinned readback

@@ -12,22 +12,24 @@
 // are running: the wait always ends; it is bounded all the same). A digit
 // that is the same in every key is skipped.
 //
+// It sorts the replicas of a prepare, and those pairs that the bucket sort
+// (pair_sort.cu) cannot take.
+//
 // What bounds it: the integer pipe (70% busy in a pass, shared-memory
 // wavefronts 50%, DRAM 31%), that is the stable ranks. Measured against a
 // histogram, two scans and a scatter per digit, with no digit skipped
 // (CUDA events): 92 M pairs 5.58 -> 3.13 ms (six digits of 46 used bits are
-// run, two skipped; 9.6 GB at 3.1 TB/s), 2.1 M pairs 249 -> 138 us, 346,000
-// pairs 158 -> 70 us, 6,700 pairs 138 -> 22 us.
+// run, two skipped; 9.6 GB at 3.1 TB/s).
 #include <algorithm>
 
-#include "stq_device.cuh"
+#include "radix_device.cuh"
 #include "stq_internal.h"
 
 namespace stq {
 
 namespace {
 
-constexpr int kBins = 256;
+constexpr int kBins = kRadixBins;
 constexpr int kMaxPasses = 8;
 constexpr int kPassBlock = 512;
 constexpr int kPassWarps = kPassBlock / 32;
@@ -218,31 +220,6 @@ __device__ __forceinline__ uint32_t look_back(const unsigned long long *status, 
   return sum;
 }
 
-// Digit of a key (digits are whole bytes).
-__device__ __forceinline__ unsigned digit_of(uint32_t k, int shift) { return __byte_perm(k, 0, 0x4440 | (shift >> 3)); }
-__device__ __forceinline__ unsigned digit_of(unsigned long long k, int shift) {
-  return digit_of(shift >= 32 ? uint32_t(k >> 32) : uint32_t(k), shift & 31);
-}
-
-// Lanes of the warp whose digit is d: one ballot per bit, four instructions
-// each. The ranking is what bounds a pass (the integer pipe is 70% busy), and
-// __match_any_sync is slower: 92 M pairs take 4.68 ms with it, 3.51 with
-// ballots as the compiler writes them, 3.16 with these.
-__device__ __forceinline__ unsigned same_digit(unsigned d) {
-  unsigned m = kFullMask;
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    unsigned v, s;  // v: lanes whose bit is set; s: 0 if this lane's is, else all ones
-    asm volatile(
-        "{ .reg .pred p; .reg .b32 t; and.b32 t, %2, %3; setp.ne.u32 p, t, 0;\n"
-        "vote.sync.ballot.b32 %0, p, 0xffffffff; selp.b32 %1, 0, 0xffffffff, p; }"
-        : "=r"(v), "=r"(s)
-        : "r"(d), "r"(1u << b));
-    m &= v ^ s;
-  }
-  return m;
-}
-
 template <typename K, bool VALS, int ITEMS>
 struct PassShared {
   static constexpr int kTile = kPassBlock * ITEMS;
@@ -356,55 +333,47 @@ radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const uns
 
 // A whole sort of at most kPassBlock * ITEMS keys by one block: keys (and
 // values) stay in registers and shared memory between the digits. A small sort
-// is all latency: 6,700 pairs take 22 us in this one launch, 30,000 pairs 60 us
-// in the launches above (8 us for each digit run, 2.4 for each skipped).
-template <typename K, bool VALS, int ITEMS>
+// is all latency: 6,600 replicas take 16 us in this one launch; in the launches
+// above each digit run costs 8 us and each skipped one 2.4.
+template <int ITEMS>
 struct BlockShared {
-  K stage[kPassBlock * ITEMS];
-  uint32_t vstage[VALS ? kPassBlock * ITEMS : 1];
+  uint32_t stage[kPassBlock * ITEMS];
+  uint32_t vstage[kPassBlock * ITEMS];
   uint32_t cnt[kPassWarps][kBins];
   uint32_t scratch[8];
-  unsigned long long any, all;  // OR and AND of the keys
+  uint32_t any, all;  // OR and AND of the keys
 };
 
-template <typename K, bool VALS, int ITEMS>
+template <int ITEMS>
 __global__ void __launch_bounds__(kPassBlock)
-radix_block_kernel(const K *k0, const K *k1, K *kout, const uint32_t *v0, const uint32_t *v1, uint32_t *vout, int n,
-                   const unsigned int *d_n, Digits dg) {
+radix_block_kernel(const uint32_t *k0, const uint32_t *k1, uint32_t *kout, const uint32_t *v0, const uint32_t *v1,
+                   uint32_t *vout, int n, const unsigned int *d_n, Digits dg) {
   if (d_n && int(*d_n) < n) n = int(*d_n);
   const bool second = dg.d_passes && (*dg.d_passes & 1u);
-  const K *kin = second ? k1 : k0;
+  const uint32_t *kin = second ? k1 : k0;
   const uint32_t *vin = second ? v1 : v0;
-  using S = BlockShared<K, VALS, ITEMS>;
+  using S = BlockShared<ITEMS>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   S &sm = *reinterpret_cast<S *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int first = warp * 32 * ITEMS + lane;
   const unsigned below = lanemask_lt();
   uint32_t *cnt = sm.cnt[warp];
-  K key[ITEMS];
-  uint32_t val[VALS ? ITEMS : 1];
-  K o = K(0), a = ~K(0);
+  uint32_t key[ITEMS], val[ITEMS], o = 0u, a = ~0u;
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
     const bool in = first + i * 32 < n;
-    key[i] = in ? kin[first + i * 32] : ~K(0);
-    if (VALS) val[i] = in ? vin[first + i * 32] : 0u;
+    key[i] = in ? kin[first + i * 32] : ~0u;
+    val[i] = in ? vin[first + i * 32] : 0u;
     if (in) o |= key[i], a &= key[i];
   }
-  if (tid == 0) sm.any = 0ull, sm.all = ~0ull;
+  if (tid == 0) sm.any = 0u, sm.all = ~0u;
   __syncthreads();
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    o |= __shfl_xor_sync(kFullMask, o, s);
-    a &= __shfl_xor_sync(kFullMask, a, s);
-  }
-  if (lane == 0) {
-    atomicOr(&sm.any, (unsigned long long)o);
-    atomicAnd(&sm.all, (unsigned long long)a);
-  }
+  o = __reduce_or_sync(kFullMask, o);
+  a = __reduce_and_sync(kFullMask, a);
+  if (lane == 0) atomicOr(&sm.any, o), atomicAnd(&sm.all, a);
   __syncthreads();
-  const K varies = K(sm.any & ~sm.all);  // bits that are not the same in every key
+  const uint32_t varies = sm.any & ~sm.all;  // bits that are not the same in every key
   for (int p = 0; p < dg.passes; ++p) {
     const int shift = dg.shift[p];
     if (((varies >> shift) & (kBins - 1)) == 0) continue;
@@ -439,7 +408,7 @@ radix_block_kernel(const K *k0, const K *k1, K *kout, const uint32_t *v0, const 
       if (first + i * 32 < n) {
         const uint32_t r = at + __popc(peers & below);
         sm.stage[r] = key[i];
-        if (VALS) sm.vstage[r] = val[i];
+        sm.vstage[r] = val[i];
       }
     }
     __syncthreads();
@@ -447,7 +416,7 @@ radix_block_kernel(const K *k0, const K *k1, K *kout, const uint32_t *v0, const 
     for (int i = 0; i < ITEMS; ++i)
       if (first + i * 32 < n) {
         key[i] = sm.stage[first + i * 32];
-        if (VALS) val[i] = sm.vstage[first + i * 32];
+        val[i] = sm.vstage[first + i * 32];
       }
     // the next digit writes the stage after two more barriers
   }
@@ -455,18 +424,8 @@ radix_block_kernel(const K *k0, const K *k1, K *kout, const uint32_t *v0, const 
   for (int i = 0; i < ITEMS; ++i)
     if (first + i * 32 < n) {
       kout[first + i * 32] = key[i];
-      if (VALS) vout[first + i * 32] = val[i];
+      vout[first + i * 32] = val[i];
     }
-}
-
-int sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
-    (void)cudaGetLastError();
-    sms = 152;
-  }
-  return sms;
 }
 
 template <typename K, bool VALS, int ITEMS>
@@ -487,15 +446,14 @@ cudaError_t launch_passes(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf
   return cudaSuccess;
 }
 
-template <typename K, bool VALS, int ITEMS>
-cudaError_t launch_block(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const Digits &dg,
+template <int ITEMS>
+cudaError_t launch_block(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const Digits &dg,
                          const unsigned int *d_n, int64_t *launches) {
-  constexpr auto kern = radix_block_kernel<K, VALS, ITEMS>;
-  constexpr size_t smem = sizeof(BlockShared<K, VALS, ITEMS>);
+  constexpr auto kern = radix_block_kernel<ITEMS>;
+  constexpr size_t smem = sizeof(BlockShared<ITEMS>);
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  kern<<<1, kPassBlock, smem, s>>>(kbuf[0], kbuf[1], kbuf[0], VALS ? vbuf[0] : nullptr, VALS ? vbuf[1] : nullptr,
-                                   VALS ? vbuf[0] : nullptr, int(n), d_n, dg);
+  kern<<<1, kPassBlock, smem, s>>>(kbuf[0], kbuf[1], kbuf[0], vbuf[0], vbuf[1], vbuf[0], int(n), d_n, dg);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
@@ -504,10 +462,6 @@ template <typename K, bool VALS>
 cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const unsigned int *d_n,
                       const Digits &dg, void *workspace, int *fault, int64_t *launches) {
   if (dg.passes == 0 || (n <= 1 && !dg.d_passes)) return cudaSuccess;
-  // one block up to its 16 keys per thread
-  if (n <= kPassBlock * 2) return launch_block<K, VALS, 2>(s, kbuf, vbuf, n, dg, d_n, launches);
-  if (n <= kPassBlock * 8) return launch_block<K, VALS, 8>(s, kbuf, vbuf, n, dg, d_n, launches);
-  if (n <= kPassBlock * 16) return launch_block<K, VALS, 16>(s, kbuf, vbuf, n, dg, d_n, launches);
   SortHead *head = static_cast<SortHead *>(workspace);
   unsigned long long *status = reinterpret_cast<unsigned long long *>(static_cast<char *>(workspace) +
                                                                       kRadixHeadBytes);
@@ -516,7 +470,7 @@ cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2],
   // large tiles write longer digit runs and look back over fewer tiles; small
   // inputs take small ones, so that every SM gets a tile. The line is at half a
   // large tile per SM: 1.0 M u32 keys take 74 us in large tiles and 91 in small
-  // ones, 346,000 pairs 78 us in large and 70 in small ones.
+  // ones, 346,000 64-bit keys 78 us in large and 70 in small ones.
   constexpr int kLarge = 16;
   static_assert(kPassBlock * kLarge >= 2 * kMinTile, "workspace sizing: status words of large tiles");
   const bool large = n >= int64_t(sm_count()) * 4096;
@@ -534,11 +488,26 @@ cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2],
 
 }  // namespace
 
+int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    (void)cudaGetLastError();
+    sms = 152;
+  }
+  return sms;
+}
+
 cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, void *workspace,
                            int *fault, int64_t *launches, const unsigned int *d_n, const unsigned int *d_passes,
                            int passes) {
-  return sort_impl<uint32_t, true>(s, kbuf, vbuf, n, d_n, Digits{passes, {0, 8, 16, 24}, d_passes}, workspace, fault,
-                                   launches);
+  const Digits dg{passes, {0, 8, 16, 24}, d_passes};
+  if (passes > 0 && (n > 1 || d_passes)) {  // one block up to its 16 keys per thread
+    if (n <= kPassBlock * 2) return launch_block<2>(s, kbuf, vbuf, n, dg, d_n, launches);
+    if (n <= kPassBlock * 8) return launch_block<8>(s, kbuf, vbuf, n, dg, d_n, launches);
+    if (n <= kPassBlock * 16) return launch_block<16>(s, kbuf, vbuf, n, dg, d_n, launches);
+  }
+  return sort_impl<uint32_t, true>(s, kbuf, vbuf, n, d_n, dg, workspace, fault, launches);
 }
 
 cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,

@@ -360,9 +360,23 @@ constexpr size_t radix_workspace_bytes(int64_t n) {
 cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, void *workspace,
                            int *fault, int64_t *launches, const unsigned int *d_n = nullptr,
                            const unsigned int *d_passes = nullptr, int passes = 4);
-// lexicographic by (first, second) as unsigned ids, in place; tmp holds n pairs
+// by digits; lexicographic by (first, second) as unsigned ids, in place; tmp holds n pairs
 cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,
                              int64_t *launches);
+// What the host needs of a pair sort's histogram, in page-locked memory.
+struct PairPlan {
+  unsigned int max_first;  // largest first id
+  unsigned int fits;       // no bucket was too long: the pairs are sorted
+};
+size_t pair_workspace_bytes(int64_t n);
+// Lexicographic sort of pairs by buckets of their first id (by digits where ids
+// have too many pairs), in place; tmp holds n pairs. May wait for the stream.
+// id_bits: bits of the largest first id of earlier sorts, kept for the next.
+cudaError_t sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, PairPlan *plan,
+                       int *id_bits, int *fault, int64_t *launches);
+// Multiprocessors of the current device.
+int sm_count();
+
 cudaError_t launch_sweep(cudaStream_t s, const SweepParams &p,
                          const SweepTuning &t, bool count_mode, int num_sms);
 // inclusive scan of box_counts[0..m) and the longest prefix whose pair sum

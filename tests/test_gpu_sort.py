@@ -1,23 +1,46 @@
-"""The device radix sort through stq_sort_pairs: sizes at the edges of its
-kernels (one block up to 1,024 / 4,096 / 8,192 pairs, tiles of 2,048 and 6,144
-pairs above), ids that use one digit, all four, or none."""
+"""The device sorts through stq_sort_pairs. Sizes at the edges of its kernels: one
+block up to 4,096 and 8,192 pairs, buckets of about 2,560 (at most 4,096) pairs
+above, segments of about 2^20 above 2^22. Ids that are few, wide, equal, or
+uneven: one first id with too many pairs for a bucket takes the radix sort, large
+groups of close pairs a bucket's digits."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2, 33, 1023, 1024, 1025, 4095, 4097, 8191, 8192, 8193, 10241, 100_003, 933_887, 933_889,
-                               2_000_003])
-@pytest.mark.parametrize("ids", ["small", "one_sided", "wide", "equal"])
-def test_sort_pairs_sizes_and_ids(ctx, cuda, n, ids):
+def draw(rng, n, ids):
+    if ids == "small":
+        return rng.integers(0, 200, (n, 2), dtype=np.uint32)
+    if ids == "wide":
+        return rng.integers(0, 1 << 32, (n, 2), dtype=np.uint32)
+    if ids == "equal":
+        return np.full((n, 2), 7, np.uint32)
+    if ids == "one_sided":
+        p = rng.integers(0, 70_000, (n, 2), dtype=np.uint32)
+        p[:, 0] = 5
+        return p
+    if ids == "groups":  # first ids of about 150 pairs each
+        p = rng.integers(0, 1 << 22, (n, 2), dtype=np.uint32)
+        p[:, 0] = rng.integers(0, max(n // 150, 1), n)
+        return p
+    if ids == "clumps":  # of about 600, in two narrow ranges of second ids
+        p = rng.integers(0, 250, (n, 2), dtype=np.uint32)
+        p[:, 1] += rng.integers(0, 2, n, dtype=np.uint32) << 30
+        p[:, 0] = rng.integers(0, max(n // 600, 1), n)
+        return p
+    if ids == "hub":  # a scene in which one box meets 1 in 50
+        p = rng.integers(0, max(n // 4, 2), (n, 2), dtype=np.uint32)
+        p[:: 50, 0] = n // 9
+        return p
+    p = rng.integers(0, max(n // 4, 2), (n, 2), dtype=np.uint32)  # "scene": 4 pairs per box
+    return np.sort(p, axis=1)
+
+
+def check(ctx, cuda, p):
     import torch
 
-    rng = np.random.default_rng(n)
-    hi = {"small": 200, "one_sided": 70_000, "wide": 1 << 32, "equal": 1}[ids]
-    p = rng.integers(0, hi, (n, 2), dtype=np.uint32)
-    if ids == "one_sided":
-        p[:, 0] = 5
+    n = len(p)
     want = p[np.lexsort((p[:, 1], p[:, 0]))]
     buf = torch.full((n + 64, 2), -7, dtype=torch.int32, device=cuda)
     buf[:n] = torch.from_numpy(p.view(np.int32)).to(cuda)
@@ -25,3 +48,23 @@ def test_sort_pairs_sizes_and_ids(ctx, cuda, n, ids):
     got = buf.cpu().numpy()
     assert np.array_equal(got[:n].view(np.uint32), want)
     assert np.all(got[n:] == -7)  # nothing written past the end
+
+
+@pytest.mark.parametrize("n", [2, 33, 1023, 4095, 4096, 4097, 8191, 8192, 8193, 10241, 100_003, 933_889, 2_000_003])
+@pytest.mark.parametrize("ids", ["small", "one_sided", "wide", "equal", "groups", "clumps", "hub", "scene"])
+def test_sort_pairs_sizes_and_ids(ctx, cuda, n, ids):
+    check(ctx, cuda, draw(np.random.default_rng(n), n, ids))
+
+
+@pytest.mark.parametrize("n", [(1 << 22) - 1, (1 << 22) + 1, 9_500_000])
+@pytest.mark.parametrize("ids", ["small", "wide", "groups", "clumps", "hub", "scene"])
+def test_sort_pairs_segments(ctx, cuda, n, ids):
+    check(ctx, cuda, draw(np.random.default_rng(n), n, ids))
+
+
+def test_sort_pairs_ids_that_grow_and_shrink(ctx, cuda):
+    """The bins' width follows the ids of earlier sorts: ids above it, and far
+    below it, sort the same."""
+    rng = np.random.default_rng(3)
+    for hi in (1000, 1 << 30, 50, 70_000, 1 << 20, 9):
+        check(ctx, cuda, rng.integers(0, hi, (60_000, 2), dtype=np.uint32))
