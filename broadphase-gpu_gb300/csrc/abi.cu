@@ -1132,13 +1132,22 @@ int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count) {
   if (!ctx || count < 0 || (count > 0 && !d_pairs)) return STQ_ERR_INVALID_ARG;
   if (count < 2) return STQ_OK;
   DeviceGuard g(ctx->device);
-  STQ_CUDA(ctx, ctx->pair_tmp.ensure(sizeof(stq_pair) * size_t(count)), "allocate pair buffer");
+  // the sort reads a pair as one word: pairs that are not on 8 bytes are sorted in a copy
+  const bool copy = reinterpret_cast<uintptr_t>(d_pairs) % sizeof(unsigned long long) != 0;
+  STQ_CUDA(ctx, ctx->pair_tmp.ensure(sizeof(stq_pair) * size_t(count) * (copy ? 2 : 1)), "allocate pair buffer");
   STQ_CUDA(ctx, ctx->sort_ws.ensure(pair_workspace_bytes(count)), "allocate sort workspace");
+  stq_pair *pairs = copy ? ctx->pair_tmp.as<stq_pair>() + count : d_pairs;
   *ctx->h_fault = 0;
   stage_begin(ctx, kPairSort);
-  STQ_CUDA(ctx, sort_pairs(ctx->stream, d_pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->sort_ws.ptr, ctx->h_plan,
+  if (copy)
+    STQ_CUDA(ctx, cudaMemcpyAsync(pairs, d_pairs, sizeof(stq_pair) * size_t(count), cudaMemcpyDeviceToDevice,
+                                  ctx->stream), "copy pairs");
+  STQ_CUDA(ctx, sort_pairs(ctx->stream, pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->sort_ws.ptr, ctx->h_plan,
                            &ctx->pair_id_bits, ctx->h_fault, &ctx->launches),
            "launch pair sort");
+  if (copy)
+    STQ_CUDA(ctx, cudaMemcpyAsync(d_pairs, pairs, sizeof(stq_pair) * size_t(count), cudaMemcpyDeviceToDevice,
+                                  ctx->stream), "copy sorted pairs");
   stage_end(ctx, kPairSort);
   STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
   collect_stages(ctx);

@@ -68,3 +68,17 @@ def test_sort_pairs_ids_that_grow_and_shrink(ctx, cuda):
     rng = np.random.default_rng(3)
     for hi in (1000, 1 << 30, 50, 70_000, 1 << 20, 9):
         check(ctx, cuda, rng.integers(0, hi, (60_000, 2), dtype=np.uint32))
+
+
+@pytest.mark.parametrize("n", [5, 5000, 20_001])
+def test_sort_pairs_on_a_four_byte_boundary(ctx, cuda, n):
+    """A pair is two 32-bit ids: any 4-byte boundary is taken."""
+    import torch
+
+    p = draw(np.random.default_rng(n), n, "scene")
+    flat = torch.full((2 * n + 3,), -7, dtype=torch.int32, device=cuda)
+    flat[1 : 2 * n + 1] = torch.from_numpy(p.view(np.int32).reshape(-1)).to(cuda)
+    ctx.sort_pairs(flat[1:], n)
+    got = flat.cpu().numpy()
+    assert np.array_equal(got[1 : 2 * n + 1].view(np.uint32).reshape(n, 2), p[np.lexsort((p[:, 1], p[:, 0]))])
+    assert got[0] == -7 and np.all(got[2 * n + 1 :] == -7)
