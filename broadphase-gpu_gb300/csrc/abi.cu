@@ -514,15 +514,16 @@ int stq_context_create(int device, void *stream, stq_context **out) {
   DeviceGuard g(device);
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   apply_options(ctx);
-  if (cudaMallocHost(&ctx->h_hdr, sizeof(BatchHeader)) != cudaSuccess ||
-      cudaMallocHost(&ctx->h_fault, sizeof(int)) != cudaSuccess ||
-      cudaMallocHost(&ctx->h_flags, sizeof(int)) != cudaSuccess ||
-      cudaMallocHost(&ctx->h_front, sizeof(FrontInfo)) != cudaSuccess ||
-      cudaMallocHost(&ctx->h_plan, sizeof(PairPlan)) != cudaSuccess ||
+  if (cudaMallocHost(&ctx->h_block, sizeof(HostBlock)) != cudaSuccess ||
       ctx->aux.ensure(sizeof(BatchHeader)) != cudaSuccess || ensure_staging(ctx, 1, 1) != STQ_OK) {
     stq_context_destroy(ctx);
     return STQ_ERR_NO_MEMORY;
   }
+  ctx->h_hdr = &ctx->h_block->hdr;
+  ctx->h_front = &ctx->h_block->front;
+  ctx->h_plan = &ctx->h_block->plan;
+  ctx->h_fault = &ctx->h_block->fault;
+  ctx->h_flags = &ctx->h_block->flags;
   *out = ctx;
   return STQ_OK;
 }
@@ -540,11 +541,7 @@ void stq_context_destroy(stq_context *ctx) {
     for (DevBuf *b : ctx->buffers())
       b->release();
     if (ctx->in_host) cudaFreeHost(ctx->in_host);
-    if (ctx->h_hdr) cudaFreeHost(ctx->h_hdr);
-    if (ctx->h_fault) cudaFreeHost(ctx->h_fault);
-    if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
-    if (ctx->h_front) cudaFreeHost(ctx->h_front);
-    if (ctx->h_plan) cudaFreeHost(ctx->h_plan);
+    if (ctx->h_block) cudaFreeHost(ctx->h_block);
     if (ctx->front_event) cudaEventDestroy(ctx->front_event);
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     if (ctx->copy_stream) {

@@ -57,6 +57,16 @@ struct GraphKey {
   }
 };
 
+// Words that kernels or copies write for the host, in one page-locked block (an
+// allocation of page-locked memory takes some 10 us).
+struct HostBlock {
+  alignas(128) BatchHeader hdr;
+  alignas(128) FrontInfo front;
+  alignas(128) PairPlan plan;
+  alignas(128) int fault;
+  alignas(128) int flags;
+};
+
 struct stq_context {
   int device = 0;
   int num_sms = 152;
@@ -90,12 +100,13 @@ struct stq_context {
   int n_scenes = 0;
   int64_t n_boxes = 0, length = 0;
   SortedScene scene;
-  BatchHeader *h_hdr = nullptr;             // pinned readback
-  int *h_fault = nullptr;  // pinned, written by a pair sort whose wait ran out
-  int *h_flags = nullptr;  // pinned, written by a box build with a bad index
-  FrontInfo *h_front = nullptr;       // pinned, written by a prepare's first half
+  HostBlock *h_block = nullptr;       // pinned; the pointers below are into it
+  BatchHeader *h_hdr = nullptr;       // readback
+  int *h_fault = nullptr;             // written by a pair sort whose wait ran out
+  int *h_flags = nullptr;             // written by a box build with a bad index
+  FrontInfo *h_front = nullptr;       // written by a prepare's first half
   cudaEvent_t front_event = nullptr;  // after it
-  PairPlan *h_plan = nullptr;         // pinned, written by a pair sort's histogram
+  PairPlan *h_plan = nullptr;         // written by a pair sort's histogram
   int pair_id_bits = 0;               // of the largest first id of the pairs sorted so far
   int passes_seen = 0;  // most digits that a replica sort of this context needed
   bool swept = false;   // the prepared scenes have been swept (their pair counters hold)

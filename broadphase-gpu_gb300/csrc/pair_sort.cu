@@ -6,8 +6,9 @@
 // A partition kernel moves the pairs to their buckets, in no order (its ranks are
 // shared-memory atomics, a third of the instructions of a radix pass's stable
 // ranks). In a bucket, pairs are grouped by first id and the leading bits of the
-// second the same way, and each pair counts the smaller ones of its group. Above 4 M pairs the same histogram and partition first cut
-// them into segments of about a million. Up to 8,192 pairs are one bucket.
+// second the same way, and each pair counts the smaller ones of its group. Above
+// 4 M pairs the same histogram and partition first cut them into segments of about
+// a million. Up to 8,192 pairs are one bucket.
 //
 // Bins hold whole ids, so ids with very many pairs make large buckets: where one
 // passes 4,096 pairs the later kernels do nothing, and once the host sees that,
