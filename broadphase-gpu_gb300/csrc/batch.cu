@@ -252,6 +252,7 @@ scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, cons
 __global__ void __launch_bounds__(kBlock)
 batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
                    const long long *__restrict__ box_off, SceneInput *inputs, SceneRecord *scenes, BatchHeader *hdr) {
+  after_previous();
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
   // moments about the tile's first box centre, in fp32 per thread (fp64 is
@@ -487,6 +488,7 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
                       SceneRecord *scenes, unsigned int *cell_base, unsigned long long *tile_reps, uint32_t *tile_off,
                       BatchHeader *hdr, FrontInfo *front, long long rep_cap, long long seg_cap, int max_passes,
                       uint2 *__restrict__ box_cells, uint32_t *__restrict__ box_q) {
+  after_previous();
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
   const SceneRecord &r = scenes[t.scene];
@@ -552,6 +554,7 @@ batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restric
                   const TileRec *__restrict__ tiles, const uint32_t *__restrict__ tile_off,
                   const SceneRecord *__restrict__ scenes, const unsigned int *__restrict__ cell_base,
                   const BatchHeader *hdr, uint32_t *k0, uint32_t *k1, uint32_t *v0, uint32_t *v1) {
+  after_previous();
   if (hdr->replicas == 0u || int(blockIdx.x) >= hdr->n_tiles) return;
   const int key_bits = hdr->key_bits;
   const bool second = hdr->passes & 1u;
@@ -618,6 +621,7 @@ batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restric
 __global__ void __launch_bounds__(kBlock)
 list_offsets_kernel(const uint32_t *__restrict__ keys, BatchHeader *__restrict__ hdr,
                     uint32_t *__restrict__ seg_scan, long long seg_cap, SortedScene scene, int64_t slots_cap) {
+  after_previous();
   // (cells past the capacity are flagged and counted as none)
   const uint32_t nseg = uint32_t(min(3ll * hdr->cells, seg_cap));
   const uint32_t R = hdr->replicas;
@@ -706,6 +710,7 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const uint32_t *__restri
                     const unsigned int *__restrict__ cell_base,
                     const SceneRecord *__restrict__ scenes, const uint32_t *__restrict__ seg_scan,
                     SortedScene scene) {
+  after_previous();
   const int64_t R = hdr->replicas;
   const int S = hdr->n_scenes;
   const int key_bits = hdr->key_bits;
@@ -812,6 +817,7 @@ int wave_blocks(const void *kernel, int64_t n) {
 
 __global__ void __launch_bounds__(kBlock)
 reset_sweep_kernel(BatchHeader *hdr, unsigned long long *scene_pairs) {
+  after_previous();
   const int S = hdr->n_scenes;
   for (int s = blockIdx.x * kBlock + threadIdx.x; s < S; s += gridDim.x * kBlock)
     scene_pairs[s] = 0ull;
@@ -829,6 +835,7 @@ reset_sweep_kernel(BatchHeader *hdr, unsigned long long *scene_pairs) {
 // between two windows of a stream while the engines move pair lists) and
 // restarts the slot's cursors for its next window.
 __global__ void window_step_kernel(WindowCounters *wc, unsigned long long *host_count) {
+  after_previous();
   if (threadIdx.x != 0) return;
   *reinterpret_cast<volatile unsigned long long *>(host_count) = wc->pairs;
   wc->work = 0;
@@ -840,44 +847,45 @@ __global__ void window_step_kernel(WindowCounters *wc, unsigned long long *host_
 }  // namespace
 
 cudaError_t launch_window_step(cudaStream_t s, WindowCounters *wc, unsigned long long *host_count) {
-  window_step_kernel<<<1, 32, 0, s>>>(wc, host_count);
+  launch_after(window_step_kernel, 1, 32, 0, s, wc, host_count);
   return cudaGetLastError();
 }
 
 cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long long *scene_pairs,
                                int scene_cap) {
-  reset_sweep_kernel<<<blocks_for(scene_cap, 64), kBlock, 0, s>>>(hdr, scene_pairs);
+  launch_after(reset_sweep_kernel, blocks_for(scene_cap, 64), kBlock, 0, s, hdr, scene_pairs);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b) {
-  batch_stats_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.box_off, b.inputs, b.scenes, b.hdr);
+  launch_after(batch_stats_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.boxes, b.tiles, b.box_off, b.inputs,
+               b.scenes, b.hdr);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap, int passes) {
-  batch_box_keys_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.boxes, b.tiles, b.box_off, b.inputs, b.scenes,
-                                                                b.cell_base, b.tile_reps, b.tile_off, b.hdr, b.front,
-                                                                rep_cap, seg_cap, passes, b.box_cells, b.box_q);
+  launch_after(batch_box_keys_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.boxes, b.tiles, b.box_off, b.inputs,
+               b.scenes, b.cell_base, b.tile_reps, b.tile_off, b.hdr, b.front, rep_cap, seg_cap, passes, b.box_cells,
+               b.box_q);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b) {
-  batch_emit_kernel<<<unsigned(b.tile_cap), kBlock, 0, s>>>(b.box_cells, b.box_q, b.tiles, b.tile_off, b.scenes,
-                                                            b.cell_base, b.hdr, b.keys[0], b.keys[1], b.vals[0],
-                                                            b.vals[1]);
+  launch_after(batch_emit_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.box_cells, b.box_q, b.tiles, b.tile_off,
+               b.scenes, b.cell_base, b.hdr, b.keys[0], b.keys[1], b.vals[0], b.vals[1]);
   return cudaGetLastError();
 }
 
 cudaError_t launch_list_offsets(cudaStream_t s, const uint32_t *keys, BatchHeader *hdr, uint32_t *seg_scan,
                                 int64_t seg_cap, const SortedScene &scene, int64_t slots_cap) {
-  list_offsets_kernel<<<blocks_for((seg_cap + 1) / (kBlock - 1) * kBlock + kBlock), kBlock, 0, s>>>(keys, hdr, seg_scan, seg_cap, scene, slots_cap);
+  launch_after(list_offsets_kernel, blocks_for((seg_cap + 1) / (kBlock - 1) * kBlock + kBlock), kBlock, 0, s, keys,
+               hdr, seg_scan, seg_cap, scene, slots_cap);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gather_cells(cudaStream_t s, const BatchBuffers &b, int64_t replicas, const SortedScene &scene) {
-  gather_cells_kernel<<<wave_blocks((const void *)gather_cells_kernel, replicas), kBlock, 0, s>>>(
-      b.boxes, b.keys[0], b.vals[0], b.box_q, b.hdr, b.cell_base, b.scenes, b.seg_scan, scene);
+  launch_after(gather_cells_kernel, wave_blocks((const void *)gather_cells_kernel, replicas), kBlock, 0, s, b.boxes,
+               b.keys[0], b.vals[0], b.box_q, b.hdr, b.cell_base, b.scenes, b.seg_scan, scene);
   return cudaGetLastError();
 }
 

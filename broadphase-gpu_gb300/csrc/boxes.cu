@@ -42,6 +42,7 @@ __device__ __forceinline__ void load_rounded(const float4 *P, int64_t i, float p
 __global__ void __launch_bounds__(256)
 round_points_kernel(const double *__restrict__ V0, const double *__restrict__ V1, int64_t nV,
                     float4 *__restrict__ P) {
+  after_previous();
   for (int64_t v = blockIdx.x * 256ll + threadIdx.x; v < nV; v += int64_t(gridDim.x) * 256) {
     float a[3], b[3];
     load_point(V0, v, a);
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(256)
 batch_round_points_kernel(const double *__restrict__ V0, const double *__restrict__ V1,
                           const long long *__restrict__ voff, const BatchHeader *hdr, int64_t vert_cap,
                           float4 *__restrict__ P) {
+  after_previous();
   const long long n = voff[hdr->n_scenes];
   const int64_t nV = n < vert_cap ? n : vert_cap;
   for (int64_t v = blockIdx.x * 256ll + threadIdx.x; v < nV; v += int64_t(gridDim.x) * 256) {
@@ -187,6 +189,7 @@ build_boxes_kernel(const double *__restrict__ V0, const double *__restrict__ V1,
                    int64_t nV, const int32_t *__restrict__ E, int64_t nE,
                    const int32_t *__restrict__ F, int64_t nF, float r_up,
                    stq_aabb *__restrict__ out, int *flags, const float4 *__restrict__ P) {
+  after_previous();
   __shared__ uint32_t stage[kBuildBlock / 32][32 * kBoxWords];
   const int lane = threadIdx.x & 31;
   const int64_t N = nV + nE + nF;
@@ -208,6 +211,7 @@ batch_build_kernel(const double *__restrict__ V0, const double *__restrict__ V1,
                    const long long *__restrict__ foff, const long long *__restrict__ box_off,
                    BatchHeader *hdr, float r_up, stq_aabb *__restrict__ out,
                    const float4 *__restrict__ P) {
+  after_previous();
   __shared__ uint32_t stage[kBuildBlock / 32][32 * kBoxWords];
   const int lane = threadIdx.x & 31;
   const int n_scenes = hdr->n_scenes;
@@ -240,6 +244,7 @@ batch_build_kernel(const double *__restrict__ V0, const double *__restrict__ V1,
 __global__ void __launch_bounds__(kBuildBlock)
 batch_build_refs_kernel(const MeshRef *__restrict__ refs, const long long *__restrict__ box_off,
                         BatchHeader *hdr, float r_up, stq_aabb *__restrict__ out) {
+  after_previous();
   __shared__ uint32_t stage[kBuildBlock / 32][32 * kBoxWords];
   const int lane = threadIdx.x & 31;
   const int n_scenes = hdr->n_scenes;
@@ -279,9 +284,9 @@ cudaError_t launch_build_boxes(cudaStream_t s, const double *V0, const double *V
                                stq_aabb *out, int *flags, float4 *points) {
   const int64_t N = nV + nE + nF;
   if (N == 0) return cudaSuccess;
-  if (nV > 0) round_points_kernel<<<grid_for(nV, 256), 256, 0, s>>>(V0, V1, nV, points);
-  build_boxes_kernel<<<grid_for(N, kBuildBlock), kBuildBlock, 0, s>>>(
-      V0, V1, nV, E, nE, F, nF, r_up, out, flags, nV > 0 ? points : nullptr);
+  if (nV > 0) launch_after(round_points_kernel, grid_for(nV, 256), 256, 0, s, V0, V1, nV, points);
+  launch_after(build_boxes_kernel, grid_for(N, kBuildBlock), kBuildBlock, 0, s, V0, V1, nV, E, nE, F, nF, r_up, out,
+               flags, nV > 0 ? points : nullptr);
   return cudaGetLastError();
 }
 
@@ -290,16 +295,16 @@ cudaError_t launch_batch_build(cudaStream_t s, const double *V0, const double *V
                                const int32_t *F, const long long *foff, const long long *box_off,
                                BatchHeader *hdr, int64_t box_cap, float r_up, stq_aabb *out,
                                float4 *points, int64_t vert_cap) {
-  batch_round_points_kernel<<<grid_for(vert_cap, 256), 256, 0, s>>>(V0, V1, voff, hdr, vert_cap, points);
-  batch_build_kernel<<<grid_for(box_cap, kBuildBlock), kBuildBlock, 0, s>>>(
-      V0, V1, voff, E, eoff, F, foff, box_off, hdr, r_up, out, points);
+  launch_after(batch_round_points_kernel, grid_for(vert_cap, 256), 256, 0, s, V0, V1, voff, hdr, vert_cap, points);
+  launch_after(batch_build_kernel, grid_for(box_cap, kBuildBlock), kBuildBlock, 0, s, V0, V1, voff, E, eoff, F, foff,
+               box_off, hdr, r_up, out, points);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_build_refs(cudaStream_t s, const MeshRef *refs, const long long *box_off,
                                     BatchHeader *hdr, int64_t box_cap, float r_up, stq_aabb *out) {
-  batch_build_refs_kernel<<<grid_for(box_cap, kBuildBlock), kBuildBlock, 0, s>>>(refs, box_off, hdr,
-                                                                                 r_up, out);
+  launch_after(batch_build_refs_kernel, grid_for(box_cap, kBuildBlock), kBuildBlock, 0, s, refs, box_off, hdr, r_up,
+               out);
   return cudaGetLastError();
 }
 

@@ -264,6 +264,7 @@ __device__ void plan_segment(const PairLevel &lv, const PairSeg &sg, int which, 
 // Histogram of the first ids of one tile of a segment (of `tile` pairs).
 __global__ void __launch_bounds__(kBlock)
 pair_hist_kernel(const unsigned long long *__restrict__ pairs, PairSeg one, PairSeg *segs, uint32_t tile, PairLevel lv) {
+  after_previous();
   __shared__ uint32_t h[kPairBins + kPairBins / 32];
   __shared__ uint32_t scratch[kWarps];
   __shared__ bool last;
@@ -320,6 +321,7 @@ template <int ITEMS>
 __global__ void __launch_bounds__(kBlock, 2)
 pair_partition_kernel(const unsigned long long *__restrict__ in, unsigned long long *__restrict__ out, PairSeg one,
                       const PairSeg *segs, PairLevel lv) {
+  after_previous();
   constexpr uint32_t TILE = kBlock * ITEMS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PartShared<ITEMS> &sm = *reinterpret_cast<PartShared<ITEMS> *>(smem_raw);
@@ -401,6 +403,7 @@ template <int THREADS, int CAP, bool AUTO>
 __global__ void __launch_bounds__(THREADS, AUTO ? 1 : 2048 / THREADS)
 pair_bucket_kernel(const unsigned long long *in, unsigned long long *out, const PairBucket *__restrict__ buckets,
                    const PairHead *head, int n) {
+  after_previous();
   constexpr int ITEMS = CAP / THREADS;
   static_assert(kGroups % THREADS == 0, "groups per thread");
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -586,7 +589,7 @@ cudaError_t launch_partition(cudaStream_t s, int64_t blocks, const unsigned long
   constexpr size_t smem = sizeof(PartShared<ITEMS>);
   const cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  kern<<<unsigned(blocks), kBlock, smem, s>>>(in, out, one, segs, lv);
+  launch_after(kern, unsigned(blocks), kBlock, smem, s, in, out, one, segs, lv);
   return cudaGetLastError();
 }
 
@@ -597,7 +600,7 @@ cudaError_t launch_buckets(cudaStream_t s, int64_t blocks, const unsigned long l
   constexpr size_t smem = sizeof(BucketShared<THREADS, CAP>);
   const cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  kern<<<unsigned(blocks), THREADS, smem, s>>>(in, out, buckets, head, n);
+  launch_after(kern, unsigned(blocks), THREADS, smem, s, in, out, buckets, head, n);
   return cudaGetLastError();
 }
 
@@ -663,7 +666,7 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
     cudaError_t e = clear(first, two ? 0 : 1, 1);
     if (e == cudaSuccess && two) e = clear(last, 1, l.segs);
     if (e != cudaSuccess) return e;
-    pair_hist_kernel<<<unsigned(div_up(n, tile)), kBlock, 0, s>>>(a, one, nullptr, uint32_t(tile), first);
+    launch_after(pair_hist_kernel, unsigned(div_up(n, tile)), kBlock, 0, s, a, one, nullptr, uint32_t(tile), first);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // every later kernel looks whether the buckets fit, and does nothing if not
     e = n >= int64_t(sm_count()) * 8192 ? launch_partition<16>(s, div_up(n, kBlock * 16), a, b, one, nullptr, first)
@@ -671,7 +674,7 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
     if (e != cudaSuccess) return e;
     *launches += 2;
     if (two) {
-      pair_hist_kernel<<<unsigned(n / kHistTile + l.segs), kBlock, 0, s>>>(b, one, segs, kHistTile, last);
+      launch_after(pair_hist_kernel, unsigned(n / kHistTile + l.segs), kBlock, 0, s, b, one, segs, kHistTile, last);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       e = launch_partition<16>(s, n / kPairPartTile + l.segs, b, a, one, segs, last);
       if (e != cudaSuccess) return e;

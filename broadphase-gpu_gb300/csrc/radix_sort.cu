@@ -99,6 +99,7 @@ template <typename K>
 __global__ void __launch_bounds__(kHistBlock)
 radix_hist_kernel(const K *__restrict__ k0, const K *__restrict__ k1, int64_t n, const unsigned int *d_n, Digits dg,
                   SortHead *head, unsigned long long *status, int tile) {
+  after_previous();
   if (d_n && int64_t(*d_n) < n) n = *d_n;
   const K *__restrict__ keys = dg.d_passes && (*dg.d_passes & 1u) ? k1 : k0;
   __shared__ uint32_t h[kMaxPasses][kBins];
@@ -237,6 +238,7 @@ template <typename K, bool VALS, int ITEMS>
 __global__ void __launch_bounds__(kPassBlock, 2)
 radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const unsigned int *d_n, int pass, int shift,
                   SortHead *head, unsigned long long *status, int *fault) {
+  after_previous();
   if (!head->run[pass]) return;
   if (d_n && int64_t(*d_n) < n) n = *d_n;
   const bool flip = head->src[pass] != 0;
@@ -348,6 +350,7 @@ template <int ITEMS>
 __global__ void __launch_bounds__(kPassBlock)
 radix_block_kernel(const uint32_t *k0, const uint32_t *k1, uint32_t *kout, const uint32_t *v0, const uint32_t *v1,
                    uint32_t *vout, int n, const unsigned int *d_n, Digits dg) {
+  after_previous();
   if (d_n && int(*d_n) < n) n = int(*d_n);
   const bool second = dg.d_passes && (*dg.d_passes & 1u);
   const uint32_t *kin = second ? k1 : k0;
@@ -438,8 +441,8 @@ cudaError_t launch_passes(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf
   const int64_t tiles = (n + kPassBlock * ITEMS - 1) / (kPassBlock * ITEMS);
   const unsigned grid = unsigned(std::min<int64_t>(tiles, int64_t(sm_count()) * 2));
   for (int p = 0; p < dg.passes; ++p) {
-    kern<<<grid, kPassBlock, smem, s>>>(kbuf[0], kbuf[1], VALS ? vbuf[0] : nullptr, VALS ? vbuf[1] : nullptr, n, d_n, p,
-                                        dg.shift[p], head, status, fault);
+    launch_after(kern, grid, kPassBlock, smem, s, kbuf[0], kbuf[1], VALS ? vbuf[0] : nullptr,
+                 VALS ? vbuf[1] : nullptr, n, d_n, p, dg.shift[p], head, status, fault);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -453,7 +456,7 @@ cudaError_t launch_block(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *cons
   constexpr size_t smem = sizeof(BlockShared<ITEMS>);
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  kern<<<1, kPassBlock, smem, s>>>(kbuf[0], kbuf[1], kbuf[0], vbuf[0], vbuf[1], vbuf[0], int(n), d_n, dg);
+  launch_after(kern, 1, kPassBlock, smem, s, kbuf[0], kbuf[1], kbuf[0], vbuf[0], vbuf[1], vbuf[0], int(n), d_n, dg);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
@@ -476,8 +479,8 @@ cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2],
   const bool large = n >= int64_t(sm_count()) * 4096;
   const int tile = large ? kPassBlock * kLarge : kMinTile;
   const int64_t hist_blocks = (n + kHistBlock * 4 - 1) / (kHistBlock * 4);
-  radix_hist_kernel<K><<<unsigned(std::min<int64_t>(hist_blocks, int64_t(sm_count()) * 4)), kHistBlock, 0, s>>>(
-      kbuf[0], kbuf[1], n, d_n, dg, head, status, tile);
+  launch_after(radix_hist_kernel<K>, unsigned(std::min<int64_t>(hist_blocks, int64_t(sm_count()) * 4)), kHistBlock, 0,
+               s, kbuf[0], kbuf[1], n, d_n, dg, head, status, tile);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   e = large ? launch_passes<K, VALS, kLarge>(s, kbuf, vbuf, n, d_n, dg, head, status, fault)

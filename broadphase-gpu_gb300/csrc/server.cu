@@ -38,6 +38,7 @@ __device__ __forceinline__ double unit(unsigned long long h) {  // [0, 1)
 __global__ void __launch_bounds__(256)
 advance_kernel(const MeshRef *__restrict__ refs, const long long *__restrict__ voff,
                const BatchHeader *hdr, int64_t vert_cap) {
+  after_previous();
   const int S = hdr->n_scenes;
   const long long total = voff[S] < vert_cap ? voff[S] : vert_cap;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
@@ -92,6 +93,7 @@ template <bool SMEM>
 __global__ void __launch_bounds__(256)
 pair_checksum_kernel(const int2 *__restrict__ pairs, long long capacity, const BatchHeader *hdr,
                      const long long *__restrict__ box_off, unsigned long long *checks) {
+  after_previous();
   extern __shared__ unsigned long long block_checks[];  // SMEM: one per scene
   const long long n = min((long long)hdr->pairs, capacity);
   const int S = hdr->n_scenes;
@@ -160,7 +162,7 @@ cudaError_t launch_advance(cudaStream_t s, const MeshRef *refs, const long long 
                            const BatchHeader *hdr, int64_t vert_cap) {
   int64_t g = (vert_cap + 255) / 256;
   g = g < 1 ? 1 : (g > 152 * 16 ? 152 * 16 : g);
-  advance_kernel<<<unsigned(g), 256, 0, s>>>(refs, voff, hdr, vert_cap);
+  launch_after(advance_kernel, unsigned(g), 256, 0, s, refs, voff, hdr, vert_cap);
   return cudaGetLastError();
 }
 
@@ -172,11 +174,11 @@ cudaError_t launch_pair_checksums(cudaStream_t s, const stq_pair *pairs, long lo
   int64_t g = (capacity / kChecksumChunk + 7) / 8;  // 8 warps per block
   g = g < 1 ? 1 : (g > 152 * 16 ? 152 * 16 : g);
   if (scene_cap <= kChecksumSmemScenes)
-    pair_checksum_kernel<true><<<unsigned(g), 256, sizeof(unsigned long long) * size_t(scene_cap), s>>>(
-        reinterpret_cast<const int2 *>(pairs), capacity, hdr, box_off, checks);
+    launch_after(pair_checksum_kernel<true>, unsigned(g), 256, sizeof(unsigned long long) * size_t(scene_cap), s,
+                 reinterpret_cast<const int2 *>(pairs), capacity, hdr, box_off, checks);
   else
-    pair_checksum_kernel<false><<<unsigned(g), 256, 0, s>>>(reinterpret_cast<const int2 *>(pairs), capacity,
-                                                            hdr, box_off, checks);
+    launch_after(pair_checksum_kernel<false>, unsigned(g), 256, 0, s, reinterpret_cast<const int2 *>(pairs), capacity,
+                 hdr, box_off, checks);
   return cudaGetLastError();
 }
 

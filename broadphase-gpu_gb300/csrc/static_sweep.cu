@@ -53,6 +53,7 @@ static __device__ __align__(256) unsigned char g_static_scratch[kScratchBytes];
 // axes: the largest ~key(min) and key(max) of each (zero before this launch).
 __global__ void static_keys_kernel(const stq_aabb *__restrict__ boxes, int n, int axis,
                                    unsigned char *scratch) {
+  after_previous();
   BatchHeader *hdr = reinterpret_cast<BatchHeader *>(scratch + kOffHdr);
   uint32_t *keys = reinterpret_cast<uint32_t *>(scratch + kOffKeys0);
   uint32_t *vals = reinterpret_cast<uint32_t *>(scratch + kOffVals0);
@@ -90,6 +91,7 @@ __global__ void static_keys_kernel(const stq_aabb *__restrict__ boxes, int n, in
 __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, int axis,
                                      const uint32_t *__restrict__ keys, const uint32_t *__restrict__ order,
                                      unsigned char *scratch) {
+  after_previous();
   float4 *yz = reinterpret_cast<float4 *>(scratch + kOffYz);
   float2 *xx = reinterpret_cast<float2 *>(scratch + kOffX);
   int4 *v = reinterpret_cast<int4 *>(scratch + kOffV);
@@ -162,8 +164,7 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   // the header and the scene's pair counter start at zero (the array keeps
   // the last call's contents); a memset on the stream, not an allocation
   if (cudaMemsetAsync(scratch + kOffHdr, 0, kScratchBytes - kOffHdr, s) != cudaSuccess) return STQ_ERR_CUDA;
-  static_keys_kernel<<<(ni + 255) / 256 > 0 ? (ni + 255) / 256 : 1, 256, 0, s>>>(d_boxes, ni, axis,
-                                                                                   scratch);
+  launch_after(static_keys_kernel, (ni + 255) / 256 > 0 ? (ni + 255) / 256 : 1, 256, 0, s, d_boxes, ni, axis, scratch);
   uint32_t *kb[2] = {reinterpret_cast<uint32_t *>(scratch + kOffKeys0),
                      reinterpret_cast<uint32_t *>(scratch + kOffKeys1)};
   uint32_t *vb[2] = {reinterpret_cast<uint32_t *>(scratch + kOffVals0),
@@ -171,7 +172,7 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   BatchHeader *hdr = reinterpret_cast<BatchHeader *>(scratch + kOffHdr);
   if (radix_sort_u32(s, kb, vb, n, scratch + kOffSortWs, &hdr->fault, nullptr) != cudaSuccess)
     return STQ_ERR_CUDA;
-  static_gather_kernel<<<blocks, 256, 0, s>>>(d_boxes, ni, axis, kb[0], vb[0], scratch);
+  launch_after(static_gather_kernel, blocks, 256, 0, s, d_boxes, ni, axis, kb[0], vb[0], scratch);
   int num_sms = 152;
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   SweepParams p;

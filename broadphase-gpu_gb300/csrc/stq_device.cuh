@@ -20,6 +20,11 @@ static_assert(offsetof(stq_aabb, min) == 4 && offsetof(stq_aabb, max) == 16 &&
               "stq_aabb field offsets must match stq::gpu::Aabb");
 
 constexpr unsigned kFullMask = 0xffffffffu;
+
+// First statement of a kernel launched by launch_after: waits until the kernels
+// before it have ended and their writes are seen. Also in blocks that return at
+// once: a kernel that ended without the wait could end before those before it.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Padding after the last sentinel of a sorted scene, so that a lane group of
 // up to 32 lanes may read past a run end without leaving the allocation.
 constexpr int kSortedPad = 256;

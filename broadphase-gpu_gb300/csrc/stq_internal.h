@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdint>
 #include <string>
+#include <utility>
 
 #include <cuda_runtime.h>
 
@@ -47,6 +48,30 @@ cudaError_t allow_smem(size_t bytes) {
   e = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
   if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev);
   return e;
+}
+
+// Launches a kernel that is placed on the device while the last blocks of the one
+// before it in the stream end, and waits at its start (after_previous). A pass of a
+// small scene is some fifteen kernels of 3 to 15 us, and the gaps between plain
+// launches a tenth of it. Whole passes, plain -> so: 2,000 boxes 134 -> 119 us,
+// 53,000 boxes 195 -> 166, 477,000 boxes 331 -> 298; large scenes gain 1% (6 M
+// boxes) to 3%. Kernels do not let the next one in earlier: its waiting blocks take
+// shared memory from the running ones' L1 cache (16 scenes of 500,000 boxes
+// 1.38 ms plain, 1.35 so, 1.55 with the next let in at the start). Errors are
+// left to cudaGetLastError.
+template <typename... P, typename... A>
+void launch_after(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
 // Device-side scalars of one sweep: counters, flags and results read back

@@ -60,6 +60,7 @@ __device__ __forceinline__ void flush_staged(const int2 *st, int n, int lane, co
 template <int G, int Q, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_kernel(const SweepParams p) {
+  after_previous();
   static_assert(32 % G == 0, "lane group must divide the warp");
   // the refill tops the ring up to one entry per group: Q >= 32 / G
   static_assert((Q & (Q - 1)) == 0 && Q >= 16 && Q >= 32 / G, "queue depth: power of two >= 16 and >= groups");
@@ -220,6 +221,7 @@ stq_sweep_kernel(const SweepParams p) {
 template <int U, int Q, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_lane_kernel(const SweepParams p) {
+  after_previous();
   static_assert(U == 1 || U == 2 || U == 4 || U == 8, "candidates per lane step: 1, 2, 4 or 8");
   static_assert((Q & (Q - 1)) == 0 && Q >= 32, "queue depth: power of two >= 32");
   constexpr int STAGE = 32 * (U + 1);  // < 32 left over + at most 32 * U new pairs
@@ -444,6 +446,7 @@ struct FlatWarp {
 template <int BLOCK, int V, bool COUNT, bool LONG>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_flat_kernel(const SweepParams p) {
+  after_previous();
   static_assert(32 * V <= kFlatRound, "queue holds a flat round");
   extern __shared__ __align__(16) unsigned char flat_smem[];
   FlatWarp &sw = reinterpret_cast<FlatWarp *>(flat_smem)[threadIdx.x >> 5];
@@ -711,7 +714,7 @@ cudaError_t launch_persistent(Kern kern, int block, cudaStream_t s, const SweepP
   const int64_t max_useful = (warps_needed + block / 32 - 1) / (block / 32);
   if (blocks > max_useful) blocks = max_useful;
   if (blocks < 1) blocks = 1;
-  kern<<<unsigned(blocks), block, smem, s>>>(p);
+  launch_after(kern, unsigned(blocks), block, smem, s, p);
   return cudaGetLastError();
 }
 
@@ -778,7 +781,7 @@ cudaError_t launch_long_runs(cudaStream_t s, const SweepParams &p, int sms) {
   constexpr size_t smem = sizeof(FlatWarp) * 8;
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  kern<<<unsigned(sms * 4), 256, smem, s>>>(p);
+  launch_after(kern, unsigned(sms * 4), 256, smem, s, p);
   return cudaGetLastError();
 }
 
@@ -820,6 +823,7 @@ __device__ __forceinline__ long long block_inclusive(long long v, long long *scr
 __global__ void __launch_bounds__(kScanBlock)
 prefix_select_kernel(const int32_t *__restrict__ c, int64_t m, long long capacity, long long *__restrict__ sums,
                      int64_t ntiles, PrefixDone *done, DevScalars *scalars) {
+  after_previous();
   __shared__ long long scratch[kScanBlock / 32];
   __shared__ long long at[2];  // the selected tile and the pairs before it
   __shared__ bool last;
@@ -956,7 +960,8 @@ cudaError_t launch_prefix_select(cudaStream_t s, const int32_t *box_counts, int6
   PrefixDone *done = reinterpret_cast<PrefixDone *>(sums + ntiles + 1);
   const cudaError_t e = cudaMemsetAsync(done, 0, sizeof(PrefixDone), s);
   if (e != cudaSuccess) return e;
-  prefix_select_kernel<<<unsigned(ntiles), kScanBlock, 0, s>>>(box_counts, m, capacity, sums, ntiles, done, scalars);
+  launch_after(prefix_select_kernel, unsigned(ntiles), kScanBlock, 0, s, box_counts, m, capacity, sums, ntiles, done,
+               scalars);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
