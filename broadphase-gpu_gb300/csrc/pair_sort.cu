@@ -8,11 +8,12 @@
 // ranks). In a bucket, pairs are grouped by first id and the leading bits of the
 // second the same way, and each pair counts the smaller ones of its group. Above
 // 4 M pairs the same histogram and partition first cut them into segments of about
-// a million. Up to 8,192 pairs are one bucket.
+// half a million. Up to 8,192 pairs are one bucket.
 //
-// Bins hold whole ids, so ids with very many pairs make large buckets: where one
-// passes 4,096 pairs the later kernels do nothing, and once the host sees that,
-// the radix sort takes over (radix_sort.cu). A bucket of large groups (one id
+// Bins hold whole ids, so ids with many pairs make large buckets. Those above
+// 4,096 pairs are left to a second launch, once the host sees that there are any
+// (in meshes of millions of boxes: a few); where one passes 8,192 the later
+// kernels do nothing, and the radix sort takes over (radix_sort.cu). A bucket of large groups (one id
 // with many pairs, close to each other) is sorted by digits in its block.
 //
 // What bounds it: instruction issue (83% of cycles in the bucket kernel, half of
@@ -37,20 +38,21 @@ constexpr int kPairBins = 1 << kPairBinBits;  // at most
 // Pairs between the places of two buckets. 92 M pairs take 2.39 ms at 2,048, 2.31 at
 // 2,560 and 2.29 at 3,072; the rest up to kBucketCap is what a bin may hold.
 constexpr uint32_t kBucket = 2560;
-constexpr int kBucketCap = 4096;          // most pairs of a bucket
+constexpr int kBucketCap = 4096;          // most pairs of a bucket that a block of 512 sorts
+constexpr int kBigCap = 8192;             // and a block of 1024
 constexpr int kGroupBits = 11;
 constexpr int kGroups = 1 << kGroupBits;  // groups of a bucket
 constexpr int kMaxGroup = 96;             // pairs of a pair's group, in the mean, that are sorted by counting
-constexpr uint32_t kSegment = 1u << 20;   // the same for segments
-constexpr int kMaxSegments = 1024;
+constexpr uint32_t kSegment = 1u << 19;   // the same for segments (at 2^20 the times are equal, and bins twice as large)
+constexpr int kMaxSegments = 2048;
 constexpr int64_t kOneLevel = 4 << 20;    // pairs that need no segments
 constexpr int64_t kTwoLevels = int64_t(kSegment) * (kMaxSegments / 2);
 constexpr int kHistTile = 65536;          // pairs per histogram block of a segment
 constexpr int kPairPartTile = kBlock * 16;  // pairs per partition block of a segment
 // buckets of a partition tile's segment: one level has up to kOneLevel / kBucket
 // windows, a segment 2 * kSegment / kBucket, each with one bucket more at most
-constexpr int kMaxTileBuckets = int(kOneLevel / kBucket) + 2;
-static_assert(kMaxTileBuckets >= int(2 * kSegment / kBucket) + 2 && kMaxTileBuckets >= kMaxSegments + 2, "partition counters");
+constexpr int kMaxTileBuckets = std::max(int(kOneLevel / kBucket), kMaxSegments) + 2;
+static_assert(kMaxTileBuckets >= int(2 * kSegment / kBucket) + 2, "partition counters");
 
 struct PairSeg {
   uint32_t begin, end;   // positions
@@ -73,6 +75,7 @@ struct PairHead {
   uint32_t buckets;     // buckets of all segments
   uint32_t segs_done;
   uint32_t fits;        // set once all segments are planned, if no bucket is too long
+  uint32_t big;         // buckets above kBucketCap
   uint32_t segs, tiles, part_tiles;  // next level's segments and tiles
   uint32_t tiles_done[kMaxSegments];
 };
@@ -89,7 +92,7 @@ int bits_of(uint32_t v) {
 // Workspace: the first level's and the last level's tables.
 struct PairLayout {
   int64_t segs = 0, buckets = 0;  // most of them
-  size_t head[2], bins[2], table[2], bucket[2], cursor[2], seg, total;
+  size_t head[2], bins[2], table[2], bucket[2], cursor[2], big, seg, total;
   static PairLayout make(int64_t n) {
     PairLayout l;
     const bool two = n > kOneLevel;
@@ -109,6 +112,7 @@ struct PairLayout {
       l.bucket[k] = take(sizeof(PairBucket) * size_t(b));
       l.cursor[k] = take(sizeof(uint32_t) * size_t(b));
     }
+    l.big = take(sizeof(uint32_t) * size_t(l.buckets));
     l.seg = take(sizeof(PairSeg) * size_t(l.segs));
     l.total = o;
     return l;
@@ -121,6 +125,7 @@ struct PairLevel {
   uint16_t *table;    // bucket of each bin, in the segment
   PairBucket *bucket;
   uint32_t *cursor;   // next place of each bucket
+  uint32_t *big;      // the buckets above kBucketCap (last level), or null
   uint32_t window;    // pairs between the places of two buckets
   uint32_t cap;       // most pairs of a bucket
   int nbins;          // bins of a segment: a power of two, kBlock to kPairBins
@@ -219,6 +224,7 @@ __device__ void plan_segment(const PairLevel &lv, const PairSeg &sg, int which, 
     bk[d].end = end;
     bk[d].span = (d + 1 < nb ? bk[d + 1].base : past) - bk[d].base;
     lv.cursor[bucket0 + d] = begin;
+    if (lv.big && end - begin > unsigned(kBucketCap)) lv.big[atomicAdd(&lv.head->big, 1u)] = bucket0 + d;
     longest = max(longest, end - begin);
   }
   longest = __reduce_max_sync(kFullMask, longest);
@@ -258,6 +264,7 @@ __device__ void plan_segment(const PairLevel &lv, const PairSeg &sg, int which, 
     lv.head->fits = fits ? 1u : 0u;
     if (!segs) lv.plan->max_first = most;
     lv.plan->fits = fits ? 1u : 0u;
+    lv.plan->big = __ldcg(&lv.head->big);
   }
 }
 
@@ -373,8 +380,9 @@ pair_partition_kernel(const unsigned long long *__restrict__ in, unsigned long l
   }
 }
 
-// Sorts one bucket (of at most CAP pairs). AUTO: the only bucket, of n pairs,
-// whose first ids are not known beforehand.
+// Sorts one bucket; one of more than CAP pairs is left. AUTO: the only bucket, of
+// n pairs, whose first ids are not known beforehand. Else with a list: the bucket
+// that the list has for the block.
 // Where the bucket has no more first ids than groups (narrow), an id's pairs are
 // cut into several groups by the leading bits of their second ids, so that the
 // groups number 2,048 whatever the pairs per id; a group's number stands for the
@@ -400,9 +408,9 @@ struct BucketShared {
 };
 
 template <int THREADS, int CAP, bool AUTO>
-__global__ void __launch_bounds__(THREADS, AUTO ? 1 : 2048 / THREADS)
+__global__ void __launch_bounds__(THREADS, THREADS == 512 && !AUTO ? 4 : 1)
 pair_bucket_kernel(const unsigned long long *in, unsigned long long *out, const PairBucket *__restrict__ buckets,
-                   const PairHead *head, int n) {
+                   const PairHead *head, const uint32_t *__restrict__ list, int n) {
   after_previous();
   constexpr int ITEMS = CAP / THREADS;
   static_assert(kGroups % THREADS == 0, "groups per thread");
@@ -413,9 +421,10 @@ pair_bucket_kernel(const unsigned long long *in, unsigned long long *out, const 
   uint32_t start = 0, base = 0, span = 0;
   if (!AUTO) {
     if (!head->fits || blockIdx.x >= head->buckets) return;
-    const PairBucket b = buckets[blockIdx.x];
+    const PairBucket b = buckets[list ? list[blockIdx.x] : blockIdx.x];
     start = b.begin;
     n = int(b.end - b.begin);
+    if (n > CAP) return;
     base = b.base;
     span = b.span;
   }
@@ -595,12 +604,12 @@ cudaError_t launch_partition(cudaStream_t s, int64_t blocks, const unsigned long
 
 template <int THREADS, int CAP, bool AUTO>
 cudaError_t launch_buckets(cudaStream_t s, int64_t blocks, const unsigned long long *in, unsigned long long *out,
-                           const PairBucket *buckets, const PairHead *head, int n) {
+                           const PairBucket *buckets, const PairHead *head, const uint32_t *list, int n) {
   constexpr auto kern = pair_bucket_kernel<THREADS, CAP, AUTO>;
   constexpr size_t smem = sizeof(BucketShared<THREADS, CAP>);
   const cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
-  launch_after(kern, unsigned(blocks), THREADS, smem, s, in, out, buckets, head, n);
+  launch_after(kern, unsigned(blocks), THREADS, smem, s, in, out, buckets, head, list, n);
   return cudaGetLastError();
 }
 
@@ -615,10 +624,10 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
   if (n < 2) return cudaSuccess;
   unsigned long long *a = reinterpret_cast<unsigned long long *>(d_pairs);
   unsigned long long *b = reinterpret_cast<unsigned long long *>(tmp);
-  if (n <= 8192) {  // one bucket
+  if (n <= kBigCap) {  // one bucket
     *launches += 1;
-    return n <= kBucketCap ? launch_buckets<512, kBucketCap, true>(s, 1, a, a, nullptr, nullptr, int(n))
-                           : launch_buckets<1024, 8192, true>(s, 1, a, a, nullptr, nullptr, int(n));
+    return n <= kBucketCap ? launch_buckets<512, kBucketCap, true>(s, 1, a, a, nullptr, nullptr, nullptr, int(n))
+                           : launch_buckets<1024, kBigCap, true>(s, 1, a, a, nullptr, nullptr, nullptr, int(n));
   }
   if (n > kTwoLevels) return radix_sort_pairs(s, d_pairs, tmp, n, ws, fault, launches);
   const PairLayout l = PairLayout::make(n);
@@ -633,7 +642,7 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
     lv.bucket = reinterpret_cast<PairBucket *>(w + l.bucket[k]);
     lv.cursor = reinterpret_cast<uint32_t *>(w + l.cursor[k]);
     lv.window = kBucket;
-    lv.cap = kBucketCap;
+    lv.cap = kBigCap;
     lv.nbins = kPairBins;
     lv.plan = plan;
     return lv;
@@ -643,6 +652,7 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
   };
   const PairLevel last = [&] {
     PairLevel lv = level(1);
+    lv.big = reinterpret_cast<uint32_t *>(w + l.big);
     if (two) lv.before = reinterpret_cast<const PairHead *>(w + l.head[0]);
     // some eight bins per bucket: every block adds its bins to the segment's
     else while (lv.nbins > kBlock && lv.nbins / 2 >= 8 * (n / int64_t(kBucket))) lv.nbins /= 2;
@@ -654,6 +664,7 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
     first.window = kSegment;
     first.cap = 2 * kSegment;
     first.next = segs;
+    first.big = nullptr;
   }
   int bin_bits = 0;
   while ((1 << bin_bits) < first.nbins) ++bin_bits;
@@ -680,10 +691,15 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *d_pairs, stq_pair *tmp, int64_t
       if (e != cudaSuccess) return e;
       *launches += 2;
     }
-    e = launch_buckets<512, kBucketCap, false>(s, l.buckets, two ? a : b, a, last.bucket, last.head, 0);
+    e = launch_buckets<512, kBucketCap, false>(s, l.buckets, two ? a : b, a, last.bucket, last.head, nullptr, 0);
     *launches += 1;
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess || plan->fits) return e;
+    if (e != cudaSuccess) return e;
+    if (plan->fits) {
+      if (plan->big == 0) return cudaSuccess;
+      *launches += 1;
+      return launch_buckets<1024, kBigCap, false>(s, plan->big, two ? a : b, a, last.bucket, last.head, last.big, 0);
+    }
     // the ids' true width, once; then ids have very many pairs
     const int bits = bits_of(plan->max_first);
     if (bits == *id_bits || tries > 0) return radix_sort_pairs(s, d_pairs, tmp, n, ws, fault, launches);

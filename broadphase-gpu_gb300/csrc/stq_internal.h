@@ -392,6 +392,7 @@ cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int
 struct PairPlan {
   unsigned int max_first;  // largest first id
   unsigned int fits;       // no bucket was too long: the pairs are sorted
+  unsigned int big;        // but for those of these buckets, which take another launch
 };
 size_t pair_workspace_bytes(int64_t n);
 // Lexicographic sort of pairs by buckets of their first id (by digits where ids

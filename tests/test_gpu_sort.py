@@ -1,8 +1,9 @@
 """The device sorts through stq_sort_pairs. Sizes at the edges of its kernels: one
 block up to 4,096 and 8,192 pairs, buckets of about 2,560 (at most 4,096) pairs
-above, segments of about 2^20 above 2^22. Ids that are few, wide, equal, or
-uneven: one first id with too many pairs for a bucket takes the radix sort, large
-groups of close pairs a bucket's digits."""
+above, segments of about 2^19 above 2^22. Ids that are few, wide, equal, or
+uneven: neighbouring ids with more than 4,096 pairs take a large bucket, one first
+id with more than 8,192 the radix sort, large groups of close pairs a bucket's
+digits."""
 import numpy as np
 import pytest
 
@@ -29,6 +30,11 @@ def draw(rng, n, ids):
         p[:, 1] += rng.integers(0, 2, n, dtype=np.uint32) << 30
         p[:, 0] = rng.integers(0, max(n // 600, 1), n)
         return p
+    if ids == "dense":  # 6,000 pairs of eight neighbouring ids
+        p = rng.integers(0, max(n // 4, 2), (n, 2), dtype=np.uint32)
+        at = rng.choice(n, min(n, 6000), replace=False)
+        p[at, 0] = n // 9 + rng.integers(0, 8, len(at))
+        return p
     if ids == "hub":  # a scene in which one box meets 1 in 50
         p = rng.integers(0, max(n // 4, 2), (n, 2), dtype=np.uint32)
         p[:: 50, 0] = n // 9
@@ -51,13 +57,13 @@ def check(ctx, cuda, p):
 
 
 @pytest.mark.parametrize("n", [2, 33, 1023, 4095, 4096, 4097, 8191, 8192, 8193, 10241, 100_003, 933_889, 2_000_003])
-@pytest.mark.parametrize("ids", ["small", "one_sided", "wide", "equal", "groups", "clumps", "hub", "scene"])
+@pytest.mark.parametrize("ids", ["small", "one_sided", "wide", "equal", "groups", "clumps", "dense", "hub", "scene"])
 def test_sort_pairs_sizes_and_ids(ctx, cuda, n, ids):
     check(ctx, cuda, draw(np.random.default_rng(n), n, ids))
 
 
 @pytest.mark.parametrize("n", [(1 << 22) - 1, (1 << 22) + 1, 9_500_000])
-@pytest.mark.parametrize("ids", ["small", "wide", "groups", "clumps", "hub", "scene"])
+@pytest.mark.parametrize("ids", ["small", "wide", "groups", "clumps", "dense", "hub", "scene"])
 def test_sort_pairs_segments(ctx, cuda, n, ids):
     check(ctx, cuda, draw(np.random.default_rng(n), n, ids))
 
