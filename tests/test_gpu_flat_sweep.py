@@ -46,3 +46,19 @@ def test_dense_windows_vs_oracle(ctx, stq, oracle, cuda, n, spread, run_cap):
         start = r.next_start
     got = np.concatenate(parts)
     assert len(got) == len(want) and np.array_equal(oracle.canonical(got), want)
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 77_823, 77_824, 77_825])
+def test_tile_edges_vs_oracle(ctx, stq, oracle, cuda, n):
+    """Tiles of 256 boxes up to 77,824 boxes, of 1,024 above; the last one of 1,
+    255 or 256 boxes."""
+    import torch
+
+    b = stq.random_boxes(n, seed=n)
+    want = oracle.broadphase(b)
+    d = torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+    cap = len(want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    r = ctx.sweep(d, n, pairs, cap, axis=-1)
+    assert r.status == stq.STQ_OK and r.count == len(want)
+    assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
