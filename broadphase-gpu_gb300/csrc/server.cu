@@ -65,18 +65,22 @@ advance_kernel(const MeshRef *__restrict__ refs, const long long *__restrict__ v
 }
 
 // XOR over each scene's pairs of mix64((lo << 32) | hi), ids local to the
-// scene. A warp takes kChecksumChunk consecutive pairs, 32 per step (one per
+// scene. A warp takes kChecksumChunk consecutive pairs, 32 at a time (one per
 // lane, coalesced), and keeps the XOR of the current scene in its lanes'
 // registers. The pair list holds runs of one scene (each sweep warp appends
 // 32 or more pairs of consecutive start positions at once), so the warp
 // reduces its registers and flushes them with one atomic per run: at a scene
-// change inside a step, the lanes still in the old scene add to the registers
+// change inside 32 pairs, the lanes still in the old scene add to the registers
 // before the flush, and the lanes of the new scene after it. A lane whose pair
-// lies in a third scene within one step adds it alone. Those XORs go to a
+// lies in a third scene within these 32 adds it alone. Those XORs go to a
 // per-block table of the scenes in shared memory when it fits (SMEM), and the
 // block adds its table to the scenes' checksums once at the end: millions of
 // runs would otherwise contend on a few dozen global addresses.
 constexpr int kChecksumChunk = 1024;
+// Pairs loaded at once by a lane. With one (and 64-bit id arithmetic) the kernel
+// waited for its loads and took a quarter of the sweep's time (100 M pairs in 0.26
+// ms), with eight 18% of it; four and two are 0.5% slower over a whole run.
+constexpr int kChecksumStep = 8;
 constexpr int kChecksumSmemScenes = 4096;  // 32 KB of shared memory
 
 __device__ __forceinline__ int scene_of(const long long *__restrict__ box_off, int S, long long id) {
@@ -113,37 +117,39 @@ pair_checksum_kernel(const int2 *__restrict__ pairs, long long capacity, const B
   for (long long base = warp * kChecksumChunk; base < n; base += nwarps * kChecksumChunk) {
     const long long end = min(base + kChecksumChunk, n);
     int cur = -1;  // warp-uniform: scene of the registers' XOR
-    long long b0 = 0, b1 = 0;
+    int b0 = 0, b1 = 0;  // its ids
     unsigned long long acc = 0;
-    for (long long q0 = base; q0 < end; q0 += 32) {
-      const long long q = q0 + lane;
-      const bool valid = q < end;
-      int2 p = make_int2(0, 0);
-      if (valid) p = pairs[q];
-      const bool in = valid && p.x >= b0 && p.x < b1;
-      if (in) {
-        const unsigned long long a = (unsigned long long)(p.x - b0), c = (unsigned long long)(p.y - b0);
-        acc ^= mix64((a << 32) | c);
+    for (long long q0 = base; q0 < end; q0 += 32 * kChecksumStep) {
+      int2 p[kChecksumStep];  // a pair past the end: ids -1, in no scene
+#pragma unroll
+      for (int u = 0; u < kChecksumStep; ++u) {
+        const long long q = q0 + 32 * u + lane;
+        p[u] = q < end ? pairs[q] : make_int2(-1, -1);
       }
-      const unsigned outm = __ballot_sync(0xffffffffu, valid && !in);
-      if (outm) {
-        // the scene changes: flush, and take the scene of the first lane outside
-        flush(cur, acc);
-        acc = 0;
-        const int leader = __ffs(outm) - 1;
-        int s = 0;
-        if (lane == leader) s = scene_of(box_off, S, p.x);
-        cur = __shfl_sync(0xffffffffu, s, leader);
-        b0 = box_off[cur];
-        b1 = box_off[cur + 1];
-        if (valid && !in) {
-          const bool in_new = p.x >= b0 && p.x < b1;
-          const int t = in_new ? cur : scene_of(box_off, S, p.x);
-          const unsigned long long a = (unsigned long long)(p.x - box_off[t]),
-                                   c = (unsigned long long)(p.y - box_off[t]);
-          const unsigned long long h = mix64((a << 32) | c);
-          if (in_new) acc ^= h;
-          else atomicXor(&acc_to[t], h);
+#pragma unroll
+      for (int u = 0; u < kChecksumStep; ++u) {
+        const bool in = unsigned(p[u].x - b0) < unsigned(b1 - b0);
+        if (in) acc ^= mix64((unsigned long long)unsigned(p[u].x - b0) << 32 | unsigned(p[u].y - b0));
+        const bool out = !in && p[u].x >= 0;
+        const unsigned outm = __ballot_sync(0xffffffffu, out);
+        if (outm) {
+          // the scene changes: flush, and take the scene of the first lane outside
+          flush(cur, acc);
+          acc = 0;
+          const int leader = __ffs(outm) - 1;
+          int s = 0;
+          if (lane == leader) s = scene_of(box_off, S, p[u].x);
+          cur = __shfl_sync(0xffffffffu, s, leader);
+          b0 = int(box_off[cur]);
+          b1 = int(box_off[cur + 1]);
+          if (out) {
+            const bool in_new = p[u].x >= b0 && p[u].x < b1;
+            const int t = in_new ? cur : scene_of(box_off, S, p[u].x);
+            const int t0 = int(box_off[t]);
+            const unsigned long long h = mix64((unsigned long long)unsigned(p[u].x - t0) << 32 | unsigned(p[u].y - t0));
+            if (in_new) acc ^= h;
+            else atomicXor(&acc_to[t], h);
+          }
         }
       }
     }
