@@ -441,12 +441,14 @@ choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__
     cell_base[S] = carry;
     const unsigned long long R = reps, lists = 3ull * carry;
     // key: list id above the top bits of the sweep-axis code, 24 bits in all (three
-    // digits) where that leaves the code 10 bits or more, else 32. At 10 bits the
+    // digits) where that leaves the code 9 bits or more, else 32. At 10 bits the
     // 6 M-box scene (14 bits of lists) tests 9% more candidates and sorts a digit
-    // less: sort + sweep 0.22 + 1.26 ms against 0.29 + 1.19 with 32 bits.
+    // less: sort + sweep 0.22 + 1.26 ms against 0.29 + 1.19 with 32 bits. With 15
+    // bits of lists, 200,000 boxes (9 bits of code): 44 + 28 -> 36 + 28 us; with 16,
+    // 256 scenes (8): the sweep's loss outweighs the digit by 50 us.
     int seg_bits = 0;
     while (seg_bits < 32 && (1ull << seg_bits) < lists) ++seg_bits;
-    const int key_bits = seg_bits <= 14 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
+    const int key_bits = seg_bits <= 15 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
     const int passes = max(seg_bits + key_bits + 7, 8) / 8;
     // more than the buffers hold: the scenes are flagged and left empty (the
     // caller without limits checks that positions fit 31 bits)
