@@ -544,6 +544,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
     const int stop = band ? jhi : total;
     int begun = 0;      // flat: starts whose run began before the current step
     int lo = 0;         // band: the lane's run begins lo positions into the step
+    uint32_t ahead = band ? p.scode[at + lane] : 0u;  // band: the next step's codes
     uint32_t hits = 0;  // band: candidates of the step that are not queued yet,
     uint32_t part = 0;  // and those of them that go next
     bool more;
@@ -556,9 +557,12 @@ stq_sweep_flat_kernel(const SweepParams p) {
           uint32_t mine = 0;  // positions of this step inside the lane's run
           if (len > 0 && lo < 32 && hi > 0)
             mine = (kFullMask << max(lo, 0)) & (hi >= 32 ? kFullMask : ~(kFullMask << hi));
-          reinterpret_cast<uint32_t *>(sw.code)[lane] = p.scode[at + lane];
+          reinterpret_cast<uint32_t *>(sw.code)[lane] = ahead;
           __syncwarp();
           at += 32;
+          // the next step's, loaded while this one is taken (6 M boxes: sweep 1.27 ms
+          // without, 1.25 with)
+          if (at < stop) ahead = p.scode[at + lane];
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint4 c = sw.code[q];
