@@ -559,7 +559,7 @@ def main():
     r = ctx.sweep_prepared(pairs, cap)
     cap = int(r.total * 1.05) + 1024
     pairs = torch.empty((cap, 2), dtype=torch.int32, device=dev)
-    # the project's autotuner picks cell scale, radix width, sweep shape,
+    # the project's autotuner picks cell scale, sweep shape,
     # lane-group width, queue depth and block size for this workload (not
     # timed); --no-tune with --options name=value,... sets them by hand instead
     # (profiling runs, which must not launch the tuner's trials)

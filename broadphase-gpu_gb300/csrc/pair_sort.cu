@@ -13,8 +13,9 @@
 // Bins hold whole ids, so ids with many pairs make large buckets. Those above
 // 4,096 pairs are left to a second launch, once the host sees that there are any
 // (in meshes of millions of boxes: a few); where one passes 8,192 the later
-// kernels do nothing, and the radix sort takes over (radix_sort.cu). A bucket of large groups (one id
-// with many pairs, close to each other) is sorted by digits in its block.
+// kernels do nothing, and the radix sort takes over (radix_sort.cu). A bucket of
+// large groups (one id with many pairs, close to each other) is sorted by digits in
+// its block.
 //
 // What bounds it: instruction issue (83% of cycles in the bucket kernel, half of
 // the time; shared memory 71%, DRAM 13%, 21 of 32 lanes active in the loops over
@@ -43,7 +44,7 @@ constexpr int kBigCap = 8192;             // and a block of 1024
 constexpr int kGroupBits = 11;
 constexpr int kGroups = 1 << kGroupBits;  // groups of a bucket
 constexpr int kMaxGroup = 96;             // pairs of a pair's group, in the mean, that are sorted by counting
-constexpr uint32_t kSegment = 1u << 19;   // the same for segments (at 2^20 the times are equal, and bins twice as large)
+constexpr uint32_t kSegment = 1u << 19;   // the same for segments (2^20: equal times, bins twice as large)
 constexpr int kMaxSegments = 2048;
 constexpr int64_t kOneLevel = 4 << 20;    // pairs that need no segments
 constexpr int64_t kTwoLevels = int64_t(kSegment) * (kMaxSegments / 2);

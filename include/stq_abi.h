@@ -136,8 +136,9 @@ int64_t stq_context_get_option(const stq_context *ctx, int option);
 const char *stq_context_last_error(const stq_context *ctx);
 /* Kernel launches this context issued since it was created. */
 int64_t stq_context_launch_count(const stq_context *ctx);
-/* Candidates (x-overlapping start box / candidate pairs) the last sweep
- * tested, a measure of the sweep's work beyond the pairs it found. */
+/* Candidates (start box / candidate pairs) the last sweep tested, a measure of
+ * the sweep's work beyond the pairs it found: the pairs that overlap on the sweep
+ * axis, and those few that share a 16-bit code of it without doing so. */
 int64_t stq_context_candidates(const stq_context *ctx);
 /* Shape of the prepared scene's (cell, type) lists: out[0] lists (3 per
  * cell), out[1] cell replicas, out[2] the longest list. Synchronises. */
@@ -158,8 +159,8 @@ int stq_build_boxes(stq_context *ctx, const double *d_V0, const double *d_V1,
 int stq_select_axis(stq_context *ctx, const stq_aabb *d_boxes, int64_t n,
                     int *axis_out);
 
-/* Sorts the boxes along `axis` into the context's sorted scene (keys,
- * bounds, vertex ids). The boxes buffer may be reused after return. */
+/* Sorts the boxes' cell replicas along `axis` into the context's sorted scene
+ * (codes, bounds, vertex ids). The boxes buffer may be reused after return. */
 int stq_prepare(stq_context *ctx, const stq_aabb *d_boxes, int64_t n,
                 int axis);
 
@@ -264,8 +265,9 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
                          int64_t capacity, int64_t *count, int64_t *total,
                          int64_t *h_scene_pairs);
 
-/* Sorts d_pairs[0..count) lexicographically on the device (deterministic
- * output order for callers that need one). */
+/* Sorts d_pairs[0..count) lexicographically, by (first, second) as unsigned ids,
+ * on the device (deterministic output order for callers that need one).
+ * Synchronises. */
 int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count);
 
 /* ---- autotuning --------------------------------------------------------------
