@@ -818,8 +818,9 @@ int wave_blocks(const void *kernel, int64_t n) {
 }
 
 __global__ void __launch_bounds__(kBlock)
-reset_sweep_kernel(BatchHeader *hdr, unsigned long long *scene_pairs) {
+reset_sweep_kernel(BatchHeader *hdr, unsigned long long *scene_pairs, const DevScalars *sel, long long capacity) {
   after_previous();
+  if (sel && sel->count <= (unsigned long long)capacity) return;
   const int S = hdr->n_scenes;
   for (int s = blockIdx.x * kBlock + threadIdx.x; s < S; s += gridDim.x * kBlock)
     scene_pairs[s] = 0ull;
@@ -854,8 +855,8 @@ cudaError_t launch_window_step(cudaStream_t s, WindowCounters *wc, unsigned long
 }
 
 cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long long *scene_pairs,
-                               int scene_cap) {
-  launch_after(reset_sweep_kernel, blocks_for(scene_cap, 64), kBlock, 0, s, hdr, scene_pairs);
+                               int scene_cap, const DevScalars *sel, long long capacity) {
+  launch_after(reset_sweep_kernel, blocks_for(scene_cap, 64), kBlock, 0, s, hdr, scene_pairs, sel, capacity);
   return cudaGetLastError();
 }
 

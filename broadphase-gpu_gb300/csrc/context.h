@@ -63,6 +63,7 @@ struct HostBlock {
   alignas(128) BatchHeader hdr;
   alignas(128) FrontInfo front;
   alignas(128) PairPlan plan;
+  alignas(128) DevScalars sel;
   alignas(128) int fault;
   alignas(128) int flags;
 };
@@ -107,8 +108,10 @@ struct stq_context {
   FrontInfo *h_front = nullptr;       // written by a prepare's first half
   cudaEvent_t front_event = nullptr;  // after it
   PairPlan *h_plan = nullptr;         // written by a pair sort's histogram
+  DevScalars *h_sel = nullptr;        // readback of an overflowing sweep's prefix
   int pair_id_bits = 0;               // of the largest first id of the pairs sorted so far
   int passes_seen = 0;  // most digits that a replica sort of this context needed
+  bool overflowed = false;  // a sweep of the prepared scenes found more pairs than the buffer held
   bool swept = false;   // the prepared scenes have been swept (their pair counters hold)
   unsigned long long *h_scene_pairs = nullptr;  // pinned readback
   int h_scene_pairs_cap = 0;
@@ -196,8 +199,8 @@ int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replic
 // launches on stream, keeping the header's statistics. timed: record the
 // launch as one sweep stage (a windowed caller times its windows as one).
 int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs, long long capacity,
-              bool count_mode, bool timed = true,
-              const SweepCursors *cursors = nullptr, cudaStream_t stream = nullptr);
+              SweepMode mode, bool timed = true, const SweepCursors *cursors = nullptr,
+              cudaStream_t stream = nullptr, const DevScalars *sel = nullptr);
 
 template <typename T>
 T *dev_at(stq_context *ctx, size_t off) {

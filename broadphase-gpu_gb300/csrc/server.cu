@@ -274,7 +274,7 @@ int enqueue_tick(stq_server *sv, bool advance) {
   const BatchBuffers b = batch_buffers(ctx, ctx->batch_boxes.as<stq_aabb>());
   STQ_TRY(enqueue_prepare_front(ctx, b, ctx->rep_cap, ctx->seg_cap));
   STQ_TRY(enqueue_prepare_back(ctx, b, -1, 4));
-  STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, sv->pairs.as<stq_pair>(), sv->pair_cap, false));
+  STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, sv->pairs.as<stq_pair>(), sv->pair_cap, kSweepEmit));
   STQ_CUDA(ctx, launch_pair_checksums(ctx->stream, sv->pairs.as<stq_pair>(), sv->pair_cap, hdr, box_off,
                                       sv->checks_dev.as<unsigned long long>(), sv->max_scenes),
            "launch checksums");

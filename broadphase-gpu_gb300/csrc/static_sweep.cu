@@ -198,10 +198,11 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   p.stats = nullptr;
   p.typed = 0;  // one list of all box types
   p.run_cap = 512;
+  p.sel = nullptr;
   p.long_list = reinterpret_cast<int2 *>(scratch + kOffLong);
   p.long_items = &hdr->long_items;
   p.long_work = &hdr->long_work;
-  if (launch_sweep(s, p, SweepTuning(), false, num_sms) != cudaSuccess) return STQ_ERR_CUDA;
+  if (launch_sweep(s, p, SweepTuning(), kSweepEmit, num_sms) != cudaSuccess) return STQ_ERR_CUDA;
   BatchHeader h;
   if (cudaMemcpyAsync(&h, hdr, sizeof(BatchHeader), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)

@@ -287,6 +287,15 @@ struct SweepParams {
   int2 *long_list;           // handed-over runs (start position, next candidate)
   unsigned int *long_items;  // their count
   unsigned int *long_work;   // warp pass grab cursor
+  const DevScalars *sel;     // if set: start positions [begin, begin + sel->prefix),
+                             // and none if sel->count pairs fit the capacity
+};
+
+// What a sweep does with its pairs.
+enum SweepMode {
+  kSweepEmit = 0,   // writes them
+  kSweepCount = 1,  // counts them per start position
+  kSweepBoth = 2,   // both
 };
 
 // ---- launch wrappers (each returns the launch error) -------------------------
@@ -365,7 +374,8 @@ cudaError_t launch_pair_checksums(cudaStream_t s, const stq_pair *pairs, long lo
                                   const BatchHeader *hdr, const long long *box_off,
                                   unsigned long long *checks, int scene_cap);
 cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long long *scene_pairs,
-                               int scene_cap);
+                               int scene_cap, const DevScalars *sel = nullptr,
+                               long long capacity = 0);
 // host_count: device address of page-locked, mapped host memory
 cudaError_t launch_window_step(cudaStream_t s, WindowCounters *wc, unsigned long long *host_count);
 
@@ -409,13 +419,15 @@ cudaError_t sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n
 int sm_count();
 
 cudaError_t launch_sweep(cudaStream_t s, const SweepParams &p,
-                         const SweepTuning &t, bool count_mode, int num_sms);
+                         const SweepTuning &t, SweepMode mode, int num_sms);
 // inclusive scan of box_counts[0..m) and the longest prefix whose pair sum
-// is <= capacity -> scalars->prefix
+// is <= capacity -> scalars->prefix; *found (or, with none, more than any
+// capacity) -> scalars->count
 size_t prefix_workspace_bytes(int64_t m);
 cudaError_t launch_prefix_select(cudaStream_t s, const int32_t *box_counts,
                                  int64_t m, long long capacity, void *workspace,
-                                 DevScalars *scalars, int64_t *launches);
+                                 DevScalars *scalars, int64_t *launches,
+                                 const unsigned long long *found);
 cudaError_t launch_brute_force(cudaStream_t s, const stq_aabb *boxes, int64_t n,
                                stq_pair *pairs, long long capacity,
                                unsigned long long *count);

@@ -45,6 +45,13 @@ __device__ __forceinline__ bool pair_hit(const PosRec &a, const PosRec &b, int t
   return x && overlap_bc(a.yz, b.yz) && (typed || valid_pair(a.v, b.v)) && !covertex(a.v, b.v);
 }
 
+// One past the last start position of a sweep, from the sizes on the device.
+__device__ __forceinline__ int sweep_end(const SweepParams &p) {
+  const int end = min(p.end, int(p.hdr->length));
+  if (!p.sel) return end;
+  return p.sel->count <= (unsigned long long)p.capacity ? p.begin : int(min((long long)end, p.begin + p.sel->prefix));
+}
+
 // Appends the warp's n staged pairs with one atomic; pairs past the capacity
 // are counted but not written.
 __device__ __forceinline__ void flush_staged(const int2 *st, int n, int lane, const SweepParams &p) {
@@ -86,7 +93,7 @@ stq_sweep_kernel(const SweepParams p) {
   PosRec kr = {};     // the current start box
   uint32_t code = 0;  // and its code
   int kf = 0;         // its scene, above the first-cell bits
-  const int end = min(p.end, int(p.hdr->length));
+  const int end = sweep_end(p);
   const int span = end - p.begin;
   unsigned tested = 0;  // candidates this lane tested (statistics)
   // warp-uniform: staged pairs, and pairs of the current scene not yet added
@@ -245,7 +252,7 @@ stq_sweep_lane_kernel(const SweepParams p) {
   PosRec kr = {};     // the start box
   uint32_t code = 0;  // and its code
   int kf = 0;         // its scene, above the first-cell bits
-  const int end = min(p.end, int(p.hdr->length));
+  const int end = sweep_end(p);
   const int span = end - p.begin;
   unsigned tested = 0;
   int staged = 0;
@@ -443,11 +450,12 @@ struct FlatWarp {
   int hits[32];                // count mode: pairs per slot
 };
 
-template <int BLOCK, int V, bool COUNT, bool LONG>
+template <int BLOCK, int V, SweepMode MODE, bool LONG>
 __global__ void __launch_bounds__(BLOCK)
 stq_sweep_flat_kernel(const SweepParams p) {
   after_previous();
   static_assert(32 * V <= kFlatRound, "queue holds a flat round");
+  constexpr bool COUNT = MODE != kSweepEmit, EMIT = MODE != kSweepCount;
   extern __shared__ __align__(16) unsigned char flat_smem[];
   FlatWarp &sw = reinterpret_cast<FlatWarp *>(flat_smem)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -460,13 +468,14 @@ stq_sweep_flat_kernel(const SweepParams p) {
   int end, span, chunk = p.chunk;
   unsigned parts = 1;  // LONG: parts of a run
   if (LONG) {
+    if (p.sel && p.sel->count <= (unsigned long long)p.capacity) return;  // the list is of an earlier sweep
     const unsigned items = *p.long_items, warps = gridDim.x * (BLOCK / 32);
     if (items == 0) return;
     parts = max(1u, min(64u, warps / items));
     end = span = int(items * parts);
     chunk = max(1, min(32, span / int(4 * warps)));
   } else {
-    end = min(p.end, int(p.hdr->length));
+    end = sweep_end(p);
     span = end - p.begin;
   }
   const int first = LONG ? 0 : p.begin;
@@ -636,9 +645,8 @@ stq_sweep_flat_kernel(const SweepParams p) {
         const int4 bv = p.v[c];
         const int4 kv = r.v;
         const bool hit = lane < n && pair_hit(PosRec{r.yz, r.x, kv}, PosRec{b, p.x[c], bv}, p.typed);
-        if (COUNT) {
-          if (hit) atomicAdd(&sw.hits[e & 31u], 1);
-        } else {
+        if (COUNT && hit) atomicAdd(&sw.hits[e & 31u], 1);
+        if (EMIT) {
           const unsigned hm = __ballot_sync(kFullMask, hit);
           if (hit) st[staged + __popc(hm & below)] = make_int2(min(kv.w, bv.w), max(kv.w, bv.w));
           staged += __popc(hm);
@@ -675,7 +683,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
       __syncwarp();
     }
   }
-  if (COUNT) return;
+  if (!EMIT) return;
   __syncwarp();
   if (staged) flush_staged(st, staged, lane, p);
   if (lane == 0 && wpairs) atomicAdd(&p.scene_pairs[wscene], wpairs);
@@ -768,9 +776,9 @@ cudaError_t launch_u(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
 }
 
 // The flat shape's blocks are 128 or 256 threads.
-template <int BLOCK, int V, bool COUNT>
+template <int BLOCK, int V, SweepMode MODE>
 cudaError_t launch_flat_block(cudaStream_t s, const SweepParams &p, int sms) {
-  constexpr auto kern = stq_sweep_flat_kernel<BLOCK, V, COUNT, false>;
+  constexpr auto kern = stq_sweep_flat_kernel<BLOCK, V, MODE, false>;
   constexpr size_t smem = sizeof(FlatWarp) * (BLOCK / 32);
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
@@ -779,9 +787,9 @@ cudaError_t launch_flat_block(cudaStream_t s, const SweepParams &p, int sms) {
 
 // The warp pass: four blocks per SM (most sweeps hand nothing over, and the
 // blocks leave at once).
-template <bool COUNT>
+template <SweepMode MODE>
 cudaError_t launch_long_runs(cudaStream_t s, const SweepParams &p, int sms) {
-  constexpr auto kern = stq_sweep_flat_kernel<256, 4, COUNT, true>;
+  constexpr auto kern = stq_sweep_flat_kernel<256, 4, MODE, true>;
   constexpr size_t smem = sizeof(FlatWarp) * 8;
   cudaError_t e = allow_smem<kern>(smem);
   if (e != cudaSuccess) return e;
@@ -791,8 +799,8 @@ cudaError_t launch_long_runs(cudaStream_t s, const SweepParams &p, int sms) {
 
 template <int V>
 cudaError_t launch_flat(cudaStream_t s, const SweepParams &p, int block, int sms) {
-  if (block == 128) return launch_flat_block<128, V, false>(s, p, sms);
-  return launch_flat_block<256, V, false>(s, p, sms);
+  if (block == 128) return launch_flat_block<128, V, kSweepEmit>(s, p, sms);
+  return launch_flat_block<256, V, kSweepEmit>(s, p, sms);
 }
 
 // ---- overflow: longest prefix of start boxes whose pairs fit ------------------
@@ -826,7 +834,7 @@ __device__ __forceinline__ long long block_inclusive(long long v, long long *scr
 
 __global__ void __launch_bounds__(kScanBlock)
 prefix_select_kernel(const int32_t *__restrict__ c, int64_t m, long long capacity, long long *__restrict__ sums,
-                     int64_t ntiles, PrefixDone *done, DevScalars *scalars) {
+                     int64_t ntiles, PrefixDone *done, DevScalars *scalars, const unsigned long long *found) {
   after_previous();
   __shared__ long long scratch[kScanBlock / 32];
   __shared__ long long at[2];  // the selected tile and the pairs before it
@@ -874,7 +882,10 @@ prefix_select_kernel(const int32_t *__restrict__ c, int64_t m, long long capacit
     run = scratch[0];
     if (within < kScanBlock) break;
   }
-  if (threadIdx.x == 0) scalars->prefix = prefix;
+  if (threadIdx.x == 0) {
+    scalars->prefix = prefix;
+    scalars->count = found ? *found : ~0ull;
+  }
 }
 
 // ---- all-pairs checker (get_collision_pairs, src/collision.cu:91-154) ---------
@@ -913,21 +924,26 @@ brute_force_kernel(const stq_aabb *__restrict__ boxes, int64_t n,
 }  // namespace
 
 static cudaError_t launch_sweep_lanes(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
-                                      bool count_mode, int num_sms);
+                                      SweepMode mode, int num_sms);
 
 cudaError_t launch_sweep(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
-                         bool count_mode, int num_sms) {
+                         SweepMode mode, int num_sms) {
   if (p.end <= p.begin) return cudaSuccess;
-  cudaError_t e = launch_sweep_lanes(s, p, t, count_mode, num_sms);
+  cudaError_t e = launch_sweep_lanes(s, p, t, mode, num_sms);
   if (e != cudaSuccess) return e;
   if (!p.run_cap) return cudaSuccess;
-  return count_mode ? launch_long_runs<true>(s, p, num_sms) : launch_long_runs<false>(s, p, num_sms);
+  switch (mode) {
+    case kSweepCount: return launch_long_runs<kSweepCount>(s, p, num_sms);
+    case kSweepBoth: return launch_long_runs<kSweepBoth>(s, p, num_sms);
+    default: return launch_long_runs<kSweepEmit>(s, p, num_sms);
+  }
 }
 
 static cudaError_t launch_sweep_lanes(cudaStream_t s, const SweepParams &p, const SweepTuning &t,
-                                      bool count_mode, int num_sms) {
-  if (count_mode)  // per-start-box counts do not depend on the tuning
-    return launch_flat_block<256, 4, true>(s, p, num_sms);
+                                      SweepMode mode, int num_sms) {
+  // per-start-box counts do not depend on the tuning
+  if (mode == kSweepCount) return launch_flat_block<256, 4, kSweepCount>(s, p, num_sms);
+  if (mode == kSweepBoth) return launch_flat_block<256, 4, kSweepBoth>(s, p, num_sms);
   if (t.shape == kShapeFlat) {
     switch (t.per_lane) {  // filter steps per round
       case 2: return launch_flat<2>(s, p, t.block, num_sms);
@@ -958,14 +974,14 @@ size_t prefix_workspace_bytes(int64_t m) {
 
 cudaError_t launch_prefix_select(cudaStream_t s, const int32_t *box_counts, int64_t m,
                                  long long capacity, void *workspace, DevScalars *scalars,
-                                 int64_t *launches) {
+                                 int64_t *launches, const unsigned long long *found) {
   const int64_t ntiles = (m + kScanTile - 1) / kScanTile;
   long long *sums = static_cast<long long *>(workspace);
   PrefixDone *done = reinterpret_cast<PrefixDone *>(sums + ntiles + 1);
   const cudaError_t e = cudaMemsetAsync(done, 0, sizeof(PrefixDone), s);
   if (e != cudaSuccess) return e;
   launch_after(prefix_select_kernel, unsigned(ntiles), kScanBlock, 0, s, box_counts, m, capacity, sums, ntiles, done,
-               scalars);
+               scalars, found);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }

@@ -62,3 +62,36 @@ def test_tile_edges_vs_oracle(ctx, stq, oracle, cuda, n):
     r = ctx.sweep(d, n, pairs, cap, axis=-1)
     assert r.status == stq.STQ_OK and r.count == len(want)
     assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+
+
+@pytest.mark.parametrize("shape", [1, 2])
+@pytest.mark.parametrize("run_cap", [0, 40])
+def test_windows_after_an_overflow(ctx, stq, oracle, cuda, shape, run_cap):
+    """Windows after the first that overflowed count while they emit (flat shape):
+    windows that overflow, the last one with room to spare, one that fits exactly,
+    and one a pair short."""
+    import torch
+
+    n = 1500
+    b = dense_boxes(stq, n, 3, 6.0)
+    want = oracle.broadphase(b)
+    d = torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+    ctx.set_option(stq.OPT_SWEEP_SHAPE, shape)
+    ctx.set_option(stq.OPT_RUN_CAP, run_cap)
+    pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+    ctx.prepare(d, n, 0)
+    for most in (len(want) // 3, len(want) // 7 + n):
+        start, parts = 0, []
+        while start < ctx.prepared_length:
+            r = ctx.sweep_prepared(pairs, most, start=start)
+            assert r.count <= most and r.next_start > start
+            assert (r.status == stq.STQ_OK) == (r.next_start == ctx.prepared_length)
+            parts.append(pairs[: r.count].cpu().numpy().copy())
+            start = r.next_start
+        got = np.concatenate(parts)
+        assert len(got) == len(want) and np.array_equal(oracle.canonical(got), want)
+    r = ctx.sweep_prepared(pairs, len(want))  # fits exactly
+    assert r.status == stq.STQ_OK and r.count == r.total == len(want)
+    assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+    r = ctx.sweep_prepared(pairs, len(want) - 1)
+    assert r.status == stq.STQ_OVERFLOW and r.total == len(want) and r.count < len(want)
