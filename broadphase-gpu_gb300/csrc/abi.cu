@@ -739,7 +739,8 @@ int stq_batch_build_boxes(stq_context *ctx, const double *d_V0, const double *d_
   STQ_CUDA(ctx, launch_batch_build(ctx->stream, d_V0, d_V1, dev_at<long long>(ctx, ctx->layout.voff),
                                    d_E, dev_at<long long>(ctx, ctx->layout.eoff), d_F,
                                    dev_at<long long>(ctx, ctx->layout.foff),
-                                   dev_at<long long>(ctx, ctx->layout.box_off), dev_hdr(ctx), N,
+                                   dev_at<long long>(ctx, ctx->layout.box_off),
+                                   dev_at<TileRec>(ctx, ctx->layout.tiles), ctx->tile_cap, dev_hdr(ctx),
                                    ref_next_up(inflation_radius), d_boxes, ctx->points.as<float4>(),
                                    std::max<int64_t>(nv_all, 1)),
            "launch batched box build");
@@ -904,8 +905,9 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     STQ_CUDA(ctx, launch_batch_build(ctx->stream, d_V0, d_V1, dev_at<long long>(ctx, ctx->layout.voff),
                                      d_E, dev_at<long long>(ctx, ctx->layout.eoff), d_F,
                                      dev_at<long long>(ctx, ctx->layout.foff),
-                                     dev_at<long long>(ctx, ctx->layout.box_off), dev_hdr(ctx),
-                                     ctx->box_cap, ref_next_up(inflation_radius),
+                                     dev_at<long long>(ctx, ctx->layout.box_off),
+                                     dev_at<TileRec>(ctx, ctx->layout.tiles), ctx->tile_cap, dev_hdr(ctx),
+                                     ref_next_up(inflation_radius),
                                      ctx->batch_boxes.as<stq_aabb>(), ctx->points.as<float4>(), vert_cap),
              "launch batched box build");
     ctx->launches += 1;  // the rounding of the positions

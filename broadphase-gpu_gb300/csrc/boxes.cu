@@ -202,71 +202,56 @@ build_boxes_kernel(const double *__restrict__ V0, const double *__restrict__ V1,
   }
 }
 
-// Batched: box t belongs to the scene s with box_off[s] <= t < box_off[s+1];
-// its id is the batch index t, its vertex ids are local to scene s.
+// Batched: kBuildParts blocks per tile (boxes of one scene), so that the scene and its
+// offsets are read once. With a search of the scene for each box, 256 scenes of 9.1 M
+// boxes took 181 us; with 1, 2, 4 and 8 blocks per tile 151, 143, 143 and 151, and 16
+// scenes of 100,000 boxes (11.2 with the search) 14.1, 12.0, 11.9 and 11.9.
+// A box's id is its batch index, its vertex ids are local to the scene.
+constexpr int kBuildParts = 4;
+template <typename Build>
+__device__ __forceinline__ void build_tile(const TileRec &t, stq_aabb *__restrict__ out, const Build &build) {
+  __shared__ uint32_t stage[kBuildBlock / 32][32 * kBoxWords];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int first = int(blockIdx.x % kBuildParts) * kBuildBlock + 32 * warp; first < t.count;
+       first += kBuildParts * kBuildBlock) {
+    const bool have = first + lane < t.count;
+    stq_aabb b;
+    if (have) b = build(t.begin + first + lane);
+    store_boxes(b, have, t.begin + first, min(t.count - first, 32), out, stage[warp], lane);
+  }
+}
+
 __global__ void __launch_bounds__(kBuildBlock)
 batch_build_kernel(const double *__restrict__ V0, const double *__restrict__ V1,
                    const long long *__restrict__ voff, const int32_t *__restrict__ E,
                    const long long *__restrict__ eoff, const int32_t *__restrict__ F,
                    const long long *__restrict__ foff, const long long *__restrict__ box_off,
-                   BatchHeader *hdr, float r_up, stq_aabb *__restrict__ out,
+                   const TileRec *__restrict__ tiles, BatchHeader *hdr, float r_up, stq_aabb *__restrict__ out,
                    const float4 *__restrict__ P) {
   after_previous();
-  __shared__ uint32_t stage[kBuildBlock / 32][32 * kBoxWords];
-  const int lane = threadIdx.x & 31;
-  const int n_scenes = hdr->n_scenes;
-  const int64_t n_boxes = hdr->n_boxes;
+  if (int(blockIdx.x / kBuildParts) >= hdr->n_tiles) return;
+  const TileRec t = tiles[blockIdx.x / kBuildParts];
+  const int s = t.scene;
+  const int64_t v0 = voff[s], e0 = eoff[s], f0 = foff[s], nV = voff[s + 1] - v0, nE = eoff[s + 1] - e0, b0 = box_off[s];
   int *flags = &hdr->flags;
-  const int64_t step = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t base = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) - lane; base < n_boxes;
-       base += step) {
-    const int64_t t = base + lane;
-    stq_aabb b;
-    if (t < n_boxes) {
-      int lo = 0, hi = n_scenes - 1;  // last scene with box_off[s] <= t
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (box_off[mid] <= t) lo = mid;
-        else hi = mid - 1;
-      }
-      const int s = lo;
-      const int64_t v0 = voff[s], e0 = eoff[s], f0 = foff[s];
-      b = build_one(V0 + 3 * v0, V1 + 3 * v0, P + 2 * v0, voff[s + 1] - v0, E + 2 * e0, eoff[s + 1] - e0,
-                    F + 3 * f0, t - box_off[s], int(t), r_up, flags);
-    }
-    store_boxes(b, t < n_boxes, base, int(n_boxes - base < 32 ? n_boxes - base : 32), out, stage[threadIdx.x >> 5],
-                lane);
-  }
+  build_tile(t, out, [&](int64_t i) {
+    return build_one(V0 + 3 * v0, V1 + 3 * v0, P + 2 * v0, nV, E + 2 * e0, nE, F + 3 * f0, i - b0, int(i), r_up, flags);
+  });
 }
 
-// Serving: scene s's mesh lives in its own allocation (MeshRef); the box id
-// is the batch index, vertex ids are local to the scene.
+// Serving: scene s's mesh lives in its own allocation (MeshRef).
 __global__ void __launch_bounds__(kBuildBlock)
 batch_build_refs_kernel(const MeshRef *__restrict__ refs, const long long *__restrict__ box_off,
-                        BatchHeader *hdr, float r_up, stq_aabb *__restrict__ out) {
+                        const TileRec *__restrict__ tiles, BatchHeader *hdr, float r_up, stq_aabb *__restrict__ out) {
   after_previous();
-  __shared__ uint32_t stage[kBuildBlock / 32][32 * kBoxWords];
-  const int lane = threadIdx.x & 31;
-  const int n_scenes = hdr->n_scenes;
-  const int64_t n_boxes = hdr->n_boxes;
-  const int64_t step = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t base = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) - lane; base < n_boxes;
-       base += step) {
-    const int64_t t = base + lane;
-    stq_aabb b;
-    if (t < n_boxes) {
-      int lo = 0, hi = n_scenes - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (box_off[mid] <= t) lo = mid;
-        else hi = mid - 1;
-      }
-      const MeshRef &m = refs[lo];
-      b = build_one(m.V0, m.V1, nullptr, m.nV, m.E, m.nE, m.F, t - box_off[lo], int(t), r_up, &hdr->flags);
-    }
-    store_boxes(b, t < n_boxes, base, int(n_boxes - base < 32 ? n_boxes - base : 32), out, stage[threadIdx.x >> 5],
-                lane);
-  }
+  if (int(blockIdx.x / kBuildParts) >= hdr->n_tiles) return;
+  const TileRec t = tiles[blockIdx.x / kBuildParts];
+  const MeshRef m = refs[t.scene];
+  const int64_t b0 = box_off[t.scene];
+  int *flags = &hdr->flags;
+  build_tile(t, out, [&](int64_t i) {
+    return build_one(m.V0, m.V1, nullptr, m.nV, m.E, m.nE, m.F, i - b0, int(i), r_up, flags);
+  });
 }
 
 int grid_for(int64_t n, int block, int cap = 152 * 32) {
@@ -293,18 +278,17 @@ cudaError_t launch_build_boxes(cudaStream_t s, const double *V0, const double *V
 cudaError_t launch_batch_build(cudaStream_t s, const double *V0, const double *V1,
                                const long long *voff, const int32_t *E, const long long *eoff,
                                const int32_t *F, const long long *foff, const long long *box_off,
-                               BatchHeader *hdr, int64_t box_cap, float r_up, stq_aabb *out,
+                               const TileRec *tiles, int tile_cap, BatchHeader *hdr, float r_up, stq_aabb *out,
                                float4 *points, int64_t vert_cap) {
   launch_after(batch_round_points_kernel, grid_for(vert_cap, 256), 256, 0, s, V0, V1, voff, hdr, vert_cap, points);
-  launch_after(batch_build_kernel, grid_for(box_cap, kBuildBlock), kBuildBlock, 0, s, V0, V1, voff, E, eoff, F, foff,
-               box_off, hdr, r_up, out, points);
+  launch_after(batch_build_kernel, unsigned(tile_cap) * kBuildParts, kBuildBlock, 0, s, V0, V1, voff, E, eoff, F, foff, box_off,
+               tiles, hdr, r_up, out, points);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_build_refs(cudaStream_t s, const MeshRef *refs, const long long *box_off,
-                                    BatchHeader *hdr, int64_t box_cap, float r_up, stq_aabb *out) {
-  launch_after(batch_build_refs_kernel, grid_for(box_cap, kBuildBlock), kBuildBlock, 0, s, refs, box_off, hdr, r_up,
-               out);
+                                    const TileRec *tiles, int tile_cap, BatchHeader *hdr, float r_up, stq_aabb *out) {
+  launch_after(batch_build_refs_kernel, unsigned(tile_cap) * kBuildParts, kBuildBlock, 0, s, refs, box_off, tiles, hdr, r_up, out);
   return cudaGetLastError();
 }
 

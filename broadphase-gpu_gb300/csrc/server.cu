@@ -268,7 +268,8 @@ int enqueue_tick(stq_server *sv, bool advance) {
                                  hdr, sv->max_boxes),
              "launch advance");
   const long long *box_off = dev_at<long long>(ctx, ctx->layout.box_off);
-  STQ_CUDA(ctx, launch_batch_build_refs(ctx->stream, sv->refs_dev.as<MeshRef>(), box_off, hdr, ctx->box_cap,
+  STQ_CUDA(ctx, launch_batch_build_refs(ctx->stream, sv->refs_dev.as<MeshRef>(), box_off,
+                                        dev_at<TileRec>(ctx, ctx->layout.tiles), ctx->tile_cap, hdr,
                                         ref_next_up(0.f), ctx->batch_boxes.as<stq_aabb>()),
            "launch box build");
   const BatchBuffers b = batch_buffers(ctx, ctx->batch_boxes.as<stq_aabb>());

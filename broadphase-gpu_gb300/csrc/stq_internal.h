@@ -354,7 +354,7 @@ cudaError_t launch_gather_cells(cudaStream_t s, const BatchBuffers &b, int64_t r
 cudaError_t launch_batch_build(cudaStream_t s, const double *V0, const double *V1,
                                const long long *voff, const int32_t *E, const long long *eoff,
                                const int32_t *F, const long long *foff, const long long *box_off,
-                               BatchHeader *hdr, int64_t box_cap, float r_up, stq_aabb *out,
+                               const TileRec *tiles, int tile_cap, BatchHeader *hdr, float r_up, stq_aabb *out,
                                float4 *points, int64_t vert_cap);
 // A scene held by the serving loop: its own device mesh and time-step state.
 struct MeshRef {
@@ -369,7 +369,7 @@ struct MeshRef {
 cudaError_t launch_advance(cudaStream_t s, const MeshRef *refs, const long long *voff,
                            const BatchHeader *hdr, int64_t vert_cap);
 cudaError_t launch_batch_build_refs(cudaStream_t s, const MeshRef *refs, const long long *box_off,
-                                    BatchHeader *hdr, int64_t box_cap, float r_up, stq_aabb *out);
+                                    const TileRec *tiles, int tile_cap, BatchHeader *hdr, float r_up, stq_aabb *out);
 cudaError_t launch_pair_checksums(cudaStream_t s, const stq_pair *pairs, long long capacity,
                                   const BatchHeader *hdr, const long long *box_off,
                                   unsigned long long *checks, int scene_cap);

@@ -261,3 +261,27 @@ def test_batch_graph_follows_small_radii(ctx, stq, oracle, cuda, scenes):
         assert np.array_equal(oracle.canonical(pairs[: res.count].cpu().numpy()), want)
         counts.add(len(want))
     assert len(counts) == 2
+
+
+@pytest.mark.parametrize("filler", [0, 80_000, 640_000])  # tiles of 256, 1,024 and 4,096 boxes
+def test_batch_build_at_tile_edges(ctx, stq, oracle, cuda, filler):
+    import torch
+
+    rng = np.random.default_rng(filler)
+    sizes = [1, 31, 33, 0, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, filler]
+    vo = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    V0, V1 = rng.normal(size=(vo[-1], 3)), rng.normal(size=(vo[-1], 3))
+    none = np.zeros(len(vo), np.int64)
+    E, F = np.zeros((0, 2), np.int32), np.zeros((0, 3), np.int32)
+    out = torch.full((int(vo[-1]) + 8, 11), -7, dtype=torch.int32, device=cuda)
+    bo = ctx.batch_build_boxes(dev(V0, cuda), dev(V1, cuda), vo, dev(E, cuda), none, dev(F, cuda), none, out)
+    assert np.array_equal(bo, vo)
+    got = out.cpu().numpy()
+    assert np.all(got[vo[-1] :] == -7)
+    got = got[: vo[-1]].reshape(-1).view(stq.AABB_DTYPE)
+    for a, b in zip(vo[:-1], vo[1:]):
+        if a == b:
+            continue
+        want = oracle.construct_boxes(V0[a:b], V1[a:b], E, F, stq.AABB_DTYPE).copy()
+        want["id"] += int(a)
+        assert np.array_equal(got[a:b], want), (a, b)
