@@ -437,7 +437,7 @@ int stq_server_create(int device, void *stream, int64_t budget_bytes, int64_t ma
       cudaEventCreateWithFlags(&sv->copy_done, cudaEventDisableTiming) != cudaSuccess)
     return bad(STQ_ERR_CUDA);
   // pipeline buffers for the largest batch, counted against the budget
-  // small ticks are cut into small tiles, of which there are fewer than kSmallBatch
+  // small ticks are cut into small tiles, of which there are at most kSmallBatch
   // / kSmallTile and one per scene
   const int64_t tiles = std::max(max_boxes / kTileBoxes, kSmallBatch / kSmallTile) + max_scenes + 1;
   if (ensure_staging(ctx, max_scenes, int(tiles)) != STQ_OK || ensure_box_buffers(ctx, max_boxes) != STQ_OK ||

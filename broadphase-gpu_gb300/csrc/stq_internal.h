@@ -190,13 +190,15 @@ struct FrontInfo {
 // host from the scene offsets), so that a block reduces per-scene values once.
 constexpr int kTileBoxes = 4096;
 // Batches of up to kSmallBatch boxes take tiles of 1,024, so that most SMs get one,
-// and those of up to kTinyBatch tiles of 256, one box per thread: whole passes with
-// tiles of 1,024 -> 256: 2,000 boxes 118 -> 107 us, 53,000 boxes 167 -> 166, 477,000
-// boxes 297 -> 318 (the last block scans the tiles).
-constexpr int kSmallTile = 1024, kTinyTile = 256;
-constexpr int64_t kSmallBatch = 152 * 4 * kSmallTile, kTinyBatch = 152 * 2 * kTinyTile;
+// those of up to kMidBatch tiles of 2,048, and those of up to kTinyBatch tiles of 256,
+// one box per thread. Whole passes with tiles of 1,024 -> 256: 2,000 boxes 118 -> 107
+// us, 53,000 boxes 167 -> 166, 477,000 boxes 297 -> 318 (the last block scans the
+// tiles); of 4,096 -> 2,048: 684,000 boxes 745 -> 737, 9.1 M boxes 3,006 -> 3,018.
+constexpr int kSmallTile = 1024, kMidTile = 2048, kTinyTile = 256;
+constexpr int64_t kTinyBatch = 152 * 2 * kTinyTile;
+constexpr int64_t kSmallBatch = 152 * 4 * kSmallTile, kMidBatch = 152 * 4 * kMidTile;
 constexpr int tile_boxes(int64_t n) {
-  return n <= kTinyBatch ? kTinyTile : (n <= kSmallBatch ? kSmallTile : kTileBoxes);
+  return n <= kTinyBatch ? kTinyTile : (n <= kSmallBatch ? kSmallTile : (n <= kMidBatch ? kMidTile : kTileBoxes));
 }
 struct TileRec {
   long long begin;  // first box of the tile

@@ -48,10 +48,10 @@ def test_dense_windows_vs_oracle(ctx, stq, oracle, cuda, n, spread, run_cap):
     assert len(got) == len(want) and np.array_equal(oracle.canonical(got), want)
 
 
-@pytest.mark.parametrize("n", [255, 256, 257, 77_823, 77_824, 77_825])
+@pytest.mark.parametrize("n", [255, 256, 257, 77_823, 77_824, 77_825, 622_592, 622_593])
 def test_tile_edges_vs_oracle(ctx, stq, oracle, cuda, n):
-    """Tiles of 256 boxes up to 77,824 boxes, of 1,024 above; the last one of 1,
-    255 or 256 boxes."""
+    """Tiles of 256 boxes up to 77,824 boxes, of 1,024 up to 622,592, of 2,048 above;
+    the last one full, one short of it, or of one box."""
     import torch
 
     b = stq.random_boxes(n, seed=n)
