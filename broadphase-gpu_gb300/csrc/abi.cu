@@ -469,8 +469,8 @@ int emit_prefix(stq_context *ctx, int64_t start, int64_t end, stq_pair *d_pairs,
   *count = int64_t(ctx->h_hdr->pairs);
   *next_start = end;
   if (found && total) *total = int64_t(ctx->h_sel->count);
-  if (found && ctx->h_sel->count <= (unsigned long long)capacity) return STQ_OK;
-  ctx->overflowed = true;
+  ctx->overflowed = !found || ctx->h_sel->count > (unsigned long long)capacity;
+  if (!ctx->overflowed) return STQ_OK;
   *next_start = start + ctx->h_sel->prefix;
   if (ctx->h_sel->prefix <= 0) return fail(ctx, STQ_ERR_CAPACITY, "the first start box has more pairs than capacity");
   if (*count > capacity) return fail(ctx, STQ_ERR_CUDA, "prefix re-sweep exceeded capacity");
@@ -803,8 +803,8 @@ int stq_sweep_prepared(stq_context *ctx, int64_t start, int64_t max_start, stq_p
   if (start < 0 || start > length) return fail(ctx, STQ_ERR_INVALID_ARG, "start out of range");
   DeviceGuard g(ctx->device);
   const int64_t end = (max_start <= 0 || start + max_start > length) ? length : start + max_start;
-  // once a sweep of the prepared scenes overflowed, the next ones count as they
-  // emit, and the whole of the overflow is queued with them. Windows of a
+  // after a sweep of the prepared scenes that overflowed, the next one counts as it
+  // emits, and the whole of the overflow is queued with it. Windows of a
   // 684,000-box scene, three of 820,000 pairs (whole pass): 790 -> 747 us
   if (ctx->overflowed && ctx->tuning.shape == kShapeFlat && end > start) {
     STQ_TRY(clear_box_counts(ctx, end - start));

@@ -111,7 +111,7 @@ struct stq_context {
   DevScalars *h_sel = nullptr;        // readback of an overflowing sweep's prefix
   int pair_id_bits = 0;               // of the largest first id of the pairs sorted so far
   int passes_seen = 0;  // most digits that a replica sort of this context needed
-  bool overflowed = false;  // a sweep of the prepared scenes found more pairs than the buffer held
+  bool overflowed = false;  // the last sweep of the prepared scenes found more pairs than fit
   bool swept = false;   // the prepared scenes have been swept (their pair counters hold)
   unsigned long long *h_scene_pairs = nullptr;  // pinned readback
   int h_scene_pairs_cap = 0;
