@@ -990,6 +990,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
   ctx->length = int64_t(h.length);
   ctx->scene.length = ctx->length;
   ctx->prepared = true;
+  ctx->swept = true;  // also by a replayed graph, which does not go through run_sweep
   if (h_scene_pairs)
     for (int s = 0; s < n_scenes; ++s) h_scene_pairs[s] = int64_t(ctx->h_scene_pairs[s]);
   const int64_t found = int64_t(h.pairs);

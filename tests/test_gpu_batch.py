@@ -243,6 +243,30 @@ def test_batch_graph_follows_buffers_that_another_call_moved(stq, oracle, cuda, 
                 ctx.set_option(stq.OPT_CELLS, 0)
 
 
+def test_scene_pairs_after_a_replayed_batch(stq, oracle, cuda, scenes):
+    """A prepare between two batches that moves no buffer: the second batch replays the
+    captured graph (no launch of its own), and the counts per scene are its own."""
+    import torch
+
+    meshes, want = scenes
+    V0, V1, E, F, vo, eo, fo = stq.concat_meshes(meshes)
+    d = [dev(x, cuda) for x in (V0, V1, E, F)]
+    cap = sum(len(w) for w in want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    b = stq.random_boxes(64, seed=3)
+    small = dev(b.view(np.int32).reshape(-1, 11), cuda)
+    with stq.Context(0, torch.cuda.current_stream(cuda).cuda_stream) as ctx:
+        for rep in range(3):
+            before = ctx.launches
+            r, per = ctx.batch_broadphase(d[0], d[1], vo, d[2], eo, d[3], fo, pairs, cap)
+            assert r.status == stq.STQ_OK
+            assert (ctx.launches == before) == (rep > 0)
+            assert np.array_equal(per, [len(w) for w in want])
+            assert np.array_equal(ctx.batch_scene_pairs(len(meshes)), per)
+            ctx.prepare(small, len(b), 0)
+            assert np.array_equal(ctx.batch_scene_pairs(1), [0])  # not swept yet
+
+
 def test_batch_graph_follows_small_radii(ctx, stq, oracle, cuda, scenes):
     """Two inflation radii below 1e-9 are two graphs: the pairs of a scene scaled
     to 1e-9 depend on which of them was asked for."""
