@@ -38,6 +38,7 @@ int fail(stq_context *ctx, int status, const char *what, cudaError_t e) {
       std::snprintf(buf, sizeof buf, "%s", what);
     ctx->error = buf;
   }
+  if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();  // reported here, not by the next launch
   return status;
 }
 
@@ -117,6 +118,7 @@ int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap) {
   scene_cap = std::max(scene_cap, ctx->scene_cap);
   tile_cap = std::max(tile_cap, ctx->tile_cap);
   const Staging lay = Staging::make(scene_cap, tile_cap);
+  ctx->scene_cap = ctx->tile_cap = 0;  // until all of it is allocated
   if (ctx->in_host) {
     STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
     cudaFreeHost(ctx->in_host);
@@ -136,6 +138,7 @@ int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap) {
   if (scene_cap > ctx->h_scene_pairs_cap) {
     if (ctx->h_scene_pairs) cudaFreeHost(ctx->h_scene_pairs);
     ctx->h_scene_pairs = nullptr;
+    ctx->h_scene_pairs_cap = 0;
     STQ_CUDA(ctx, cudaMallocHost(&ctx->h_scene_pairs, sizeof(unsigned long long) * size_t(scene_cap)),
              "allocate pinned scene counters");
     ctx->h_scene_pairs_cap = scene_cap;
@@ -237,7 +240,9 @@ int ensure_box_buffers(stq_context *ctx, int64_t box_cap) {
   return STQ_OK;
 }
 
-int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap) {
+namespace {
+
+int grow_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap) {
   const size_t r = size_t(std::max<int64_t>(rep_cap, 1));
   for (int b = 0; b < 2; ++b) {
     STQ_CUDA(ctx, ctx->keys[b].ensure(sizeof(uint32_t) * r), "allocate keys");
@@ -247,7 +252,6 @@ int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap)
   // three lists (vertices, edges, faces) per cell, each followed by a sentinel
   const int64_t segs = std::max<int64_t>(3 * cells_cap, ctx->seg_cap);
   STQ_CUDA(ctx, ctx->seg_scan.ensure(sizeof(uint32_t) * size_t(segs + 1)), "allocate segment offsets");
-  ctx->seg_cap = segs;
   const size_t slots = r + size_t(segs) + 1 + kSortedPad;
   STQ_CUDA(ctx, ctx->yz.ensure(sizeof(float4) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->xx.ensure(sizeof(float2) * slots), "allocate sorted scene");
@@ -257,9 +261,26 @@ int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap)
   STQ_CUDA(ctx, ctx->partner.ensure(sizeof(int) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->run_end.ensure(sizeof(int) * slots), "allocate sorted scene");
   STQ_CUDA(ctx, ctx->long_list.ensure(sizeof(int2) * slots), "allocate long-run list");
+  ctx->seg_cap = segs;
   ctx->rep_cap = int64_t(r);
   ctx->slot_cap = int64_t(slots);
   return STQ_OK;
+}
+
+}  // namespace
+
+int ensure_replica_buffers(stq_context *ctx, int64_t rep_cap, int64_t cells_cap) {
+  const int st = grow_replica_buffers(ctx, rep_cap, cells_cap);
+  if (st != STQ_OK) {
+    // the buffers are of any size now: a prepare must not take them for those of
+    // the scenes before (has_room), and what was allocated is given back
+    ctx->prepared = false;
+    ctx->rep_cap = ctx->slot_cap = ctx->seg_cap = 0;
+    for (DevBuf *b : {&ctx->keys[0], &ctx->keys[1], &ctx->vals[0], &ctx->vals[1], &ctx->sort_ws, &ctx->seg_scan, &ctx->yz,
+                      &ctx->xx, &ctx->vv, &ctx->flag, &ctx->scode, &ctx->partner, &ctx->run_end, &ctx->long_list})
+      b->release();
+  }
+  return st;
 }
 
 int bits_for(int64_t v) {
@@ -888,6 +909,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
   const int64_t T = std::max<int64_t>(tiles_for(box_off.data(), n_scenes), 1);
   const int64_t rep_cap = std::max<int64_t>(int64_t(ctx->budget) * N, 1);
   const int64_t cells_cap = N / 16 + n_scenes + 1;
+  ctx->prepared = false;  // the buffers of the prepared scenes are reused
   STQ_TRY(ensure_staging(ctx, n_scenes, int(T)));
   STQ_TRY(ensure_box_buffers(ctx, N));
   STQ_TRY(ensure_replica_buffers(ctx, rep_cap, cells_cap));
@@ -952,6 +974,8 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     key.opts[16] = int64_t(radius_bits);
     key.stream = caller;
     for (const DevBuf *b : ctx->buffers()) key.bufs.push_back(b->ptr);
+    key.bufs.push_back(ctx->in_host);
+    key.bufs.push_back(ctx->h_scene_pairs);
     int st = STQ_OK;
     if (!ctx->graph || !(key == ctx->graph_key)) {
       if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
@@ -1159,14 +1183,14 @@ int stq_sort_pairs(stq_context *ctx, stq_pair *d_pairs, int64_t count) {
   // the sort reads a pair as one word: pairs that are not on 8 bytes are sorted in a copy
   const bool copy = reinterpret_cast<uintptr_t>(d_pairs) % sizeof(unsigned long long) != 0;
   STQ_CUDA(ctx, ctx->pair_tmp.ensure(sizeof(stq_pair) * size_t(count) * (copy ? 2 : 1)), "allocate pair buffer");
-  STQ_CUDA(ctx, ctx->sort_ws.ensure(pair_workspace_bytes(count)), "allocate sort workspace");
+  STQ_CUDA(ctx, ctx->pair_ws.ensure(pair_workspace_bytes(count)), "allocate sort workspace");
   stq_pair *pairs = copy ? ctx->pair_tmp.as<stq_pair>() + count : d_pairs;
   *ctx->h_fault = 0;
   stage_begin(ctx, kPairSort);
   if (copy)
     STQ_CUDA(ctx, cudaMemcpyAsync(pairs, d_pairs, sizeof(stq_pair) * size_t(count), cudaMemcpyDeviceToDevice,
                                   ctx->stream), "copy pairs");
-  STQ_CUDA(ctx, sort_pairs(ctx->stream, pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->sort_ws.ptr, ctx->h_plan,
+  STQ_CUDA(ctx, sort_pairs(ctx->stream, pairs, ctx->pair_tmp.as<stq_pair>(), count, ctx->pair_ws.ptr, ctx->h_plan,
                            &ctx->pair_id_bits, ctx->h_fault, &ctx->launches),
            "launch pair sort");
   if (copy)

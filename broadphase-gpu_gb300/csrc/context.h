@@ -90,6 +90,7 @@ struct stq_context {
   DevBuf scenes, cell_base, scene_pairs, box_cells, box_q, tile_reps, tile_off, keys[2], vals[2], sort_ws;
   DevBuf points;  // fp64 vertex positions rounded to float once (box builds)
   DevBuf yz, xx, vv, flag, scode, partner, run_end, box_counts, prefix_ws, pair_tmp;
+  DevBuf pair_ws;  // pair sorts' own: a prepare relies on sort_ws as it sized it
   DevBuf long_list;  // runs handed from the lane sweep to the warp pass
   DevBuf seg_scan;  // first sorted replica of each (cell, type) list
   int64_t seg_cap = 0;
@@ -149,7 +150,7 @@ struct stq_context {
   std::vector<DevBuf *> buffers() {
     return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &box_cells, &box_q, &tile_reps, &tile_off, &keys[0], &keys[1],
             &vals[0], &vals[1], &sort_ws, &yz, &xx, &vv, &flag, &scode, &partner, &run_end, &long_list, &seg_scan, &box_counts,
-            &prefix_ws, &pair_tmp, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh, &aux, &window_pairs,
+            &prefix_ws, &pair_tmp, &pair_ws, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh, &aux, &window_pairs,
             &window_long_list, &window_cursors};
   }
 };

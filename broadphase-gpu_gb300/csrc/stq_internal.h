@@ -25,7 +25,12 @@ struct DevBuf {
     bytes = 0;
     size_t rounded = (want + 4095) & ~size_t(4095);
     cudaError_t e = cudaMalloc(&ptr, rounded);
-    if (e == cudaSuccess) bytes = rounded;
+    if (e == cudaSuccess) {
+      bytes = rounded;
+    } else {
+      ptr = nullptr;
+      (void)cudaGetLastError();  // a refused allocation is no error of the next launch
+    }
     return e;
   }
   void release() {

@@ -69,3 +69,55 @@ def test_bad_boxes_after_good_ones(ctx, stq, oracle, cuda):
         r = ctx.sweep_prepared(small, len(want) // 2, start=r.next_start)
         got.append(small[: r.count].cpu().numpy().copy())
     assert np.array_equal(oracle.canonical(np.concatenate(got)), want)
+
+
+@pytest.mark.parametrize("left", [2500 << 20, 1500 << 20, 300 << 20])
+def test_refused_allocations_leave_the_context_usable(stq, oracle, cuda, left):
+    """The device's memory is held but for `left` bytes, so that the buffers of a large
+    scene and a pair sort's are refused at different places. What fitted before fits
+    after: the same small scene, against the oracle."""
+    import torch
+
+    b = scene(stq, 4000, 0.05, seed=7)
+    want = oracle.broadphase(b)
+    d, n = dev(b, cuda), len(b)
+    pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+    # 12 boxes across every cell of a 2,048 x 2,048 grid: 50 M replicas, 5 GB of buffers
+    big = scene(stq, 12, 0.05, seed=8)
+    big["min"], big["max"] = 0.0, 1.0
+    big = dev(big, cuda)
+    held = None
+
+    def refused(call, *args):  # (an exception that is kept would keep the held memory)
+        try:
+            call(*args)
+        except stq.STQError as e:
+            return e.status
+        return stq.STQ_OK
+
+    with stq.Context(0, torch.cuda.current_stream(cuda).cuda_stream) as ctx:
+
+        def check():
+            r = ctx.sweep(d, n, pairs, len(want) + 16)
+            assert r.status == stq.STQ_OK and r.count == len(want)
+            ctx.sort_pairs(pairs, r.count)
+            assert np.array_equal(pairs[: r.count].cpu().numpy(), oracle.canonical(want))
+
+        check()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info(cuda)[0]
+        held = torch.empty(free - left, dtype=torch.uint8, device=cuda)
+        try:
+            ctx.set_option(stq.OPT_CELLS, 2048)
+            assert refused(ctx.prepare, big, 12, 0) == stq.STQ_ERR_NO_MEMORY and ctx.prepared_length == -1
+            assert refused(ctx.sweep_prepared, pairs, 16) == stq.STQ_ERR_NOT_PREPARED
+            ctx.set_option(stq.OPT_CELLS, 0)
+            check()
+            # pairs (of the held memory, never read) whose second buffer fits, but not
+            # the tables: half a byte per pair
+            count = (torch.cuda.mem_get_info(cuda)[0] - (8 << 20)) // 8
+            assert refused(ctx.sort_pairs, held, count) == stq.STQ_ERR_NO_MEMORY
+            check()
+        finally:
+            del held
+            torch.cuda.empty_cache()
