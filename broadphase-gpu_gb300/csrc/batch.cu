@@ -360,10 +360,11 @@ __device__ __forceinline__ Range cell_range(const stq_aabb &x, int a, float ob, 
   int b, c;
   axes_bc(a, b, c);
   Range r;
+  // (a box in a grid has min <= max, or a NaN bound, which is refused: cell 0)
   r.b0 = cell_coord(x.min[b], ob, ib, nb);
-  r.b1 = cell_coord(x.max[b], ob, ib, nb);
+  r.b1 = max(cell_coord(x.max[b], ob, ib, nb), r.b0);
   r.c0 = cell_coord(x.min[c], oc, ic, nc);
-  r.c1 = cell_coord(x.max[c], oc, ic, nc);
+  r.c1 = max(cell_coord(x.max[c], oc, ic, nc), r.c0);
   return r;
 }
 
@@ -451,10 +452,12 @@ choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__
     const int key_bits = seg_bits <= 15 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
     const int passes = max(seg_bits + key_bits + 7, 8) / 8;
     // more than the buffers hold: the scenes are flagged and left empty (the
-    // caller without limits checks that positions fit 31 bits)
-    const bool fits = R < 0xffffffffull && (rep_cap < 0 || ((long long)R <= rep_cap && (long long)lists <= seg_cap &&
-                                                            passes <= max_passes));
-    if (!fits) atomicOr(&hdr->flags, kFlagReplicaOverflow);
+    // caller without limits checks that positions fit 31 bits). So are scenes with a
+    // bad box: what follows is queued already
+    const bool bad = hdr->flags != 0;
+    const bool fits = !bad && R < 0xffffffffull &&
+                      (rep_cap < 0 || ((long long)R <= rep_cap && (long long)lists <= seg_cap && passes <= max_passes));
+    if (!fits && !bad) atomicOr(&hdr->flags, kFlagReplicaOverflow);
     hdr->replicas = fits ? unsigned(R) : 0u;
     hdr->cells = fits ? carry : 0u;
     hdr->lists = fits ? unsigned(lists) : 0u;

@@ -71,6 +71,37 @@ def test_bad_boxes_after_good_ones(ctx, stq, oracle, cuda):
     assert np.array_equal(oracle.canonical(np.concatenate(got)), want)
 
 
+@pytest.mark.parametrize("field,axis", [(f, a) for f in ("min", "max") for a in range(3)])
+@pytest.mark.parametrize("bits", [0x7FC00000, 0xFFC00000])  # NaN, and NaN with the sign set
+def test_a_nan_of_either_sign_is_refused(ctx, stq, oracle, cuda, field, axis, bits):
+    """In the first box, one in the middle and the last one of scenes in grids, by the whole
+    sweep and by prepare; the scene without it before and after."""
+    import torch
+
+    n = 3000
+    b = scene(stq, n, 0.04, seed=9)
+    want = oracle.broadphase(b)
+    good = dev(b, cuda)
+    pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+    for at in (0, n // 2, n - 1):
+        bad = b.copy()
+        bad[field].view(np.uint32)[at, axis] = bits
+        bad = dev(bad, cuda)
+        for cells in (0, 40):
+            ctx.set_option(stq.OPT_CELLS, cells)
+            for boxes in (good, bad, good):
+                calls = (lambda: ctx.sweep(boxes, n, pairs, len(pairs), axis=-1),
+                         lambda: ctx.batch_prepare(boxes, [0, 1, n], axis=0))
+                for k, call in enumerate(calls):
+                    if boxes is bad:
+                        with pytest.raises(stq.STQError) as e:
+                            call()
+                        assert e.value.status == stq.STQ_ERR_INVALID_INPUT and ctx.prepared_length == -1
+                    else:
+                        r = call()
+                        assert k or np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+
+
 @pytest.mark.parametrize("left", [2500 << 20, 1500 << 20, 300 << 20])
 def test_refused_allocations_leave_the_context_usable(stq, oracle, cuda, left):
     """The device's memory is held but for `left` bytes, so that the buffers of a large
