@@ -627,6 +627,7 @@ __global__ void __launch_bounds__(kBlock)
 list_offsets_kernel(const uint32_t *__restrict__ keys, BatchHeader *__restrict__ hdr,
                     uint32_t *__restrict__ seg_scan, long long seg_cap, SortedScene scene, int64_t slots_cap) {
   after_previous();
+  if (hdr->fault) return;  // the replicas are not sorted
   // (cells past the capacity are flagged and counted as none)
   const uint32_t nseg = uint32_t(min(3ll * hdr->cells, seg_cap));
   const uint32_t R = hdr->replicas;
@@ -716,6 +717,7 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const uint32_t *__restri
                     const SceneRecord *__restrict__ scenes, const uint32_t *__restrict__ seg_scan,
                     SortedScene scene) {
   after_previous();
+  if (hdr->fault) return;  // the replicas are not sorted
   const int64_t R = hdr->replicas;
   const int S = hdr->n_scenes;
   const int key_bits = hdr->key_bits;

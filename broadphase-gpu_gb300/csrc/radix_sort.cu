@@ -37,8 +37,12 @@ constexpr int kMinTile = kRadixMinTile;  // smallest tile of a pass
 static_assert(kMinTile == kPassBlock * 4, "smallest tile: four keys per thread");
 constexpr int kHistBlock = 512;
 // polls of one status word before a block gives up (each is a load from L2,
-// some 0.5 us; a predecessor's counts take a few microseconds)
-constexpr int kSpinLimit = 1 << 20;
+// some 0.5 us; a predecessor's counts take a few microseconds). A test builds the
+// sort with 0: every tile but the first gives up.
+#ifndef STQ_SORT_POLL_LIMIT
+#define STQ_SORT_POLL_LIMIT (1 << 20)
+#endif
+constexpr int kPollLimit = STQ_SORT_POLL_LIMIT;
 
 // Head of the workspace, cleared before every sort; the tiles' status words
 // follow it.
@@ -48,6 +52,7 @@ struct SortHead {
   uint32_t done;                     // blocks of the histogram kernel that are done
   uint32_t run[kMaxPasses];          // the pass is run (not skipped)
   uint32_t src[kMaxPasses];          // buffer that the pass reads
+  uint32_t fault;                    // a wait gave up: nothing more is written
 };
 
 static_assert(sizeof(SortHead) <= kRadixHeadBytes, "workspace sizing");
@@ -68,6 +73,10 @@ __device__ __forceinline__ unsigned long long load_status(const unsigned long lo
 }
 __device__ __forceinline__ void store_status(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ bool faulted(const SortHead *head) {
+  return *reinterpret_cast<const volatile uint32_t *>(&head->fault) != 0u;
 }
 
 // Exclusive scan of v over the first 256 threads of the block (every thread
@@ -185,12 +194,18 @@ radix_hist_kernel(const K *__restrict__ k0, const K *__restrict__ k1, int64_t n,
 // of the tiles before it, eight at a time, back to one that holds its own sum.
 // Status word: (2 * pass + 1) << 32 | count of the tile, or (2 * pass + 2) << 32
 // | sum up to and with the tile; smaller tags are from earlier passes.
-__device__ __forceinline__ uint32_t look_back(const unsigned long long *status, int64_t tile, int d, uint32_t tag,
-                                              bool *timeout) {
+// *timeout: a word did not come, here or in another block of the pass.
+__device__ __forceinline__ uint32_t look_back(const SortHead *head, const unsigned long long *status, int64_t tile, int d,
+                                              uint32_t tag, bool *timeout) {
   uint32_t sum = 0;
-  int spins = 0;
+  int polls = 0;
   int64_t t = tile - 1;
   while (t >= 0) {
+    if (polls == kPollLimit || (polls % 1024 == 1023 && faulted(head))) {
+      *timeout = true;
+      break;
+    }
+    ++polls;
     unsigned long long w[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -203,19 +218,16 @@ __device__ __forceinline__ uint32_t look_back(const unsigned long long *status, 
       if (g < tag) {
         wait = true;
         t -= i;
+        if (i > 0) polls = 0;
       } else {
         sum += uint32_t(w[i]);
         if (g == tag + 1) t = -1;
       }
     }
     if (t < 0) break;
-    if (wait) {
-      if (++spins > kSpinLimit) {
-        *timeout = true;
-        break;
-      }
-    } else {
+    if (!wait) {
       t -= 8;
+      polls = 0;
     }
   }
   return sum;
@@ -239,7 +251,7 @@ __global__ void __launch_bounds__(kPassBlock, 2)
 radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const unsigned int *d_n, int pass, int shift,
                   SortHead *head, unsigned long long *status, int *fault) {
   after_previous();
-  if (!head->run[pass]) return;
+  if (!head->run[pass] || head->fault) return;
   if (d_n && int64_t(*d_n) < n) n = *d_n;
   const bool flip = head->src[pass] != 0;
   const K *__restrict__ kin = flip ? k1 : k0;
@@ -256,7 +268,7 @@ radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const uns
   uint32_t *cnt = sm.cnt[warp];
   const unsigned below = lanemask_lt();
   while (true) {
-    if (tid == 0) sm.tile = int64_t(atomicAdd(&head->ticket[pass], 1u));
+    if (tid == 0) sm.tile = faulted(head) ? tiles : int64_t(atomicAdd(&head->ticket[pass], 1u));
     for (int i = lane; i < kBins; i += 32) cnt[i] = 0;
     __syncthreads();  // also: the tile before has been written out
     const int64_t tile = sm.tile;
@@ -313,14 +325,18 @@ radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const uns
     // 3. the digits' first output positions
     bool timeout = false;
     if (tid < kBins) {
-      const uint32_t before = look_back(status, tile, tid, tag, &timeout);
-      if (tile > 0) store_status(status + tile * kBins + tid, (unsigned long long)(tag + 1u) << 32 | (before + total));
+      const uint32_t before = look_back(head, status, tile, tid, tag, &timeout);
+      if (tile > 0 && !timeout) store_status(status + tile * kBins + tid, (unsigned long long)(tag + 1u) << 32 | (before + total));
       sm.out_base[tid] = head->hist[pass][tid] + before - base;
     }
-    // a wait that gave up leaves wrong positions: nothing is written then
+    // a wait that gave up leaves wrong positions: nothing is written then, here, by
+    // the tiles that wait for this one, or in a later pass
     if (__syncthreads_or(timeout)) {
-      if (tid == 0) *fault = 1;
-      continue;
+      if (tid == 0) {
+        *reinterpret_cast<volatile uint32_t *>(&head->fault) = 1u;
+        *reinterpret_cast<volatile int *>(fault) = 1;
+      }
+      return;
     }
     // 4. out, digit by digit
 #pragma unroll 4

@@ -92,6 +92,7 @@ __global__ void static_gather_kernel(const stq_aabb *__restrict__ boxes, int n, 
                                      const uint32_t *__restrict__ keys, const uint32_t *__restrict__ order,
                                      unsigned char *scratch) {
   after_previous();
+  if (reinterpret_cast<const BatchHeader *>(scratch + kOffHdr)->fault) return;  // the boxes are not sorted
   float4 *yz = reinterpret_cast<float4 *>(scratch + kOffYz);
   float2 *xx = reinterpret_cast<float2 *>(scratch + kOffX);
   int4 *v = reinterpret_cast<int4 *>(scratch + kOffV);

@@ -45,8 +45,10 @@ __device__ __forceinline__ bool pair_hit(const PosRec &a, const PosRec &b, int t
   return x && overlap_bc(a.yz, b.yz) && (typed || valid_pair(a.v, b.v)) && !covertex(a.v, b.v);
 }
 
-// One past the last start position of a sweep, from the sizes on the device.
+// One past the last start position of a sweep, from the sizes on the device (none
+// if a wait of the sort ran out: there is no sorted scene then).
 __device__ __forceinline__ int sweep_end(const SweepParams &p) {
+  if (p.hdr->fault) return p.begin;
   const int end = min(p.end, int(p.hdr->length));
   if (!p.sel) return end;
   return p.sel->count <= (unsigned long long)p.capacity ? p.begin : int(min((long long)end, p.begin + p.sel->prefix));
@@ -469,6 +471,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
   unsigned parts = 1;  // LONG: parts of a run
   if (LONG) {
     if (p.sel && p.sel->count <= (unsigned long long)p.capacity) return;  // the list is of an earlier sweep
+    if (p.hdr->fault) return;
     const unsigned items = *p.long_items, warps = gridDim.x * (BLOCK / 32);
     if (items == 0) return;
     parts = max(1u, min(64u, warps / items));
