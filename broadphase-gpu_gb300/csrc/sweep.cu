@@ -420,6 +420,8 @@ stq_sweep_lane_kernel(const SweepParams p) {
 // which would keep one lane, group or warp busy long after the others finished).
 // The warp's starts are entries of that list, and when there are fewer of them
 // than warps each run is cut into as many equal parts as give every warp one.
+// Parts are taken in slices of at most kLongSlice candidates, so that the warp's
+// 32 together are within 31 bits, and an offset in a run within the queue's 27.
 struct FlatStart {
   float4 yz;      // the start box (PosRec)
   int4 v;
@@ -442,6 +444,7 @@ constexpr int kBandRatio = 6;
 constexpr int kFlatStage = 192;
 constexpr int kFlatRound = 256;  // candidates queued at once by a band step (or 32 V by a flat one)
 constexpr int kFlatQueue = 32 + kFlatRound;
+constexpr int kLongSlice = 1 << 25;
 struct FlatWarp {
   FlatStart rec[32];
   int2 lookup[32];             // flat form: code_start of a start's code, and joff: its
@@ -488,36 +491,46 @@ stq_sweep_flat_kernel(const SweepParams p) {
   int staged = 0, queued = 0;
   int wscene = 0;
   unsigned long long wpairs = 0;
+  int k = 0, j = 0, len = 0;  // the lane's start and run (this slice of it)
+  int rest = 0;               // LONG: what comes after the slice
 
   while (true) {
-    if (next_k >= chunk_end) {
-      int c = 0;
-      if (lane == 0) c = LONG ? int(atomicAdd(p.long_work, unsigned(chunk))) : atomicAdd(p.work, chunk);
-      c = __shfl_sync(kFullMask, c, 0);
-      if (c >= span) break;
-      next_k = first + c;
-      chunk_end = min(next_k + chunk, end);
-    }
-    const int take = min(32, chunk_end - next_k);
-    int k = next_k + lane;
-    next_k += take;
-    // 1. Runs (that of the position after a list is empty).
-    int len = 0, j = 0;
-    if (LONG) {
-      if (lane < take) {
-        const int2 it = p.long_list[unsigned(k) / parts];
-        const int part = int(unsigned(k) % parts), run_end = p.run_end[it.x];
-        const int each = (run_end - it.y + int(parts) - 1) / int(parts);
-        k = it.x;
-        j = it.y + part * each;
-        len = max(min(each, run_end - j), 0);
+    if (LONG && __any_sync(kFullMask, rest > 0)) {
+      j += len;
+      len = min(rest, kLongSlice);
+      rest -= len;
+    } else {
+      if (next_k >= chunk_end) {
+        int c = 0;
+        if (lane == 0) c = LONG ? int(atomicAdd(p.long_work, unsigned(chunk))) : atomicAdd(p.work, chunk);
+        c = __shfl_sync(kFullMask, c, 0);
+        if (c >= span) break;
+        next_k = first + c;
+        chunk_end = min(next_k + chunk, end);
       }
-    } else if (lane < take) {
-      j = p.partner[k];
-      len = max(p.run_end[k] - j, 0);
-      if (p.run_cap && len > p.run_cap) {  // a long run: the warp pass takes the rest
-        p.long_list[atomicAdd(p.long_items, 1u)] = make_int2(k, j + p.run_cap);
-        len = p.run_cap;
+      const int take = min(32, chunk_end - next_k);
+      k = next_k + lane;
+      next_k += take;
+      // 1. Runs (that of the position after a list is empty).
+      len = 0, j = 0;
+      if (LONG) {
+        if (lane < take) {
+          const int2 it = p.long_list[unsigned(k) / parts];
+          const int part = int(unsigned(k) % parts), run_end = p.run_end[it.x];
+          const int each = int((unsigned(run_end - it.y) + parts - 1u) / parts);
+          k = it.x;
+          j = it.y + min(part * each, run_end - it.y);
+          rest = min(each, run_end - j);
+          len = min(rest, kLongSlice);
+          rest -= len;
+        }
+      } else if (lane < take) {
+        j = p.partner[k];
+        len = max(p.run_end[k] - j, 0);
+        if (p.run_cap && len > p.run_cap) {  // a long run: the warp pass takes the rest
+          p.long_list[atomicAdd(p.long_items, 1u)] = make_int2(k, j + p.run_cap);
+          len = p.run_cap;
+        }
       }
     }
     const unsigned nz = __ballot_sync(kFullMask, len > 0);

@@ -95,3 +95,31 @@ def test_windows_after_an_overflow(ctx, stq, oracle, cuda, shape, run_cap):
     assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
     r = ctx.sweep_prepared(pairs, len(want) - 1)
     assert r.status == stq.STQ_OVERFLOW and r.total == len(want) and r.count < len(want)
+
+
+def test_runs_of_tens_of_millions(ctx, stq, cuda):
+    """2,500 boxes along the whole axis above 70 M points on it: one list, in which 32 of
+    the long runs together have more candidates than 31 bits count. The long boxes all
+    meet each other and no point; a point meets none."""
+    import torch
+
+    n, long = 70_000_000, 2500
+    boxes = torch.zeros((n + long, 11), dtype=torch.int32, device=cuda)
+    i = torch.arange(n + long, dtype=torch.int32, device=cuda)
+    boxes[:, 0] = i
+    x = (i[:n] + 0x3F800000).view(torch.float32)  # 70 M floats from 1 on
+    f = boxes.view(torch.float32)
+    f[:n, 1] = x
+    f[:n, 4] = x
+    f[n:, 1] = 0.5
+    f[n:, 4] = float(x[-1])
+    f[n:, [2, 3, 5, 6]] = 1.0  # y and z of the long boxes
+    boxes[:, 7], boxes[:, 8], boxes[:, 9] = 2 * i, 2 * i + 1, -2 * i - 1  # edges without a common vertex
+    ctx.set_option(stq.OPT_CELLS, 1)
+    want = long * (long - 1) // 2
+    pairs = torch.empty((want + 16, 2), dtype=torch.int32, device=cuda)
+    r = ctx.sweep(boxes, n + long, pairs, want + 16, axis=0)
+    assert r.status == stq.STQ_OK and r.count == want
+    ctx.sort_pairs(pairs, want)
+    a, b = torch.triu_indices(long, long, 1, device=cuda).to(torch.int32)
+    assert torch.equal(pairs[:want, 0], a + n) and torch.equal(pairs[:want, 1], b + n)
