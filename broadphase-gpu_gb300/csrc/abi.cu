@@ -204,12 +204,17 @@ int upload_staging(stq_context *ctx) {
   return STQ_OK;
 }
 
+// Tiles to launch blocks for: the staged batch's, or, in a graph, any batch's.
+static int grid_tiles(stq_context *ctx) {
+  return ctx->capturing ? ctx->tile_cap : std::max(host_at<BatchHeader>(ctx, ctx->layout.hdr)->n_tiles, 1);
+}
+
 BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
   BatchBuffers b;
   b.boxes = boxes;
   b.box_off = dev_at<long long>(ctx, ctx->layout.box_off);
   b.tiles = dev_at<TileRec>(ctx, ctx->layout.tiles);
-  b.tile_cap = ctx->tile_cap;
+  b.tile_cap = grid_tiles(ctx);
   b.inputs = dev_at<SceneInput>(ctx, ctx->layout.inputs);
   b.scene_pairs = ctx->scene_pairs.as<unsigned long long>();
   b.scenes = ctx->scenes.as<SceneRecord>();
@@ -299,13 +304,27 @@ int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_c
   return STQ_OK;
 }
 
-int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes) {
+SceneSizes scene_sizes(const stq_context *ctx, int64_t N, int S) {
+  // the automatic grid keeps to the budget and to N / 16 cells (one per scene at
+  // least); in a requested grid a box may be in every cell
+  const int64_t side = std::max<int64_t>(ctx->options[STQ_OPT_CELLS], 1);
+  SceneSizes z;
+  z.replicas = std::min(ctx->rep_cap, N * (side > 1 ? side * side : ctx->budget));
+  z.lists = std::min(ctx->seg_cap, 3 * (side > 1 ? S * side * side : N / 16 + S));
+  z.positions = std::min(ctx->slot_cap, z.replicas + z.lists + 1 + kSortedPad);
+  const double likely = 1.125 * double(N) * (ctx->density > 0.0 ? ctx->density : double(ctx->budget));
+  z.likely = std::min(z.replicas, int64_t(likely) + 256);
+  return z;
+}
+
+int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes, const SceneSizes *sizes) {
   STQ_CUDA(ctx, launch_batch_emit(ctx->stream, b), "launch replica emit");
   stage_end(ctx, kKeys);
   stage_begin(ctx, kSort);
-  const int64_t r = replicas >= 0 ? replicas : ctx->rep_cap;
+  const int64_t r = replicas >= 0 ? replicas : (sizes ? sizes->replicas : ctx->rep_cap);
   STQ_CUDA(ctx, radix_sort_u32(ctx->stream, b.keys, b.vals, r, ctx->sort_ws.ptr, &b.hdr->fault, &ctx->launches,
-                               replicas >= 0 ? nullptr : &b.hdr->replicas, &b.hdr->passes, passes),
+                               replicas >= 0 ? nullptr : &b.hdr->replicas, &b.hdr->passes, passes,
+                               sizes ? sizes->likely : r),
            "launch replica sort");
   stage_end(ctx, kSort);
   ctx->scene.yz = ctx->yz.as<float4>();
@@ -316,7 +335,8 @@ int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replic
   ctx->scene.partner = ctx->partner.as<int>();
   ctx->scene.run_end = ctx->run_end.as<int>();
   stage_begin(ctx, kGather);
-  STQ_CUDA(ctx, launch_list_offsets(ctx->stream, b.keys[0], b.hdr, b.seg_scan, b.seg_cap, ctx->scene, ctx->slot_cap),
+  STQ_CUDA(ctx, launch_list_offsets(ctx->stream, b.keys[0], b.hdr, b.seg_scan, b.seg_cap, ctx->scene, ctx->slot_cap,
+                                    sizes ? sizes->lists : b.seg_cap),
            "launch list offsets");
   STQ_CUDA(ctx, launch_gather_cells(ctx->stream, b, r, ctx->scene), "launch gather");
   stage_end(ctx, kGather);
@@ -342,6 +362,7 @@ int take_front(stq_context *ctx, int S, int64_t N, bool *again) {
   }
   ctx->n_scenes = S;
   ctx->n_boxes = N;
+  if (N > 0) ctx->density = double(f.replicas) / double(N);
   ctx->length = f.replicas > 0 ? int64_t(f.replicas + 3 * f.cells) - 1 : 0;
   ctx->scene.length = ctx->length;
   ctx->prepared = true;
@@ -353,9 +374,9 @@ bool has_room(const stq_context *ctx, int64_t N) {
   return ctx->passes_seen > 0 && ctx->rep_cap >= N && ctx->seg_cap > 0;
 }
 
-// Queues a whole prepare for the buffers that the context has.
+// Queues a prepare: all of it, for the buffers that the context has, or its first half.
 int enqueue_prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_off, int S, const int *axes, int axis,
-                    bool *whole) {
+                    bool whole) {
   ctx->prepared = false;
   ctx->swept = false;
   ctx->overflowed = false;
@@ -365,11 +386,13 @@ int enqueue_prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *bo
   fill_staging(ctx, box_off, S, axes, axis, nullptr, nullptr, nullptr);
   STQ_TRY(upload_staging(ctx));
   const BatchBuffers b = batch_buffers(ctx, d_boxes);
-  STQ_TRY(enqueue_prepare_front(ctx, b, *whole ? ctx->rep_cap : -1, ctx->seg_cap, ctx->passes_seen));
+  // (what the second half is not launched for counts as not fitting)
+  const SceneSizes sizes = scene_sizes(ctx, N, S);
+  STQ_TRY(enqueue_prepare_front(ctx, b, whole ? sizes.replicas : -1, sizes.lists, ctx->passes_seen));
   if (!ctx->front_event)
     STQ_CUDA(ctx, cudaEventCreateWithFlags(&ctx->front_event, cudaEventDisableTiming), "create event");
   STQ_CUDA(ctx, cudaEventRecord(ctx->front_event, ctx->stream), "record prepare");
-  if (*whole) STQ_TRY(enqueue_prepare_back(ctx, b, -1, ctx->passes_seen));
+  if (whole) STQ_TRY(enqueue_prepare_back(ctx, b, -1, ctx->passes_seen, &sizes));
   return STQ_OK;
 }
 
@@ -377,11 +400,13 @@ int enqueue_prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *bo
 // count when the buffers of earlier scenes may hold it, so that the stream does
 // not idle while the host waits for that count; if they do not, or there are
 // none, they are sized (an eighth more than needed, for the next step of a
-// moving scene) and the second half is queued then.
-int prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_off, int S, const int *axes, int axis) {
+// moving scene) and the second half is queued then. fits: false where the caller has
+// seen that they do not.
+int prepare(stq_context *ctx, const stq_aabb *d_boxes, const int64_t *box_off, int S, const int *axes, int axis,
+            bool fits = true) {
   const int64_t N = box_off[S];
-  for (bool whole = has_room(ctx, N);; whole = false) {
-    STQ_TRY(enqueue_prepare(ctx, d_boxes, box_off, S, axes, axis, &whole));
+  for (bool whole = fits && has_room(ctx, N);; whole = false) {
+    STQ_TRY(enqueue_prepare(ctx, d_boxes, box_off, S, axes, axis, whole));
     STQ_CUDA(ctx, cudaEventSynchronize(ctx->front_event), "wait for prepare");
     bool again = false;
     STQ_TRY(take_front(ctx, S, N, &again));
@@ -418,11 +443,10 @@ int run_sweep(stq_context *ctx, int64_t begin, int64_t end, stq_pair *pairs,
   p.run_end = ctx->scene.run_end;
   p.begin = int32_t(begin);
   p.end = int32_t(std::min<int64_t>(end, INT32_MAX));
-  // start positions per work grab: at least ~4 grabs per resident warp
-  const int64_t span = std::min<int64_t>(end, ctx->slot_cap) - begin;
-  const int64_t want = int64_t(ctx->num_sms) * 64 * 4;
-  const int64_t chunk = ((std::max<int64_t>(span, 0) / want) + 31) / 32 * 32;
-  p.chunk = int32_t(chunk < 32 ? 32 : (chunk > ctx->tuning.chunk ? ctx->tuning.chunk : chunk));
+  // start positions per work grab: at least ~4 grabs per resident warp (taken from
+  // the positions that there are: end may be a capacity)
+  p.grabs = ctx->num_sms * 64 * 4;
+  p.chunk = ctx->tuning.chunk;
   p.pairs = pairs;
   p.capacity = capacity;
   p.count = &hdr->pairs;
@@ -761,7 +785,7 @@ int stq_batch_build_boxes(stq_context *ctx, const double *d_V0, const double *d_
                                    d_E, dev_at<long long>(ctx, ctx->layout.eoff), d_F,
                                    dev_at<long long>(ctx, ctx->layout.foff),
                                    dev_at<long long>(ctx, ctx->layout.box_off),
-                                   dev_at<TileRec>(ctx, ctx->layout.tiles), ctx->tile_cap, dev_hdr(ctx),
+                                   dev_at<TileRec>(ctx, ctx->layout.tiles), grid_tiles(ctx), dev_hdr(ctx),
                                    ref_next_up(inflation_radius), d_boxes, ctx->points.as<float4>(),
                                    std::max<int64_t>(nv_all, 1)),
            "launch batched box build");
@@ -846,9 +870,9 @@ int stq_sweep(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int axis, in
       max_start <= 0 && count && next_start && capacity >= 0 && (capacity == 0 || d_pairs) && has_room(ctx, n)) {
     DeviceGuard g(ctx->device);
     const int64_t off[2] = {0, n};
-    bool whole = true, again = false;
-    STQ_TRY(enqueue_prepare(ctx, d_boxes, off, 1, nullptr, axis, &whole));
-    STQ_TRY(run_sweep(ctx, 0, ctx->slot_cap, d_pairs, capacity, kSweepEmit));
+    bool again = false;
+    STQ_TRY(enqueue_prepare(ctx, d_boxes, off, 1, nullptr, axis, true));
+    STQ_TRY(run_sweep(ctx, 0, scene_sizes(ctx, n, 1).positions, d_pairs, capacity, kSweepEmit));
     STQ_CUDA(ctx, cudaMemcpyAsync(ctx->h_hdr, dev_hdr(ctx), sizeof(BatchHeader), cudaMemcpyDeviceToHost, ctx->stream),
              "read back batch header");
     STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");
@@ -862,8 +886,10 @@ int stq_sweep(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int axis, in
       }
       return finish_sweep(ctx, 0, ctx->length, d_pairs, capacity, count, next_start, total);
     }
+    STQ_TRY(prepare(ctx, d_boxes, off, 1, nullptr, axis, false));
+  } else {
+    STQ_TRY(stq_prepare(ctx, d_boxes, n, axis));
   }
-  STQ_TRY(stq_prepare(ctx, d_boxes, n, axis));
   return stq_sweep_prepared(ctx, start, max_start, d_pairs, capacity, count, next_start, total);
 }
 
@@ -928,7 +954,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
                                      d_E, dev_at<long long>(ctx, ctx->layout.eoff), d_F,
                                      dev_at<long long>(ctx, ctx->layout.foff),
                                      dev_at<long long>(ctx, ctx->layout.box_off),
-                                     dev_at<TileRec>(ctx, ctx->layout.tiles), ctx->tile_cap, dev_hdr(ctx),
+                                     dev_at<TileRec>(ctx, ctx->layout.tiles), grid_tiles(ctx), dev_hdr(ctx),
                                      ref_next_up(inflation_radius),
                                      ctx->batch_boxes.as<stq_aabb>(), ctx->points.as<float4>(), vert_cap),
              "launch batched box build");
@@ -1027,6 +1053,12 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
 
 namespace {
 
+// Start positions of a scene of n boxes, by the density of the scenes before.
+int64_t likely_positions(const stq_context *ctx, int64_t n) {
+  const SceneSizes z = scene_sizes(ctx, n, 1);
+  return std::min(z.positions, z.likely + z.lists);
+}
+
 // Prepares the boxes and sweeps them into h_pairs. The start positions are cut into
 // windows (STQ_OPT_HOST_WINDOWS, default 16) that alternate between two
 // slots: even windows sweep on the context's stream into e2e_pairs, odd
@@ -1047,7 +1079,7 @@ int sweep_to_host(stq_context *ctx, const stq_aabb *d_boxes, int64_t n, int axis
   constexpr int64_t kMinWindow = int64_t(1) << 19;  // start positions
   // too small for two windows, whatever its replicas: prepared and swept in one
   const bool one = capacity == 0 || ctx->options[STQ_OPT_HOST_OVERLAP] == 2 ||
-                   (has_room(ctx, n) && ctx->slot_cap < 2 * kMinWindow);
+                   (has_room(ctx, n) && likely_positions(ctx, n) < 2 * kMinWindow);
   if (!one) STQ_TRY(stq_prepare(ctx, d_boxes, n, axis));
   const size_t pair_bytes = sizeof(stq_pair) * size_t(capacity > 0 ? capacity : 1);
   STQ_CUDA(ctx, ctx->e2e_pairs.ensure(pair_bytes), "allocate pair staging");

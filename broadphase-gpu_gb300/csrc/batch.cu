@@ -885,8 +885,8 @@ cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b) {
 }
 
 cudaError_t launch_list_offsets(cudaStream_t s, const uint32_t *keys, BatchHeader *hdr, uint32_t *seg_scan,
-                                int64_t seg_cap, const SortedScene &scene, int64_t slots_cap) {
-  launch_after(list_offsets_kernel, blocks_for((seg_cap + 1) / (kBlock - 1) * kBlock + kBlock), kBlock, 0, s, keys,
+                                int64_t seg_cap, const SortedScene &scene, int64_t slots_cap, int64_t lists) {
+  launch_after(list_offsets_kernel, blocks_for((lists + 1) / (kBlock - 1) * kBlock + kBlock), kBlock, 0, s, keys,
                hdr, seg_scan, seg_cap, scene, slots_cap);
   return cudaGetLastError();
 }

@@ -112,6 +112,7 @@ struct stq_context {
   DevScalars *h_sel = nullptr;        // readback of an overflowing sweep's prefix
   int pair_id_bits = 0;               // of the largest first id of the pairs sorted so far
   int passes_seen = 0;  // most digits that a replica sort of this context needed
+  double density = 0.0;  // replicas per box of the last prepared scenes
   bool overflowed = false;  // the last sweep of the prepared scenes found more pairs than fit
   bool swept = false;   // the prepared scenes have been swept (their pair counters hold)
   unsigned long long *h_scene_pairs = nullptr;  // pinned readback
@@ -159,6 +160,15 @@ struct stq_context {
 namespace stq {
 namespace ctxops {
 
+// What the host knows of scenes before the device has counted their replicas:
+// launches take their shape from these, not from the capacities that larger scenes
+// left behind.
+struct SceneSizes {
+  int64_t replicas, lists, positions;  // at most
+  int64_t likely;                      // replicas, by the density of the scenes before
+};
+SceneSizes scene_sizes(const stq_context *ctx, int64_t N, int S);
+
 struct DeviceGuard {
   int prev = -1;
   bool changed = false;
@@ -191,8 +201,9 @@ int enqueue_prepare_front(stq_context *ctx, const BatchBuffers &b, int64_t rep_c
 // Replica emit in box order, their sort by (list, sweep-axis code), list offsets
 // and the sorted scene. replicas: the replica count, or -1 when only the device
 // knows it (graph capture, serving, a prepare that is not waited for). passes:
-// digits of the sort to launch.
-int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes);
+// digits of the sort to launch. sizes: of these scenes (null: the buffers').
+int enqueue_prepare_back(stq_context *ctx, const BatchBuffers &b, int64_t replicas, int passes,
+                         const SceneSizes *sizes = nullptr);
 // Launches one sweep over start positions [begin, end). With cursors null it
 // first clears the batch header's pair counter, cursors, per-scene counts and
 // statistics and uses them and the context's long-run list; otherwise it uses

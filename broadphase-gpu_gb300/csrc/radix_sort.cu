@@ -479,7 +479,7 @@ cudaError_t launch_block(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *cons
 
 template <typename K, bool VALS>
 cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2], int64_t n, const unsigned int *d_n,
-                      const Digits &dg, void *workspace, int *fault, int64_t *launches) {
+                      const Digits &dg, void *workspace, int *fault, int64_t *launches, int64_t likely) {
   if (dg.passes == 0 || (n <= 1 && !dg.d_passes)) return cudaSuccess;
   SortHead *head = static_cast<SortHead *>(workspace);
   unsigned long long *status = reinterpret_cast<unsigned long long *>(static_cast<char *>(workspace) +
@@ -492,7 +492,7 @@ cudaError_t sort_impl(cudaStream_t s, K *const kbuf[2], uint32_t *const vbuf[2],
   // ones, 346,000 64-bit keys 78 us in large and 70 in small ones.
   constexpr int kLarge = 16;
   static_assert(kPassBlock * kLarge >= 2 * kMinTile, "workspace sizing: status words of large tiles");
-  const bool large = n >= int64_t(sm_count()) * 4096;
+  const bool large = likely >= int64_t(sm_count()) * 4096 || n > kRadixMinTiles * kMinTile;
   const int tile = large ? kPassBlock * kLarge : kMinTile;
   const int64_t hist_blocks = (n + kHistBlock * 4 - 1) / (kHistBlock * 4);
   launch_after(radix_hist_kernel<K>, unsigned(std::min<int64_t>(hist_blocks, int64_t(sm_count()) * 4)), kHistBlock, 0,
@@ -519,14 +519,14 @@ int sm_count() {
 
 cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, void *workspace,
                            int *fault, int64_t *launches, const unsigned int *d_n, const unsigned int *d_passes,
-                           int passes) {
+                           int passes, int64_t likely) {
   const Digits dg{passes, {0, 8, 16, 24}, d_passes};
   if (passes > 0 && (n > 1 || d_passes)) {  // one block up to its 16 keys per thread
     if (n <= kPassBlock * 2) return launch_block<2>(s, kbuf, vbuf, n, dg, d_n, launches);
     if (n <= kPassBlock * 8) return launch_block<8>(s, kbuf, vbuf, n, dg, d_n, launches);
     if (n <= kPassBlock * 16) return launch_block<16>(s, kbuf, vbuf, n, dg, d_n, launches);
   }
-  return sort_impl<uint32_t, true>(s, kbuf, vbuf, n, d_n, dg, workspace, fault, launches);
+  return sort_impl<uint32_t, true>(s, kbuf, vbuf, n, d_n, dg, workspace, fault, launches, likely < 0 ? n : likely);
 }
 
 cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,
@@ -537,7 +537,7 @@ cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int
                                reinterpret_cast<unsigned long long *>(tmp)};
   return sort_impl<unsigned long long, false>(s, kb, nullptr, n, nullptr,
                                               Digits{8, {32, 40, 48, 56, 0, 8, 16, 24}, nullptr},
-                                              workspace, fault, launches);
+                                              workspace, fault, launches, n);
 }
 
 }  // namespace stq

@@ -277,7 +277,8 @@ struct SweepParams {
   const int *partner;        // first candidate position of each start position
   const int *run_end;        // one past its last candidate
   int32_t begin, end;        // start positions [begin, min(end, hdr->length))
-  int32_t chunk;             // start positions per grab
+  int32_t chunk;             // start positions per grab, at most
+  int32_t grabs;             // and as many as make this number of grabs (0: chunk)
   stq_pair *pairs;
   long long capacity;
   unsigned long long *count;
@@ -350,9 +351,9 @@ cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t
 // replicas in box order (1 launch)
 cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b);
 // list offsets from the sorted keys (and the longest list); the empty position
-// after every list and the padding after the last
+// after every list and the padding after the last. lists: to launch blocks for
 cudaError_t launch_list_offsets(cudaStream_t s, const uint32_t *keys, BatchHeader *hdr, uint32_t *seg_scan,
-                                int64_t seg_cap, const SortedScene &scene, int64_t slots_cap);
+                                int64_t seg_cap, const SortedScene &scene, int64_t slots_cap, int64_t lists);
 
 cudaError_t launch_gather_cells(cudaStream_t s, const BatchBuffers &b, int64_t replicas, const SortedScene &scene);
 // Batched box build: scene s has vertices [voff[s], voff[s+1]) etc.; box ids
@@ -391,22 +392,24 @@ cudaError_t launch_window_step(cudaStream_t s, WindowCounters *wc, unsigned long
 // (the result is then not sorted). d_n (may be null): on the device, the number
 // of elements (at most n).
 constexpr int kRadixMinTile = 2048;       // keys of the smallest tile of a pass
+constexpr int64_t kRadixMinTiles = 1 << 13;  // most tiles of that size
 constexpr size_t kRadixHeadBytes = 8704;  // digit counts, cursors
 // Workspace of a sort of up to n elements: the head and 256 status words per
 // tile. The smallest tiles are used below a fixed size, larger ones (at least
 // twice as long) above it.
 constexpr size_t radix_workspace_bytes(int64_t n) {
   const size_t tiles = size_t((n > 0 ? n : 1) + kRadixMinTile - 1) / kRadixMinTile;
-  const size_t half = (tiles + 1) / 2, small_max = size_t(1) << 13;
+  const size_t half = (tiles + 1) / 2, small_max = size_t(kRadixMinTiles);
   const size_t small = tiles < small_max ? tiles : small_max;
   return kRadixHeadBytes + sizeof(unsigned long long) * 256 * (small > half ? small : half);
 }
 // result in kbuf[0], vbuf[0]. d_passes (may be null: 4): on the device, the
 // number of low digits to sort by, at most `passes`; the input is then in
-// buffer *d_passes & 1, else in buffer 0.
+// buffer *d_passes & 1, else in buffer 0. likely: the expected number of elements
+// (-1: n); the tile size follows it.
 cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *const vbuf[2], int64_t n, void *workspace,
                            int *fault, int64_t *launches, const unsigned int *d_n = nullptr,
-                           const unsigned int *d_passes = nullptr, int passes = 4);
+                           const unsigned int *d_passes = nullptr, int passes = 4, int64_t likely = -1);
 // by digits; lexicographic by (first, second) as unsigned ids, in place; tmp holds n pairs
 cudaError_t radix_sort_pairs(cudaStream_t s, stq_pair *pairs, stq_pair *tmp, int64_t n, void *workspace, int *fault,
                              int64_t *launches);

@@ -22,6 +22,7 @@
 // Runs longer than a cap go to a warp pass (the flat kernel over a list). Refill,
 // hand-out and pair output use __ballot_sync/__popc compaction: no
 // shared-memory atomics, and one global atomic per 32 or more pairs.
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -52,6 +53,11 @@ __device__ __forceinline__ int sweep_end(const SweepParams &p) {
   const int end = min(p.end, int(p.hdr->length));
   if (!p.sel) return end;
   return p.sel->count <= (unsigned long long)p.capacity ? p.begin : int(min((long long)end, p.begin + p.sel->prefix));
+}
+
+// Start positions per grab of a sweep over `span` of them.
+__device__ __forceinline__ int sweep_chunk(const SweepParams &p, int span) {
+  return p.grabs ? max(32, min(p.chunk, (span / p.grabs + 31) / 32 * 32)) : p.chunk;
 }
 
 // Appends the warp's n staged pairs with one atomic; pairs past the capacity
@@ -96,7 +102,7 @@ stq_sweep_kernel(const SweepParams p) {
   uint32_t code = 0;  // and its code
   int kf = 0;         // its scene, above the first-cell bits
   const int end = sweep_end(p);
-  const int span = end - p.begin;
+  const int span = end - p.begin, chunk = sweep_chunk(p, span);
   unsigned tested = 0;  // candidates this lane tested (statistics)
   // warp-uniform: staged pairs, and pairs of the current scene not yet added
   // to its counter
@@ -111,14 +117,14 @@ stq_sweep_kernel(const SweepParams p) {
     while (qsize < E && more) {
       if (next_k >= chunk_end) {
         int c = 0;
-        if (lane == 0) c = atomicAdd(p.work, p.chunk);
+        if (lane == 0) c = atomicAdd(p.work, chunk);
         c = __shfl_sync(kFullMask, c, 0);
         if (c >= span) {
           more = false;
           break;
         }
         next_k = p.begin + c;
-        chunk_end = min(next_k + p.chunk, end);
+        chunk_end = min(next_k + chunk, end);
       }
       const int take = min(32, min(Q - qsize, chunk_end - next_k));
       const int kk = next_k + lane;
@@ -255,7 +261,7 @@ stq_sweep_lane_kernel(const SweepParams p) {
   uint32_t code = 0;  // and its code
   int kf = 0;         // its scene, above the first-cell bits
   const int end = sweep_end(p);
-  const int span = end - p.begin;
+  const int span = end - p.begin, chunk = sweep_chunk(p, span);
   unsigned tested = 0;
   int staged = 0;
   int wscene = 0;
@@ -267,14 +273,14 @@ stq_sweep_lane_kernel(const SweepParams p) {
     while (qsize < 32 && more) {
       if (next_k >= chunk_end) {
         int c = 0;
-        if (lane == 0) c = atomicAdd(p.work, p.chunk);
+        if (lane == 0) c = atomicAdd(p.work, chunk);
         c = __shfl_sync(kFullMask, c, 0);
         if (c >= span) {
           more = false;
           break;
         }
         next_k = p.begin + c;
-        chunk_end = min(next_k + p.chunk, end);
+        chunk_end = min(next_k + chunk, end);
       }
       const int take = min(32, min(Q - qsize, chunk_end - next_k));
       const int kk = next_k + lane;
@@ -470,7 +476,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
   int2 *st = sw.stage;
   uint32_t *qu = sw.queue;
 
-  int end, span, chunk = p.chunk;
+  int end, span, chunk;
   unsigned parts = 1;  // LONG: parts of a run
   if (LONG) {
     if (p.sel && p.sel->count <= (unsigned long long)p.capacity) return;  // the list is of an earlier sweep
@@ -483,6 +489,7 @@ stq_sweep_flat_kernel(const SweepParams p) {
   } else {
     end = sweep_end(p);
     span = end - p.begin;
+    chunk = sweep_chunk(p, span);
   }
   const int first = LONG ? 0 : p.begin;
   const bool multi = p.hdr->n_scenes > 1;
@@ -737,7 +744,8 @@ cudaError_t launch_persistent(Kern kern, int block, cudaStream_t s, const SweepP
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   // persistent grid: all resident blocks, capped by the available work
-  const int64_t warps_needed = (int64_t(p.end - p.begin) + p.chunk - 1) / p.chunk;
+  const int64_t chunk = p.grabs ? std::min(p.chunk, 32) : p.chunk;
+  const int64_t warps_needed = (int64_t(p.end) - p.begin + chunk - 1) / chunk;
   int64_t blocks = int64_t(num_sms) * per_sm;
   const int64_t max_useful = (warps_needed + block / 32 - 1) / (block / 32);
   if (blocks > max_useful) blocks = max_useful;

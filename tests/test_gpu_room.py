@@ -71,6 +71,32 @@ def test_bad_boxes_after_good_ones(ctx, stq, oracle, cuda):
     assert np.array_equal(oracle.canonical(np.concatenate(got)), want)
 
 
+def test_launches_follow_the_scene_not_the_buffers(stq, oracle, cuda):
+    """A small scene on a context that has held a large one is launched like on one that
+    has not, and a scene that outgrows the buffers is prepared twice, not three times."""
+    import torch
+
+    small, large = (300, scene(stq, 300, 0.05, seed=1)), (60_000, scene(stq, 60_000, 0.02, seed=2))
+    pairs = torch.empty((1 << 20, 2), dtype=torch.int32, device=cuda)
+    boxes = {n: dev(b, cuda) for n, b in (small, large)}
+    want = {n: oracle.broadphase(b) for n, b in (small, large)}
+
+    def launches(ctx, n):
+        before = ctx.launches
+        r = ctx.sweep(boxes[n], n, pairs, 1 << 20)
+        assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want[n])
+        return ctx.launches - before
+
+    stream = torch.cuda.current_stream(cuda).cuda_stream
+    with stq.Context(0, stream) as a, stq.Context(0, stream) as b:
+        first = launches(a, 300)
+        again = launches(a, 300)
+        first_large = launches(b, 60_000)
+        assert launches(b, 300) == again  # no wait, the sort in one launch
+        assert launches(a, 60_000) <= again + first_large
+        assert first <= again
+
+
 @pytest.mark.parametrize("field,axis", [(f, a) for f in ("min", "max") for a in range(3)])
 @pytest.mark.parametrize("bits", [0x7FC00000, 0xFFC00000])  # NaN, and NaN with the sign set
 def test_a_nan_of_either_sign_is_refused(ctx, stq, oracle, cuda, field, axis, bits):
