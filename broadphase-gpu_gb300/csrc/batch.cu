@@ -197,14 +197,16 @@ scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, cons
       median[q] = k == 0 ? 0.f : 0.75f * exp2f(float(k - kHistBias));
     }
   }
-  // sweep-axis code segments: their ends are quantiles of the sample, the first
-  // and the last reach to the scene's bounds
+  // sweep-axis code segments: the ends of the inner ones are quantiles of the sample;
+  // the first and the last reach from it to the scene's bounds
   if (threadIdx.x >= 64 && threadIdx.x < 64 + kSplits) {
     const int i = threadIdx.x - 64;
-    const int m = int(n < kSampleMins ? (n > 0 ? n : 1) : kSampleMins);
-    const float lo = key_float(key_of(lo_key, axis)), hi = key_float(key_of(hi_key, axis));
-    const float s0 = i == 0 && isfinite(lo) ? lo : sorted[i * m / kSplits];
-    const float s1 = i == kSplits - 1 ? (isfinite(hi) ? hi : sorted[m - 1]) : sorted[(i + 1) * m / kSplits];
+    // samples taken: above
+    const int m = n > kSampleMins ? int(min(n, (long long)kSampleBoxes) + 3) / 4 : max(int(n), 1);
+    static_assert(kSampleBoxes / kBlock == 4, "every fourth sample gives a minimum");
+    constexpr int kInner = kSplits - 2;
+    const float s0 = i == 0 ? key_float(key_of(lo_key, axis)) : sorted[(i - 1) * (m - 1) / kInner];
+    const float s1 = i == kSplits - 1 ? key_float(key_of(hi_key, axis)) : sorted[i * (m - 1) / kInner];
     const float w = s1 - s0;
     r.split[i] = s0;
     r.split_inv[i] = w > 0.f && isfinite(w) ? float(kSplitSteps) / w : 0.f;
@@ -237,6 +239,8 @@ scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, cons
   if (!(Lc > 0.f) || !isfinite(Lc)) nc = 1;
   GridParams &g = r.grid;
   g.axis = axis;
+  g.key_lo = key_of(lo_key, axis);
+  g.key_span = max(key_of(hi_key, axis), g.key_lo) - g.key_lo;
   g.ob = lob;
   g.oc = loc;
   g.Lb = Lb;
@@ -447,9 +451,17 @@ choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__
     // less: sort + sweep 0.22 + 1.26 ms against 0.29 + 1.19 with 32 bits. With 15
     // bits of lists, 200,000 boxes (9 bits of code): 44 + 28 -> 36 + 28 us; with 16,
     // 256 scenes (8): the sweep's loss outweighs the digit by 50 us.
+    // Batches of few, long lists (one cell: plain sweeps, inverted boxes, boxes on a line)
+    // have what the list id leaves of 32 bits: where a 16-bit code is shared by a part
+    // of a list, that part is tested all with all. 300,000 boxes of one cell in 200
+    // clusters: 65.8 M candidates with codes, 0.8 M so, whole sweep 207 -> 148 us; evenly
+    // spread, where codes are as good, the fourth digit costs 20 us (136 -> 157).
+    // Shorter lists lose less than the digit costs.
     int seg_bits = 0;
     while (seg_bits < 32 && (1ull << seg_bits) < lists) ++seg_bits;
-    const int key_bits = seg_bits <= 15 ? min(kAxisCodeBits, 24 - seg_bits) : min(kAxisCodeBits, max(32 - seg_bits, 0));
+    const bool exact = seg_bits <= 8 && R >= 4096ull * lists;
+    const int code_bits = min(kAxisCodeBits, seg_bits <= 15 ? 24 - seg_bits : max(32 - seg_bits, 0));
+    const int key_bits = exact ? 32 - seg_bits : code_bits;
     const int passes = max(seg_bits + key_bits + 7, 8) / 8;
     // more than the buffers hold: the scenes are flagged and left empty (the
     // caller without limits checks that positions fit 31 bits). So are scenes with a
@@ -466,6 +478,7 @@ choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__
     hdr->length = fits && carry > 0 && R > 0 ? unsigned(R + lists - 1) : 0u;
     hdr->max_list = 0u;
     hdr->key_bits = key_bits;
+    hdr->exact = exact ? 1 : 0;
     hdr->passes = unsigned(passes);
     front->replicas = R;
     front->cells = carry;
@@ -554,14 +567,22 @@ __device__ __forceinline__ uint32_t cells_count(uint2 r, int shift) {
          (((r.y >> 11 & 2047u) >> shift) - ((r.y & 2047u) >> shift) + 1u);
 }
 
+// Sweep-axis bits of a bound's key where the batch's keys are exact: monotone, the
+// bounds of inverted boxes clamped to the scene's.
+__device__ __forceinline__ uint32_t exact_code(float v, const GridParams &g, int key_bits) {
+  const uint32_t above = min(max(float_key(v), g.key_lo) - g.key_lo, g.key_span);
+  return above >> max(32 - __clz(g.key_span) - key_bits, 0);
+}
+
 __global__ void __launch_bounds__(kBlock)
-batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restrict__ box_q,
+batch_emit_kernel(const stq_aabb *__restrict__ boxes, const uint2 *__restrict__ box_cells, uint32_t *box_q,
                   const TileRec *__restrict__ tiles, const uint32_t *__restrict__ tile_off,
                   const SceneRecord *__restrict__ scenes, const unsigned int *__restrict__ cell_base,
                   const BatchHeader *hdr, uint32_t *k0, uint32_t *k1, uint32_t *v0, uint32_t *v1) {
   after_previous();
   if (hdr->replicas == 0u || int(blockIdx.x) >= hdr->n_tiles) return;
   const int key_bits = hdr->key_bits;
+  const bool exact = hdr->exact != 0;
   const bool second = hdr->passes & 1u;
   uint32_t *__restrict__ keys = second ? k1 : k0;
   uint32_t *__restrict__ vals = second ? v1 : v0;
@@ -590,7 +611,13 @@ batch_emit_kernel(const uint2 *__restrict__ box_cells, const uint32_t *__restric
     uint32_t n = 0, q = 0;
     if (i < w1) {
       r = box_cells[t.begin + i];
-      q = (box_q[t.begin + i] & 0xffffu) >> (kAxisCodeBits - key_bits);
+      if (exact) {  // (the gather takes the maximum's code from the same bits)
+        const stq_aabb &x = boxes[t.begin + i];
+        q = exact_code(x.min[g.axis], g, key_bits);
+        box_q[t.begin + i] = exact_code(x.max[g.axis], g, key_bits) << (32 - key_bits);
+      } else {
+        q = (box_q[t.begin + i] & 0xffffu) >> (kAxisCodeBits - key_bits);
+      }
       n = cells_count(r, sh);
     }
     uint32_t x = n;
@@ -726,7 +753,7 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const uint32_t *__restri
     const uint32_t key = keys[p];
     const uint32_t bi = order[p];
     const stq_aabb &x = boxes[bi];
-    const uint32_t qmax = (box_q[bi] >> 16) >> (kAxisCodeBits - key_bits);
+    const uint32_t qmax = (box_q[bi] >> 1) >> (31 - key_bits);  // its leading bits (none where key_bits is 0)
     const unsigned int seg = key >> key_bits;
     const unsigned int cell = seg / 3u, type = seg - 3u * cell;
     int lo = 0, hi = S - 1;  // scene of the cell
@@ -879,7 +906,7 @@ cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t
 }
 
 cudaError_t launch_batch_emit(cudaStream_t s, const BatchBuffers &b) {
-  launch_after(batch_emit_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.box_cells, b.box_q, b.tiles, b.tile_off,
+  launch_after(batch_emit_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.boxes, b.box_cells, b.box_q, b.tiles, b.tile_off,
                b.scenes, b.cell_base, b.hdr, b.keys[0], b.keys[1], b.vals[0], b.vals[1]);
   return cudaGetLastError();
 }

@@ -120,15 +120,19 @@ struct GridParams {
   int shift;      // cell coordinate = level-0 coordinate >> shift (the chosen
                   // level; kCoordBits when no level fits: one cell)
   float sb, sc;   // code steps (64 per cell of the chosen level) per unit length
+  uint32_t key_lo, key_span;  // float keys on the sweep axis: the least minimum, and up to
+                              // the largest maximum (long lists, see BatchHeader::exact)
 };
 
 constexpr int kGridLevels = 6;  // level L halves the level-0 grid L times
 constexpr int kCoordBits = 11;  // level-0 cell coordinates are below 2^11
 static_assert(kMaxGridSide <= (1 << kCoordBits), "level-0 cell coordinates fit kCoordBits");
 
-// Sweep-axis codes: 16 bits, 64 segments of 1,024 steps. The segments hold
-// about the same number of boxes each (their ends are quantiles of a sample), so
-// that no spread of the boxes, however uneven, puts many of them on one step.
+// Sweep-axis codes: 16 bits, 64 segments of 1,024 steps. The inner segments hold
+// about the same number of boxes each (their ends are quantiles of a sample), the
+// first and the last those before and after the sample, 1 in 256 each: a box far away
+// widens the steps of no others. A segment with a gap in it still puts many boxes on
+// few steps: batches of few, long lists have keys of more bits (BatchHeader::exact).
 constexpr int kSplits = 64;
 constexpr int kSplitSteps = 1024;
 constexpr int kAxisCodeBits = 16;
@@ -175,6 +179,8 @@ struct BatchHeader {
   int n_tiles;              // input: entries of the tile table
   unsigned int max_list;    // longest (cell, type) list
   int key_bits;             // sweep-axis bits of a replica key (the list id is above)
+  int exact;                // they are the leading bits of the minimum's float key above
+                            // the scene's least, not of its 16-bit code
   unsigned long long candidates;  // candidates tested by the last sweep
   unsigned int lists;       // (cell, type) lists: 3 * cells
   int fault;                // a bounded wait between blocks ran out
@@ -328,7 +334,8 @@ struct BatchBuffers {
   FrontInfo *front;             // page-locked
   uint2 *box_cells;             // per box: cell range and type
                                 // (b0 | b1 << 11 | type << 22, c0 | c1 << 11)
-  uint32_t *box_q;              // per box: sweep-axis codes of its min | its max << 16
+  uint32_t *box_q;              // per box: sweep-axis codes of its min | its max << 16 (exact
+                                // keys: the max's alone, in the leading bits)
   unsigned long long *tile_reps;  // per tile: replicas of each grid level
   uint32_t *tile_off;           // per tile: first replica
   uint32_t *keys[2];            // replica keys: list id << key_bits | sweep-axis code

@@ -97,6 +97,77 @@ def test_windows_after_an_overflow(ctx, stq, oracle, cuda, shape, run_cap):
     assert r.status == stq.STQ_OVERFLOW and r.total == len(want) and r.count < len(want)
 
 
+def overlaps_on_x(b, axis):
+    """Pairs that overlap on the axis, of two edges or of a vertex and a face."""
+    kind = (b["vertex_ids"][:, 1] >= 0).astype(int) + (b["vertex_ids"][:, 2] >= 0)
+    lo, hi = b["min"][:, axis], b["max"][:, axis]
+    order = [np.argsort(lo[kind == k], kind="stable") for k in range(3)]
+    v, e, f = ((lo[kind == k][order[k]], hi[kind == k][order[k]]) for k in range(3))
+    to = lambda x, bound, side="right": np.searchsorted(x[0], bound, side)  # noqa: E731
+    edges = (to(e, e[1]) - np.arange(len(e[0])) - 1).sum()
+    return int(edges + (to(f, v[1]) - to(f, v[0], "left")).sum() + (to(v, f[1]) - to(v, f[0])).sum())
+
+
+@pytest.mark.parametrize("spread", ["even", "far", "far both", "clusters"])
+@pytest.mark.parametrize("axis", [0, 2])
+def test_candidates_of_one_long_list(ctx, stq, oracle, cuda, spread, axis):
+    """However the boxes lie on the sweep axis, one list's candidates are those that
+    overlap on it: a box far away or gaps do not put boxes on one code."""
+    import torch
+
+    n = 60_000
+    b = stq.random_boxes(n, sliver_frac=0.0, seed=4)
+    rng = np.random.default_rng(4)
+    lo = rng.uniform(0, 1, (n, 3)).astype(np.float32)
+    if spread == "clusters":
+        lo[:, axis] = (rng.integers(0, 150, n) + 1e-3 * lo[:, axis]) / 150
+    if spread in ("far", "far both"):
+        lo[17, axis] = 1e4
+    if spread == "far both":
+        lo[18, axis] = -1e5
+    b["min"], b["max"] = lo, lo + np.float32(1e-6 if spread == "clusters" else 1e-3)
+    want, real = oracle.broadphase(b), overlaps_on_x(b, axis)
+    pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+    ctx.set_option(stq.OPT_CELLS, 1)
+    d = torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+    for _ in range(2):
+        r = ctx.sweep(d, n, pairs, len(want) + 16, axis=axis)
+        assert r.count == len(want)
+        assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+        assert real <= ctx.candidates <= 1.01 * real + 100
+
+
+@pytest.mark.parametrize("n", [12_287, 12_288, 12_289, 40_000])
+def test_long_list_keys_vs_oracle(ctx, stq, oracle, cuda, n):
+    """Either side of the line from which a list's keys are those of the minima (4,096
+    boxes per list, three lists in a scene): negative and equal minima, both zeros,
+    infinite bounds, and boxes inverted on the sweep axis."""
+    import torch
+
+    b = dense_boxes(stq, n, n, 400.0)
+    centre = 0.5 * (b["min"] + b["max"]) - np.float32(200)
+    centre[:, 1:] /= 40
+    b["min"], b["max"] = centre - np.float32(0.5), centre + np.float32(0.5)
+    for side in ("min", "max"):
+        b[side][: n // 2, 0] = np.round(b[side][: n // 2, 0])  # (-0 among them)
+    b["max"][5, 0], b["min"][6, 0], b["max"][7, 1], b["min"][8, 2] = np.inf, -np.inf, np.inf, -np.inf
+    b["min"][9, 0], b["max"][9, 0] = 1.25, -3.75
+    b["min"][10, 0], b["max"][10, 0] = 150.125, -np.inf
+    want = oracle.broadphase(b)
+    d = torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+    pairs = torch.empty((len(want) + 16, 2), dtype=torch.int32, device=cuda)
+    ctx.set_option(stq.OPT_CELLS, 1)
+    for _ in range(2):
+        r = ctx.sweep(d, n, pairs, len(want) + 16, axis=0)
+        assert r.count == len(want)
+        assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+    ctx.batch_prepare(d, [0, 0, n // 2, n], axis=0)  # lists half as long, an empty scene between
+    r = ctx.sweep_prepared(pairs, len(want) + 16)
+    halves = [oracle.broadphase(b[: n // 2]), oracle.broadphase(b[n // 2 :])]
+    want = np.concatenate([h for h in halves if len(h)])
+    assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), oracle.canonical(want))
+
+
 def test_runs_of_tens_of_millions(ctx, stq, cuda):
     """2,500 boxes along the whole axis above 70 M points on it: one list, in which 32 of
     the long runs together have more candidates than 31 bits count. The long boxes all
