@@ -999,7 +999,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
     std::memcpy(&radius_bits, &inflation_radius, sizeof radius_bits);
     key.opts[16] = int64_t(radius_bits);
     key.stream = caller;
-    for (const DevBuf *b : ctx->buffers()) key.bufs.push_back(b->ptr);
+    for (const DevBuf *b : ctx->batch_buffers()) key.bufs.push_back(b->ptr);
     key.bufs.push_back(ctx->in_host);
     key.bufs.push_back(ctx->h_scene_pairs);
     int st = STQ_OK;

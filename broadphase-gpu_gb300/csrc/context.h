@@ -45,8 +45,8 @@ struct Staging {
 
 struct GraphKey {
   const void *ptr[7] = {};
-  // every buffer of the context: any call on it may have moved one since the
-  // capture (a sort of more pairs than the batch has replicas, a larger scene)
+  // the buffers that the graph addresses, device and page-locked: any call on the
+  // context may have moved one since the capture (a larger scene)
   std::vector<const void *> bufs;
   int64_t sizes[9] = {};
   int64_t opts[17] = {};  // every context option, then the inflation radius
@@ -147,12 +147,19 @@ struct stq_context {
   double stage_ms[kStages] = {};
   int64_t stage_calls[kStages] = {};
 
-  // every device buffer of the context
-  std::vector<DevBuf *> buffers() {
+  // the device buffers that a captured batch addresses (GraphKey)
+  std::vector<DevBuf *> batch_buffers() {
     return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &box_cells, &box_q, &tile_reps, &tile_off, &keys[0], &keys[1],
-            &vals[0], &vals[1], &sort_ws, &yz, &xx, &vv, &flag, &scode, &partner, &run_end, &long_list, &seg_scan, &box_counts,
-            &prefix_ws, &pair_tmp, &pair_ws, &batch_boxes, &e2e_boxes, &e2e_pairs, &e2e_mesh, &aux, &window_pairs,
-            &window_long_list, &window_cursors};
+            &vals[0], &vals[1], &sort_ws, &yz, &xx, &vv, &flag, &scode, &partner, &run_end, &long_list, &seg_scan,
+            &batch_boxes};
+  }
+  // every device buffer
+  std::vector<DevBuf *> buffers() {
+    std::vector<DevBuf *> all = batch_buffers();
+    for (DevBuf *b : {&box_counts, &prefix_ws, &pair_tmp, &pair_ws, &e2e_boxes, &e2e_pairs, &e2e_mesh, &aux, &window_pairs,
+                      &window_long_list, &window_cursors})
+      all.push_back(b);
+    return all;
   }
 };
 

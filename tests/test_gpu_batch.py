@@ -267,6 +267,32 @@ def test_scene_pairs_after_a_replayed_batch(stq, oracle, cuda, scenes):
             assert np.array_equal(ctx.batch_scene_pairs(1), [0])  # not swept yet
 
 
+def test_batch_graph_outlives_growing_buffers_of_other_calls(ctx, stq, oracle, cuda, scenes):
+    """Sorts of ever more pairs, an overflow's counts and a host call's copies are none of
+    the captured batch's buffers: it is replayed (no launch of its own), not captured again."""
+    import torch
+
+    meshes, want = scenes
+    V0, V1, E, F, vo, eo, fo = stq.concat_meshes(meshes)
+    d = [dev(x, cuda) for x in (V0, V1, E, F)]
+    cap = sum(len(w) for w in want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    few = stq.random_boxes(3000, seed=3)
+    for rep in range(4):
+        before = ctx.launches
+        r, per = ctx.batch_broadphase(d[0], d[1], vo, d[2], eo, d[3], fo, pairs, cap)
+        assert (ctx.launches == before) == (rep > 0)
+        assert np.array_equal(per, [len(w) for w in want])
+        if rep == 0:
+            ctx.sweep_prepared(pairs, cap // 2)  # overflows
+        elif rep == 1:
+            many = torch.randint(0, 1 << 20, (cap, 2), dtype=torch.int32, device=cuda)
+            ctx.sort_pairs(many, cap // 2)
+            ctx.sort_pairs(many, cap)
+        else:
+            ctx.sweep_host(few, np.zeros((1 << 16 << rep, 2), np.int32), axis=0)
+
+
 def test_batch_graph_follows_small_radii(ctx, stq, oracle, cuda, scenes):
     """Two inflation radii below 1e-9 are two graphs: the pairs of a scene scaled
     to 1e-9 depend on which of them was asked for."""
