@@ -129,6 +129,9 @@ int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap) {
   ctx->in_host_bytes = lay.total;
   STQ_CUDA(ctx, ctx->in_dev.ensure(lay.total), "allocate staging");
   STQ_CUDA(ctx, ctx->scenes.ensure(sizeof(SceneRecord) * size_t(scene_cap)), "allocate scenes");
+  STQ_CUDA(ctx, ctx->scene_sums.ensure(sizeof(SceneSums) * size_t(scene_cap)), "allocate scene sums");
+  STQ_CUDA(ctx, cudaMemsetAsync(ctx->scene_sums.ptr, 0, ctx->scene_sums.bytes, ctx->stream), "clear scene sums");
+  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");  // (the context's stream may change)
   STQ_CUDA(ctx, ctx->cell_base.ensure(sizeof(unsigned) * size_t(scene_cap + 1)), "allocate cell bases");
   STQ_CUDA(ctx, ctx->scene_pairs.ensure(sizeof(unsigned long long) * size_t(scene_cap)),
            "allocate scene pair counters");
@@ -171,14 +174,6 @@ void fill_staging(stq_context *ctx, const int64_t *box_off, int S, const int *ax
     in[s].cells_opt = int(ctx->options[STQ_OPT_CELLS]);
     in[s].cell_scale = ctx->cell_scale;
     in[s].tiles = 0;  // counted below
-    for (int k = 0; k < 3; ++k) {
-      in[s].s1[k] = in[s].s2[k] = 0.0;
-      in[s].lo_key[k] = 0xffffffffu;
-      in[s].hi_key[k] = 0u;
-    }
-    in[s].inverted = 0;
-    in[s].done = 0;
-    for (int l = 0; l < kGridLevels; ++l) in[s].level_reps[l] = 0;
   }
   TileRec *tr = host_at<TileRec>(ctx, L.tiles);
   int t = 0;
@@ -216,6 +211,7 @@ BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes) {
   b.tiles = dev_at<TileRec>(ctx, ctx->layout.tiles);
   b.tile_cap = grid_tiles(ctx);
   b.inputs = dev_at<SceneInput>(ctx, ctx->layout.inputs);
+  b.sums = ctx->scene_sums.as<SceneSums>();
   b.scene_pairs = ctx->scene_pairs.as<unsigned long long>();
   b.scenes = ctx->scenes.as<SceneRecord>();
   b.cell_base = ctx->cell_base.as<unsigned>();

@@ -93,20 +93,20 @@ __device__ __forceinline__ float inv_side(int n, float L) { return n > 1 ? float
 // median box extent (from a strided sample of the scene's boxes), at most
 // 2048 cells per axis and at most max(1, n / max(16, 8 x cell_scale)) cells.
 __device__ __forceinline__ void
-scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, const SceneInput &in, SceneRecord &r,
-             int scene, BatchHeader *hdr) {
+scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, const SceneInput &in, SceneSums &sums,
+             SceneRecord &r, int scene, BatchHeader *hdr) {
   // the accumulators were written by other blocks' atomics: read them from L2
   uint32_t lo_key[3], hi_key[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) lo_key[k] = __ldcg(&in.lo_key[k]), hi_key[k] = __ldcg(&in.hi_key[k]);
-  const bool inverted = __ldcg(&in.inverted) != 0;
+  for (int k = 0; k < 3; ++k) lo_key[k] = ~__ldcg(&sums.lo_not[k]), hi_key[k] = __ldcg(&sums.hi_key[k]);
+  const bool inverted = __ldcg(&sums.inverted) != 0;
   int axis = in.axis_mode;
   if (axis < 0) {
     __shared__ double var[3];
     if (threadIdx.x < 3) {
       const double m = n > 0 ? 2.0 * double(n) : 1.0;
-      const double mean = __ldcg(&in.s1[threadIdx.x]) / m;
-      var[threadIdx.x] = __ldcg(&in.s2[threadIdx.x]) - m * mean * mean;
+      const double mean = __ldcg(&sums.s1[threadIdx.x]) / m;
+      var[threadIdx.x] = __ldcg(&sums.s2[threadIdx.x]) - m * mean * mean;
     }
     __syncthreads();
     axis = 0;
@@ -213,6 +213,12 @@ scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, cons
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
+  for (int k = 0; k < 3; ++k) {  // for the next prepare
+    sums.s1[k] = sums.s2[k] = 0.0;
+    sums.lo_not[k] = sums.hi_key[k] = 0u;
+  }
+  sums.inverted = 0;
+  sums.done = 0u;
   const float lob = key_float(key_of(lo_key, b)), hib = key_float(key_of(hi_key, b));
   const float loc = key_float(key_of(lo_key, c)), hic = key_float(key_of(hi_key, c));
   const float Lb = hib - lob, Lc = hic - loc;
@@ -255,7 +261,8 @@ scene_policy(const stq_aabb *__restrict__ boxes, long long b0, long long n, cons
 // ---- 1. statistics: one tile (one scene) per block ------------------------------
 __global__ void __launch_bounds__(kBlock)
 batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
-                   const long long *__restrict__ box_off, SceneInput *inputs, SceneRecord *scenes, BatchHeader *hdr) {
+                   const long long *__restrict__ box_off, const SceneInput *__restrict__ inputs, SceneSums *sums,
+                   SceneRecord *scenes, BatchHeader *hdr) {
   after_previous();
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
@@ -315,7 +322,7 @@ batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict
     wflag[warp] = fl;
   }
   __syncthreads();
-  SceneInput &r = inputs[t.scene];
+  SceneSums &r = sums[t.scene];
   __shared__ bool last;
   if (warp == 0) {
     double tot = 0.0;  // lane k < 6: moment k of the block
@@ -335,7 +342,7 @@ batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict
       const double ck = k == 0 ? c[0] : (k == 1 ? c[1] : c[2]), n = double(t.count);
       if (lane < 3) {
         atomicAdd(&r.s1[k], tot + 2.0 * n * ck);
-        atomicMin(&r.lo_key[k], key);
+        atomicMax(&r.lo_not[k], ~key);
       } else {
         atomicAdd(&r.s2[k], tot + 2.0 * ck * a1 + 2.0 * n * ck * ck);
         atomicMax(&r.hi_key[k], key);
@@ -346,13 +353,13 @@ batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict
     // the block whose tile is the scene's last goes on to its policy
     __threadfence();
     __syncwarp();
-    if (lane == 0) last = atomicAdd(&r.done, 1u) + 1u == unsigned(r.tiles);
+    if (lane == 0) last = atomicAdd(&r.done, 1u) + 1u == unsigned(inputs[t.scene].tiles);
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
   const long long first = box_off[t.scene];
-  scene_policy(boxes, first, box_off[t.scene + 1] - first, r, scenes[t.scene], t.scene, hdr);
+  scene_policy(boxes, first, box_off[t.scene + 1] - first, inputs[t.scene], r, scenes[t.scene], t.scene, hdr);
 }
 
 struct Range {
@@ -372,79 +379,89 @@ __device__ __forceinline__ Range cell_range(const stq_aabb &x, int a, float ob, 
   return r;
 }
 
-// ---- 4. the finest level within the replica budget, cell bases, key layout, by the
-// block that finished the box keys
-__device__ __forceinline__ void
-choose_levels(const long long *__restrict__ box_off, const TileRec *__restrict__ tiles, const SceneInput *inputs,
-              SceneRecord *scenes, unsigned int *cell_base, const unsigned long long *tile_reps, uint32_t *tile_off,
-              BatchHeader *hdr, FrontInfo *front, long long rep_cap, long long seg_cap, int max_passes) {
-  __shared__ uint32_t scratch[kBlock / 32];
-  __shared__ unsigned long long reps;
-  if (threadIdx.x == 0) reps = 0;
-  __syncthreads();
-  const int S = hdr->n_scenes;
-  const long long budget = hdr->budget;
-  unsigned int carry = 0;
-  for (int base = 0; base < S; base += kBlock) {
-    const int s = base + threadIdx.x;
-    unsigned int cells = 0;
-    if (s < S) {
-      SceneRecord &r = scenes[s];
-      const SceneInput &in = inputs[s];
-      unsigned long long level_reps[kGridLevels];
+// ---- 4. the finest level of a scene within the replica budget, by one thread of the
+// block that finished the scene's box keys; returns its replicas
+__device__ __forceinline__ unsigned long long choose_level(const SceneInput &in, const unsigned long long (&level_reps)[kGridLevels],
+                                                           GridParams &g, long long n, long long budget) {
+  int level = kCoordBits;  // none fits: every coordinate shifts to cell 0
+  unsigned long long used = (unsigned long long)n;  // one cell: each box once
+  if (in.cells_opt > 1) {
+    level = 0;  // a requested grid is kept as is
+    used = level_reps[0];
+  } else {
 #pragma unroll
-      for (int l = 0; l < kGridLevels; ++l) level_reps[l] = __ldcg(&in.level_reps[l]);
-      const long long n = box_off[s + 1] - box_off[s];
-      int level = kCoordBits;  // none fits: every coordinate shifts to cell 0
-      unsigned long long used = (unsigned long long)n;  // one cell: each box once
-      if (in.cells_opt > 1) {
-        level = 0;  // a requested grid is kept as is
-        used = level_reps[0];
-      } else {
-#pragma unroll
-        for (int l = kGridLevels - 1; l >= 0; --l)
-          if ((long long)level_reps[l] <= budget * n) {
-            level = l;
-            used = level_reps[l];
-          }
+    for (int l = kGridLevels - 1; l >= 0; --l)
+      if ((long long)level_reps[l] <= budget * n) {
+        level = l;
+        used = level_reps[l];
       }
-      GridParams &g = r.grid;
-      g.shift = level;
-      g.nb = ((g.nb0 - 1) >> level) + 1;
-      g.nc = ((g.nc0 - 1) >> level) + 1;
-      g.ncells = g.nb * g.nc;
-      atomicAdd(&reps, used);
-      // 64 code steps per cell of the chosen level; a cell is 2^level level-0
-      // cells, of which there are nb0 over Lb (one cell: the whole extent)
-      const float steps = 64.f / float(1 << level);
-      g.sb = g.Lb > 0.f && isfinite(g.Lb) ? (level >= kCoordBits ? 64.f : steps * float(g.nb0)) / g.Lb : 0.f;
-      g.sc = g.Lc > 0.f && isfinite(g.Lc) ? (level >= kCoordBits ? 64.f : steps * float(g.nc0)) / g.Lc : 0.f;
-      cells = unsigned(g.ncells);
-    }
-    uint32_t total;
-    const unsigned int excl = carry + block_exclusive(cells, &total, scratch);
-    if (s < S) cell_base[s] = excl;
+  }
+  g.shift = level;
+  g.nb = ((g.nb0 - 1) >> level) + 1;
+  g.nc = ((g.nc0 - 1) >> level) + 1;
+  g.ncells = g.nb * g.nc;
+  // 64 code steps per cell of the chosen level; a cell is 2^level level-0
+  // cells, of which there are nb0 over Lb (one cell: the whole extent)
+  const float steps = 64.f / float(1 << level);
+  g.sb = g.Lb > 0.f && isfinite(g.Lb) ? (level >= kCoordBits ? 64.f : steps * float(g.nb0)) / g.Lb : 0.f;
+  g.sc = g.Lc > 0.f && isfinite(g.Lc) ? (level >= kCoordBits ? 64.f : steps * float(g.nc0)) / g.Lc : 0.f;
+  return used;
+}
+
+// Exclusive scan, by the block, of value(0 .. n - 1) into out; returns the total. Each
+// thread takes several consecutive values where there are more than threads: their
+// loads are in flight together, and one scan serves them all.
+template <typename Value>
+__device__ __forceinline__ uint32_t scan_into(int n, uint32_t *out, uint32_t *scratch, const Value &value) {
+  constexpr int kMost = 8;
+  const int per = min(kMost, (n + kBlock - 1) / kBlock);
+  uint32_t carry = 0;
+  for (int base = 0; base < n; base += kBlock * per) {
+    const int i0 = base + int(threadIdx.x) * per;
+    uint32_t v[kMost], sum = 0, total;
+#pragma unroll
+    for (int u = 0; u < kMost; ++u) v[u] = u < per && i0 + u < n ? value(i0 + u) : 0u;
+#pragma unroll
+    for (int u = 0; u < kMost; ++u) sum += v[u];
+    uint32_t at = carry + block_exclusive(sum, &total, scratch);
+#pragma unroll
+    for (int u = 0; u < kMost; ++u)
+      if (u < per && i0 + u < n) {
+        out[i0 + u] = at;
+        at += v[u];
+      }
     carry += total;
   }
-  __syncthreads();
+  return carry;
+}
+
+// What choose_level found, kept in the block for a batch of one scene.
+struct OneScene {
+  unsigned long long used;
+  uint32_t cells;
+  int level;
+};
+
+// Cell bases, the tiles' first replicas and the key layout, by the block that finished
+// the box keys. (20,000 scenes of 20 boxes: the keys stage took 1,172 us with the levels
+// chosen here, one scene per thread.)
+__device__ __forceinline__ void
+lay_out(const TileRec *__restrict__ tiles, const SceneRecord *scenes, const OneScene &one, unsigned int *cell_base,
+        const unsigned long long *tile_reps, uint32_t *tile_off, BatchHeader *hdr, FrontInfo *front, long long rep_cap,
+        long long seg_cap, int max_passes) {
+  __shared__ uint32_t scratch[kBlock / 32];
+  const int S = hdr->n_scenes;
+  const uint32_t carry = scan_into(S, cell_base, scratch, [&](int s) {
+    return S == 1 ? one.cells : uint32_t(__ldcg(&scenes[s].grid.ncells));
+  });
   // every tile's first replica, at its scene's level
-  const int n_tiles = hdr->n_tiles;
-  uint32_t at = 0;
-  for (int base = 0; base < n_tiles; base += kBlock) {
-    const int t = base + threadIdx.x;
-    uint32_t n = 0;
-    if (t < n_tiles) {
-      const int level = scenes[tiles[t].scene].grid.shift;
-      n = level < kGridLevels ? uint32_t(__ldcg(&tile_reps[size_t(t) * kGridLevels + level])) : uint32_t(tiles[t].count);
-    }
-    uint32_t total;
-    const uint32_t off = at + block_exclusive(n, &total, scratch);
-    if (t < n_tiles) tile_off[t] = off;
-    at += total;
-  }
+  scan_into(hdr->n_tiles, tile_off, scratch, [&](int t) {
+    const int level = S == 1 ? one.level : __ldcg(&scenes[tiles[t].scene].grid.shift);
+    return level < kGridLevels ? uint32_t(__ldcg(&tile_reps[size_t(t) * kGridLevels + level])) : uint32_t(tiles[t].count);
+  });
   if (threadIdx.x == 0) {
     cell_base[S] = carry;
-    const unsigned long long R = reps, lists = 3ull * carry;
+    const unsigned long long R = S == 1 ? one.used : __ldcg(&hdr->used), lists = 3ull * carry;
     // key: list id above the top bits of the sweep-axis code, 24 bits in all (three
     // digits) where that leaves the code 9 bits or more, else 32. At 10 bits the
     // 6 M-box scene (14 bits of lists) tests 9% more candidates and sorts a digit
@@ -502,7 +519,7 @@ __device__ __forceinline__ uint32_t axis_code(float v, const float *split, const
 
 __global__ void __launch_bounds__(kBlock)
 batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict__ tiles,
-                      const long long *__restrict__ box_off, SceneInput *inputs,
+                      const long long *__restrict__ box_off, const SceneInput *__restrict__ inputs, SceneSums *sums,
                       SceneRecord *scenes, unsigned int *cell_base, unsigned long long *tile_reps, uint32_t *tile_off,
                       BatchHeader *hdr, FrontInfo *front, long long rep_cap, long long seg_cap, int max_passes,
                       uint2 *__restrict__ box_cells, uint32_t *__restrict__ box_q) {
@@ -542,21 +559,47 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
   for (int l = 0; l < kGridLevels; ++l) wide[l] = reps[l];
   block_sums(wide, tot, red);
   __shared__ bool last;
+  __shared__ OneScene one;
   if (threadIdx.x == 0) {
+    const SceneInput &in = inputs[t.scene];
+    SceneSums &sum = sums[t.scene];
+    const unsigned tiles_all = unsigned(hdr->n_tiles);
 #pragma unroll
     for (int l = 0; l < kGridLevels; ++l) {
-      if (tot[l]) atomicAdd(&inputs[t.scene].level_reps[l], tot[l]);
       tile_reps[size_t(blockIdx.x) * kGridLevels + l] = tot[l];
+      if (in.tiles > 1 && tot[l]) atomicAdd(&sum.level_reps[l], tot[l]);
     }
-    // the block whose tile is the batch's last goes on to the levels
+    // the block whose tile is the scene's last chooses its level (in a batch of one
+    // scene, the one that goes on)
+    bool scene_last = in.tiles == 1;
+    if (!scene_last) {
+      __threadfence();
+      if (unsigned(in.tiles) != tiles_all) {
+        scene_last = atomicAdd(&sum.keys_done, 1u) + 1u == unsigned(in.tiles);
+      } else {
+        scene_last = last = atomicAdd(&hdr->keys_done, 1u) + 1u == tiles_all;
+      }
+      if (scene_last) {  // the other blocks' sums, cleared for the next prepare
+        __threadfence();
+#pragma unroll
+        for (int l = 0; l < kGridLevels; ++l) tot[l] = __ldcg(&sum.level_reps[l]), sum.level_reps[l] = 0ull;
+        sum.keys_done = 0u;
+      }
+    }
+    if (scene_last) {
+      GridParams &sg = scenes[t.scene].grid;
+      const unsigned long long used = choose_level(in, tot, sg, box_off[t.scene + 1] - box_off[t.scene], hdr->budget);
+      if (unsigned(in.tiles) == tiles_all) one = OneScene{used, uint32_t(sg.ncells), sg.shift};
+      else if (used) atomicAdd(&hdr->used, used);
+    }
+    // the block whose tile is the batch's last goes on to the layout
     __threadfence();
-    last = atomicAdd(&hdr->keys_done, 1u) + 1u == unsigned(hdr->n_tiles);
+    if (unsigned(in.tiles) != tiles_all || in.tiles == 1) last = atomicAdd(&hdr->keys_done, 1u) + 1u == tiles_all;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  choose_levels(box_off, tiles, inputs, scenes, cell_base, tile_reps, tile_off, hdr, front, rep_cap, seg_cap,
-                max_passes);
+  lay_out(tiles, scenes, one, cell_base, tile_reps, tile_off, hdr, front, rep_cap, seg_cap, max_passes);
 }
 
 // ---- 5. replica keys in box order: (list id << key_bits) | sweep-axis code, where
@@ -894,13 +937,13 @@ cudaError_t launch_reset_sweep(cudaStream_t s, BatchHeader *hdr, unsigned long l
 
 cudaError_t launch_batch_stats(cudaStream_t s, const BatchBuffers &b) {
   launch_after(batch_stats_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.boxes, b.tiles, b.box_off, b.inputs,
-               b.scenes, b.hdr);
+               b.sums, b.scenes, b.hdr);
   return cudaGetLastError();
 }
 
 cudaError_t launch_batch_box_keys(cudaStream_t s, const BatchBuffers &b, int64_t rep_cap, int64_t seg_cap, int passes) {
   launch_after(batch_box_keys_kernel, unsigned(b.tile_cap), kBlock, 0, s, b.boxes, b.tiles, b.box_off, b.inputs,
-               b.scenes, b.cell_base, b.tile_reps, b.tile_off, b.hdr, b.front, rep_cap, seg_cap, passes, b.box_cells,
+               b.sums, b.scenes, b.cell_base, b.tile_reps, b.tile_off, b.hdr, b.front, rep_cap, seg_cap, passes, b.box_cells,
                b.box_q);
   return cudaGetLastError();
 }

@@ -87,7 +87,7 @@ struct stq_context {
   DevBuf in_dev;
   char *in_host = nullptr;
   size_t in_host_bytes = 0;
-  DevBuf scenes, cell_base, scene_pairs, box_cells, box_q, tile_reps, tile_off, keys[2], vals[2], sort_ws;
+  DevBuf scenes, scene_sums, cell_base, scene_pairs, box_cells, box_q, tile_reps, tile_off, keys[2], vals[2], sort_ws;
   DevBuf points;  // fp64 vertex positions rounded to float once (box builds)
   DevBuf yz, xx, vv, flag, scode, partner, run_end, box_counts, prefix_ws, pair_tmp;
   DevBuf pair_ws;  // pair sorts' own: a prepare relies on sort_ws as it sized it
@@ -149,7 +149,7 @@ struct stq_context {
 
   // the device buffers that a captured batch addresses (GraphKey)
   std::vector<DevBuf *> batch_buffers() {
-    return {&points, &in_dev, &scenes, &cell_base, &scene_pairs, &box_cells, &box_q, &tile_reps, &tile_off, &keys[0], &keys[1],
+    return {&points, &in_dev, &scenes, &scene_sums, &cell_base, &scene_pairs, &box_cells, &box_q, &tile_reps, &tile_off, &keys[0], &keys[1],
             &vals[0], &vals[1], &sort_ws, &yz, &xx, &vv, &flag, &scode, &partner, &run_end, &long_list, &seg_scan,
             &batch_boxes};
   }

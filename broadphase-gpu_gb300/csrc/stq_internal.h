@@ -145,18 +145,23 @@ struct SceneRecord {
   GridParams grid;
 };
 
-// Per-scene inputs, written by the host before every prepare with the
-// accumulators at their start values.
+// Per-scene inputs, written by the host before every prepare.
 struct SceneInput {
   int axis_mode;        // -1: largest variance, else the axis
   int cells_opt;        // 0 automatic, 1 no cells, k > 1 a k x k grid
   float cell_scale;     // automatic cell side in median box extents
   int tiles;            // tiles of the scene
-  // accumulators
-  double s1[3], s2[3];                // sum(min + max), sum(min^2 + max^2)
-  unsigned int lo_key[3], hi_key[3];  // order-preserving min / max bounds
-  int inverted;                       // some box has min > max on an axis
-  unsigned int done;                  // tiles whose statistics are in
+};
+
+// Per-scene accumulators of a prepare, on the device: zero before it, and cleared by
+// the blocks that read them (uploaded with the inputs, 20,000 scenes were 3 MB to fill
+// and copy).
+struct SceneSums {
+  double s1[3], s2[3];               // sum(min + max), sum(min^2 + max^2)
+  unsigned int lo_not[3], hi_key[3]; // order-preserving keys of the bounds: ~ of the least, the largest
+  int inverted;                      // some box has min > max on an axis
+  unsigned int done;                 // tiles whose statistics are in
+  unsigned int keys_done, pad;       // tiles whose box keys are
   unsigned long long level_reps[kGridLevels];  // replicas per grid level
 };
 
@@ -186,6 +191,7 @@ struct BatchHeader {
   int fault;                // a bounded wait between blocks ran out
   unsigned int passes;      // digits of the replica sort; its input is in buffer passes & 1
   unsigned int keys_done;   // tiles whose box keys and level counts are in
+  unsigned long long used;  // replicas of all scenes at their levels, accumulated
 };
 
 // What the host needs of a prepare's first half, written by the device to
@@ -326,7 +332,8 @@ struct BatchBuffers {
   const long long *box_off;     // n_scenes + 1 box offsets
   const TileRec *tiles;         // n_tiles entries
   int tile_cap;
-  SceneInput *inputs;           // n_scenes entries
+  const SceneInput *inputs;     // n_scenes entries
+  SceneSums *sums;              // n_scenes entries, zero between prepares
   unsigned long long *scene_pairs;  // n_scenes pair counters
   SceneRecord *scenes;
   unsigned int *cell_base;      // n_scenes + 1

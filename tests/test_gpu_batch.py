@@ -188,6 +188,37 @@ def test_batch_skewed_boxes_mixed_axes(ctx, stq, oracle, cuda):
     check_batch(oracle, pairs[: r.count].cpu().numpy(), bo, want, ctx.batch_scene_pairs(len(sizes)))
 
 
+@pytest.mark.parametrize("count", [256, 257, 2048, 2049, 5000])
+def test_batches_of_many_small_scenes(ctx, stq, oracle, cuda, count):
+    """More scenes (and tiles) than threads of the block that lays them out, empty ones
+    and one of several tiles among them."""
+    rng = np.random.default_rng(count)
+    kinds = []
+    for k in range(12):
+        b = stq.random_boxes(5 * k, sliver_frac=0.0, seed=k) if k else np.zeros(0, stq.AABB_DTYPE)
+        c = rng.uniform(0, 1, (len(b), 3)).astype(np.float32)
+        b["min"], b["max"] = c, c + np.float32(0.3)
+        kinds.append((b, oracle.broadphase(b) if k else np.zeros((0, 2), np.int32)))
+    b = stq.random_boxes(3000, sliver_frac=0.0, seed=20)
+    kinds.append((b, oracle.broadphase(b)))
+    pick = rng.integers(0, 12, count)
+    pick[[3, count - 2]] = 12
+    bo = np.concatenate([[0], np.cumsum([len(kinds[k][0]) for k in pick])]).astype(np.int64)
+    boxes = np.concatenate([kinds[k][0] for k in pick])
+    boxes["id"] = np.arange(len(boxes))
+    import torch
+
+    want = [kinds[k][1] for k in pick]
+    cap = sum(len(w) for w in want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    ctx.batch_prepare(dev(boxes.view(np.int32).reshape(-1, 11), cuda), bo)
+    r = ctx.sweep_prepared(pairs, cap)
+    assert r.status == stq.STQ_OK
+    assert np.array_equal(ctx.batch_scene_pairs(count), [len(w) for w in want])
+    all_want = np.concatenate([w + o for w, o in zip(want, bo[:-1])])
+    assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), oracle.canonical(all_want))
+
+
 def test_autotune_keeps_results_exact_and_caches(ctx, stq, oracle, cuda, scenes):
     import torch
 
