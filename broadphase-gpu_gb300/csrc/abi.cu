@@ -130,8 +130,7 @@ int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap) {
   STQ_CUDA(ctx, ctx->in_dev.ensure(lay.total), "allocate staging");
   STQ_CUDA(ctx, ctx->scenes.ensure(sizeof(SceneRecord) * size_t(scene_cap)), "allocate scenes");
   STQ_CUDA(ctx, ctx->scene_sums.ensure(sizeof(SceneSums) * size_t(scene_cap)), "allocate scene sums");
-  STQ_CUDA(ctx, cudaMemsetAsync(ctx->scene_sums.ptr, 0, ctx->scene_sums.bytes, ctx->stream), "clear scene sums");
-  STQ_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "synchronise stream");  // (the context's stream may change)
+  ctx->sums_clear = false;
   STQ_CUDA(ctx, ctx->cell_base.ensure(sizeof(unsigned) * size_t(scene_cap + 1)), "allocate cell bases");
   STQ_CUDA(ctx, ctx->scene_pairs.ensure(sizeof(unsigned long long) * size_t(scene_cap)),
            "allocate scene pair counters");
@@ -192,7 +191,17 @@ void fill_staging(stq_context *ctx, const int64_t *box_off, int S, const int *ax
   h->n_tiles = t;
 }
 
+// Clears newly allocated accumulators, on the stream that uses them next (a graph's
+// are cleared before the capture).
+int clear_sums(stq_context *ctx) {
+  if (ctx->sums_clear) return STQ_OK;
+  STQ_CUDA(ctx, cudaMemsetAsync(ctx->scene_sums.ptr, 0, ctx->scene_sums.bytes, ctx->stream), "clear scene sums");
+  ctx->sums_clear = true;
+  return STQ_OK;
+}
+
 int upload_staging(stq_context *ctx) {
+  if (!ctx->capturing) STQ_TRY(clear_sums(ctx));
   STQ_CUDA(ctx, cudaMemcpyAsync(ctx->in_dev.ptr, ctx->in_host, ctx->layout.total,
                                 cudaMemcpyHostToDevice, ctx->stream),
            "upload batch inputs");
@@ -933,6 +942,7 @@ int stq_batch_broadphase(stq_context *ctx, const double *d_V0, const double *d_V
   const int64_t cells_cap = N / 16 + n_scenes + 1;
   ctx->prepared = false;  // the buffers of the prepared scenes are reused
   STQ_TRY(ensure_staging(ctx, n_scenes, int(T)));
+  STQ_TRY(clear_sums(ctx));
   STQ_TRY(ensure_box_buffers(ctx, N));
   STQ_TRY(ensure_replica_buffers(ctx, rep_cap, cells_cap));
   STQ_CUDA(ctx, ctx->batch_boxes.ensure(sizeof(stq_aabb) * size_t(std::max<int64_t>(N, 1))),

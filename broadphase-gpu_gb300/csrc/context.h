@@ -111,6 +111,7 @@ struct stq_context {
   PairPlan *h_plan = nullptr;         // written by a pair sort's histogram
   DevScalars *h_sel = nullptr;        // readback of an overflowing sweep's prefix
   int pair_id_bits = 0;               // of the largest first id of the pairs sorted so far
+  bool sums_clear = false;  // scene_sums holds zeros between prepares
   int passes_seen = 0;  // most digits that a replica sort of this context needed
   double density = 0.0;  // replicas per box of the last prepared scenes
   bool overflowed = false;  // the last sweep of the prepared scenes found more pairs than fit
@@ -195,6 +196,7 @@ int64_t tiles_for(const int64_t *box_off, int S);
 int ensure_staging(stq_context *ctx, int scene_cap, int tile_cap);
 void fill_staging(stq_context *ctx, const int64_t *box_off, int S, const int *axes, int axis,
                   const int64_t *voff, const int64_t *eoff, const int64_t *foff);
+int clear_sums(stq_context *ctx);
 int upload_staging(stq_context *ctx);
 BatchBuffers batch_buffers(stq_context *ctx, const stq_aabb *boxes);
 int ensure_box_buffers(stq_context *ctx, int64_t box_cap);
