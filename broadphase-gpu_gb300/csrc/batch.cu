@@ -697,11 +697,11 @@ __global__ void __launch_bounds__(kBlock)
 list_offsets_kernel(const uint32_t *__restrict__ keys, BatchHeader *__restrict__ hdr,
                     uint32_t *__restrict__ seg_scan, long long seg_cap, SortedScene scene, int64_t slots_cap) {
   after_previous();
-  if (hdr->fault) return;  // the replicas are not sorted
-  // (cells past the capacity are flagged and counted as none)
+  // (cells past the capacity are flagged and counted as none; the loads together)
   const uint32_t nseg = uint32_t(min(3ll * hdr->cells, seg_cap));
   const uint32_t R = hdr->replicas;
   const int key_bits = hdr->key_bits;
+  if (hdr->fault) return;  // the replicas are not sorted
   auto empty = [&](int64_t k) {
     if (k < slots_cap) {
       scene.partner[k] = int(k);
@@ -787,8 +787,7 @@ gather_cells_kernel(const stq_aabb *__restrict__ boxes, const uint32_t *__restri
                     const SceneRecord *__restrict__ scenes, const uint32_t *__restrict__ seg_scan,
                     SortedScene scene) {
   after_previous();
-  if (hdr->fault) return;  // the replicas are not sorted
-  const int64_t R = hdr->replicas;
+  const int64_t R = hdr->fault ? 0 : hdr->replicas;  // (none where they are not sorted)
   const int S = hdr->n_scenes;
   const int key_bits = hdr->key_bits;
   for (int64_t p = blockIdx.x * int64_t(kBlock) + threadIdx.x; p < R;
@@ -903,7 +902,7 @@ reset_sweep_kernel(BatchHeader *hdr, unsigned long long *scene_pairs, const DevS
     hdr->pairs = 0ull;
     hdr->work = 0;
     hdr->long_items = 0u;
-    hdr->long_work = 0u;
+    hdr->long_work = 0ull;
     hdr->candidates = 0ull;
   }
 }
@@ -918,7 +917,7 @@ __global__ void window_step_kernel(WindowCounters *wc, unsigned long long *host_
   *reinterpret_cast<volatile unsigned long long *>(host_count) = wc->pairs;
   wc->work = 0;
   wc->long_items = 0u;
-  wc->long_work = 0u;
+  wc->long_work = 0ull;
   __threadfence_system();
 }
 

@@ -48,14 +48,22 @@ constexpr int kPollLimit = STQ_SORT_POLL_LIMIT;
 // follow it.
 struct SortHead {
   uint32_t hist[kMaxPasses][kBins];  // digit counts, then first positions
-  uint32_t ticket[kMaxPasses];       // next tile of each pass
+  uint32_t ticket[kMaxPasses];       // next tile of each pass; kNoTile and more: a wait gave up
   uint32_t done;                     // blocks of the histogram kernel that are done
   uint32_t run[kMaxPasses];          // the pass is run (not skipped)
   uint32_t src[kMaxPasses];          // buffer that the pass reads
-  uint32_t fault;                    // a wait gave up: nothing more is written
 };
 
 static_assert(sizeof(SortHead) <= kRadixHeadBytes, "workspace sizing");
+
+// Added to the tickets of a pass, and no later pass run, once a wait gave up: the words
+// that blocks read anyway (a word of its own cost each tile of a pass 0.7 us).
+constexpr uint32_t kNoTile = 1u << 30;
+
+__device__ __forceinline__ void give_up(SortHead *head, int pass) {
+  atomicMax(&head->ticket[pass], kNoTile);
+  for (int q = pass + 1; q < kMaxPasses; ++q) head->run[q] = 0u;
+}
 
 // Bits of each digit of a sort, lowest first.
 struct Digits {
@@ -73,10 +81,6 @@ __device__ __forceinline__ unsigned long long load_status(const unsigned long lo
 }
 __device__ __forceinline__ void store_status(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-__device__ __forceinline__ bool faulted(const SortHead *head) {
-  return *reinterpret_cast<const volatile uint32_t *>(&head->fault) != 0u;
 }
 
 // Exclusive scan of v over the first 256 threads of the block (every thread
@@ -195,13 +199,14 @@ radix_hist_kernel(const K *__restrict__ k0, const K *__restrict__ k1, int64_t n,
 // Status word: (2 * pass + 1) << 32 | count of the tile, or (2 * pass + 2) << 32
 // | sum up to and with the tile; smaller tags are from earlier passes.
 // *timeout: a word did not come, here or in another block of the pass.
-__device__ __forceinline__ uint32_t look_back(const SortHead *head, const unsigned long long *status, int64_t tile, int d,
-                                              uint32_t tag, bool *timeout) {
+__device__ __forceinline__ uint32_t look_back(const uint32_t *ticket, const unsigned long long *status, int64_t tile,
+                                              int d, uint32_t tag, bool *timeout) {
   uint32_t sum = 0;
   int polls = 0;
   int64_t t = tile - 1;
   while (t >= 0) {
-    if (polls == kPollLimit || (polls % 1024 == 1023 && faulted(head))) {
+    if (polls == kPollLimit ||
+        (polls % 1024 == 1023 && *reinterpret_cast<const volatile uint32_t *>(ticket) >= kNoTile)) {
       *timeout = true;
       break;
     }
@@ -251,7 +256,7 @@ __global__ void __launch_bounds__(kPassBlock, 2)
 radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const unsigned int *d_n, int pass, int shift,
                   SortHead *head, unsigned long long *status, int *fault) {
   after_previous();
-  if (!head->run[pass] || head->fault) return;
+  if (!head->run[pass]) return;
   if (d_n && int64_t(*d_n) < n) n = *d_n;
   const bool flip = head->src[pass] != 0;
   const K *__restrict__ kin = flip ? k1 : k0;
@@ -268,7 +273,7 @@ radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const uns
   uint32_t *cnt = sm.cnt[warp];
   const unsigned below = lanemask_lt();
   while (true) {
-    if (tid == 0) sm.tile = faulted(head) ? tiles : int64_t(atomicAdd(&head->ticket[pass], 1u));
+    if (tid == 0) sm.tile = int64_t(atomicAdd(&head->ticket[pass], 1u));
     for (int i = lane; i < kBins; i += 32) cnt[i] = 0;
     __syncthreads();  // also: the tile before has been written out
     const int64_t tile = sm.tile;
@@ -325,7 +330,7 @@ radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const uns
     // 3. the digits' first output positions
     bool timeout = false;
     if (tid < kBins) {
-      const uint32_t before = look_back(head, status, tile, tid, tag, &timeout);
+      const uint32_t before = look_back(&head->ticket[pass], status, tile, tid, tag, &timeout);
       if (tile > 0 && !timeout) store_status(status + tile * kBins + tid, (unsigned long long)(tag + 1u) << 32 | (before + total));
       sm.out_base[tid] = head->hist[pass][tid] + before - base;
     }
@@ -333,7 +338,7 @@ radix_pass_kernel(K *k0, K *k1, uint32_t *v0, uint32_t *v1, int64_t n, const uns
     // the tiles that wait for this one, or in a later pass
     if (__syncthreads_or(timeout)) {
       if (tid == 0) {
-        *reinterpret_cast<volatile uint32_t *>(&head->fault) = 1u;
+        give_up(head, pass);
         *reinterpret_cast<volatile int *>(fault) = 1;
       }
       return;

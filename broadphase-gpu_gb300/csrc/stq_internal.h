@@ -176,7 +176,7 @@ struct BatchHeader {
   unsigned int length;      // sweep positions: R + 3 * cells - 1
   int work;                 // sweep grab cursor
   unsigned int long_items;  // runs handed from the lane sweep to the warp pass
-  unsigned int long_work;   // warp pass grab cursor
+  unsigned long long long_work;  // warp pass grab cursor
   unsigned long long pairs; // pairs found by the last sweep
   long long prefix;         // overflow: start positions of the prefix that fits
   int axis;                 // sweep axis of scene 0
@@ -267,8 +267,7 @@ struct WindowCounters {
   unsigned long long pairs;  // pairs found
   int work;                  // grab cursor
   unsigned int long_items;   // runs handed to the warp pass
-  unsigned int long_work;    // warp pass grab cursor
-  int pad;
+  unsigned long long long_work;  // warp pass grab cursor
 };
 
 // Where one sweep launch keeps its counters and handed-over runs.
@@ -277,7 +276,7 @@ struct SweepCursors {
   int *work;
   int2 *long_list;
   unsigned int *long_items;
-  unsigned int *long_work;
+  unsigned long long *long_work;
 };
 
 struct SweepParams {
@@ -306,7 +305,7 @@ struct SweepParams {
                              // pass; 0 = never
   int2 *long_list;           // handed-over runs (start position, next candidate)
   unsigned int *long_items;  // their count
-  unsigned int *long_work;   // warp pass grab cursor
+  unsigned long long *long_work;  // warp pass grab cursor
   const DevScalars *sel;     // if set: start positions [begin, begin + sel->prefix),
                              // and none if sel->count pairs fit the capacity
 };

@@ -49,8 +49,7 @@ __device__ __forceinline__ bool pair_hit(const PosRec &a, const PosRec &b, int t
 // One past the last start position of a sweep, from the sizes on the device (none
 // if a wait of the sort ran out: there is no sorted scene then).
 __device__ __forceinline__ int sweep_end(const SweepParams &p) {
-  if (p.hdr->fault) return p.begin;
-  const int end = min(p.end, int(p.hdr->length));
+  const int end = p.hdr->fault ? p.begin : min(p.end, int(p.hdr->length));
   if (!p.sel) return end;
   return p.sel->count <= (unsigned long long)p.capacity ? p.begin : int(min((long long)end, p.begin + p.sel->prefix));
 }
@@ -425,9 +424,9 @@ stq_sweep_lane_kernel(const SweepParams p) {
 // LONG: the warp pass over the runs that were handed over (longer than run_cap,
 // which would keep one lane, group or warp busy long after the others finished).
 // The warp's starts are entries of that list, and when there are fewer of them
-// than warps each run is cut into as many equal parts as give every warp one.
-// Parts are taken in slices of at most kLongSlice candidates, so that the warp's
-// 32 together are within 31 bits, and an offset in a run within the queue's 27.
+// than warps each run is cut into as many equal parts as give every warp one; at
+// least into as many as keep a part within kLongPart candidates, so that the warp's
+// 32 together are within 31 bits, and an offset in a part within the queue's 27.
 struct FlatStart {
   float4 yz;      // the start box (PosRec)
   int4 v;
@@ -450,7 +449,7 @@ constexpr int kBandRatio = 6;
 constexpr int kFlatStage = 192;
 constexpr int kFlatRound = 256;  // candidates queued at once by a band step (or 32 V by a flat one)
 constexpr int kFlatQueue = 32 + kFlatRound;
-constexpr int kLongSlice = 1 << 25;
+constexpr unsigned kLongPart = 1u << 25;
 struct FlatWarp {
   FlatStart rec[32];
   int2 lookup[32];             // flat form: code_start of a start's code, and joff: its
@@ -476,68 +475,65 @@ stq_sweep_flat_kernel(const SweepParams p) {
   int2 *st = sw.stage;
   uint32_t *qu = sw.queue;
 
-  int end, span, chunk;
+  using Index = typename std::conditional<LONG, long long, int>::type;  // a part of a run, or a start position
+  Index end, span;
+  int chunk;
   unsigned parts = 1;  // LONG: parts of a run
   if (LONG) {
     if (p.sel && p.sel->count <= (unsigned long long)p.capacity) return;  // the list is of an earlier sweep
-    if (p.hdr->fault) return;
     const unsigned items = *p.long_items, warps = gridDim.x * (BLOCK / 32);
     if (items == 0) return;
-    parts = max(1u, min(64u, warps / items));
-    end = span = int(items * parts);
-    chunk = max(1, min(32, span / int(4 * warps)));
+    parts = max(max(1u, min(64u, warps / items)), (p.hdr->length + kLongPart - 1u) / kLongPart);
+    end = span = Index(items) * parts;
+    chunk = int(max(Index(1), min(Index(32), span / Index(4 * warps))));
   } else {
     end = sweep_end(p);
     span = end - p.begin;
     chunk = sweep_chunk(p, span);
   }
-  const int first = LONG ? 0 : p.begin;
+  const Index first = LONG ? 0 : p.begin;
   const bool multi = p.hdr->n_scenes > 1;
-  int next_k = 0, chunk_end = 0;
+  Index next_k = 0, chunk_end = 0;
   unsigned long long tested = 0;  // warp-uniform
   int staged = 0, queued = 0;
   int wscene = 0;
   unsigned long long wpairs = 0;
-  int k = 0, j = 0, len = 0;  // the lane's start and run (this slice of it)
-  int rest = 0;               // LONG: what comes after the slice
 
   while (true) {
-    if (LONG && __any_sync(kFullMask, rest > 0)) {
-      j += len;
-      len = min(rest, kLongSlice);
-      rest -= len;
-    } else {
-      if (next_k >= chunk_end) {
-        int c = 0;
-        if (lane == 0) c = LONG ? int(atomicAdd(p.long_work, unsigned(chunk))) : atomicAdd(p.work, chunk);
-        c = __shfl_sync(kFullMask, c, 0);
-        if (c >= span) break;
-        next_k = first + c;
-        chunk_end = min(next_k + chunk, end);
+    if (next_k >= chunk_end) {
+      Index c = 0;
+      if constexpr (LONG) {
+        if (lane == 0) c = Index(atomicAdd(p.long_work, (unsigned long long)chunk));
+      } else {
+        if (lane == 0) c = atomicAdd(p.work, chunk);
       }
-      const int take = min(32, chunk_end - next_k);
-      k = next_k + lane;
-      next_k += take;
-      // 1. Runs (that of the position after a list is empty).
-      len = 0, j = 0;
-      if (LONG) {
-        if (lane < take) {
-          const int2 it = p.long_list[unsigned(k) / parts];
-          const int part = int(unsigned(k) % parts), run_end = p.run_end[it.x];
-          const int each = int((unsigned(run_end - it.y) + parts - 1u) / parts);
-          k = it.x;
-          j = it.y + min(part * each, run_end - it.y);
-          rest = min(each, run_end - j);
-          len = min(rest, kLongSlice);
-          rest -= len;
-        }
-      } else if (lane < take) {
-        j = p.partner[k];
-        len = max(p.run_end[k] - j, 0);
-        if (p.run_cap && len > p.run_cap) {  // a long run: the warp pass takes the rest
-          p.long_list[atomicAdd(p.long_items, 1u)] = make_int2(k, j + p.run_cap);
-          len = p.run_cap;
-        }
+      c = __shfl_sync(kFullMask, c, 0);
+      if (c >= span) break;
+      next_k = first + c;
+      chunk_end = min(next_k + chunk, end);
+    }
+    const int take = int(min(Index(32), chunk_end - next_k));
+    const Index at_k = next_k + lane;
+    next_k += take;
+    // 1. Runs (that of the position after a list is empty).
+    int k = int(at_k), len = 0, j = 0;
+    if constexpr (LONG) {
+      if (lane < take) {
+        const unsigned item = span >> 32 ? unsigned(at_k / parts) : unsigned(at_k) / parts;
+        const int part = int(at_k - Index(item) * parts);
+        const int2 it = p.long_list[item];
+        const int run_end = p.run_end[it.x];
+        const int each = int((unsigned(run_end - it.y) + parts - 1u) / parts);
+        k = it.x;
+        j = it.y + part * each;
+        len = max(min(each, run_end - j), 0);
+      }
+    } else if (lane < take) {
+      j = p.partner[k];
+      len = max(p.run_end[k] - j, 0);
+      if (p.run_cap && len > p.run_cap) {  // a long run: the warp pass takes the rest
+        p.long_list[atomicAdd(p.long_items, 1u)] = make_int2(k, j + p.run_cap);
+        len = p.run_cap;
       }
     }
     const unsigned nz = __ballot_sync(kFullMask, len > 0);
