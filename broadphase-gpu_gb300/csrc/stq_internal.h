@@ -168,30 +168,32 @@ struct SceneSums {
 // Device-side header of a prepared batch: sizes read by every kernel, so a
 // captured graph can be replayed for any batch within its capacities.
 struct BatchHeader {
+  // what kernels read first, on one line of 128 bytes
   long long n_boxes;        // input: boxes in the batch
   int n_scenes;             // input: scenes
-  int flags;                // kFlag* bits
+  int n_tiles;              // input: entries of the tile table
   unsigned int replicas;    // R, cell replicas
   unsigned int cells;       // total cells of all scenes
   unsigned int length;      // sweep positions: R + 3 * cells - 1
-  int work;                 // sweep grab cursor
-  unsigned int long_items;  // runs handed from the lane sweep to the warp pass
-  unsigned long long long_work;  // warp pass grab cursor
-  unsigned long long pairs; // pairs found by the last sweep
-  long long prefix;         // overflow: start positions of the prefix that fits
-  int axis;                 // sweep axis of scene 0
-  int budget;               // replica budget: replicas <= budget * boxes per scene
-  int n_tiles;              // input: entries of the tile table
-  unsigned int max_list;    // longest (cell, type) list
+  unsigned int lists;       // (cell, type) lists: 3 * cells
+  int fault;                // a bounded wait between blocks ran out
   int key_bits;             // sweep-axis bits of a replica key (the list id is above)
   int exact;                // they are the leading bits of the minimum's float key above
                             // the scene's least, not of its 16-bit code
-  unsigned long long candidates;  // candidates tested by the last sweep
-  unsigned int lists;       // (cell, type) lists: 3 * cells
-  int fault;                // a bounded wait between blocks ran out
   unsigned int passes;      // digits of the replica sort; its input is in buffer passes & 1
-  unsigned int keys_done;   // tiles whose box keys and level counts are in
+  int budget;               // replica budget: replicas <= budget * boxes per scene
+  int flags;                // kFlag* bits
+  int axis;                 // sweep axis of scene 0
+  unsigned int max_list;    // longest (cell, type) list
+  // counters
+  alignas(128) unsigned long long pairs;  // pairs found by the last sweep
+  int work;                 // sweep grab cursor
+  unsigned int long_items;  // runs handed from the lane sweep to the warp pass
+  unsigned long long long_work;  // warp pass grab cursor
+  unsigned long long candidates; // candidates tested by the last sweep
+  long long prefix;         // overflow: start positions of the prefix that fits
   unsigned long long used;  // replicas of all scenes at their levels, accumulated
+  unsigned int keys_done;   // tiles whose box keys and level counts are in
 };
 
 // What the host needs of a prepare's first half, written by the device to
