@@ -76,7 +76,7 @@ advance_kernel(const MeshRef *__restrict__ refs, const long long *__restrict__ v
 // per-block table of the scenes in shared memory when it fits (SMEM), and the
 // block adds its table to the scenes' checksums once at the end: millions of
 // runs would otherwise contend on a few dozen global addresses.
-constexpr int kChecksumChunk = 1024;
+constexpr int kChecksumChunk = 1024;  // at most; as many pairs as a warp loads at once where there are few
 // Pairs loaded at once by a lane. With one (and 64-bit id arithmetic) the kernel
 // waited for its loads and took a quarter of the sweep's time (100 M pairs in 0.26
 // ms), with eight 18% of it; four and two are 0.5% slower over a whole run.
@@ -114,8 +114,12 @@ pair_checksum_kernel(const int2 *__restrict__ pairs, long long capacity, const B
     for (int o = 16; o > 0; o >>= 1) acc ^= __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0 && cur >= 0 && acc) atomicXor(&acc_to[cur], acc);
   };
-  for (long long base = warp * kChecksumChunk; base < n; base += nwarps * kChecksumChunk) {
-    const long long end = min(base + kChecksumChunk, n);
+  // (a chunk is a chain of loads and, at every change of the scene, a search: 360,000
+  // pairs of 4 scenes take 42 us in chunks of 1,024, 17 in chunks of 256)
+  constexpr long long kLeast = 32 * kChecksumStep;
+  const long long chunk = max(kLeast, min((long long)kChecksumChunk, (n / nwarps + kLeast - 1) / kLeast * kLeast));
+  for (long long base = warp * chunk; base < n; base += nwarps * chunk) {
+    const long long end = min(base + chunk, n);
     int cur = -1;  // warp-uniform: scene of the registers' XOR
     int b0 = 0, b1 = 0;  // its ids
     unsigned long long acc = 0;
