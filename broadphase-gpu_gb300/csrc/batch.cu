@@ -266,6 +266,7 @@ batch_stats_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restrict
   after_previous();
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
+  if (threadIdx.x == 0) want_l2(&sums[t.scene]);
   // moments about the tile's first box centre, in fp32 per thread (fp64 is
   // slow on this part); the block combines them in fp64 and shifts them back
   float c[3];
@@ -526,6 +527,7 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
   after_previous();
   if (int(blockIdx.x) >= hdr->n_tiles) return;
   const TileRec t = tiles[blockIdx.x];
+  if (threadIdx.x == 0) want_l2(&sums[t.scene].level_reps), want_l2(&hdr->keys_done);
   const SceneRecord &r = scenes[t.scene];
   const GridParams g = r.grid;
   __shared__ float split[kSplits], inv[kSplits];

@@ -25,6 +25,10 @@ constexpr unsigned kFullMask = 0xffffffffu;
 // before it have ended and their writes are seen. Also in blocks that return at
 // once: a kernel that ended without the wait could end before those before it.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Asks for the line of p in L2: for words that are first met by an atomic at a kernel's
+// end, and may be in device memory.
+__device__ __forceinline__ void want_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Padding after the last sentinel of a sorted scene, so that a lane group of
 // up to 32 lanes may read past a run end without leaving the allocation.
 constexpr int kSortedPad = 256;
