@@ -210,14 +210,22 @@ struct FrontInfo {
 constexpr int kTileBoxes = 4096;
 // Batches of up to kSmallBatch boxes take tiles of 1,024, so that most SMs get one,
 // those of up to kMidBatch tiles of 2,048, and those of up to kTinyBatch tiles of 256,
-// one box per thread. Whole passes with tiles of 1,024 -> 256: 2,000 boxes 118 -> 107
-// us, 53,000 boxes 167 -> 166, 477,000 boxes 297 -> 318 (the last block scans the
-// tiles); of 4,096 -> 2,048: 684,000 boxes 745 -> 737, 9.1 M boxes 3,006 -> 3,018.
+// one box per thread (the lines are two or four tiles for each of 152 SMs). Whole passes
+// with tiles of 1,024 -> 256: 2,000 boxes 118 -> 107 us, 53,000 boxes 167 -> 166, 477,000
+// boxes 297 -> 318 (the last block scans the tiles); sweeps with tiles of 1,024, 2,048
+// and 4,096: 650,000 boxes 239, 227, 239 us, 1 M 295, 288, 297, 1.2 M 346, 343, 350; 9.1 M
+// boxes with 2,048 and 4,096: 3,018, 3,006.
 constexpr int kSmallTile = 1024, kMidTile = 2048, kTinyTile = 256;
 constexpr int64_t kTinyBatch = 152 * 2 * kTinyTile;
 constexpr int64_t kSmallBatch = 152 * 4 * kSmallTile, kMidBatch = 152 * 4 * kMidTile;
 constexpr int tile_boxes(int64_t n) {
   return n <= kTinyBatch ? kTinyTile : (n <= kSmallBatch ? kSmallTile : (n <= kMidBatch ? kMidTile : kTileBoxes));
+}
+// Most tiles of a batch of up to n boxes, but for one more per scene.
+constexpr int64_t most_tiles(int64_t n) {
+  int64_t t = n / kTileBoxes;
+  for (const int64_t v : {kTinyBatch / kTinyTile, kSmallBatch / kSmallTile, kMidBatch / kMidTile}) t = t > v ? t : v;
+  return t;
 }
 struct TileRec {
   long long begin;  // first box of the tile

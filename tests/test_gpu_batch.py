@@ -366,3 +366,8 @@ def test_batch_build_at_tile_edges(ctx, stq, oracle, cuda, filler):
         want = oracle.construct_boxes(V0[a:b], V1[a:b], E, F, stq.AABB_DTYPE).copy()
         want["id"] += int(a)
         assert np.array_equal(got[a:b], want), (a, b)
+
+
+def test_batch_build_at_edges_of_the_largest_tiles(ctx, stq, oracle, cuda):
+    """As above in a batch above 1,245,184 boxes, whose tiles are of 4,096."""
+    test_batch_build_at_tile_edges(ctx, stq, oracle, cuda, 1_240_000)

@@ -64,6 +64,22 @@ def test_tile_edges_vs_oracle(ctx, stq, oracle, cuda, n):
     assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
 
 
+@pytest.mark.parametrize("n", [1_245_184, 1_245_185])
+def test_large_tile_edges_vs_oracle(ctx, stq, oracle, cuda, n):
+    """Tiles of 2,048 boxes up to 1,245,184 boxes, of 4,096 above."""
+    import torch
+
+    b = stq.random_boxes(n, sliver_frac=0.0, seed=n)
+    want = oracle.broadphase(b)
+    d = torch.from_numpy(b.view(np.int32).reshape(-1, 11).copy()).to(cuda)
+    cap = len(want) + 16
+    pairs = torch.empty((cap, 2), dtype=torch.int32, device=cuda)
+    for _ in range(2):
+        r = ctx.sweep(d, n, pairs, cap, axis=-1)
+        assert r.status == stq.STQ_OK and r.count == len(want)
+        assert np.array_equal(oracle.canonical(pairs[: r.count].cpu().numpy()), want)
+
+
 @pytest.mark.parametrize("shape", [1, 2])
 @pytest.mark.parametrize("run_cap", [0, 40])
 def test_windows_after_an_overflow(ctx, stq, oracle, cuda, shape, run_cap):
