@@ -548,7 +548,7 @@ batch_box_keys_kernel(const stq_aabb *__restrict__ boxes, const TileRec *__restr
     box_q[bi] = axis_code(x.min[g.axis], split, inv) | axis_code(x.max[g.axis], split, inv) << 16;
     // level-0 coordinates fit kCoordBits = 11 bits
     const Range q = cell_range(x, g.axis, g.ob, g.ib, g.nb0, g.oc, g.ic, g.nc0);
-    const unsigned type = unsigned(type_of(x.vertex_ids[1], x.vertex_ids[2]));
+    const unsigned type = unsigned(box_type(x.vertex_ids[1], x.vertex_ids[2]));
     box_cells[bi] = make_uint2(unsigned(q.b0) | unsigned(q.b1) << 11 | type << 22,
                                unsigned(q.c0) | unsigned(q.c1) << 11);
 #pragma unroll

@@ -526,7 +526,9 @@ cudaError_t radix_sort_u32(cudaStream_t s, uint32_t *const kbuf[2], uint32_t *co
                            int *fault, int64_t *launches, const unsigned int *d_n, const unsigned int *d_passes,
                            int passes, int64_t likely) {
   const Digits dg{passes, {0, 8, 16, 24}, d_passes};
-  if (passes > 0 && (n > 1 || d_passes)) {  // one block up to its 16 keys per thread
+  // one block up to its 16 keys per thread. 1,000, 4,000 and 8,000 keys with 2, 8 and 16
+  // per thread: 7.5, 13.2 and 18.0 us (with 16: 17.5, 17.8); in launches per digit 20, 23, 26
+  if (passes > 0 && (n > 1 || d_passes)) {
     if (n <= kPassBlock * 2) return launch_block<2>(s, kbuf, vbuf, n, dg, d_n, launches);
     if (n <= kPassBlock * 8) return launch_block<8>(s, kbuf, vbuf, n, dg, d_n, launches);
     if (n <= kPassBlock * 16) return launch_block<16>(s, kbuf, vbuf, n, dg, d_n, launches);

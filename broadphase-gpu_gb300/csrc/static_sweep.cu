@@ -186,9 +186,9 @@ extern "C" int stq_sweep_static(const stq_aabb *d_boxes, int64_t n, int axis, st
   p.run_end = reinterpret_cast<const int *>(scratch + kOffRunEnd);
   p.begin = 0;
   p.end = ni;
-  // start boxes per warp: 8 where 32 would leave warps without any (65,536 boxes
-  // are 2,048 warps of 32)
-  p.chunk = n <= int64_t(num_sms) * 48 * 32 ? 8 : 32;
+  // start boxes per warp: 32 would leave warps without any (65,536 boxes are 2,048
+  // warps of 32)
+  p.chunk = 8;
   p.grabs = 0;
   p.pairs = d_pairs;
   p.capacity = capacity;

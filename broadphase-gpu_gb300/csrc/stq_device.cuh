@@ -81,12 +81,6 @@ __device__ __forceinline__ float key_float(uint32_t k) {
   return __uint_as_float(b);
 }
 
-// Box type from the signs of vertexIds (src/aabb.cu:12-31): vertex 0, edge
-// 1, face 2.
-__device__ __forceinline__ int type_of(int v1, int v2) {
-  return v2 >= 0 ? 2 : (v1 >= 0 ? 1 : 0);
-}
-
 // Cell coordinate of a bound: clamp(floor((v - origin) * inv), 0, n - 1),
 // with round-to-nearest float steps. Each step is monotone non-decreasing in
 // v, so a <= b implies cell(a) <= cell(b): a point inside a box's range has
