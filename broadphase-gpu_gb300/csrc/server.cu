@@ -457,8 +457,13 @@ int stq_server_create(int device, void *stream, int64_t budget_bytes, int64_t ma
   std::memset(sv->voff_host, 0, sizeof(long long) * size_t(max_scenes + 1));
   size_t free_b = 0, total = 0;
   cudaMemGetInfo(&free_b, &total);
+  // (what grows with the boxes; the tables per scene and tile are small change that
+  // would refuse budgets of a few hundred KB)
   sv->fixed = 0;
-  for (const DevBuf *b : ctx->buffers()) sv->fixed += int64_t(b->bytes);
+  for (const DevBuf *b : {&ctx->keys[0], &ctx->keys[1], &ctx->vals[0], &ctx->vals[1], &ctx->sort_ws, &ctx->seg_scan, &ctx->yz,
+                          &ctx->xx, &ctx->vv, &ctx->flag, &ctx->scode, &ctx->partner, &ctx->run_end, &ctx->box_cells,
+                          &ctx->box_q, &ctx->batch_boxes})
+    sv->fixed += int64_t(b->bytes);
   if (sv->fixed >= budget_bytes) return bad(STQ_ERR_NO_MEMORY);
   *out = sv.release();
   return STQ_OK;

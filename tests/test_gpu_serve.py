@@ -160,3 +160,11 @@ def test_budget_admits_in_arrival_order(stq, cuda):
     with pytest.raises(stq.STQError):
         with stq.Server(0, None, budget_bytes=8 << 30, max_boxes=1000, max_scenes=2) as sv:
             sv.submit(meshes[0], steps=1, sigma=0.0, seed=0)
+
+
+@pytest.mark.parametrize("boxes,scenes,held", [(100, 1, 106_496), (100, 256, 172_032), (5000, 256, 2_138_112),
+                                               (20_000, 256, 8_179_712), (1 << 20, 32, 422_117_376)])
+def test_small_budgets_are_accepted(stq, cuda, boxes, scenes, held):
+    """Budgets just above what a server of that size has always counted for its buffers."""
+    with stq.Server(0, None, budget_bytes=held + 1, max_boxes=boxes, max_scenes=scenes) as sv:
+        assert sv.stats()["bytes"] <= held
