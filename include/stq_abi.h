@@ -138,7 +138,7 @@ const char *stq_context_last_error(const stq_context *ctx);
 int64_t stq_context_launch_count(const stq_context *ctx);
 /* Candidates (start box / candidate pairs) the last sweep tested, a measure of
  * the sweep's work beyond the pairs it found: the pairs that overlap on the sweep
- * axis, and those few that share a 16-bit code of it without doing so. */
+ * axis, and those that share a step of its code (or key) without doing so. */
 int64_t stq_context_candidates(const stq_context *ctx);
 /* Shape of the prepared scene's (cell, type) lists: out[0] lists (3 per
  * cell), out[1] cell replicas, out[2] the longest list. Synchronises. */
