@@ -7,10 +7,10 @@
 // scene along x. Here every scene of a batch gets its own sweep axis and
 // y/z cell grid, all scenes' cells get global ids, and one sort orders every
 // replica by (cell, box type, sweep-axis code). The code is a monotone 16-bit
-// image of the minimum (where lists are few and long, more bits of it): a list is sorted up to boxes of one code, its runs hold
-// every candidate of a code that can overlap, and the sweep tests the sweep axis
-// exactly for the pairs that pass its filter. So the whole key fits 24 or 32
-// bits, and the boxes need no sort of their own.
+// image of the minimum (more bits of it where lists are few and long): a list is
+// sorted up to boxes of one code, its runs hold every candidate of a code that can
+// overlap, and the sweep tests the sweep axis exactly for the pairs that pass its
+// filter. So the whole key fits 24 or 32 bits, and the boxes need no sort of their own.
 //
 // All sizes are read from the BatchHeader on the device, so one captured
 // graph serves any batch within the buffer capacities.

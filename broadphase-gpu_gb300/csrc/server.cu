@@ -443,7 +443,8 @@ int stq_server_create(int device, void *stream, int64_t budget_bytes, int64_t ma
   // pipeline buffers for the largest batch, counted against the budget
   // (small ticks are cut into small tiles)
   const int64_t tiles = most_tiles(max_boxes) + max_scenes + 1;
-  if (ensure_staging(ctx, max_scenes, int(tiles)) != STQ_OK || clear_sums(ctx) != STQ_OK || ensure_box_buffers(ctx, max_boxes) != STQ_OK ||
+  if (ensure_staging(ctx, max_scenes, int(tiles)) != STQ_OK || clear_sums(ctx) != STQ_OK ||
+      ensure_box_buffers(ctx, max_boxes) != STQ_OK ||
       ensure_replica_buffers(ctx, int64_t(ctx->budget) * max_boxes, max_boxes / 16 + max_scenes + 1) != STQ_OK ||
       ctx->batch_boxes.ensure(sizeof(stq_aabb) * size_t(max_boxes)) != cudaSuccess ||
       sv->refs_dev.ensure(sizeof(MeshRef) * size_t(max_scenes)) != cudaSuccess ||
